@@ -25,32 +25,13 @@ __global__ void pool_keys_kernel(const T *__restrict__ keys, int64_t n_pools, in
 
 // ------------------------------------------------------------------------------------------------ Ward
 
-constexpr int kWardThreads = 256;
+constexpr int kWardAnyThreads = 256;
 
-// Dot of the caller's row (registers when D > 0, shared memory otherwise) with a shared-memory row.
-template <int D>
-__device__ __forceinline__ float ward_dot(const float *mine, const float *other, int d) {
-  float acc = 0.0f;
-  if (D > 0) {
-#pragma unroll
-    for (int k = 0; k < D; k += 4) {
-      float4 o = *reinterpret_cast<const float4 *>(other + k);
-      acc = fmaf(mine[k], o.x, acc);
-      acc = fmaf(mine[k + 1], o.y, acc);
-      acc = fmaf(mine[k + 2], o.z, acc);
-      acc = fmaf(mine[k + 3], o.w, acc);
-    }
-  } else {
-    for (int k = 0; k < d; ++k) acc = fmaf(mine[k], other[k], acc);
-  }
-  return acc;
-}
-
-// One CTA merges one cluster block. Shared memory: the key sums [P][stride] and a few per-row vectors.
+// Any number of dims (the other widths are in ward.cu): one CTA merges one cluster block, every row searching all of its
+// partners every round. Shared memory: the key sums [P][stride] and a few per-row vectors.
 // Rows are stored at a stride of d + 4 floats, which keeps float4 alignment and spreads rows over banks.
-template <int D>
-__global__ void __launch_bounds__(kWardThreads)
-    ward_kernel(const float *__restrict__ pool_keys, const float *__restrict__ pool_sizes, float uniform_size, int P,
+__global__ void __launch_bounds__(kWardAnyThreads)
+    ward_any_kernel(const float *__restrict__ pool_keys, const float *__restrict__ pool_sizes, float uniform_size, int P,
                 int d, int bucket_count, float bucket_cap, int max_rounds, int64_t *__restrict__ labels,
                 uint8_t *__restrict__ reached, int32_t *__restrict__ rounds_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -60,18 +41,18 @@ __global__ void __launch_bounds__(kWardThreads)
   float *sq = sz + P;                                        // [P]
   float *al = sq + P;                                        // [P]
   float *best_cost = al + P;                                 // [P]
-  float *cand_cost = best_cost + P;                          // [kWardThreads]
-  int *best = reinterpret_cast<int *>(cand_cost + kWardThreads);  // [P]
-  int *cand_j = best + P;                                    // [kWardThreads]
-  int *parent = cand_j + kWardThreads;                       // [P]
+  float *cand_cost = best_cost + P;                          // [kWardAnyThreads]
+  int *best = reinterpret_cast<int *>(cand_cost + kWardAnyThreads);  // [P]
+  int *cand_j = best + P;                                    // [kWardAnyThreads]
+  int *parent = cand_j + kWardAnyThreads;                       // [P]
   int *state = parent + P;                                   // [P] 0 dead, 1 alive; bit 1 = mutual, bit 2 = kept
   __shared__ int n_alive_s, merged_s;
 
   const int tid = threadIdx.x;
   const int64_t block = blockIdx.x;
   const float *src = pool_keys + block * (int64_t)P * d;
-  for (int e = tid; e < P * d; e += kWardThreads) ks[(e / d) * stride + (e % d)] = src[e];
-  for (int i = tid; i < P; i += kWardThreads) {
+  for (int e = tid; e < P * d; e += kWardAnyThreads) ks[(e / d) * stride + (e % d)] = src[e];
+  for (int i = tid; i < P; i += kWardAnyThreads) {
     sz[i] = pool_sizes ? pool_sizes[block * P + i] : uniform_size;
     parent[i] = i;
     state[i] = 1;
@@ -80,12 +61,12 @@ __global__ void __launch_bounds__(kWardThreads)
   __syncthreads();
 
   // Threads a row when the block has fewer rows than the CTA has threads: each takes every tpr-th partner.
-  const int tpr = P >= kWardThreads ? 1 : kWardThreads / P;
+  const int tpr = P >= kWardAnyThreads ? 1 : kWardAnyThreads / P;
   int rounds = 0;
   for (int round = 0; round < max_rounds; ++round) {
     const int merges_left = n_alive_s - bucket_count;
     if (merges_left <= 0) break;
-    for (int i = tid; i < P; i += kWardThreads) {
+    for (int i = tid; i < P; i += kWardAnyThreads) {
       const float *row = ks + (size_t)i * stride;
       float s = 0.0f;
       for (int k = 0; k < d; ++k) s = fmaf(row[k], row[k], s);
@@ -96,22 +77,19 @@ __global__ void __launch_bounds__(kWardThreads)
     __syncthreads();
 
     // Cheapest allowed partner of every row, the first minimum in ascending partner order.
-    for (int base = 0; base < P * tpr; base += kWardThreads) {
+    for (int base = 0; base < P * tpr; base += kWardAnyThreads) {
       const int slot = base + tid;
       const int i = slot / tpr, sub = slot - i * tpr;
       float bc = INFINITY;
       int bj = 0;
       if (i < P && (state[i] & 1)) {
-        float mine[D > 0 ? D : 1];
         const float *row = ks + (size_t)i * stride;
-        if (D > 0) {
-#pragma unroll
-          for (int k = 0; k < D; ++k) mine[k] = row[k];
-        }
         const float szi = sz[i], sqi = sq[i], ali = al[i];
         for (int j = sub; j < P; j += tpr) {
           if (j == i || !(state[j] & 1) || __fadd_rn(szi, sz[j]) > bucket_cap) continue;
-          const float g = ward_dot<D>(D > 0 ? mine : row, ks + (size_t)j * stride, d);
+          const float *other = ks + (size_t)j * stride;
+          float g = 0.0f;
+          for (int k = 0; k < d; ++k) g = fmaf(row[k], other[k], g);
           const float m2 = __fadd_rn(__fadd_rn(sqi, sq[j]), __fmul_rn(2.0f, g));
           const float merged = sqrtf(m2 > 0.0f ? m2 : 0.0f);
           const float cost = __fsub_rn(__fadd_rn(ali, al[j]), merged);
@@ -148,13 +126,13 @@ __global__ void __launch_bounds__(kWardThreads)
     __syncthreads();
 
     // Mutual cheapest pairs, held by their lower row.
-    for (int i = tid; i < P; i += kWardThreads) {
+    for (int i = tid; i < P; i += kWardAnyThreads) {
       const bool mutual = best_cost[i] < INFINITY && best[best[i]] == i && i < best[i];
       state[i] = (state[i] & 1) | (mutual ? 2 : 0);
     }
     __syncthreads();
     // The cheapest merges_left of them merge, a tie to the lower row.
-    for (int i = tid; i < P; i += kWardThreads) {
+    for (int i = tid; i < P; i += kWardAnyThreads) {
       if (!(state[i] & 2)) continue;
       const float ci = best_cost[i];
       int rank = 0;
@@ -167,12 +145,12 @@ __global__ void __launch_bounds__(kWardThreads)
     }
     __syncthreads();
     if (merged_s == 0) break;
-    for (int e = tid; e < P * d; e += kWardThreads) {
+    for (int e = tid; e < P * d; e += kWardAnyThreads) {
       const int i = e / d, c = e - i * d;
       if (state[i] & 4) ks[(size_t)i * stride + c] = __fadd_rn(ks[(size_t)i * stride + c], ks[(size_t)best[i] * stride + c]);
     }
     __syncthreads();
-    for (int i = tid; i < P; i += kWardThreads) {
+    for (int i = tid; i < P; i += kWardAnyThreads) {
       if (!(state[i] & 4)) continue;
       const int a = best[i];
       sz[i] = __fadd_rn(sz[i], sz[a]);
@@ -182,12 +160,12 @@ __global__ void __launch_bounds__(kWardThreads)
     if (tid == 0) n_alive_s -= merged_s;
     ++rounds;
     __syncthreads();
-    for (int i = tid; i < P; i += kWardThreads) state[i] &= 1;
+    for (int i = tid; i < P; i += kWardAnyThreads) state[i] &= 1;
     __syncthreads();
   }
 
   // Survivors numbered by their first pool; a merge keeps the lower pool, so a root is its bucket's first pool.
-  for (int i = tid; i < P; i += kWardThreads) {
+  for (int i = tid; i < P; i += kWardAnyThreads) {
     int r = i;
     while (parent[r] != r) r = parent[r];
     int number = -1;
@@ -201,8 +179,8 @@ __global__ void __launch_bounds__(kWardThreads)
 }
 
 static size_t ward_smem_bytes(int P, int d) {
-  return sizeof(float) * ((size_t)P * (d + 4) + 4 * (size_t)P + kWardThreads) +
-         sizeof(int) * (3 * (size_t)P + kWardThreads);
+  return sizeof(float) * ((size_t)P * (d + 4) + 4 * (size_t)P + kWardAnyThreads) +
+         sizeof(int) * (3 * (size_t)P + kWardAnyThreads);
 }
 
 // ------------------------------------------------------------------------------------------------ bucket table
@@ -305,18 +283,16 @@ LSA_API int lsa_pool_keys(const void *index_keys, int key_dtype, int64_t n_pools
 }
 
 namespace lsa {
-size_t ward_large_workspace_bytes(int64_t G, int P, int d);
-int ward_large_run(const float *pool_keys, const float *pool_sizes, float uniform_size, int64_t G, int P, int d,
-                   int bucket_count, float bucket_cap, int max_rounds, int64_t *labels, uint8_t *reached,
-                   int32_t *rounds, void *workspace, cudaStream_t s);
-// Blocks up to this many pools (at 64 dims) are merged by one CTA out of shared memory.
-constexpr int kWardOneCtaPools = 512;
+bool ward_cluster_takes(int d);
+size_t ward_cluster_workspace_bytes(int64_t G, int P, int d);
+int ward_cluster_run(const float *pool_keys, const float *pool_sizes, float uniform_size, int64_t G, int P, int d,
+                     int bucket_count, float bucket_cap, int max_rounds, int64_t *labels, uint8_t *reached,
+                     int32_t *rounds, void *workspace, cudaStream_t s);
 }  // namespace lsa
 
 LSA_API size_t lsa_ward_merge_workspace_bytes(int64_t blocks, int P, int d) {
-  if (blocks <= 0 || P <= 0 || d <= 0) return 0;
-  if (P <= lsa::kWardOneCtaPools && lsa::ward_smem_bytes(P, d) <= 227 * 1024) return 0;
-  return lsa::ward_large_workspace_bytes(blocks, P, d);
+  if (blocks <= 0 || P <= 0 || d <= 0 || !lsa::ward_cluster_takes(d)) return 0;
+  return lsa::ward_cluster_workspace_bytes(blocks, P, d);
 }
 
 LSA_API int lsa_ward_merge(const float *pool_keys, const float *pool_sizes, float uniform_pool_size, int64_t blocks,
@@ -328,34 +304,20 @@ LSA_API int lsa_ward_merge(const float *pool_keys, const float *pool_sizes, floa
               LSA_ERR_ARGUMENT);
   LSA_REQUIRE(P <= 4096 && d <= 1024, LSA_ERR_UNSUPPORTED);
   if (blocks == 0) return LSA_OK;
-  const size_t need = lsa_ward_merge_workspace_bytes(blocks, P, d);
-  if (need > 0) {
-    LSA_REQUIRE(d == 16 || d == 32 || d == 64, LSA_ERR_UNSUPPORTED);
-    LSA_REQUIRE(workspace, LSA_ERR_NULL);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (lsa::ward_cluster_takes(d)) {
+    const size_t need = lsa_ward_merge_workspace_bytes(blocks, P, d);
+    LSA_REQUIRE(need == 0 || workspace, LSA_ERR_NULL);
     LSA_REQUIRE(workspace_bytes >= need, LSA_ERR_WORKSPACE);
-    return lsa::ward_large_run(pool_keys, pool_sizes, uniform_pool_size, blocks, P, d, bucket_count, bucket_cap,
-                               max_rounds, labels, reached, rounds, workspace, (cudaStream_t)stream);
+    return lsa::ward_cluster_run(pool_keys, pool_sizes, uniform_pool_size, blocks, P, d, bucket_count, bucket_cap,
+                                 max_rounds, labels, reached, rounds, workspace, s);
   }
   const size_t smem = lsa::ward_smem_bytes(P, d);
-  cudaStream_t s = (cudaStream_t)stream;
-#define LSA_WARD_LAUNCH(DD)                                                                                       \
-  do {                                                                                                            \
-    if (cudaFuncSetAttribute(lsa::ward_kernel<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=     \
-        cudaSuccess)                                                                                              \
-      return LSA_ERR_LAUNCH;                                                                                      \
-    lsa::ward_kernel<DD><<<(unsigned)blocks, lsa::kWardThreads, smem, s>>>(                                       \
-        pool_keys, pool_sizes, uniform_pool_size, P, d, bucket_count, bucket_cap, max_rounds, labels, reached,    \
-        rounds);                                                                                                  \
-  } while (0)
-  if (d == 64)
-    LSA_WARD_LAUNCH(64);
-  else if (d == 32)
-    LSA_WARD_LAUNCH(32);
-  else if (d == 16)
-    LSA_WARD_LAUNCH(16);
-  else
-    LSA_WARD_LAUNCH(0);
-#undef LSA_WARD_LAUNCH
+  LSA_REQUIRE(P <= 512 && smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
+  if (cudaFuncSetAttribute(lsa::ward_any_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return LSA_ERR_LAUNCH;
+  lsa::ward_any_kernel<<<(unsigned)blocks, lsa::kWardAnyThreads, smem, s>>>(
+      pool_keys, pool_sizes, uniform_pool_size, P, d, bucket_count, bucket_cap, max_rounds, labels, reached, rounds);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

@@ -140,6 +140,23 @@ def test_large_block_ward_is_bit_exact(ops, oracle, G, P, d, count, cap, sizes):
     assert np.array_equal(rounds.cpu().numpy(), want_rounds)
 
 
+@pytest.mark.parametrize("G,P,d,count,cap,sizes", [(7, 1, 64, 1, 8.0, 1.0), (3, 5, 32, 2, 8.0, 1.0), (1, 65, 64, 8, 640.0, 64.0),
+                                                     (9, 128, 64, 64, 16.0, 4.0), (150, 96, 16, 12, 64.0, 4.0),
+                                                     (2, 512, 64, 64, 32.0, 2.0), (2, 513, 64, 257, 2.0, 1.0),
+                                                     (80, 640, 16, 320, 2.0, 1.0), (1, 4096, 64, 2048, 2.0, 1.0)])
+def test_ward_blocks_over_one_to_eight_ctas_are_bit_exact(ops, oracle, G, P, d, count, cap, sizes):
+    """One pool, a ragged second tile, blocks of a CTA and of a cluster, key sums in shared memory up to 512 pools and in
+    the workspace above, both tile heights; and sizes that differ, so that rows close at different times."""
+    keys = unit_rows(mixture(G * P, d, 24, 0.4, G + P + d)).reshape(G, P, d) * np.float32(2.0)
+    rng = np.random.default_rng(P)
+    for size_rows in (np.full((G, P), sizes, dtype=np.float32), sizes * rng.integers(1, 4, (G, P)).astype(np.float32)):
+        want, want_reached, want_rounds = oracle.ward_rounds(keys, size_rows, count, cap, return_rounds=True)
+        got, reached, rounds = ops.ward_rounds(cuda(keys), cuda(size_rows), count, cap, return_rounds=True)
+        assert np.array_equal(got.cpu().numpy(), want)
+        assert np.array_equal(reached.cpu().numpy(), want_reached)
+        assert np.array_equal(rounds.cpu().numpy(), want_rounds)
+
+
 def test_ward_golden_and_adversarial_cases(ops, oracle):
     g = golden("ward")
     for tag in "abcde":
