@@ -185,38 +185,68 @@ static size_t ward_smem_bytes(int P, int d) {
 
 // ------------------------------------------------------------------------------------------------ bucket table
 
-// One CTA per cluster block. Phase 1: a warp per bucket walks the pools in order, 32 at a time, and lists their
-// positions. Phase 2: a thread per (bucket, dim) adds the bucket's keys one by one in position order, eight loads in
-// flight at a time (the order of the additions is what the results are pinned to; the loads may run ahead of it).
+// A cluster block's buckets, a run of them a CTA (grid: blocks x runs). Phase 1: one warp walks the block's pools in
+// order, 32 a step, and gives every pool its place in its bucket (the pools of the same label before it: those of the
+// step by a match over the warp, those of the steps before by a count a bucket) - a walk over P labels, where a warp a
+// bucket walks P labels for every bucket; the CTA then writes the positions. Phase 2: a thread per (bucket, dim) adds the
+// bucket's keys one by one in position order, sixteen loads in flight and the next sixteen ids behind them (the order of
+// the additions is what the results are pinned to; the loads may run ahead of it).
+constexpr int kTableThreads = 256;
+constexpr int kTableAhead = 16;
+constexpr int kTablePools = 2048;  // pools of a step of phase 1
+
 template <typename T>
-__global__ void bucket_table_kernel(const T *__restrict__ index_keys, const int64_t *__restrict__ labels, int P,
-                                    int pool_size, int d, int bucket_count, int bucket_cap, int64_t first_position,
-                                    int32_t *__restrict__ members, int32_t *__restrict__ sizes,
-                                    float *__restrict__ key_sums, float *__restrict__ centroids,
-                                    uint16_t *__restrict__ centroids_bf16, int32_t *__restrict__ status) {
+__global__ void __launch_bounds__(kTableThreads)
+    bucket_table_kernel(const T *__restrict__ index_keys, const int64_t *__restrict__ labels, int P, int pool_size, int d,
+                        int bucket_count, int run, int bucket_cap, int64_t first_position,
+                        int32_t *__restrict__ members, int32_t *__restrict__ sizes, float *__restrict__ key_sums,
+                        float *__restrict__ centroids, uint16_t *__restrict__ centroids_bf16,
+                        int32_t *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float *sums = reinterpret_cast<float *>(smem_raw);  // [bucket_count][d]
   const int64_t block = blockIdx.x;
   const int64_t block_keys = (int64_t)P * pool_size;
-  const int64_t row0 = block * bucket_count;
+  const int first_bucket = blockIdx.y * run, buckets = min(run, bucket_count - first_bucket);
+  const int64_t row0 = block * bucket_count + first_bucket;
   const int64_t *lab = labels + block * P;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  for (int b = warp; b < bucket_count; b += warps) {
-    int32_t *row = members + (row0 + b) * bucket_cap;
-    int pools = 0;  // pools of the bucket so far
-    for (int p0 = 0; p0 < P; p0 += 32) {
-      const int p = p0 + lane;
-      const bool mine = p < P && lab[p] == b;
-      const unsigned votes = __ballot_sync(0xffffffffu, mine);
-      if (mine) {
-        const int at = (pools + __popc(votes & ((1u << lane) - 1))) * pool_size;
-        for (int j = 0; j < pool_size; ++j)
-          if (at + j < bucket_cap) row[at + j] = (int32_t)(first_position + block * block_keys + (int64_t)p * pool_size + j);
-      }
-      pools += __popc(votes);
+  const int lane = threadIdx.x & 31;
+  int *pools_of = reinterpret_cast<int *>(smem_raw);  // [run] pools of a bucket so far
+  int *place = pools_of + run;                        // [step] a pool's bucket of this run, or -1
+  int *before = place + kTablePools;                  // [step] and the bucket's pools before it
+  float *sums = reinterpret_cast<float *>(before + kTablePools);  // [run][d]
+  for (int b = threadIdx.x; b < buckets; b += blockDim.x) pools_of[b] = 0;
+  for (int from = 0; from < P; from += kTablePools) {
+    const int pools = min(kTablePools, P - from);
+    for (int p = threadIdx.x; p < pools; p += blockDim.x) {
+      const int64_t b = lab[from + p] - first_bucket;
+      place[p] = b >= 0 && b < buckets ? (int)b : -1;
     }
-    const int64_t listed = (int64_t)pools * pool_size;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      for (int p0 = 0; p0 < pools; p0 += 32) {
+        const int p = p0 + lane, b = p < pools ? place[p] : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, b);
+        const int rank = __popc(same & ((1u << lane) - 1));
+        const int so_far = b >= 0 ? pools_of[b] : 0;
+        if (b >= 0) before[p] = so_far + rank;
+        __syncwarp();
+        if (b >= 0 && rank == 0) pools_of[b] = so_far + __popc(same);
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < pools; p += blockDim.x) {
+      const int b = place[p];
+      if (b < 0) continue;
+      int32_t *row = members + (row0 + b) * bucket_cap;
+      const int64_t at = (int64_t)before[p] * pool_size, position = first_position + block * block_keys + (int64_t)(from + p) * pool_size;
+      for (int j = 0; j < pool_size && at + j < bucket_cap; ++j) row[at + j] = (int32_t)(position + j);
+    }
+    __syncthreads();
+  }
+  for (int b = threadIdx.x >> 5; b < buckets; b += kTableThreads / 32) {
+    const int64_t listed = (int64_t)pools_of[b] * pool_size;
     const int n = (int)(listed < bucket_cap ? listed : bucket_cap);
+    int32_t *row = members + (row0 + b) * bucket_cap;
     for (int j = n + lane; j < bucket_cap; j += 32) row[j] = LSA_PAD;
     if (lane == 0) {
       sizes[row0 + b] = n;
@@ -225,18 +255,26 @@ __global__ void bucket_table_kernel(const T *__restrict__ index_keys, const int6
   }
   __syncthreads();
   if (!key_sums && !centroids && !centroids_bf16) return;
-  for (int e = threadIdx.x; e < bucket_count * d; e += blockDim.x) {
+  for (int e = threadIdx.x; e < buckets * d; e += blockDim.x) {
     const int b = e / d, c = e - b * d;
     const int32_t *row = members + (row0 + b) * bucket_cap;
     const int n = sizes[row0 + b];
     float acc = 0.0f;
-    for (int j0 = 0; j0 < n; j0 += 8) {
-      float v[8];
+    int32_t id[kTableAhead];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        v[j] = j0 + j < n ? load_as_float<T>(index_keys, (int64_t)(row[j0 + j] - first_position) * d + c) : 0.0f;
+    for (int j = 0; j < kTableAhead; ++j) id[j] = j < n ? row[j] : 0;
+    for (int j0 = 0; j0 < n; j0 += kTableAhead) {
+      float v[kTableAhead];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < kTableAhead; ++j)
+        v[j] = j0 + j < n ? load_as_float<T>(index_keys, (int64_t)(id[j] - first_position) * d + c) : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kTableAhead; ++j) {
+        const int next = j0 + kTableAhead + j;
+        id[j] = next < n ? row[next] : 0;
+      }
+#pragma unroll
+      for (int j = 0; j < kTableAhead; ++j)
         if (j0 + j < n) acc = __fadd_rn(acc, v[j]);
     }
     sums[e] = acc;
@@ -244,15 +282,15 @@ __global__ void bucket_table_kernel(const T *__restrict__ index_keys, const int6
   }
   __syncthreads();
   if (!centroids && !centroids_bf16) return;
-  float *norms = sums + (size_t)bucket_count * d;  // [bucket_count]
-  for (int b = threadIdx.x; b < bucket_count; b += blockDim.x) {
+  float *norms = sums + (size_t)run * d;  // [run]
+  for (int b = threadIdx.x; b < buckets; b += blockDim.x) {
     float ss = 0.0f;
     for (int c = 0; c < d; ++c) ss = fmaf(sums[b * d + c], sums[b * d + c], ss);
     const float nrm = sqrtf(ss);
     norms[b] = nrm > 1e-30f ? nrm : 1e-30f;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < bucket_count * d; e += blockDim.x) {
+  for (int e = threadIdx.x; e < buckets * d; e += blockDim.x) {
     const int b = e / d;
     const float value = __fdiv_rn(sums[e], norms[b]);
     if (centroids) centroids[row0 * d + e] = value;
@@ -333,23 +371,32 @@ LSA_API int lsa_bucket_table(const void *index_keys, int key_dtype, const int64_
   const bool sums = key_sums || centroids || centroids_bf16;
   LSA_REQUIRE(!sums || index_keys, LSA_ERR_NULL);
   if (blocks == 0) return LSA_OK;
-  const size_t smem = sums ? sizeof(float) * ((size_t)bucket_count * d + bucket_count) : 0;
-  LSA_REQUIRE(smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
+  // (a block's sums and norms beside one another in one CTA's shared memory: the size this call has always taken)
+  LSA_REQUIRE(!sums || sizeof(float) * ((size_t)bucket_count * d + bucket_count) <= 227 * 1024, LSA_ERR_UNSUPPORTED);
   cudaStream_t s = (cudaStream_t)stream;
-  const int threads = 256;
+  // CTAs a block: enough to give every SM four, and no fewer than a run's sums fit shared memory with the pools' places.
+  const int sms = lsa::sm_count();
+  const size_t fixed = sizeof(int) * 2 * lsa::kTablePools, a_bucket = sizeof(int) + (sums ? sizeof(float) * ((size_t)d + 1) : 0);
+  int64_t runs = (4 * (int64_t)sms + blocks - 1) / blocks;
+  runs = runs < bucket_count ? runs : bucket_count;
+  int run = (int)((bucket_count + runs - 1) / runs);
+  while (run > 1 && fixed + run * a_bucket > 200 * 1024) run = (run + 1) / 2;
+  const size_t smem = fixed + run * a_bucket;
+  LSA_REQUIRE(smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
+  const dim3 grid((unsigned)blocks, (unsigned)((bucket_count + run - 1) / run));
   if (key_dtype == LSA_DTYPE_F32) {
     if (cudaFuncSetAttribute(lsa::bucket_table_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return LSA_ERR_LAUNCH;
-    lsa::bucket_table_kernel<float><<<(unsigned)blocks, threads, smem, s>>>(
-        (const float *)index_keys, labels, P, pool_size, d, bucket_count, bucket_cap, first_position, members, sizes,
+    lsa::bucket_table_kernel<float><<<grid, lsa::kTableThreads, smem, s>>>(
+        (const float *)index_keys, labels, P, pool_size, d, bucket_count, run, bucket_cap, first_position, members, sizes,
         key_sums, centroids, centroids_bf16, status);
   } else {
     if (cudaFuncSetAttribute(lsa::bucket_table_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return LSA_ERR_LAUNCH;
-    lsa::bucket_table_kernel<uint16_t><<<(unsigned)blocks, threads, smem, s>>>(
-        (const uint16_t *)index_keys, labels, P, pool_size, d, bucket_count, bucket_cap, first_position, members,
+    lsa::bucket_table_kernel<uint16_t><<<grid, lsa::kTableThreads, smem, s>>>(
+        (const uint16_t *)index_keys, labels, P, pool_size, d, bucket_count, run, bucket_cap, first_position, members,
         sizes, key_sums, centroids, centroids_bf16, status);
   }
   LSA_LAUNCH_CHECK();

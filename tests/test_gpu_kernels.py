@@ -219,6 +219,29 @@ def test_kmeans_bucketing_matches_its_restatement(ops, oracle):
     assert np.array_equal(centroids.cpu().numpy().view(np.int32), want_centroids.view(np.int32))
 
 
+@pytest.mark.parametrize("G,P,pool,count,cap", [(1, 33, 3, 5, 40), (2, 2049, 1, 1024, 3), (700, 40, 2, 8, 8), (1, 5000, 1, 7, 900)])
+def test_bucket_table_of_ragged_blocks(ops, G, P, pool, count, cap):
+    """Pools past a step of the walk, buckets over their cap (cut, and counted), labels past the table (left out), one
+    bucket a CTA and many: against the walk as written."""
+    rng = np.random.default_rng(P)
+    labels = rng.integers(0, count + 1, (G, P))
+    keys = rng.standard_normal((G * P * pool, 32), dtype=np.float32)
+    members, sizes, sums, cent, _, status = ops.bucket_table(cuda(keys), cuda(labels), pool, count, cap)
+    want, over = np.full((G * count, cap), -1, np.int32), 0
+    for g in range(G):
+        for b in range(count):
+            ids = (g * P * pool + np.flatnonzero(labels[g] == b)[:, None] * pool + np.arange(pool)).reshape(-1)
+            over += len(ids) > cap
+            want[g * count + b, :min(len(ids), cap)] = ids[:cap]
+    assert np.array_equal(members.cpu().numpy(), want) and int(status) == over
+    assert np.array_equal(sizes.cpu().numpy(), (want >= 0).sum(1))
+    for row in rng.integers(0, G * count, 20):  # added one by one, ascending: fp32, so equal and not close
+        acc = np.zeros(32, np.float32)
+        for i in want[row][want[row] >= 0]:
+            acc = acc + keys[i]
+        assert np.array_equal(sums.cpu().numpy()[row], acc)
+
+
 def test_bucket_table_is_bit_exact(ops, oracle):
     for name, (pool, bucket, cap, block) in {"flat_small": (4, 8, 16, 64), "flat_c1like": (16, 64, 128, 512)}.items():
         g = golden(name)
