@@ -180,6 +180,45 @@ def test_ward_golden_and_adversarial_cases(ops, oracle):
     assert not reached.any() and torch.equal(labels.cpu(), torch.arange(16).expand(2, 16))
 
 
+@pytest.mark.parametrize("cap,m,top_p,top_k,rows", [(1, 90, 70, 33, 70), (16, 300, 130, 900, 70), (17, 200, 64, 500, 9),
+                                                     (63, 80, 33, 2079, 70), (64, 80, 40, 700, 70), (65, 128, 128, 8320, 70),
+                                                     (100, 90, 90, 2000, 70), (1280, 40, 30, 20000, 65)])
+def test_lists_over_narrow_and_wide_buckets_are_the_oracles(ops, oracle, cap, m, top_p, top_k, rows):
+    """Picks walked as one run of places (up to 64 members a bucket), a CTA a row over runs of members (wider buckets, long
+    lists) and a warp a row: ragged and empty buckets, empty picks, the cut inside a pick, window and sinks, rows at early
+    positions, a row's own budgets, and an owner's range."""
+    rng = np.random.default_rng(cap * 7 + m)
+    sizes = rng.integers(0, cap + 1, m)
+    order = rng.permutation(m * cap).astype(np.int32)
+    members, at = np.full((m, cap), -1, np.int32), 0
+    for b in range(m):
+        members[b, :sizes[b]] = np.sort(order[at:at + sizes[b]])
+        at += sizes[b]
+    picked = np.stack([rng.permutation(m)[:top_p] if top_p <= m else np.r_[rng.permutation(m), -np.ones(top_p - m)]
+                       for _ in range(rows)]).astype(np.int32)
+    picked[rng.random(picked.shape) < 0.1] = -1
+    positions = rng.integers(0, m * cap + 50, rows)
+    positions[:3] = 0, 1, m * cap + 40
+    for sink, window in ((0, 1), (4, 37)):
+        want, want_len = oracle.expand(picked, positions, members, top_k, sink, window)
+        got, lens, status = ops.expand(cuda(picked), cuda(positions), cuda(members), top_k, sink, window)
+        assert np.array_equal(got.cpu().numpy(), want) and np.array_equal(lens.cpu().numpy(), want_len) and not int(status)
+    cut = int(np.median(positions))
+    want, want_len = oracle.expand(picked, positions, members, top_k, 4, 37, early_budget=(cut, top_k // 3 + 1, top_p // 2 + 1))
+    early = cuda(positions) < cut
+    row_p = torch.where(early, top_p // 2 + 1, top_p).to(torch.int32)
+    row_k = torch.where(early, top_k // 3 + 1, top_k).to(torch.int32)
+    got, lens, _ = ops.expand(cuda(picked), cuda(positions), cuda(members), top_k, 4, 37, row_p, row_k)
+    assert np.array_equal(got.cpu().numpy(), want) and np.array_equal(lens.cpu().numpy(), want_len)
+    half = m * cap // 2
+    parts = [ops.expand(cuda(picked), cuda(positions), cuda(members), top_k, 4, 37, row_p, row_k, owner=owner)[:2]
+             for owner in ((0, half), (half, 1 << 40))]
+    for r in range(rows):
+        ids = want[r][:want_len[r]]
+        for (lists, lengths), mine in zip(parts, (ids < half, ids >= half)):
+            assert np.array_equal(lists[r].cpu().numpy()[:int(lengths[r])], ids[mine])
+
+
 def test_linear_layers_over_a_few_rows(ops):
     """The decode-row maps: heads summed or read side by side, GELU or not, unit rows or not, against fp32 torch on
     the same bf16 values (the hidden layer of the two-layer map is rounded to bf16, as the batched map rounds it)."""
