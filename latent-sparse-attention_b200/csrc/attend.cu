@@ -24,7 +24,10 @@ struct AttendParams {
   float scale_log2;
 };
 
-// DH: head dim (64 or 128). NT: 8-head tiles a group needs (1 or 2). W: warps a CTA. STAGES: ring depth.
+// DH: head dim (64 or 128). NT: 8-head tiles a group needs (1 or 2). W: warps a CTA, at most. STAGES: ring depth.
+// What bounds a chunk of prefill rows is the gather's bytes out of L2 (10 to 11 TB/s in the 256-byte rows of 1,024-byte
+// tokens): stages of 16 keys with 14 warps an SM, or three stages a warp, moved the same or less (1.70 ms became 1.73 to
+// 2.30 over 16,384 rows of 1,100 keys and 2 KV heads).
 template <int DH, int NT, int W, int STAGES>
 __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p) {
   constexpr int ROW_BYTES = DH * 2;
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t item = (int64_t)blockIdx.x * W + warp;
+  const int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
   dependents_may_launch();
   wait_for_earlier_grids();
   if (item >= p.R * p.splits * p.Hkv) return;
@@ -388,14 +391,19 @@ __global__ void __launch_bounds__(128)
 template <int DH, int NT, int W, int STAGES>
 static int launch_attend(const AttendParams &p, cudaStream_t s) {
   constexpr int WARP_BYTES = STAGES * 2 * kKeysPerStage * DH * 2 + 16;
-  const size_t smem = (size_t)W * WARP_BYTES;
+  const int64_t items = p.R * p.splits * p.Hkv;
+  // A decode step has fewer items than the SMs have room for warps: they are spread over all SMs, so that an item has an
+  // SM's copies to itself as far as there are SMs (a row's 64 items of 385 keys: 23.4 us on ten SMs, 14.5 on 64; 128 items
+  // of 190 keys: 12.1 on 19 SMs, 7.3 on 128).
+  const int64_t spread = (items + sm_count() - 1) / sm_count();
+  const int warps = (int)(spread < W ? spread : W);
+  const size_t smem = (size_t)warps * WARP_BYTES;
   if (cudaFuncSetAttribute(sparse_attend_kernel<DH, NT, W, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return LSA_ERR_LAUNCH;
-  const int64_t items = p.R * p.splits * p.Hkv;
-  const int64_t grid = (items + W - 1) / W;
+  const int64_t grid = (items + warps - 1) / warps;
   if (grid > INT32_MAX) return LSA_ERR_ARGUMENT;
-  launch(p.R <= kChainedRows, sparse_attend_kernel<DH, NT, W, STAGES>, dim3((unsigned)grid), dim3(W * 32), smem, s, p);
+  launch(p.R <= kChainedRows, sparse_attend_kernel<DH, NT, W, STAGES>, dim3((unsigned)grid), dim3(warps * 32), smem, s, p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

@@ -246,6 +246,24 @@ def test_linear_layers_over_a_few_rows(ops):
         ops.rows_linear(torch.zeros(9, 64, device="cuda", dtype=torch.bfloat16), wide)
 
 
+def test_a_rows_gather_does_not_depend_on_the_rows_beside_it(ops):
+    """Items are spread one warp a CTA while there are fewer than SMs, up to seven a CTA: the same bits either way."""
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    for Hq, Hkv, dh in ((8, 2, 128), (24, 2, 128), (8, 2, 64)):
+        q = torch.randn(260, Hq, dh, generator=gen, device="cuda").bfloat16()
+        k, v = (torch.randn(900, Hkv, dh, generator=gen, device="cuda").bfloat16() for _ in range(2))
+        ids = torch.stack([torch.randperm(900, generator=gen, device="cuda")[:333] for _ in range(260)]).to(torch.int32)
+        lens = torch.randint(0, 334, (260,), generator=gen, device="cuda", dtype=torch.int32)
+        for splits in (1, 3, 16):
+            whole, whole_lse = ops.sparse_attend(q, k, v, ids, lens, dh ** -0.5, splits=splits)
+            for n in (1, 5, 80):
+                part, lse = ops.sparse_attend(q[:n], k, v, ids[:n], lens[:n], dh ** -0.5, splits=splits)
+                if splits == 1:
+                    assert torch.equal(part, whole[:n]) and torch.equal(lse, whole_lse[:n])
+                else:  # (the merge of the splits goes by the number of rows: fp32 sums of up to 16 terms, rounded to bf16)
+                    assert (part.float() - whole[:n].float()).abs().max() <= 2 ** -8 * whole.float().abs().max()
+
+
 def test_kmeans_bucketing_matches_its_restatement(ops, oracle):
     """A variant with no reference code: config 1's shapes - 1,024 pools, 256 centres, 32 dims, 10 rounds."""
     keys = unit_rows(mixture(16384, 32, 64, 0.3, 8))
