@@ -342,7 +342,7 @@ class FlatLayer:
         Every intermediate lives in buffers the layer keeps, so after the first call a step allocates nothing but
         its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
         `band` reads the window and the sinks as dense tiles; `bucket_major` reads the selected keys bucket by bucket
-        where the shapes allow (both off: every row gathers its whole list).
+        where the shapes allow and it is the faster read (both off: every row gathers its whole list).
         """
         T = q.shape[0]
         index = self.build_index(k, reuse_buffers=not return_index)
@@ -403,6 +403,15 @@ class FlatLayer:
         main.wait_stream(self._copy_out)
         return out_host
 
+    @property
+    def _reads_by_bucket(self) -> bool:
+        """Whether reading the selected keys bucket by bucket is the faster read. It costs a partial output a (row, pick,
+        query head), whatever the bucket holds; the gather costs the bytes of a pick's keys once a KV head. Measured on a
+        B200, bucket-major against gather, whole prefills: buckets of 8 keys under groups of 4, 8 and 5 heads 22.3 / 13.3,
+        35.1 / 13.6 and 82.7 / 39.8 ms (24,576 tokens); buckets of 32 keys under groups of 4, 5 and 8 heads 19.0 / 32.6,
+        69.7 / 137.5 and 29.7 / 34.0 ms (131,072 tokens): the two meet near four keys a query head of the group."""
+        return self.design.bucket_size >= 4 * (self.heads // self.kv_heads)
+
     def prefill_rows(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, band: bool = True, bucket_major: bool = True) -> torch.Tensor:
         """The read of consecutive query rows [n, Hq, dh] at positions start.. over a cache whose index is built,
@@ -418,7 +427,8 @@ class FlatLayer:
         banded = band and self.design.sink_size <= 64 and k.shape[0] >= stop
         lse = self._buffer("lse", (n, self.heads), torch.float32, dev)
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
-        if banded and bucket_major and ops.bucket_attend_supported(rows, k, self.design.bucket_cap):
+        if banded and bucket_major and self._reads_by_bucket and \
+                ops.bucket_attend_supported(rows, k, self.design.bucket_cap):
             # The band and the read of the selected keys meet only in the merge, and one waits on the tensor pipe
             # while the other is bound by instruction issue: the band runs on a stream of its own beside them.
             main = torch.cuda.current_stream(dev)
