@@ -134,12 +134,15 @@ class FlatLayer:
     # ---- buffers
 
     def _buffer(self, name: str, shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
-        """A tensor that lives as long as the layer: a step allocates nothing once every shape has been seen."""
-        key = (name, tuple(shape), dtype, str(device))
-        held = self._buffers.get(key)
-        if held is None:
-            held = self._buffers[key] = torch.empty(shape, device=device, dtype=dtype)
-        return held
+        """A tensor that lives as long as the layer: a step allocates nothing once every shape has been seen. (Fewer rows
+        than a buffer of that name has are its leading ones: a ragged chunk allocates nothing beside a whole one.)"""
+        key = (name, tuple(shape[1:]), dtype, str(device))
+        held = self._buffers.setdefault(key, [])  # ascending: a call that outgrows them adds one, and none moves
+        for buffer in held:
+            if buffer.shape[0] >= shape[0]:
+                return buffer[:shape[0]]
+        held.append(torch.empty(shape, device=device, dtype=dtype))
+        return held[-1]
 
     def _takes_tensor_cores(self, x: torch.Tensor) -> bool:
         """Heads packed densely in bf16 with a 16-byte aligned row pitch: the layout a TMA descriptor can walk."""
@@ -185,7 +188,7 @@ class FlatLayer:
         d, d_idx = self.design, self.index_dim
         blocks = T // d.cluster_block_size
         P, rows = d.cluster_block_size // d.pool_size, blocks * d.block_bucket_count
-        make = (lambda name, shape, dtype: self._buffer(name, shape, dtype, dev)) if reuse_buffers else \
+        make = (lambda name, shape, dtype: self._buffer(f"{name} of {T}", shape, dtype, dev)) if reuse_buffers else \
             (lambda name, shape, dtype: torch.empty(shape, device=dev, dtype=dtype))
         bufs = {"keys": make("index keys", (T, d_idx), torch.float32),
                 "pools": make("pools", (blocks, P, d_idx), torch.float32),
@@ -347,9 +350,11 @@ class FlatLayer:
         T = q.shape[0]
         index = self.build_index(k, reuse_buffers=not return_index)
         out = torch.empty_like(q) if out is None else out
-        for start in range(0, T, chunk):
-            stop = min(T, start + chunk)
-            self.prefill_rows(q[start:stop], start, k, v, index, out[start:stop], band, bucket_major)
+        whole = min(T, self._whole_until(index)) if band else 0  # (rows that read everything make chunks of their own)
+        for first, end in ((0, whole), (whole, T)):
+            for start in range(first, end, chunk):
+                stop = min(end, start + chunk)
+                self.prefill_rows(q[start:stop], start, k, v, index, out[start:stop], band, bucket_major)
         return (out, index) if return_index else out
 
     def prefill_from_host(self, q_host: torch.Tensor, k_host: torch.Tensor, v_host: torch.Tensor,
@@ -403,6 +408,18 @@ class FlatLayer:
         main.wait_stream(self._copy_out)
         return out_host
 
+    def _whole_until(self, index: FlatIndex) -> int:
+        """The first position whose read leaves anything out. A row before it picks every bucket it sees, no cut bites,
+        and the window covers what is in no closed block yet: its list is all the keys up to its own, so a dense causal
+        read is the same read (and scores, picks and lists nothing). 0 where a design has no such rows."""
+        d = self.design
+        if d.window_size < d.cluster_block_size or d.early_budget is not None:
+            return 0
+        by_picks = (d.top_p // d.block_bucket_count + 1) * d.cluster_block_size
+        by_index = (index.buckets.bucket_centroids.shape[0] // d.block_bucket_count + 1) * d.cluster_block_size
+        until = min(by_picks, by_index, d.top_k + d.window_size + d.sink_size)
+        return until // 128 * 128  # (whole tiles of query rows)
+
     @property
     def _reads_by_bucket(self) -> bool:
         """Whether reading the selected keys bucket by bucket is the faster read. It costs a partial output a (row, pick,
@@ -418,6 +435,21 @@ class FlatLayer:
         into `out` [n, Hq, dh] bf16 - one chunk of a prefill, or one rank's rows of a chunk."""
         n, dev = rows.shape[0], rows.device
         stop = start + n
+        if band and self.design.sink_size <= 64 and k.shape[0] >= stop and start < self._whole_until(index):
+            # (a tensor-core row costs 1.4 ps a key and head here: 0.17 us for the 3,000 keys of a row of 40 heads, against
+            # 0.5 us for its window and 64 picked buckets)
+            whole = min(n, self._whole_until(index) - start)
+            with probe.region("band"):
+                dense, _ = ops.band_attend(rows[:whole], k, v, start, start + whole, 0, self.scale,
+                                           out=self._buffer("dense out", (whole, self.heads, self.head_dim),
+                                                            torch.float32, dev),
+                                           lse=self._buffer("dense lse", (whole, self.heads), torch.float32, dev),
+                                           status=self._attend_status)
+                out[:whole].copy_(dense)
+            if whole == n:
+                return out
+            self.prefill_rows(rows[whole:], start + whole, k, v, index, out[whole:], band, bucket_major)
+            return out
         positions = torch.arange(start, stop, device=dev)
         with probe.region("index map"):
             index_queries = self.index_queries(rows, out=self._buffer("index queries", (n, self.index_dim),

@@ -95,3 +95,37 @@ def test_prefill_from_pinned_host_memory_is_the_resident_prefill():
         layer.prefill_from_host(q, k, v, out, chunk=2048)
         torch.cuda.current_stream().synchronize()
         assert torch.equal(out, want.cpu())
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,dh,chunk,sizes", [
+    (1500, 8, 2, 128, 512, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=600,
+                                sink_size=4, window_size=150)),   # the key budget runs out first, inside a chunk
+    (1500, 8, 2, 128, 2048, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=640,
+                                 sink_size=0, window_size=128)),  # the picks run out first
+    (777, 5, 1, 64, 300, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=4096,
+                              sink_size=4, window_size=256)),     # every row reads everything
+    (700, 8, 2, 128, 256, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=256, top_p=64, top_k=600,
+                               sink_size=4, window_size=100)),    # a window short of a block: no row is read densely
+])
+def test_rows_that_read_everything_are_read_densely(oracle, T, Hq, Hkv, dh, chunk, sizes):
+    """Rows before a design leaves anything out take the dense causal read; from there on the lists: both equal the gather
+    of every row's whole list, and the boundary lies where the oracle's lists first leave a key out."""
+    from lsa_b200.layer import FlatDesign
+
+    design = FlatDesign(**sizes)
+    layer, _ = _layer(Hq, Hkv, dh, 64, design, T)
+    q, k, v = layer_inputs(T, Hq, Hkv, dh, 16, T + 2)
+    Q, K, V = (cuda(a, torch.bfloat16) for a in (q, k, v))
+    out, index = layer.prefill(Q, K, V, chunk=chunk, return_index=True)
+    gathered = layer.prefill(Q, K, V, chunk=chunk, band=False, bucket_major=False)
+    err = (out.float() - gathered.float()).abs()
+    assert err.max() <= 2e-2 and err.mean() <= 2e-3, (err.max(), err.mean())
+    positions = np.arange(T)
+    _, lengths = layer.select(layer.index_queries(Q), cuda(positions), index)
+    everything = lengths.cpu().numpy() == positions + 1
+    until = layer._whole_until(index)
+    if design.window_size < design.cluster_block_size:
+        assert until == 0
+    else:
+        assert everything[:until].all() and (until >= T or not everything[until:].all())
+    layer.check()
