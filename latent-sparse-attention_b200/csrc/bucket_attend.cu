@@ -502,7 +502,9 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
                   m >= 0 && m < INT32_MAX && bucket_cap >= 1 && top_k >= 1 && sink >= 0 && window >= 1 &&
                   R * top_p < INT32_MAX && scale > 0.0f,
               LSA_ERR_ARGUMENT);
-  LSA_REQUIRE(dh == 128 && bucket_cap <= lsa::kBktKeys && Hq / Hkv <= 8, LSA_ERR_UNSUPPORTED);
+  const bool tensor_memory = !(flags & LSA_BUCKET_WARP_MMA) && R * top_p * Hq < INT32_MAX;
+  LSA_REQUIRE(dh == 128 && bucket_cap <= (tensor_memory ? lsa::kBktKeysTc : lsa::kBktKeys) && Hq / Hkv <= 8,
+              LSA_ERR_UNSUPPORTED);
   LSA_REQUIRE(kv_row_stride % 8 == 0 && kv_head_stride % 8 == 0 && ((uintptr_t)k % 16) == 0 &&
                   ((uintptr_t)v % 16) == 0 && q_row_stride % 8 == 0 && q_head_stride % 8 == 0 &&
                   ((uintptr_t)q % 16) == 0,
@@ -533,7 +535,6 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
   p.kv_row_stride = kv_row_stride, p.kv_head_stride = kv_head_stride;
   p.top_p = top_p, p.cap = bucket_cap, p.top_k = top_k, p.sink = sink, p.window = window;
   p.Hq = Hq, p.Hkv = Hkv, p.group = Hq / Hkv;
-  const bool tensor_memory = !(flags & LSA_BUCKET_WARP_MMA) && R * top_p * Hq < INT32_MAX;
   p.segment = tensor_memory ? lsa::kBktSegmentTc : lsa::kBktSegment;
   p.scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t s = (cudaStream_t)stream;

@@ -5,7 +5,8 @@
 
 namespace lsa {
 
-constexpr int kBktKeys = 64;     // members a bucket may hold here (the tile of keys a CTA stages)
+constexpr int kBktKeys = 64;     // members a bucket may hold in the warp-level pass (the tile of keys a CTA stages)
+constexpr int kBktKeysTc = 128;  // and in the tcgen05 pass
 constexpr int kBktSegment = 128;  // (row, pick) pairs a CTA of the warp-level pass runs through its bucket
 constexpr int kBktSegmentTc = 256;  // and of the tcgen05 pass: twice the tiles for one staging of the bucket
 constexpr int kBktTile = 16;     // query rows a warp multiplies at once
@@ -36,8 +37,7 @@ struct BucketParams {
   float scale_log2;
 };
 
-// The attend pass on the fifth-generation tensor cores (bucket_attend_tc.cu); `variant` picks a descriptor form
-// while the kernel is being validated.
+// The attend pass on the fifth-generation tensor cores (bucket_attend_tc.cu).
 int launch_bucket_attend_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t stream);
 
 }  // namespace lsa

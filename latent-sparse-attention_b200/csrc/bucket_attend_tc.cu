@@ -7,19 +7,21 @@
 //
 //   S [128 x keys]  = Q [128 x 128] . K^T           tcgen05.mma, A = the tile's query rows, B = the bucket's keys,
 //                                                   both K-major planes of 64 dims with the 128-byte swizzle
-//   P               = exp2(S - rowmax) / rowsum on the row's key range, bf16, written back to shared memory
+//   P               = exp2(S - rowmax) on the row's key range, bf16, written back to shared memory (divided by the
+//                     row's sum first where a thread can hold the whole row: buckets of up to 64 keys)
 //   O [128 x 128]   = P [128 x keys] . V            A = P (K-major), B = the bucket's values AS STORED
 //                                                   ([key][dim] planes: an MN-major operand)
 //
-// Eight warps. Together they gather the query rows of the tile after next (a row of 256 bytes a half warp) and send
-// the finished tile's rows out in the same shape. For the softmax and the unloading of O a row has TWO threads, one
-// in warp q and one in warp 4 + q (both may read the tensor-memory lanes of quarter q): they take alternate groups
-// of 8 keys of S, swap their maxima and sums through shared memory, and take a half of O's columns each. The row's instruction stream is what bounds this kernel, so it
-// is cut in two. A lane of warp 0 also issues the MMAs, at the points where the warp would wait for their results
-// anyway: a ninth warp for that would cost every thread 32 registers (five warps on a scheduler instead of four).
-//
-// The tiles of a CTA overlap: the tensor cores multiply S of tile i + 1 while the workers unload O of tile i, and
-// the query rows of tile i + 2 are on their way by then. Two CTAs share an SM and fill one another's waits.
+// Two warpgroups, each with tiles of its own (every other tile of the segment), its own query buffer and its own 128
+// columns of tensor memory (O takes the columns of S, which has been read by then). A warp copies, multiplies and writes
+// out ITS 32 rows, so between the hand-overs to the tensor cores nothing waits for another warp; lane 0 of a
+// warpgroup's first warp issues its products. Two CTAs share an SM (buckets of up to 64 keys), so four tiles are under
+// way on it and fill one another's waits. What bounds it is the instruction stream around the products and the chain
+// copy - product - softmax - product - copy of a tile: 0.85 G warp instructions a launch of 8,192 rows x 64 picks x 40 heads,
+// issued on 41 % of the cycles. (With both warpgroups on ONE tile, two threads a row, swapping maxima and sums and waiting
+// for one another six times a tile, it was 1.2 G; a 131,072-token prompt spends 35.3 ms here against 41.1.) Buckets of 65
+// to 128 members take twice the shared memory, so one CTA an SM, and a thread reads its row of S twice; against the gather
+// of every row's list a 16,384-token prompt of 64-key buckets reads in 0.78 ms instead of 1.8.
 //
 // Shared-memory operands are written by ordinary and asynchronous copies (the generic proxy), so a proxy fence stands
 // before every hand-over to the tensor cores. Every wait on an mbarrier is bounded; a wait that gives up raises the
@@ -31,44 +33,42 @@
 namespace lsa {
 
 constexpr int kTcThreads = 256;
-constexpr int kTcRows = 128;                    // rows of a tile
-constexpr int kTcPlane = 64 * 128;              // a plane of 64 rows x 128 bytes (keys or values, 64 dims)
-constexpr int kTcQPlane = kTcRows * 128;        // a plane of the query tile or of P
-constexpr int kTcKOff = 0;                      // K: 2 planes
-constexpr int kTcVOff = 2 * kTcPlane;           // V: 2 planes
-constexpr int kTcQOff = 4 * kTcPlane;           // Q: 2 buffers of 2 planes
-// P takes the first plane of the tile's own query buffer (the first product is over when P is written), and the
-// finished rows of O are staged in the whole of it (the second product is over by then).
-constexpr int kTcSmem = kTcQOff + 4 * kTcQPlane + 1024;  // + room to align the base to 1,024 bytes
-constexpr int kTcTmemCols = 256;                // S in columns 0-63, O in 64-191
-static_assert(kBktSegmentTc == kTcThreads && kBktKeys == 64, "a thread a pair of the segment; 64 keys a bucket");
+constexpr int kTcRows = 128;                    // rows of a tile: a warpgroup's threads
+constexpr int kTcQPlane = kTcRows * 128;        // a plane (64 dims) of the query tile, of P (64 keys) or of finished rows
+constexpr int kTcTmemCols = 256;                // 128 columns a warpgroup: S, then O
+static_assert(kBktSegmentTc == kTcThreads, "a thread a pair of the segment");
+
+// Shared memory: K and V (2 planes of 64 dims each), then a query buffer of two planes a warpgroup. P takes the query
+// buffer's planes (the first product is over when P is written), and the finished rows of O are staged in the whole of it
+// (the second product is over by then).
+template <int KEYS>
+constexpr int tc_smem() {
+  return 4 * KEYS * 128 + 2 * 2 * kTcQPlane + 1024;  // + room to align the base to 1,024 bytes
+}
 
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// the two warps of a quarter of the rows
-__device__ __forceinline__ void quarter_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory"); }
 
-
-template <int DH>
-__global__ void __launch_bounds__(kTcThreads, 2) bucket_attend_tc_kernel(BucketParams p) {
+// KEYS: members a bucket may hold, 64 or 128.
+template <int DH, int KEYS>
+__global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_tc_kernel(BucketParams p) {
   static_assert(DH == 128, "two planes of 64 dims");
+  constexpr int kPlane = KEYS * 128;           // a plane of KEYS rows x 64 dims
+  constexpr int kKOff = 0, kVOff = 2 * kPlane, kQOff = 4 * kPlane;
+  constexpr int kWords = KEYS / 32;
+  constexpr bool kHeld = KEYS == 64;           // a thread holds its whole row of S
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ int32_t ids_s[kBktKeys];
+  __shared__ int32_t ids_s[KEYS];
   __shared__ int32_t pairs_s[kBktSegmentTc];   // the segment's pairs, -1 past its end
   __shared__ int32_t qrows_s[kBktSegmentTc];   // their query rows
   __shared__ int32_t hi_s[kBktSegmentTc];      // members of the bucket they read
-  // of the rows of a tile (a ring of three tiles): where the query row starts in q (-1 past the end), which slot of
-  // the partial outputs it fills, and the end of its key range
-  __shared__ int64_t src_s[3][kTcRows];
-  __shared__ int32_t dst_s[3][kTcRows];  // (the caller has checked that the slots fit 31 bits)
-  __shared__ int32_t end_s[3][kTcRows];
-  __shared__ float swap_max_s[2][kTcRows], swap_sum_s[2][kTcRows];
-  __shared__ __align__(8) uint64_t bars[3];
+  __shared__ int64_t src_s[2][kTcRows];        // where the query rows of a warpgroup's tile start in q, -1 past the end
+  __shared__ __align__(8) uint64_t bars[6];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
-  __shared__ uint32_t valid_s[2];  // which members of the bucket name a row of the cache
+  __shared__ uint32_t valid_s[kWords];         // which members of the bucket name a row of the cache
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y;
@@ -81,13 +81,15 @@ __global__ void __launch_bounds__(kTcThreads, 2) bucket_attend_tc_kernel(BucketP
   const int n_rows = n_pairs * p.group;
   const int n_tiles = (n_rows + kTcRows - 1) / kTcRows;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  // bar_w: the workers tell the MMA lane that operands are in place; bar_s / bar_o: a product has finished
-  const uint32_t bar_w = smem_u32(&bars[0]), bar_s = smem_u32(&bars[1]), bar_o = smem_u32(&bars[2]);
+  const int wg = warp >> 2;                  // the warpgroup
+  const int quarter = warp & 3;              // the 32 tensor-memory lanes (and tile rows) this warp has
+  const int row = quarter * 32 + lane;       // the tile row (= tensor-memory lane)
+  // of the warpgroup - bar_w: its threads tell its issuing lane that operands are in place (queries, then P, of every
+  // tile); bar_s / bar_o: a product has finished
+  const uint32_t bar_w = smem_u32(&bars[wg]), bar_s = smem_u32(&bars[2 + wg]), bar_o = smem_u32(&bars[4 + wg]);
 
   if (tid == 0) {
-    mbar_init(bar_w, kTcThreads);
-    mbar_init(bar_s, 1);
-    mbar_init(bar_o, 1);
+    for (int i = 0; i < 6; ++i) mbar_init(smem_u32(&bars[i]), i < 2 ? kTcRows : 1);
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -96,10 +98,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) bucket_attend_tc_kernel(BucketP
                  "r"(kTcTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  for (int i = tid; i < kBktKeys; i += kTcThreads) ids_s[i] = i < p.cap ? p.members[bucket * p.cap + i] : LSA_PAD;
+  for (int i = tid; i < KEYS; i += kTcThreads) ids_s[i] = i < p.cap ? p.members[bucket * p.cap + i] : LSA_PAD;
   // The segment's pairs, fetched beside the member ids (one round of loads for both). The starts pass has counted the
   // keys a pair takes; its run of members starts where the sinks end, which is added once the ids are in.
-  if (tid < kBktSegmentTc) {
+  {
     int32_t pair = -1, take = 0;
     if (tid < n_pairs) {
       pair = p.order[first + tid];
@@ -110,286 +112,284 @@ __global__ void __launch_bounds__(kTcThreads, 2) bucket_attend_tc_kernel(BucketP
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_s;
+  const uint32_t tmem = tmem_base_s + wg * DH;
+  const uint32_t buf = base + kQOff + wg * 2 * kTcQPlane;  // the warpgroup's query buffer
 
-  // members of the bucket: the ids before the first pad
-  int n_members;
-  {
-    const unsigned low = __ballot_sync(0xffffffffu, ids_s[lane] >= 0),
-                   high = __ballot_sync(0xffffffffu, ids_s[lane + 32] >= 0);
-    n_members = low != 0xffffffffu ? __ffs(~low) - 1 : (high != 0xffffffffu ? 32 + __ffs(~high) - 1 : 64);
-    n_members = min(n_members, p.cap);
+  // members of the bucket: the ids before the first pad; and which of them name a row of the cache handed in (a key
+  // outside it is staged as zeros and masked out of the softmax, as the row-by-row read skips such ids)
+  int n_members = 0;
+  bool all_valid = true, ended = false;
+#pragma unroll
+  for (int w = 0; w < kWords; ++w) {
+    const int32_t id = ids_s[32 * w + lane];
+    const unsigned some = __ballot_sync(0xffffffffu, id >= 0), valid = __ballot_sync(0xffffffffu, id >= 0 && id < p.slots);
+    if (!ended) n_members += some != 0xffffffffu ? __ffs(~some) - 1 : 32;
+    ended = ended || some != 0xffffffffu;
+    all_valid = all_valid && valid == some;
+    if (tid == 0) valid_s[w] = valid;
   }
-  // members that name a row of the cache handed in: a key outside it is staged as zeros and masked out of the softmax,
-  // as the row-by-row read skips such ids
-  // (the word stays in shared memory and only a flag in a register: every member is in the cache as a rule, and a
-  // 64-bit word held through the tile loop costs this kernel spills)
-  bool all_valid;
-  {
-    const uint32_t v_lo = __ballot_sync(0xffffffffu, ids_s[lane] >= 0 && ids_s[lane] < p.slots),
-                   v_hi = __ballot_sync(0xffffffffu, ids_s[lane + 32] >= 0 && ids_s[lane + 32] < p.slots);
-    all_valid = __popc(v_lo) + __popc(v_hi) == n_members;
-    if (tid == 0) valid_s[0] = v_lo, valid_s[1] = v_hi;
-  }
-  // which of keys c0 .. c0 + 7 name a row of the cache, a bit each
+  n_members = min(n_members, p.cap);
+  // (the words stay in shared memory and only a flag in a register: every member is in the cache as a rule)
   auto valid_byte = [&](int c0) { return all_valid ? 0xFFu : (valid_s[c0 >> 5] >> (c0 & 31)) & 0xFFu; };
   const int n_keys = max(16, (n_members + 15) & ~15);  // the N of S and the K of O: whole 16-key steps
+  int lo_key = 0;
+  {
+    int hi = n_members;
+    while (lo_key < hi) {
+      const int mid = (lo_key + hi) >> 1;
+      if (ids_s[mid] < p.sink) lo_key = mid + 1; else hi = mid;
+    }
+  }
+  // The bucket's keys and values of this KV head: chunk c of member j goes to plane c / 8, row j, 16-byte slot
+  // (c % 8) ^ (j % 8) - the layout a tensor-map copy with the 128-byte swizzle would write.
+  {
+    const uint16_t *k_head = p.k + (int64_t)h * p.kv_head_stride, *v_head = p.v + (int64_t)h * p.kv_head_stride;
+#pragma unroll 2
+    for (int e = tid; e < n_keys * 16; e += kTcThreads) {
+      const int r = e >> 4, chunk = e & 15;
+      const int32_t id = ids_s[r];
+      const bool ok = id >= 0 && id < p.slots;
+      const int64_t off = ok ? (int64_t)id * p.kv_row_stride + chunk * 8 : 0;
+      const uint32_t dst = (chunk >> 3) * kPlane + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
+      cp_async_16(base + kKOff + dst, k_head + off, ok ? 16 : 0);
+      cp_async_16(base + kVOff + dst, v_head + off, ok ? 16 : 0);
+    }
+    cp_async_commit();
+  }
+  const uint32_t group_inverse = (65536u + (uint32_t)p.group - 1) / (uint32_t)p.group;  // flat / group, exact here
+  int hi_key = 0;       // of this thread's row: the end of its key range,
+  int32_t slot = -1;    // and the slot of the partial outputs it fills (the caller has checked that slots fit 31 bits)
+  auto list_rows = [&](int tile) {
+    const int flat = tile * kTcRows + row;
+    const bool ok = flat < n_rows;
+    const int pl = ok ? (int)((uint32_t)flat * group_inverse >> 16) : 0;
+    const int head = h * p.group + (flat - pl * p.group);
+    src_s[wg][row] = ok ? (int64_t)qrows_s[pl] * p.q_row_stride + (int64_t)head * p.q_head_stride : -1;
+    slot = ok ? pairs_s[pl] * p.Hq + head : -1;
+    hi_key = ok ? lo_key + hi_s[pl] : 0;
+    __syncwarp();
+  };
+  // The warp's query rows of a tile: half a warp copies a row of 256 bytes, in the layout of the keys.
+  const int chunk = lane & 15;
+  const uint32_t lane_at = (chunk >> 3) * kTcQPlane + quarter * 32 * 128;
+  auto gather_q = [&] {
+#pragma unroll 8
+    for (int j = 0; j < 16; ++j) {
+      const int r = 2 * j + (lane >> 4);  // of the warp's 32
+      const int64_t from = src_s[wg][quarter * 32 + r];
+      cp_async_16(buf + lane_at + r * 128 + (((chunk & 7) ^ (r & 7)) << 4), p.q + (from >= 0 ? from + chunk * 8 : 0),
+                  from >= 0 ? 16 : 0);
+    }
+    cp_async_commit();
+  };
+  // The issuing lane's turn (the whole warp waits so that its lanes stay together): false once the CTA has given up.
+  auto my_turn = [&](uint32_t parity) {
+    if (__all_sync(0xffffffffu, !abort_s && mbar_wait(bar_w, parity))) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return true;
+    }
+    abort_s = 1;
+    return false;
+  };
 
-  // Step k of the MMAs (warp 0; the whole warp waits so that its lanes stay together, lane 0 issues): once the k-th
-  // hand-over of the threads is complete, O of tile k - 1 and S of tile k.
-  auto issue_products = [&](int k) {
-    if (!__all_sync(0xffffffffu, !abort_s && mbar_wait(bar_w, k & 1))) {
-      abort_s = 1;
-      return;
+  const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+  if (wg < n_tiles) {
+    list_rows(wg);
+    gather_q();
+  }
+  cp_async_wait<0>();
+  proxy_fence();
+  __syncthreads();  // K and V are in place (a warpgroup without tiles has copied its share too)
+  for (int tile = wg, n = 0; tile < n_tiles; tile += 2, ++n) {
+    const uint32_t parity = n & 1;
+    if (n > 0) {
+      cp_async_wait<0>();
+      proxy_fence();
     }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (lane != 0) return;
-    if (k >= 1) {  // O = P V: 16 keys are 32 bytes along P's rows, 16 rows (2,048 bytes) down V's planes
-      const uint32_t p_buf = base + kTcQOff + ((k - 1) & 1) * 2 * kTcQPlane;
-      for (int s = 0; s < n_keys / 16; ++s)
-        umma_bf16(tmem_base + 64, smem_desc_sw128(p_buf) + 2 * s, smem_desc_mn_sw128(base + kTcVOff + s * 2048, kTcPlane),
-                  umma_idesc(DH, true), s != 0);
-      umma_commit(bar_o);
-    }
-    if (k < n_tiles) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
-      const uint32_t q_buf = base + kTcQOff + (k & 1) * 2 * kTcQPlane;
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    mbar_arrive(bar_w);  // this thread's part of the tile's queries is in place, and it has read its row of the last O
+    if (quarter == 0 && my_turn(0) && lane == 0) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
 #pragma unroll
       for (int plane = 0; plane < 2; ++plane)
 #pragma unroll
         for (int s = 0; s < 4; ++s)
-          umma_bf16(tmem_base, smem_desc_sw128(q_buf + plane * kTcQPlane) + 2 * s,
-                    smem_desc_sw128(base + kTcKOff + plane * kTcPlane) + 2 * s, umma_idesc(n_keys), (plane | s) != 0);
+          umma_bf16(tmem, smem_desc_sw128(buf + plane * kTcQPlane) + 2 * s,
+                    smem_desc_sw128(base + kKOff + plane * kPlane) + 2 * s, umma_idesc(n_keys), (plane | s) != 0);
       umma_commit(bar_s);
     }
-  };
-  {
-    const int w = tid;                         // the thread's place in the shared copies
-    const int quarter = warp & 3;              // the 32 tensor-memory lanes this warp may read
-    const int half = warp >> 2;                // which of the row's two threads
-    const int row = quarter * 32 + lane;       // the tile row (= tensor-memory lane)
-    auto members_below = [&](int64_t bound) {
-      int lo = 0, hi = n_members;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (ids_s[mid] < bound) lo = mid + 1; else hi = mid;
+    __syncwarp();
+    // A group of 8 keys that lies inside the key range of every row of the warp needs no masks: most do.
+    const int hi_min = __reduce_min_sync(0xffffffffu, hi_key);
+    auto whole = [&](int c0) { return c0 >= lo_key && c0 + 8 <= hi_min && valid_byte(c0) == 0xFFu; };
+    // ---- softmax of the row: P is the A operand of the second product. (One decision a warp on a wait: the
+    // tensor-memory loads are warp-wide instructions.)
+    bool go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_s, parity));
+    if (!go) abort_s = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t sv[kHeld ? kWords : 1][32];
+    // keys 32 c .. 32 c + 31 of the row, the masked ones at -inf
+    auto load_keys = [&](int c, uint32_t (&v)[32]) {
+      if (go) tmem_load_32(lane_addr + 32 * c, v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c0 = 32 * c + 8 * j;
+        if (c0 >= n_keys || whole(c0)) continue;
+        const uint32_t vb = valid_byte(c0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {  // (bitwise logic and selects: branches here would diverge lane by lane)
+          const bool ok = (c0 + i >= lo_key) & (c0 + i < hi_key) & (bool)((vb >> i) & 1u);
+          v[8 * j + i] = ok ? v[8 * j + i] : 0xFF800000u;
+        }
       }
-      return lo;
     };
-    const int lo_key = members_below(p.sink);
-    // The bucket's keys and values of this KV head: chunk c of member j goes to plane c / 8, row j, 16-byte slot
-    // (c % 8) ^ (j % 8) - the layout a tensor-map copy with the 128-byte swizzle would write.
-    {
-      const uint16_t *k_head = p.k + (int64_t)h * p.kv_head_stride, *v_head = p.v + (int64_t)h * p.kv_head_stride;
-#pragma unroll 2
-      for (int e = w; e < kBktKeys * 16; e += kTcThreads) {
-        const int r = e >> 4, chunk = e & 15;
-        const int32_t id = ids_s[r];
-        const bool ok = id >= 0 && id < p.slots;
-        const int64_t off = ok ? (int64_t)id * p.kv_row_stride + chunk * 8 : 0;
-        const uint32_t dst = (chunk >> 3) * kTcPlane + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
-        cp_async_16(base + kTcKOff + dst, k_head + off, ok ? 16 : 0);
-        cp_async_16(base + kTcVOff + dst, v_head + off, ok ? 16 : 0);
+    // (four running maxima, and four running sums below: one chain of 64 dependent operations is what a thread with few
+    // warps beside it waits on)
+    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int c = 0; c < kWords; ++c) {
+      if (32 * c >= n_keys) continue;
+      uint32_t (&v)[32] = sv[kHeld ? c : 0];
+      load_keys(c, v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (32 * c + 8 * j >= n_keys) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[8 * j + i]));
       }
     }
-    // Rows come in, are listed and go out a QUARTER at a time: the two warps that share the tensor-memory lanes of 32
-    // rows also copy those rows, so the only barriers inside a tile are between those two warps.
-    const int w64 = half * 32 + lane;  // the thread's place among the 64 of its quarter
-    auto list_rows = [&](int tile) {
-      if (half != 0) return;
-      const int flat = tile * kTcRows + row;
-      const bool ok = flat < n_rows;
-      const int pl = ok ? flat / p.group : 0;
-      const int head = h * p.group + (flat - pl * p.group);
-      src_s[tile % 3][row] = ok ? (int64_t)qrows_s[pl] * p.q_row_stride + (int64_t)head * p.q_head_stride : -1;
-      dst_s[tile % 3][row] = ok ? pairs_s[pl] * p.Hq + head : -1;
-      end_s[tile % 3][row] = ok ? lo_key + hi_s[pl] : 0;
-    };
-    // The query rows of a tile: half a warp copies a row of 256 bytes, in the layout of the keys.
-    auto gather_q = [&](int tile) {
-      const uint32_t buf = base + kTcQOff + (tile & 1) * 2 * kTcQPlane;
-#pragma unroll 4
-      for (int j = 0; j < 32 * 16 / 64; ++j) {
-        const int e = j * 64 + w64;
-        const int r = quarter * 32 + (e >> 4), chunk = e & 15;
-        const int64_t from = src_s[tile % 3][r];
-        cp_async_16(buf + (chunk >> 3) * kTcQPlane + r * 128 + (((chunk & 7) ^ (r & 7)) << 4),
-                    p.q + (from >= 0 ? from + chunk * 8 : 0), from >= 0 ? 16 : 0);
-      }
-    };
-    list_rows(0);
-    if (n_tiles > 1) list_rows(1);
-    quarter_sync(quarter);  // and the first tiles' rows of this quarter
-    gather_q(0);
-    cp_async_commit();
-    if (n_tiles > 1) gather_q(1);
-    cp_async_commit();
-    cp_async_wait<1>();
-    proxy_fence();
-    mbar_arrive(bar_w);  // K, V and the first tile's queries are in place
-    if (warp == 0) issue_products(0);
-
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    for (int tile = 0; tile < n_tiles; ++tile) {
-      const uint32_t parity = tile & 1;
-      const uint32_t buf = base + kTcQOff + parity * 2 * kTcQPlane;
-      const int hi_key = end_s[tile % 3][row];
-      const int64_t slot = dst_s[tile % 3][row];
-      // ---- softmax of the row: P, bf16 and already divided by the row's sum, is the A operand of the second product.
-      // This thread has the groups of 8 keys 2 j + half. (One decision a warp on the wait: the tensor-memory loads
-      // are warp-wide instructions.)
-      bool go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_s, parity));
-      if (!go) abort_s = 1;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // A group of 8 keys that lies inside the key range of every row of the warp needs no masks: most do.
-      uint32_t sv[4][8];
-      bool active[4], whole[4];
+    const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+    const float m_row = mx == -INFINITY ? 0.0f : mx * p.scale_log2;  // (finite, so that a masked key gives exp2(-inf) = 0)
+    float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto exponentials = [&](int c, uint32_t (&v)[32]) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int c0 = (2 * j + half) * 8;
-        active[j] = c0 < n_keys;
-        whole[j] = __all_sync(0xffffffffu, c0 >= lo_key && c0 + 8 <= hi_key) && valid_byte(c0) == 0xFFu;
-        if (go && active[j]) tmem_load_8(lane_addr + c0, sv[j]);
-      }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      // (four running maxima, and four running sums below: one chain of 32 dependent operations is what a thread
-      // with few warps beside it waits on)
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (32 * c + 8 * j >= n_keys) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c0 = (2 * j + half) * 8;
-        if (!active[j]) continue;
-        if (whole[j]) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sv[j][c]));
-        } else {
-          const uint32_t vb = valid_byte(c0);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {  // (bitwise logic and selects: branches here would diverge lane by lane)
-            const bool ok = (c0 + c >= lo_key) & (c0 + c < hi_key) & (bool)((vb >> c) & 1u);
-            mx4[c & 3] = fmaxf(mx4[c & 3], ok ? __uint_as_float(sv[j][c]) : -INFINITY);
-          }
+        for (int i = 0; i < 8; ++i) {
+          const float e = fast_exp2(fmaf(__uint_as_float(v[8 * j + i]), p.scale_log2, -m_row));
+          l4[i & 3] += e;
+          v[8 * j + i] = __float_as_uint(e);
         }
       }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      swap_max_s[half][row] = mx;
-      quarter_sync(quarter);
-      mx = fmaxf(mx, swap_max_s[half ^ 1][row]);
-      const float m_row = mx == -INFINITY ? 0.0f : mx * p.scale_log2;  // (finite, so that a masked key gives exp2(-inf) = 0)
-      float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    };
+    // 16-byte slot (key / 8 % 8) ^ (row % 8) of the row, in the plane of the key's 64
+    auto store_p = [&](int c, uint32_t (&v)[32], float by) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int c0 = (2 * j + half) * 8;
-        if (!active[j]) continue;
-        if (whole[j]) {
+        const int c8 = 4 * c + j;
+        if (8 * c8 >= n_keys) continue;
+        uint32_t w[4];
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float e = fast_exp2(fmaf(__uint_as_float(sv[j][c]), p.scale_log2, -m_row));
-            l4[c & 3] += e;
-            sv[j][c] = __float_as_uint(e);
-          }
-        } else {
-          const uint32_t vb = valid_byte(c0);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const bool ok = (c0 + c >= lo_key) & (c0 + c < hi_key) & (bool)((vb >> c) & 1u);
-            const float e = fast_exp2(fmaf(ok ? __uint_as_float(sv[j][c]) : -INFINITY, p.scale_log2, -m_row));
-            l4[c & 3] += e;
-            sv[j][c] = __float_as_uint(e);
-          }
+        for (int i = 0; i < 4; ++i) {
+          const float a = __uint_as_float(v[8 * j + 2 * i]), b = __uint_as_float(v[8 * j + 2 * i + 1]);
+          w[i] = kHeld ? pack_bf16x2(a * by, b * by) : pack_bf16x2(a, b);
         }
-      }
-      float l_row = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-      swap_sum_s[half][row] = l_row;
-      quarter_sync(quarter);
-      l_row += swap_sum_s[half ^ 1][row];
-      const float inv = l_row > 0.0f ? 1.0f / l_row : 0.0f;
-      const uint32_t p_row = buf + row * 128;  // 16-byte slot (c / 8) ^ (row % 8) of the row
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c8 = 2 * j + half;
-        if (!active[j]) continue;
-        uint32_t v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          v[i] = pack_bf16x2(__uint_as_float(sv[j][2 * i]) * inv, __uint_as_float(sv[j][2 * i + 1]) * inv);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p_row + ((c8 ^ (row & 7)) << 4)), "r"(v[0]),
-                     "r"(v[1]), "r"(v[2]), "r"(v[3])
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (c8 >> 3) * kTcQPlane + row * 128 +
+                                                                       (((c8 & 7) ^ (row & 7)) << 4)),
+                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
                      : "memory");
       }
-      if (go && half == 0 && slot >= 0)
-        p.part_lse[slot] = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
-      cp_async_wait<0>();  // the next tile's queries (sent a tile ago) have landed too
-      proxy_fence();
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(bar_w);
-      if (warp == 0) issue_products(tile + 1);
-      // ---- O of the tile: out of tensor memory into the tile's (spent) query buffer, this thread's half of the
-      // columns, then out in whole rows
-      go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_o, parity));
-      if (!go) abort_s = 1;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (go) {
+    };
+#pragma unroll
+    for (int c = 0; c < kWords; ++c) {
+      if (32 * c >= n_keys) continue;
+      uint32_t (&v)[32] = sv[kHeld ? c : 0];
+      if constexpr (!kHeld) load_keys(c, v);
+      exponentials(c, v);
+      if constexpr (!kHeld) store_p(c, v, 1.0f);
+    }
+    const float l_row = (l4[0] + l4[1]) + (l4[2] + l4[3]);
+    const float inv = l_row > 0.0f ? 1.0f / l_row : 0.0f;
+    if constexpr (kHeld) {
+#pragma unroll
+      for (int c = 0; c < kWords; ++c)
+        if (32 * c < n_keys) store_p(c, sv[c], inv);
+    }
+    if (go && slot >= 0) p.part_lse[slot] = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+    proxy_fence();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    mbar_arrive(bar_w);
+    if (quarter == 0 && my_turn(1) && lane == 0) {  // O = P V: 16 keys are 32 bytes along P's rows, 2,048 down V's planes
+      for (int s = 0; s < n_keys / 16; ++s)
+        umma_bf16(tmem, smem_desc_sw128(buf + (s >> 2) * kTcQPlane) + 2 * (s & 3),
+                  smem_desc_mn_sw128(base + kVOff + s * 2048, kPlane), umma_idesc(DH, true), s != 0);
+      umma_commit(bar_o);
+    }
+    __syncwarp();
+    // ---- O of the tile: out of tensor memory into the tile's (spent) query buffer, then out in whole rows
+    go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_o, parity));
+    if (!go) abort_s = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (go) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
         uint32_t r[2][32];
-        tmem_load_32(lane_addr + 64 + half * (DH / 2), r[0]);
-        tmem_load_32(lane_addr + 64 + half * (DH / 2) + 32, r[1]);
+        tmem_load_32(lane_addr + half * 64, r[0]);
+        tmem_load_32(lane_addr + half * 64 + 32, r[1]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint32_t a = pack_bf16x2(__uint_as_float(r[c][8 * i]), __uint_as_float(r[c][8 * i + 1]));
-            const uint32_t b = pack_bf16x2(__uint_as_float(r[c][8 * i + 2]), __uint_as_float(r[c][8 * i + 3]));
-            const uint32_t d = pack_bf16x2(__uint_as_float(r[c][8 * i + 4]), __uint_as_float(r[c][8 * i + 5]));
-            const uint32_t f = pack_bf16x2(__uint_as_float(r[c][8 * i + 6]), __uint_as_float(r[c][8 * i + 7]));
-            // (the thread's half of the columns is a plane of the buffer, laid out as the query rows were: a quarter's
-            // rows stay inside the bytes that the quarter itself fills again)
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float a = __uint_as_float(r[c][8 * i + 2 * k]), b = __uint_as_float(r[c][8 * i + 2 * k + 1]);
+              w[k] = kHeld ? pack_bf16x2(a, b) : pack_bf16x2(a * inv, b * inv);
+            }
+            // (64 columns are a plane of the buffer, laid out as the query rows were: a warp's rows stay inside the bytes
+            // that the warp itself fills again)
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + half * kTcQPlane + row * 128 +
                                                                            (((c * 4 + i) ^ (row & 7)) << 4)),
-                         "r"(a), "r"(b), "r"(d), "r"(f)
+                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
                          : "memory");
           }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      quarter_sync(quarter);  // the quarter's rows are staged
-      if (go) {
-#pragma unroll 4
-        for (int j = 0; j < 32 * 16 / 64; ++j) {
-          const int e = j * 64 + w64;
-          const int r = quarter * 32 + (e >> 4), chunk = e & 15;
-          const int64_t to = dst_s[tile % 3][r];
-          if (to < 0) continue;
-          uint4 piece;
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
-                       : "r"(buf + (chunk >> 3) * kTcQPlane + r * 128 + (((chunk & 7) ^ (r & 7)) << 4)));
-          *reinterpret_cast<uint4 *>(p.part_out + to * DH + chunk * 8) = piece;
-        }
-      }
-      if (tile + 2 < n_tiles) list_rows(tile + 2);
-      quarter_sync(quarter);  // the quarter's rows have been read out, and those of the tile after next are listed
-      if (tile + 2 < n_tiles) gather_q(tile + 2);
-      cp_async_commit();
     }
-    cp_async_wait<0>();
+    __syncwarp();  // the warp's rows are staged
+    if (go) {
+#pragma unroll 4
+      for (int j = 0; j < 16; ++j) {
+        const int r = 2 * j + (lane >> 4);
+        const int32_t to = __shfl_sync(0xffffffffu, slot, r);
+        if (to < 0) continue;
+        uint4 piece;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
+                     : "r"(buf + lane_at + r * 128 + (((chunk & 7) ^ (r & 7)) << 4)));
+        *reinterpret_cast<uint4 *>(p.part_out + (int64_t)to * DH + chunk * 8) = piece;
+      }
+    }
+    __syncwarp();  // and have been read out
+    if (tile + 2 < n_tiles) {
+      list_rows(tile + 2);
+      gather_q();
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTcTmemCols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_s), "r"(kTcTmemCols));
   }
   // A CTA that gave up leaves stale partials behind: the status word tells the host that the call's output is void.
   if (tid == 0 && abort_s && p.status) atomicAdd(p.status, 1);
 }
 
-int launch_bucket_attend_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t stream) {
-  auto kernel = bucket_attend_tc_kernel<128>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
+template <int KEYS>
+static int launch_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t stream) {
+  auto kernel = bucket_attend_tc_kernel<128, KEYS>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem<KEYS>()) != cudaSuccess)
     return LSA_ERR_LAUNCH;
   const dim3 grid((unsigned)segment_bound, (unsigned)p.Hkv);
-  kernel<<<grid, kTcThreads, kTcSmem, stream>>>(p);
+  kernel<<<grid, kTcThreads, tc_smem<KEYS>(), stream>>>(p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
+}
+
+int launch_bucket_attend_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t stream) {
+  return p.cap <= 64 ? launch_tc<64>(p, segment_bound, stream) : launch_tc<128>(p, segment_bound, stream);
 }
 
 }  // namespace lsa

@@ -460,7 +460,8 @@ class FlatLayer:
         lse = self._buffer("lse", (n, self.heads), torch.float32, dev)
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
         if banded and bucket_major and self._reads_by_bucket and \
-                ops.bucket_attend_supported(rows, k, self.design.bucket_cap):
+                ops.bucket_attend_supported(rows, k, self.design.bucket_cap, self.design.top_p,
+                                            not self.bucket_tensor_memory):
             # The band and the read of the selected keys meet only in the merge, and one waits on the tensor pipe
             # while the other is bound by instruction issue: the band runs on a stream of its own beside them.
             main = torch.cuda.current_stream(dev)

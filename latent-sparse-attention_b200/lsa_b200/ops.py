@@ -654,9 +654,13 @@ def latent_attend(q: torch.Tensor, latent: torch.Tensor, ids: torch.Tensor, leng
     return out, lse
 
 
-def bucket_attend_supported(q: torch.Tensor, k: torch.Tensor, bucket_cap: int) -> bool:
-    """Whether `bucket_attend` takes these shapes (else: `expand` + `sparse_attend`)."""
-    return q.shape[2] == 128 and bucket_cap <= 64 and q.shape[1] % k.shape[1] == 0 and q.shape[1] // k.shape[1] <= 8
+def bucket_attend_supported(q: torch.Tensor, k: torch.Tensor, bucket_cap: int, top_p: int | None = None,
+                            warp_mma: bool = False) -> bool:
+    """Whether `bucket_attend` takes these shapes (else: `expand` + `sparse_attend`). Buckets of 65 to 128 members are the
+    tensor-memory pass's alone, which numbers a chunk's (row, pick, head) partials in 31 bits."""
+    wide = top_p is not None and not warp_mma and q.shape[0] * top_p * q.shape[1] < 2**31 - 1
+    return q.shape[2] == 128 and bucket_cap <= (128 if wide else 64) and q.shape[1] % k.shape[1] == 0 \
+        and q.shape[1] // k.shape[1] <= 8
 
 
 def bucket_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, picked: torch.Tensor, positions: torch.Tensor,

@@ -145,3 +145,42 @@ def test_full_buckets_a_bucket_across_the_sinks_and_a_bucket_with_many_pairs(ora
     got_s, _ = ops.bucket_attend(rows_q, K[:short], V[:short], pk, pos, mem, top_k, sink, window, scale,
                                  warp_mma=warp_mma)
     _close(got_s.float().cpu().numpy(), want_s.float().cpu().numpy(), "short cache")
+
+
+@pytest.mark.parametrize("cap,Hq,Hkv", [(65, 8, 2), (96, 3, 1), (128, 16, 2), (128, 1, 1)])
+def test_bucket_major_read_of_wide_buckets(cap, Hq, Hkv):
+    """Buckets of 65 to 128 members, filled from none to all: a pair's range cut by the sinks, the window and the top-k,
+    members past the cache handed in, segments of one pair and of more than two tiles. The gather path is the oracle's
+    read (checked above); both round P and the output to bf16."""
+    from lsa_b200 import ops
+
+    rng = np.random.default_rng(cap + Hq)
+    T, m, R, top_p, sink, window = 4000, 40, 300, 9, 4, 64
+    sizes = rng.integers(0, cap + 1, m)
+    sizes[:3] = cap, 1, 64
+    order, members, at = rng.permutation(T).astype(np.int32), np.full((m, cap), -1, np.int32), 0
+    for b in range(m):
+        sizes[b] = min(sizes[b], T - at)
+        members[b, :sizes[b]] = np.sort(order[at:at + sizes[b]])
+        at += sizes[b]
+    picked = np.stack([rng.permutation(m)[:top_p] for _ in range(R)]).astype(np.int32)
+    picked[:, 0] = 0  # (a bucket every row picks: segments of 256 pairs)
+    positions = np.sort(rng.integers(T // 2, T, R))
+    gen = torch.Generator(device="cuda").manual_seed(cap)
+    Q = torch.randn(R, Hq, 128, generator=gen, device="cuda").bfloat16()
+    K, V = (torch.randn(T, Hkv, 128, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    assert ops.bucket_attend_supported(Q, K, cap, top_p) and not ops.bucket_attend_supported(Q, K, cap, top_p, warp_mma=True)
+    pk, mem, pos = cuda(picked), cuda(members), cuda(positions)
+    for slots in (T, T - 1500):
+        for top_k in (10000, 333):
+            lists, lens, _ = ops.expand(pk, pos, mem, top_k, sink, window, local=False)
+            want, want_lse = ops.sparse_attend(Q, K[:slots], V[:slots], lists, lens, 128 ** -0.5)
+            status = torch.zeros(1, dtype=torch.int32, device="cuda")
+            out, lse = ops.bucket_attend(Q, K[:slots], V[:slots], pk, pos, mem, top_k, sink, window, 128 ** -0.5,
+                                         status=status)
+            assert int(status) == 0
+            _close(out.float().cpu().numpy(), want.float().cpu().numpy(), (slots, top_k))
+            some = torch.isfinite(want_lse)
+            assert torch.equal(some, torch.isfinite(lse)) and (lse - want_lse)[some].abs().max() <= 2e-2
+    with pytest.raises(ValueError):
+        ops.bucket_attend(Q, K, V, pk, pos, mem, 100, sink, window, 128 ** -0.5, warp_mma=True)
