@@ -157,6 +157,13 @@ int lsa_gather_sum(const void *src, int src_dtype, const void *index, int index_
                    int d, int64_t index_base, float *out, void *stream);
 
 /* ---------------------------------------------------------------------------------------------------------
+ * The buckets every row sees: visible[r] = min(positions[r] / block * per_block, limit), those of the cluster blocks
+ * closed before its own (src/lsa/core/reference.py:228-232). positions [R] int64, visible [R] int32 out.
+ * --------------------------------------------------------------------------------------------------------- */
+int lsa_visible_buckets(const int64_t *positions, int64_t R, int64_t block, int64_t per_block, int64_t limit,
+                        int32_t *visible, void *stream);
+
+/* ---------------------------------------------------------------------------------------------------------
  * Flat search, prefill form: score every visible bucket, keep the top_p packed keys of each row.
  * Reference: read / _read_row (src/lsa/core/reference.py:228-265); served Selector.read_flat
  * (src/lsa/sglang/index/selector.py:370-423), ScanSelect (src/lsa/core/kernels/scan_select.py:189-385), packed

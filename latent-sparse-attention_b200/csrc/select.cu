@@ -1395,6 +1395,28 @@ LSA_API int lsa_dense_scores(const float *queries, int64_t R, int d, const float
   return LSA_OK;
 }
 
+namespace lsa {
+__global__ void __launch_bounds__(256)
+    visible_buckets_kernel(const int64_t *__restrict__ positions, int64_t R, int64_t block, int64_t per_block,
+                           int64_t limit, int32_t *__restrict__ visible) {
+  const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (r >= R) return;
+  const int64_t pos = positions[r], seen = (pos >= 0 ? pos / block : -((block - 1 - pos) / block)) * per_block;
+  visible[r] = (int32_t)(seen < limit ? seen : limit);
+}
+}  // namespace lsa
+
+LSA_API int lsa_visible_buckets(const int64_t *positions, int64_t R, int64_t block, int64_t per_block, int64_t limit,
+                                int32_t *visible, void *stream) {
+  LSA_REQUIRE(positions && visible, LSA_ERR_NULL);
+  LSA_REQUIRE(R >= 0 && block >= 1 && per_block >= 1 && limit >= 0 && limit <= INT32_MAX, LSA_ERR_ARGUMENT);
+  if (R == 0) return LSA_OK;
+  lsa::visible_buckets_kernel<<<(unsigned)((R + 255) / 256), 256, 0, (cudaStream_t)stream>>>(positions, R, block, per_block,
+                                                                                           limit, visible);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
 LSA_API int lsa_flat_select(const float *queries, int64_t R, int d, const float *centroids, int64_t m,
                             const int32_t *visible, const int32_t *row_top_p, int top_p, int32_t bucket_id_base,
                             int64_t *keys_out, int32_t *picked_out, void *stream) {

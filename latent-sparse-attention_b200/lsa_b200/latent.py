@@ -176,13 +176,15 @@ class LatentLayer(FlatLayer):
         d, b = self.design, index.buckets
         with probe.region("index map"):
             index_queries = self.index_queries(q)
-        visible = (positions.to(torch.int64) // d.cluster_block_size * d.block_bucket_count).clamp_max(
-            b.bucket_centroids.shape[0]).to(torch.int32)
+        visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
         with probe.region("select"):
             _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p,
                                                splits=select_splits)
         with probe.region("expand"):
-            lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size)
+            outs = (torch.empty(q.shape[0], d.list_width, device=q.device, dtype=torch.int32),
+                    torch.empty(q.shape[0], device=q.device, dtype=torch.int32), self._expand_status)
+            lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
+                                           outs=outs)
         with probe.region("attend"):
             out, _ = ops.latent_attend(q, latent, lists, lengths, self.scale, value_dim=self.value_dim, splits=splits,
                                        warp_mma=warp_mma, status=self._attend_status)

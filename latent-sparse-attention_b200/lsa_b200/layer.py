@@ -271,8 +271,7 @@ class FlatLayer:
         d, b, dev = self.design, index.buckets, index_queries.device
         R = index_queries.shape[0]
         positions = positions.to(torch.int64)
-        visible = (positions // d.cluster_block_size * d.block_bucket_count).clamp_max(
-            b.bucket_centroids.shape[0]).to(torch.int32)
+        visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
         row_p = row_k = None
         if d.early_budget is not None:
             early = positions < d.early_budget.position
@@ -298,6 +297,12 @@ class FlatLayer:
                                             row_p, max_visible=bound, keys=keys, picked=picked,
                                             status=self._scan_status, workspace=work, lengths=index.lengths,
                                             radius=index.radius)
+            elif R <= 8 and row_p is None and d.top_p <= 128 and keys is None and b.bucket_centroids.shape[1] in (32, 64):
+                # A decode step: a CTA sorts a thousand candidates of one row in registers, and more are split over CTAs
+                # and merged (one row over 1,024 buckets: 32.1 us in the kernel whose CTA holds 16 rows, 16.7 in this one).
+                m = b.bucket_centroids.shape[0]
+                _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p,
+                                                   splits=1 if m <= 1024 else min(32, -(-m // 512)))
             else:
                 _, picked = ops.flat_select(index_queries, b.bucket_centroids, visible, d.top_p, row_p, keys=keys,
                                             picked=picked)
@@ -310,14 +315,17 @@ class FlatLayer:
         d, b, dev = self.design, index.buckets, index_queries.device
         R = index_queries.shape[0]
         picked, positions, row_p, row_k = self.pick(index_queries, positions, index, reuse_buffers, last_position)
-        outs = None
         if reuse_buffers:
-            outs = (self._buffer("lists", (R, d.list_width), torch.int32, dev),
-                    self._buffer("lengths", (R,), torch.int32, dev), self._expand_status)
+            lists, lengths = (self._buffer("lists", (R, d.list_width), torch.int32, dev),
+                              self._buffer("lengths", (R,), torch.int32, dev))
+        else:
+            lists = torch.empty(R, d.list_width, device=dev, dtype=torch.int32)
+            lengths = torch.empty(R, device=dev, dtype=torch.int32)
         with probe.region("expand"):
             # (the layer's own buffers are read by their lengths: nothing is padded there)
             lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
-                                           row_p, row_k, outs=outs, local=local, pad=not reuse_buffers)
+                                           row_p, row_k, outs=(lists, lengths, self._expand_status), local=local,
+                                           pad=not reuse_buffers)
         return lists, lengths
 
     def attend(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, lists: torch.Tensor, lengths: torch.Tensor,

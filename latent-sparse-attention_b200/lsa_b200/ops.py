@@ -235,6 +235,15 @@ def kmeans(pools: torch.Tensor, init_centroids: torch.Tensor, iters: int):
     return centroids, assign
 
 
+def visible_buckets(positions: torch.Tensor, block_size: int, block_buckets: int, limit: int) -> torch.Tensor:
+    """The buckets each of `positions` [R] sees [R] int32: those of the cluster blocks closed before its own, `limit` at
+    most (src/lsa/core/reference.py:228-232)."""
+    positions = _contig(positions.to(torch.int64))
+    visible = torch.empty(positions.shape[0], device=positions.device, dtype=torch.int32)
+    call("lsa_visible_buckets", ptr(positions), positions.shape[0], block_size, block_buckets, limit, ptr(visible), stream())
+    return visible
+
+
 def flat_select(index_queries: torch.Tensor, centroids: torch.Tensor, visible: torch.Tensor, top_p: int,
                 row_top_p: torch.Tensor | None = None, bucket_id_base: int = 0, keys: torch.Tensor | None = None,
                 picked: torch.Tensor | None = None):

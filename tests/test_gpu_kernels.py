@@ -680,3 +680,40 @@ def test_topk_attention_reproduces_the_reference(oracle):
 def test_cpu_tensors_are_refused(ops):
     with pytest.raises(RuntimeError, match="no CPU path"):
         ops.pool_keys(torch.zeros(1, 16, 8), 4)
+
+
+def test_few_row_paths_of_a_decode_step(ops, oracle):
+    """The buckets a position sees against torch's; a few rows' scan split over CTAs against the chunk's scan, key for key;
+    the few-row map's vector loads against its plain ones, bit for bit; merges of up to 33 parts against 64-bit sums."""
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    positions = torch.tensor([0, 1, 1023, 1024, 5000, 1 << 40], device="cuda")
+    for block, per, limit in ((1024, 32, 100), (64, 8, 1 << 30), (1, 1, 0)):
+        want = (positions // block * per).clamp_max(limit).to(torch.int32)
+        assert torch.equal(ops.visible_buckets(positions, block, per, limit), want)
+    for d, m in ((64, 1), (64, 1024), (64, 1025), (32, 5000)):
+        rows = torch.nn.functional.normalize(torch.randn(8, d, generator=gen, device="cuda"), dim=1)
+        cent = torch.nn.functional.normalize(torch.randn(m, d, generator=gen, device="cuda"), dim=1)
+        visible = torch.randint(0, m + 1, (8,), generator=gen, device="cuda", dtype=torch.int32)
+        visible[0] = m
+        for keep in (1, 64, 128):
+            want, _ = ops.flat_select(rows, cent, visible, keep)
+            got, _ = ops.flat_select_decode(rows, cent, None, visible, keep, splits=1 if m <= 1024 else -(-m // 512))
+            assert torch.equal(got, want)
+    x = torch.randn(5, 10, 128, generator=gen, device="cuda").bfloat16()
+    for cols in (64, 128):
+        w = torch.randn(256, cols, generator=gen, device="cuda").bfloat16()
+        shifted = torch.empty(256 * cols + 1, device="cuda", dtype=torch.bfloat16)[1:].view(256, cols).copy_(w)
+        got, plain = ops.index_map(x, w, group=5), ops.index_map(x, shifted, group=5)
+        assert torch.equal(got, plain) and shifted.data_ptr() % 16 != 0
+        want = torch.nn.functional.normalize(x.double().view(5, 2, 5, 128).sum(2).view(5, 256) @ w.double(), dim=1)
+        assert (got.double() - want).abs().max() <= 1e-5  # (256 fp32 terms in eight partial sums, unit rows)
+    for n in (1, 2, 15, 16, 17, 32, 33):
+        for dh in (8, 128, 264):
+            parts = torch.randn(n, 1030, dh, generator=gen, device="cuda")
+            lses = 3 * torch.randn(n, 1030, generator=gen, device="cuda")
+            lses[0, 5], lses[:, 6] = -float("inf"), -float("inf")
+            out, lse = ops.lse_merge(parts, lses)
+            weights = torch.softmax(lses.double(), 0).nan_to_num(0.0)
+            assert (out.double() - (weights[..., None] * parts.double()).sum(0)).abs().max() <= 1e-5
+            assert (lse - torch.logsumexp(lses.double(), 0))[torch.isfinite(lse)].abs().max() <= 1e-5
+            assert not torch.isfinite(lse[6]) and not out[6].any()
