@@ -24,7 +24,8 @@ struct BucketParams {
   int32_t *counts;         // [m + 1] pairs of each bucket
   int32_t *offsets;        // [m + 1] exclusive scan of counts
   int32_t *seg_offsets;    // [m + 1] exclusive scan of ceil(counts / segment)
-  int32_t *cursors;        // [m]
+  int4 *ends;              // [m] first member, last member, members
+  int32_t *ranks;          // [R * top_p] a pair's place among its bucket's
   int32_t *order;          // [R * top_p] pair ids grouped by bucket
   int32_t *takes;          // [R * top_p] keys of its bucket a pair reads (0 = none), by pair
   int32_t *order_takes;    // [R * top_p] the same beside `order`, so a CTA fetches both with one round of loads
