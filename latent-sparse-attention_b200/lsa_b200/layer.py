@@ -51,6 +51,16 @@ class FlatDesign:
     def list_width(self) -> int:
         return self.top_k + self.window_size + self.sink_size
 
+    def whole_until(self, buckets: int) -> int:
+        """The first position whose read leaves anything out, over an index of `buckets` buckets. A row before it picks
+        every bucket it sees, no cut bites, and the window covers what is in no closed block yet: its list is all the keys
+        up to its own, so a dense causal read is the same read (and scores, picks and lists nothing). 0 where a design has
+        no such rows; else whole tiles of 128 query rows."""
+        if self.window_size < self.cluster_block_size or self.early_budget is not None:
+            return 0
+        by_buckets = (min(self.top_p, buckets) // self.block_bucket_count + 1) * self.cluster_block_size
+        return min(by_buckets, self.list_width) // 128 * 128
+
 
 class FlatIndex:
     """A request's index: its index keys and the buckets of its closed cluster blocks (and, where the tensor-core
@@ -417,16 +427,7 @@ class FlatLayer:
         return out_host
 
     def _whole_until(self, index: FlatIndex) -> int:
-        """The first position whose read leaves anything out. A row before it picks every bucket it sees, no cut bites,
-        and the window covers what is in no closed block yet: its list is all the keys up to its own, so a dense causal
-        read is the same read (and scores, picks and lists nothing). 0 where a design has no such rows."""
-        d = self.design
-        if d.window_size < d.cluster_block_size or d.early_budget is not None:
-            return 0
-        by_picks = (d.top_p // d.block_bucket_count + 1) * d.cluster_block_size
-        by_index = (index.buckets.bucket_centroids.shape[0] // d.block_bucket_count + 1) * d.cluster_block_size
-        until = min(by_picks, by_index, d.top_k + d.window_size + d.sink_size)
-        return until // 128 * 128  # (whole tiles of query rows)
+        return self.design.whole_until(index.buckets.bucket_centroids.shape[0])
 
     @property
     def _reads_by_bucket(self) -> bool:

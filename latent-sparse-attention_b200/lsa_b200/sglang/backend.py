@@ -174,16 +174,21 @@ class GroupedQueryIndexer:
         rows = forward_batch.lsa_rows
         self.ready().maintain(forward_batch.rids, rows, ends_of(forward_batch, len(rows)))
 
-    def select(self, q: torch.Tensor, k: torch.Tensor, forward_batch: Any) -> torch.Tensor:
+    def whole_rows(self, forward_batch: Any) -> list:
+        """Of each request of a prefill batch, the leading rows that read every key whatever is selected."""
+        return self.ready().whole_rows(forward_batch.extend_seq_lens_cpu, forward_batch.extend_prefix_lens_cpu)
+
+    def select(self, q: torch.Tensor, k: torch.Tensor, forward_batch: Any, skip: list | None = None) -> torch.Tensor:
         """Select for every query of a forward, from the heads attention was handed: q [T, Hq * dh] or [T, Hq, dh]
         rotated on the prefix alone, k [T, Hkv, dh] the same, already in the pool at `out_cache_loc`. Returns KV
-        slots [T, width] int32, -1 padded, valid entries first."""
+        slots [T, width] int32, -1 padded, valid entries first; with `skip` of the rows past each request's leading
+        ones alone."""
         index = self.ready()
         inputs = index_space.key_and_query(q, k, self.geometry, self.heads)
         positions, slots = forward_batch.positions, forward_batch.out_cache_loc.long()
         if forward_batch.forward_mode.is_extend():
             return index.extend(inputs, positions, slots, forward_batch.lsa_rows, forward_batch.extend_seq_lens_cpu,
-                                forward_batch.extend_prefix_lens_cpu)
+                                forward_batch.extend_prefix_lens_cpu, skip)
         return index.decode(inputs, positions, slots, forward_batch.req_pool_indices.long())
 
 
@@ -271,6 +276,43 @@ def save(backend: Any, layer: Any, k: torch.Tensor, v: torch.Tensor, forward_bat
     backend.token_to_kv_pool.set_kv_buffer(layer, forward_batch.out_cache_loc, k, v)
 
 
+def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, layer: Any, indexer: Any,
+               forward_batch: Any) -> torch.Tensor | None:
+    """A prefill batch with prompts that start in it: the rows that read every key up to their own take the dense causal
+    read of the batch's own keys and values, the others their lists. None where no row does, or where the pool does not
+    hold what the batch hands over (another dtype)."""
+    lengths = list(forward_batch.extend_seq_lens_cpu)
+    whole = indexer.whole_rows(forward_batch)
+    heads, head_dim = layer.tp_q_head_num, layer.head_dim
+    keys, values = _pool(backend, layer)
+    kv_heads = keys.shape[1]
+    if not any(whole) or {t.dtype for t in (q, k, v, keys, values)} != {torch.bfloat16} or head_dim not in (64, 128) \
+            or heads // kv_heads > 16 or keys.shape[2] != head_dim or values.shape[1:] != keys.shape[1:] \
+            or k[0].numel() != v[0].numel() or k[0].numel() != kv_heads * head_dim or sum(lengths) != q.shape[0]:
+        return None
+    tokens = q.shape[0]
+    lists = indexer.select(q, k, forward_batch, whole)
+    q = q.contiguous().view(tokens, heads, head_dim)
+    k, v = (x.contiguous().view(tokens, kv_heads, head_dim) for x in (k, v))
+    out = torch.empty(tokens, heads, head_dim, device=q.device, dtype=q.dtype)
+    rest, first = [], 0
+    for count, dense in zip(lengths, whole, strict=True):
+        if dense:
+            piece = slice(first, first + dense)
+            out[piece] = ops.band_attend(q[piece], k[piece], v[piece], 0, dense, 0, layer.scaling)[0]
+        if dense < count:
+            rest.append(slice(first + dense, first + count))
+        first += count
+    if rest:
+        read = sparse_read(backend, torch.cat([q[piece] for piece in rest]), layer, lists).view(-1, heads, head_dim)
+        at = 0
+        for piece in rest:
+            n = piece.stop - piece.start
+            out[piece] = read[at:at + n]
+            at += n
+    return out.view(tokens, heads * head_dim)
+
+
 def select_and_read(original: Any, self: Any, *args: Any, **kwargs: Any) -> Any:
     """Serve a layer's attention from its selection, or hand any other call to the backend as it was
     (backend.py:784-822). `original` is `forward_extend` or `forward_decode`; `self` the attention backend."""
@@ -290,6 +332,9 @@ def select_and_read(original: Any, self: Any, *args: Any, **kwargs: Any) -> Any:
     if arguments.get("save_kv_cache", True):
         save(self, layer, k, v, forward_batch, shard)
     if shard.size == 1:
-        return sparse_read(self, q, layer, indexer.select(q, k, forward_batch))
+        out = None
+        if mode.is_extend() and arguments.get("save_kv_cache", True) and isinstance(indexer, GroupedQueryIndexer):
+            out = whole_read(self, q, k, v, layer, indexer, forward_batch)
+        return sparse_read(self, q, layer, indexer.select(q, k, forward_batch)) if out is None else out
     every_head = gather_heads(q, layer)
     return group_read(self, every_head, layer, indexer.select(every_head, k, forward_batch), shard)

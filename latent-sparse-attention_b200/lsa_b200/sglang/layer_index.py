@@ -393,8 +393,17 @@ class LayerIndex:
             from lsa_b200.sglang.consistency import check_same_index
             check_same_index(self.selector.cache, rows, self.shard.reduce, self.shard.size)
 
+    def whole_rows(self, lengths: Sequence, starts: Sequence) -> list:
+        """Of each request of a prefill batch, how many of its new rows read every key up to their own whatever is
+        selected (`FlatDesign.whole_until`): rows of a prompt that starts in this batch, so that all of their keys are in
+        it."""
+        design = self.selector.cache.design
+        blocks = [count // design.cluster_block_size for count in lengths]
+        return [min(count, design.whole_until(held * design.block_bucket_count)) if int(start) == 0 else 0
+                for count, start, held in zip(lengths, starts, blocks, strict=True)]
+
     def extend(self, inputs: KeyAndQuery, positions: torch.Tensor, slots: torch.Tensor, rows: Sequence,
-               lengths: Sequence, starts: Sequence) -> torch.Tensor:
+               lengths: Sequence, starts: Sequence, skip: Sequence | None = None) -> torch.Tensor:
         """Write the keys of a prefill batch and select for its queries, request by request.
 
         Args:
@@ -403,21 +412,23 @@ class LayerIndex:
             slots: Each new token's KV slot [S] int64.
             rows: The requests' table rows; lengths: new tokens of each; starts: position of each request's first
                 new token, from the scheduler - no device read.
+            skip: Leading rows of each request that need no list (`whole_rows`); their keys are indexed all the same.
 
         Returns:
-            KV slots [S, width] int32, -1 padded, valid entries first.
+            KV slots [S, width] int32, -1 padded, valid entries first, of the rows not skipped.
         """
+        skip = [0] * len(lengths) if skip is None else skip
         index_queries, index_keys = self.project(inputs, slots)
         starts = [int(start) for start in starts]
         self.check_starts(positions, lengths, starts)
         lists, first = [], 0
-        for row, count, start in zip(rows, lengths, starts, strict=True):
+        for row, count, start, past in zip(rows, lengths, starts, skip, strict=True):
             stop = first + count
             held = self.selector.cache.end(row)
             if held != start:  # (`maintain` brings a cached prefix's keys in before the forward)
                 raise ValueError(f"request {row}'s index holds {held} keys and its chunk starts at {start}")
-            lists.append(self.selector.prefill(row, index_queries[first:stop], positions[first:stop],
-                                               index_keys[first:stop], start))
+            lists.append(self.selector.prefill(row, index_queries[first + past:stop], positions[first + past:stop],
+                                               index_keys[first:stop], start + past))
             first = stop
         self.check(rows)
         return torch.cat(lists) if lists else torch.empty(0, self.settings.width, device=slots.device,

@@ -338,3 +338,68 @@ def test_a_decode_group_reads_each_key_on_the_rank_that_owns_its_slot():
         layer.maintain(["a"], [rows[0]], [n])
         assert torch.equal(layer.decode(step, position, slots[n:], row), want)
         assert layer.selector.cache.buckets_of(rows[0]) == n // 256 * 16
+
+
+def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypatch):
+    """Prompts that start in a prefill batch: their leading rows take the dense read, the rest their lists, and the output is
+    the lists' read of every row; a continued prompt and a batch that leaves its keys unsaved take lists alone. (A prompt of
+    less than a block has no list to compare with: it is held to the causal read in 64 bits.)"""
+    from lsa_b200.sglang import backend, index_space, settings
+
+    rng = np.random.default_rng(4)
+    lengths = [1500, 700, 90]
+    rows, table, data, slots_total = _requests(lengths, rng)
+    block = {"indexer": dict(pool_size=4, bucket_size=8, bucket_cap=16, top_p=64, top_k=400,
+                             sink_size=4, window_size=128)}
+    design = settings.parse({**block, "serving": {}})
+    geometry = index_space.Geometry(HQ, HKV, DH, ROTARY, (0,))
+    maps = tuple(torch.from_numpy(bf16_round(rng.standard_normal((geometry.key_dim, design.indexer.index_dim),
+                                                                 dtype=np.float32) / 14)).cuda().bfloat16() for _ in range(2))
+    layer = types.SimpleNamespace(layer_id=0, tp_q_head_num=HQ, tp_k_head_num=HKV, head_dim=DH, scaling=DH ** -0.5)
+
+    def served(dense: bool, save: bool = True):
+        monkeypatch.setattr(backend, "ROWS", {})
+        runner = types.SimpleNamespace(pool=Pool(slots_total), req_to_token=cuda(table))
+        engine = Engine(runner)
+        indexer = backend.GroupedQueryIndexer(0, geometry, design, engine, maps=maps)
+        engine.lsa_indexers = {0: indexer}
+        if not dense:
+            monkeypatch.setattr(indexer, "whole_rows", lambda batch: [0] * len(batch.rids))
+        outs, taken = [], []
+        for first, stops in (([0, 0], [1200, 700]), ([1200], [1500])):  # a batch of prompts, then the first goes on
+            some = range(len(stops))
+            parts = [np.concatenate([data[i][x][a:b] for i, a, b in zip(some, first, stops)]) for x in range(3)]
+            positions = np.concatenate([np.arange(a, b) for a, b in zip(first, stops)])
+            slots = np.concatenate([table[rows[i], a:b] for i, a, b in zip(some, first, stops)])
+            batch = _batch(True, [rows[i] for i in some], [f"r{i}" for i in some], positions, slots, stops,
+                           [b - a for a, b in zip(first, stops)])
+            q, k, v = (cuda(x, torch.bfloat16) for x in parts)
+            if not save:
+                runner.pool.set_kv_buffer(layer, batch.out_cache_loc, k, v)
+            backend.maintain_all(engine, batch)
+            outs.append(backend.select_and_read(Engine.forward_extend, engine, q.view(len(positions), HQ * DH), k, v, layer,
+                                                batch, **({} if save else {"save_kv_cache": False})))
+            taken.append(indexer.whole_rows(batch))
+        return outs, taken
+
+    dense, taken = served(True)
+    lists, _ = served(False)
+    assert taken == [[512, 512], [0]], taken
+    unsaved, _ = served(True, save=False)
+    for got, want, plain in zip(dense, lists, unsaved):
+        assert torch.equal(plain, want)
+        gap = (got.float() - want.float()).abs()
+        assert gap.max() <= 2e-2 and gap.mean() <= 2e-3, (gap.max(), gap.mean())
+    # the short prompt
+    monkeypatch.setattr(backend, "ROWS", {})
+    engine = Engine(types.SimpleNamespace(pool=Pool(slots_total), req_to_token=cuda(table)))
+    engine.lsa_indexers = {0: backend.GroupedQueryIndexer(0, geometry, design, engine, maps=maps)}
+    batch = _batch(True, [rows[2]], ["short"], np.arange(90), table[rows[2], :90], [90], [90])
+    q, k, v = (cuda(x[:90], torch.bfloat16) for x in data[2])
+    backend.maintain_all(engine, batch)
+    got = backend.select_and_read(Engine.forward_extend, engine, q.view(90, HQ * DH), k, v, layer, batch)
+    k64, v64 = (x.double().repeat_interleave(HQ // HKV, dim=1) for x in (k, v))
+    scores = torch.einsum("qhd,khd->hqk", q.double(), k64) * DH ** -0.5
+    scores.masked_fill_(torch.ones(90, 90, device="cuda").triu(1).bool(), -float("inf"))
+    want = torch.einsum("hqk,khd->qhd", scores.softmax(-1), v64).reshape(90, HQ * DH)
+    assert (got.double() - want).abs().max() <= 2e-2
