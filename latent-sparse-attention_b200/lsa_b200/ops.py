@@ -16,6 +16,13 @@ def _contig(t: torch.Tensor) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _as(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """t in `dtype`, contiguous. (A conversion that has nothing to do still costs the host a microsecond.)"""
+    if t.dtype != dtype:
+        t = t.to(dtype)
+    return t if t.is_contiguous() else t.contiguous()
+
+
 def index_map(x: torch.Tensor, index_map_weight: torch.Tensor | None, group: int = 1, dh_off: int = 0,
               dh_used: int | None = None, normalize: bool = True, out_dtype: torch.dtype = torch.float32,
               also_bf16: bool = False, out: torch.Tensor | None = None):
@@ -217,8 +224,8 @@ def kmeans(pools: torch.Tensor, init_centroids: torch.Tensor, iters: int):
     """k-means bucketing (no counterpart in the reference): `iters` Lloyd iterations over pool keys
     [n, d] from `init_centroids` [k, d]; returns (centroids [k, d] fp32, assignment [n] int32). Assignment is the
     exact fixed-order argmax of pool . centroid (a tie to the lower cluster)."""
-    pools = _contig(pools.float())
-    centroids = _contig(init_centroids.float()).clone()
+    pools = _as(pools, torch.float32)
+    centroids = _as(init_centroids, torch.float32).clone()
     n, d = pools.shape
     k = centroids.shape[0]
     every = torch.full((n,), k, device=pools.device, dtype=torch.int32)
@@ -238,7 +245,7 @@ def kmeans(pools: torch.Tensor, init_centroids: torch.Tensor, iters: int):
 def visible_buckets(positions: torch.Tensor, block_size: int, block_buckets: int, limit: int) -> torch.Tensor:
     """The buckets each of `positions` [R] sees [R] int32: those of the cluster blocks closed before its own, `limit` at
     most (src/lsa/core/reference.py:228-232)."""
-    positions = _contig(positions.to(torch.int64))
+    positions = _as(positions, torch.int64)
     visible = torch.empty(positions.shape[0], device=positions.device, dtype=torch.int32)
     call("lsa_visible_buckets", ptr(positions), positions.shape[0], block_size, block_buckets, limit, ptr(visible), stream())
     return visible
@@ -248,11 +255,11 @@ def flat_select(index_queries: torch.Tensor, centroids: torch.Tensor, visible: t
                 row_top_p: torch.Tensor | None = None, bucket_id_base: int = 0, keys: torch.Tensor | None = None,
                 picked: torch.Tensor | None = None):
     """Top-p packed keys and bucket ids of every row (src/lsa/core/reference.py:228-265)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64) if keys is None else keys
     picked = torch.empty(R, top_p, device=q.device, dtype=torch.int32) if picked is None else picked
-    call("lsa_flat_select", ptr(q), R, d, ptr(c), c.shape[0], ptr(_contig(visible.to(torch.int32))),
+    call("lsa_flat_select", ptr(q), R, d, ptr(c), c.shape[0], ptr(_as(visible, torch.int32)),
          ptr(row_top_p), top_p, bucket_id_base, ptr(keys), ptr(picked), stream())
     return keys, picked
 
@@ -262,13 +269,13 @@ def dense_scores(index_queries: torch.Tensor, centroids: torch.Tensor, counts: t
     """Every (row, bucket) score at its own column [R, width] fp32 (-inf past a row's count), or with `keys` the
     packed keys [R, width] int64 (src/lsa/core/kernels/scan_select.py:24-58, triton/paged.py:61-101); through
     `pages` [R, max_pages] where a cache holds its buckets in pages of `page_rows`."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     width = c.shape[0] if width is None else width
     out = torch.empty(R, width, device=q.device, dtype=torch.int64 if keys else torch.float32)
-    pages = None if pages is None else _contig(pages.to(torch.int32))
+    pages = None if pages is None else _as(pages, torch.int32)
     call("lsa_dense_scores", ptr(q), R, d, ptr(c), ptr(pages), pages.shape[1] if pages is not None else 0, page_rows,
-         ptr(_contig(counts.to(torch.int32))), width, bucket_id_base, None if keys else ptr(out),
+         ptr(_as(counts, torch.int32)), width, bucket_id_base, None if keys else ptr(out),
          ptr(out) if keys else None, stream())
     return out
 
@@ -278,7 +285,7 @@ def scan_centre(centroids: torch.Tensor, centre: torch.Tensor | None = None, out
     """The tensor-core scan's N operand: `centroids` [rows, 64] fp32 less `centre` [64] (None: no centre), rounded to
     bf16 into `out`; the length of every row into `lengths` [rows] fp32, and `radius` [1] fp32 raised to the greatest
     of them (start it at zero; a run of rows at a time as an index grows). Returns (out, lengths, radius)."""
-    c = _contig(centroids.float())
+    c = _as(centroids, torch.float32)
     out = torch.empty(c.shape, device=c.device, dtype=torch.bfloat16) if out is None else out
     lengths = torch.empty(c.shape[0], device=c.device, dtype=torch.float32) if lengths is None else lengths
     radius = torch.zeros(1, device=c.device, dtype=torch.float32) if radius is None else radius
@@ -286,7 +293,7 @@ def scan_centre(centroids: torch.Tensor, centre: torch.Tensor | None = None, out
         raise ValueError(f"out must be a contiguous bfloat16 {tuple(c.shape)}")
     if lengths.shape != (c.shape[0],) or lengths.dtype != torch.float32 or not lengths.is_contiguous():
         raise ValueError(f"lengths must be a contiguous float32 [{c.shape[0]}]")
-    call("lsa_scan_centre", ptr(c), c.shape[0], c.shape[1], ptr(None if centre is None else _contig(centre.float())),
+    call("lsa_scan_centre", ptr(c), c.shape[0], c.shape[1], ptr(None if centre is None else _as(centre, torch.float32)),
          ptr(out), ptr(lengths), ptr(radius), stream())
     return out, lengths, radius
 
@@ -301,7 +308,7 @@ def scan_select(index_queries: torch.Tensor, centroids: torch.Tensor, centroids_
     (src/lsa/core/kernels/cutedsl/blackwell/bucket_scan.py:63-836, src/lsa/core/kernels/scan_select.py:189-385).
     `centroids_bf16`, `lengths` and `radius` come from `scan_centre` (without them: the plain bf16 rounding of
     centroids no longer than 1). `max_visible` is the host's bound on `visible` (0: all of the centroids)."""
-    q, c, cb = _contig(index_queries.float()), _contig(centroids.float()), _contig(centroids_bf16)
+    q, c, cb = _as(index_queries, torch.float32), _as(centroids, torch.float32), _contig(centroids_bf16)
     R, d = q.shape
     if cb.dtype != torch.bfloat16 or cb.shape != c.shape:
         raise ValueError("centroids_bf16 must be a bfloat16 matrix of the centroids' shape")
@@ -311,7 +318,7 @@ def scan_select(index_queries: torch.Tensor, centroids: torch.Tensor, centroids_
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8)
     call("lsa_scan_select", ptr(q), R, d, ptr(c), ptr(cb), ptr(lengths), ptr(radius), c.shape[0],
-         ptr(_contig(visible.to(torch.int32))), ptr(row_top_p), top_p, bucket_id_base, int(max_visible), ptr(keys),
+         ptr(_as(visible, torch.int32)), ptr(row_top_p), top_p, bucket_id_base, int(max_visible), ptr(keys),
          ptr(picked), ptr(status), ptr(workspace), workspace.numel() * workspace.element_size(), stream(),
          launches=8 if _scan_samples(c.shape[0], top_p, int(max_visible)) else 1)
     return keys, picked
@@ -329,14 +336,14 @@ def _scan_samples(m: int, top_p: int, max_visible: int) -> bool:
 def flat_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, request_first: torch.Tensor | None,
                        visible: torch.Tensor, top_p: int, splits: int = 1, workspace: torch.Tensor | None = None):
     """Decode-form flat scan (src/lsa/sglang/index/selector.py:603-660): few rows, their buckets split over CTAs."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64)
     picked = torch.empty(R, top_p, device=q.device, dtype=torch.int32)
     need = query("lsa_flat_select_decode_workspace_bytes", R, top_p, splits)
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
-    call("lsa_flat_select_decode", ptr(q), R, d, ptr(c), ptr(request_first), ptr(_contig(visible.to(torch.int32))),
+    call("lsa_flat_select_decode", ptr(q), R, d, ptr(c), ptr(request_first), ptr(_as(visible, torch.int32)),
          top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
          launches=1 if splits == 1 else 2)
@@ -348,8 +355,8 @@ def flat_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, page
                       workspace: torch.Tensor | None = None):
     """The decode scan through each request's page table (src/lsa/core/kernels/triton/paged.py:61-101): logical
     bucket i of request r is row i % page_rows of page pages[r, i // page_rows]. Returns (keys, logical ids)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
-    pages = _contig(pages.to(torch.int32))
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
+    pages = _as(pages, torch.int32)
     R, d = q.shape
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64)
     picked = torch.empty(R, top_p, device=q.device, dtype=torch.int32)
@@ -357,7 +364,7 @@ def flat_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, page
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
     call("lsa_flat_select_paged", ptr(q), R, d, ptr(c), c.shape[0], ptr(pages), pages.shape[1], page_rows,
-         ptr(_contig(counts.to(torch.int32))), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
+         ptr(_as(counts, torch.int32)), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
          launches=1 if splits == 1 else 2)
     return keys, picked
@@ -396,7 +403,7 @@ def shape_build(index_keys: torch.Tensor, centroids: torch.Tensor, members: torc
     src/lsa/core/kernels/triton/shape.py:849-886): each bucket's covariance about its centroid, diagonalised exactly,
     kept as `rank` packed sign directions, their variances and a floor. `index_keys` [rows, d] fp32 holds the keys at
     positions key_base.. ; `members` [m, cap] are positions, -1 padded. `out`: a table's rows to write into."""
-    keys, c, mem = _contig(index_keys.float()), _contig(centroids.float()), _contig(members.to(torch.int32))
+    keys, c, mem = _as(index_keys, torch.float32), _as(centroids, torch.float32), _as(members, torch.int32)
     m, d = c.shape
     if out is None:
         out = ShapeTable(torch.empty(m, rank, d // 8, device=c.device, dtype=torch.uint8),
@@ -416,13 +423,13 @@ def shaped_select(index_queries: torch.Tensor, centroids: torch.Tensor, shapes: 
                   keys: torch.Tensor | None = None, picked: torch.Tensor | None = None):
     """`flat_select` over shaped buckets: a bucket scores as its estimated best key
     (src/lsa/core/reference.py:229-230, src/lsa/core/shape.py:123-137)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     basis, variances, floor = _shape_args(shapes, d)
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64) if keys is None else keys
     picked = torch.empty(R, top_p, device=q.device, dtype=torch.int32) if picked is None else picked
     call("lsa_shaped_select", ptr(q), R, d, ptr(c), c.shape[0], ptr(basis), ptr(variances), ptr(floor),
-         basis.shape[1], float(shapes.deviations), ptr(_contig(visible.to(torch.int32))), ptr(row_top_p), top_p,
+         basis.shape[1], float(shapes.deviations), ptr(_as(visible, torch.int32)), ptr(row_top_p), top_p,
          bucket_id_base, ptr(keys), ptr(picked), stream())
     return keys, picked
 
@@ -431,7 +438,7 @@ def shaped_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, s
                          request_first: torch.Tensor | None, visible: torch.Tensor, top_p: int, splits: int = 1,
                          workspace: torch.Tensor | None = None):
     """`flat_select_decode` over shaped buckets (src/lsa/core/kernels/triton/shape.py:659-717)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     basis, variances, floor = _shape_args(shapes, d)
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64)
@@ -440,7 +447,7 @@ def shaped_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, s
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
     call("lsa_shaped_select_decode", ptr(q), R, d, ptr(c), ptr(basis), ptr(variances), ptr(floor), basis.shape[1],
-         float(shapes.deviations), ptr(request_first), ptr(_contig(visible.to(torch.int32))), top_p, splits, ptr(keys),
+         float(shapes.deviations), ptr(request_first), ptr(_as(visible, torch.int32)), top_p, splits, ptr(keys),
          ptr(picked), ptr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0,
          stream(), launches=1 if splits == 1 else 2)
     return keys, picked
@@ -451,8 +458,8 @@ def shaped_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, sh
                         workspace: torch.Tensor | None = None):
     """`flat_select_paged` over shaped buckets, the shapes paged as the centroids are
     (src/lsa/core/kernels/triton/shape.py:573-717). Returns (keys, logical ids)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
-    pages = _contig(pages.to(torch.int32))
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
+    pages = _as(pages, torch.int32)
     R, d = q.shape
     basis, variances, floor = _shape_args(shapes, d)
     keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64)
@@ -462,7 +469,7 @@ def shaped_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, sh
         workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
     call("lsa_shaped_select_paged", ptr(q), R, d, ptr(c), c.shape[0], ptr(basis), ptr(variances), ptr(floor),
          basis.shape[1], float(shapes.deviations), ptr(pages), pages.shape[1], page_rows,
-         ptr(_contig(counts.to(torch.int32))), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
+         ptr(_as(counts, torch.int32)), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
          launches=1 if splits == 1 else 2)
     return keys, picked
@@ -472,10 +479,10 @@ def shaped_scores(index_queries: torch.Tensor, centroids: torch.Tensor, shapes: 
                   rows: torch.Tensor | None = None, width: int | None = None) -> torch.Tensor:
     """Shaped scores written out [R, width] fp32: row r against the table rows `rows[r]` (-1: -inf), or against the
     first `width` table rows (src/lsa/core/kernels/triton/shape.py:281-343,407-450)."""
-    q, c = _contig(index_queries.float()), _contig(centroids.float())
+    q, c = _as(index_queries, torch.float32), _as(centroids, torch.float32)
     R, d = q.shape
     basis, variances, floor = _shape_args(shapes, d)
-    rows = None if rows is None else _contig(rows.to(torch.int32))
+    rows = None if rows is None else _as(rows, torch.int32)
     width = (c.shape[0] if width is None else width) if rows is None else rows.shape[1]
     out = torch.empty(R, width, device=q.device, dtype=torch.float32)
     call("lsa_shaped_scores", ptr(q), R, d, ptr(c), c.shape[0], ptr(basis), ptr(variances), ptr(floor), basis.shape[1],
@@ -498,7 +505,7 @@ def page_fingerprints(stored: torch.Tensor, page_rows: int, word_weights: torch.
         raise ValueError(f"{count} rows are not whole pages of {page_rows}")
     if position_weights.shape[0] != page_rows or word_weights.shape[0] * 8 < stored.shape[1] * size:
         raise ValueError("the weights cover a page's positions and a row's words")
-    slots = None if slots is None else _contig(slots.to(torch.int64))
+    slots = None if slots is None else _as(slots, torch.int64)
     owned = None if owned is None else _contig(owned.to(torch.uint8))
     out = torch.empty(count // page_rows, device=stored.device, dtype=torch.int64)
     call("lsa_page_fingerprints", ptr(stored), stored.stride(0) * size, stored.shape[1] * size, ptr(slots),
@@ -521,10 +528,10 @@ def beam_step(index_queries: torch.Tensor, vectors: torch.Tensor, carried: torch
               open_first: torch.Tensor, open_end: torch.Tensor, keep: int, children: torch.Tensor | None = None,
               splits: int = 1, workspace: torch.Tensor | None = None):
     """One level of the beam (src/lsa/core/hierarchy.py:402-451): kept rows, or their children when given."""
-    q, v = _contig(index_queries.float()), _contig(vectors.float())
+    q, v = _as(index_queries, torch.float32), _as(vectors, torch.float32)
     R, d = q.shape
     n_carried = 0 if carried is None else carried.shape[1]
-    carried = None if carried is None else _contig(carried.to(torch.int32))
+    carried = None if carried is None else _as(carried, torch.int32)
     kept = keys = carried_out = None
     fanout = 0
     if children is not None:
@@ -538,7 +545,7 @@ def beam_step(index_queries: torch.Tensor, vectors: torch.Tensor, carried: torch
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
     call("lsa_beam_step_split", ptr(q), R, d, ptr(v), v.shape[0], ptr(carried), n_carried,
-         ptr(_contig(open_first.to(torch.int32))), ptr(_contig(open_end.to(torch.int32))), keep, ptr(children),
+         ptr(_as(open_first, torch.int32)), ptr(_as(open_end, torch.int32)), keep, ptr(children),
          fanout, splits, ptr(kept), ptr(keys), ptr(carried_out), ptr(workspace) if need else None, need, stream(),
          launches=1 if splits <= 1 else 2)
     return carried_out if children is not None else (kept, keys)
@@ -563,7 +570,7 @@ def expand(picked: torch.Tensor, positions: torch.Tensor, members: torch.Tensor,
     first, end = owner if owner is not None else (0, _lib.INT64_MAX)
     # dealt = (granule, world, rank): keep the ids of this rank's granules, stored as rows of its own cache
     granule, world, rank = dealt if dealt is not None else (1, 1, 0)
-    call("lsa_expand", ptr(picked), R, top_p, ptr(_contig(positions.to(torch.int64))), ptr(members),
+    call("lsa_expand", ptr(picked), R, top_p, ptr(_as(positions, torch.int64)), ptr(members),
          members.shape[0], members.shape[1], ptr(row_top_p), ptr(row_top_k), top_k, sink, window, ptr(page_table),
          page_size, first, end, granule, world, rank, (0 if local else 1) | (0 if pad else 2), ptr(selected), ptr(lengths),
          ptr(status), stream())
@@ -582,12 +589,12 @@ def expand_batched(picked: torch.Tensor, positions: torch.Tensor, row_request: t
     selected = torch.empty(R, top_k + window + sink, device=picked.device, dtype=torch.int32)
     lengths = torch.empty(R, device=picked.device, dtype=torch.int32)
     status = torch.zeros(1, device=picked.device, dtype=torch.int32)
-    bucket_pages = None if bucket_pages is None else _contig(bucket_pages.to(torch.int32))
-    kv_pages = None if kv_pages is None else _contig(kv_pages.to(torch.int32))
-    call("lsa_expand_batched", ptr(picked), R, top_p, ptr(_contig(positions.to(torch.int64))), ptr(members),
+    bucket_pages = None if bucket_pages is None else _as(bucket_pages, torch.int32)
+    kv_pages = None if kv_pages is None else _as(kv_pages, torch.int32)
+    call("lsa_expand_batched", ptr(picked), R, top_p, ptr(_as(positions, torch.int64)), ptr(members),
          members.shape[0], members.shape[1], None, None, top_k, sink, window, ptr(kv_pages), kv_page_size, 0,
          _lib.INT64_MAX, 1, 1, 0, 0 if local else 1,
-         ptr(None if row_request is None else _contig(row_request.to(torch.int32))),
+         ptr(None if row_request is None else _as(row_request, torch.int32)),
          kv_pages.shape[1] if kv_pages is not None else 0, ptr(bucket_pages),
          bucket_pages.shape[1] if bucket_pages is not None else 0,
          bucket_pages.shape[1] if bucket_pages is not None else 0, bucket_page_rows, ptr(selected), ptr(lengths),
@@ -698,11 +705,11 @@ def bucket_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, picked: tor
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8)
     call("lsa_bucket_attend", ptr(q), R, Hq, dh, q.stride(0), q.stride(1), ptr(k), ptr(v), slots, Hkv, k.stride(0),
-         k.stride(1), ptr(picked), top_p, ptr(_contig(positions.to(torch.int64))), ptr(members), members.shape[0],
+         k.stride(1), ptr(picked), top_p, ptr(_as(positions, torch.int64)), ptr(members), members.shape[0],
          members.shape[1], ptr(row_top_p), ptr(row_top_k), top_k, sink, window, ptr(init[0]) if init else None,
          ptr(init[1]) if init else None, float(scale), ptr(out), ptr(lse), 1 if warp_mma else 0,
          init_ready.cuda_event if init_ready is not None else None, ptr(status), ptr(workspace),
-         workspace.numel() * workspace.element_size(), stream(), launches=6)
+         workspace.numel() * workspace.element_size(), stream(), launches=7)
     return out, lse
 
 
@@ -731,7 +738,7 @@ def lse_merge(parts: torch.Tensor, lses: torch.Tensor, out_dtype=torch.float32):
     log-sum-exps."""
     if parts.dtype != torch.bfloat16 or parts.shape[0] >= 16 or parts.shape[-1] % 8:
         parts = parts.float()
-    parts, lses = _contig(parts), _contig(lses.float())
+    parts, lses = _contig(parts), _as(lses, torch.float32)
     n, dh = parts.shape[0], parts.shape[-1]
     rows = lses.numel() // n
     out = torch.empty(parts.shape[1:], device=parts.device, dtype=out_dtype)
