@@ -184,7 +184,7 @@ class LatentLayer(FlatLayer):
             outs = (torch.empty(q.shape[0], d.list_width, device=q.device, dtype=torch.int32),
                     torch.empty(q.shape[0], device=q.device, dtype=torch.int32), self._expand_status)
             lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
-                                           outs=outs)
+                                           outs=outs, pad=False)  # (the read goes by the lengths)
         with probe.region("attend"):
             out, _ = ops.latent_attend(q, latent, lists, lengths, self.scale, value_dim=self.value_dim, splits=splits,
                                        warp_mma=warp_mma, status=self._attend_status)
