@@ -34,6 +34,7 @@ struct BucketParams {
   float *part_lse;         // [R * top_p, Hq]
   int64_t R, m, slots, q_row_stride, q_head_stride, kv_row_stride, kv_head_stride;
   int top_p, cap, top_k, sink, window, Hq, Hkv, group;
+  int heads_a_cta;         // KV heads a CTA of the tcgen05 pass takes, one after another
   int segment;             // pairs a segment, at most: kBktSegment or kBktSegmentTc
   float scale_log2;
 };

@@ -19,7 +19,7 @@
 // way on it and fill one another's waits. What bounds it is the instruction stream around the products and the chain
 // copy - product - softmax - product - copy of a tile: 0.85 G warp instructions a launch of 8,192 rows x 64 picks x 40 heads,
 // issued on 41 % of the cycles. (With both warpgroups on ONE tile, two threads a row, swapping maxima and sums and waiting
-// for one another six times a tile, it was 1.2 G; a 131,072-token prompt spends 35.3 ms here against 41.1.) Buckets of 65
+// for one another six times a tile, it was 1.2 G; a 131,072-token prompt spent 41.1 ms here, and 35.3 after that step.) Buckets of 65
 // to 128 members take twice the shared memory, so one CTA an SM, and a thread reads its row of S twice; against the gather
 // of every row's list a 16,384-token prompt of 64-key buckets reads in 0.78 ms instead of 1.8.
 //
@@ -71,7 +71,6 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
   __shared__ uint32_t valid_s[kWords];         // which members of the bucket name a row of the cache
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.y;
   const int seg = blockIdx.x;
   // (the table holds a slot for every CTA of the grid: the segment is asked for beside the count, not after it)
   const int4 info = p.segments[seg];
@@ -140,9 +139,9 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
       if (ids_s[mid] < p.sink) lo_key = mid + 1; else hi = mid;
     }
   }
-  // The bucket's keys and values of this KV head: chunk c of member j goes to plane c / 8, row j, 16-byte slot
+  // The bucket's keys and values of a KV head: chunk c of member j goes to plane c / 8, row j, 16-byte slot
   // (c % 8) ^ (j % 8) - the layout a tensor-map copy with the 128-byte swizzle would write.
-  {
+  auto stage_kv = [&](int h) {
     const uint16_t *k_head = p.k + (int64_t)h * p.kv_head_stride, *v_head = p.v + (int64_t)h * p.kv_head_stride;
 #pragma unroll 2
     for (int e = tid; e < n_keys * 16; e += kTcThreads) {
@@ -155,11 +154,11 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
       cp_async_16(base + kVOff + dst, v_head + off, ok ? 16 : 0);
     }
     cp_async_commit();
-  }
+  };
   const uint32_t group_inverse = (65536u + (uint32_t)p.group - 1) / (uint32_t)p.group;  // flat / group, exact here
   int hi_key = 0;       // of this thread's row: the end of its key range,
   int32_t slot = -1;    // and the slot of the partial outputs it fills (the caller has checked that slots fit 31 bits)
-  auto list_rows = [&](int tile) {
+  auto list_rows = [&](int h, int tile) {
     const int flat = tile * kTcRows + row;
     const bool ok = flat < n_rows;
     const int pl = ok ? (int)((uint32_t)flat * group_inverse >> 16) : 0;
@@ -193,182 +192,189 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
   };
 
   const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-  if (wg < n_tiles) {
-    list_rows(wg);
-    gather_q();
-  }
-  cp_async_wait<0>();
-  proxy_fence();
-  __syncthreads();  // K and V are in place (a warpgroup without tiles has copied its share too)
-  for (int tile = wg, n = 0; tile < n_tiles; tile += 2, ++n) {
-    const uint32_t parity = n & 1;
-    if (n > 0) {
-      cp_async_wait<0>();
-      proxy_fence();
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    mbar_arrive(bar_w);  // this thread's part of the tile's queries is in place, and it has read its row of the last O
-    if (quarter == 0 && my_turn(0) && lane == 0) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
-#pragma unroll
-      for (int plane = 0; plane < 2; ++plane)
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-          umma_bf16(tmem, smem_desc_sw128(buf + plane * kTcQPlane) + 2 * s,
-                    smem_desc_sw128(base + kKOff + plane * kPlane) + 2 * s, umma_idesc(n_keys), (plane | s) != 0);
-      umma_commit(bar_s);
-    }
-    __syncwarp();
-    // A group of 8 keys that lies inside the key range of every row of the warp needs no masks: most do.
-    const int hi_min = __reduce_min_sync(0xffffffffu, hi_key);
-    auto whole = [&](int c0) { return c0 >= lo_key && c0 + 8 <= hi_min && valid_byte(c0) == 0xFFu; };
-    // ---- softmax of the row: P is the A operand of the second product. (One decision a warp on a wait: the
-    // tensor-memory loads are warp-wide instructions.)
-    bool go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_s, parity));
-    if (!go) abort_s = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t sv[kHeld ? kWords : 1][32];
-    // keys 32 c .. 32 c + 31 of the row, the masked ones at -inf
-    auto load_keys = [&](int c, uint32_t (&v)[32]) {
-      if (go) tmem_load_32(lane_addr + 32 * c, v);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c0 = 32 * c + 8 * j;
-        if (c0 >= n_keys || whole(c0)) continue;
-        const uint32_t vb = valid_byte(c0);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {  // (bitwise logic and selects: branches here would diverge lane by lane)
-          const bool ok = (c0 + i >= lo_key) & (c0 + i < hi_key) & (bool)((vb >> i) & 1u);
-          v[8 * j + i] = ok ? v[8 * j + i] : 0xFF800000u;
-        }
-      }
-    };
-    // (four running maxima, and four running sums below: one chain of 64 dependent operations is what a thread with few
-    // warps beside it waits on)
-    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int c = 0; c < kWords; ++c) {
-      if (32 * c >= n_keys) continue;
-      uint32_t (&v)[32] = sv[kHeld ? c : 0];
-      load_keys(c, v);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (32 * c + 8 * j >= n_keys) continue;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[8 * j + i]));
-      }
-    }
-    const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-    const float m_row = mx == -INFINITY ? 0.0f : mx * p.scale_log2;  // (finite, so that a masked key gives exp2(-inf) = 0)
-    float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    auto exponentials = [&](int c, uint32_t (&v)[32]) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (32 * c + 8 * j >= n_keys) continue;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float e = fast_exp2(fmaf(__uint_as_float(v[8 * j + i]), p.scale_log2, -m_row));
-          l4[i & 3] += e;
-          v[8 * j + i] = __float_as_uint(e);
-        }
-      }
-    };
-    // 16-byte slot (key / 8 % 8) ^ (row % 8) of the row, in the plane of the key's 64
-    auto store_p = [&](int c, uint32_t (&v)[32], float by) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c8 = 4 * c + j;
-        if (8 * c8 >= n_keys) continue;
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float a = __uint_as_float(v[8 * j + 2 * i]), b = __uint_as_float(v[8 * j + 2 * i + 1]);
-          w[i] = kHeld ? pack_bf16x2(a * by, b * by) : pack_bf16x2(a, b);
-        }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (c8 >> 3) * kTcQPlane + row * 128 +
-                                                                       (((c8 & 7) ^ (row & 7)) << 4)),
-                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
-                     : "memory");
-      }
-    };
-#pragma unroll
-    for (int c = 0; c < kWords; ++c) {
-      if (32 * c >= n_keys) continue;
-      uint32_t (&v)[32] = sv[kHeld ? c : 0];
-      if constexpr (!kHeld) load_keys(c, v);
-      exponentials(c, v);
-      if constexpr (!kHeld) store_p(c, v, 1.0f);
-    }
-    const float l_row = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-    const float inv = l_row > 0.0f ? 1.0f / l_row : 0.0f;
-    if constexpr (kHeld) {
-#pragma unroll
-      for (int c = 0; c < kWords; ++c)
-        if (32 * c < n_keys) store_p(c, sv[c], inv);
-    }
-    if (go && slot >= 0) p.part_lse[slot] = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
-    proxy_fence();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    mbar_arrive(bar_w);
-    if (quarter == 0 && my_turn(1) && lane == 0) {  // O = P V: 16 keys are 32 bytes along P's rows, 2,048 down V's planes
-      for (int s = 0; s < n_keys / 16; ++s)
-        umma_bf16(tmem, smem_desc_sw128(buf + (s >> 2) * kTcQPlane) + 2 * (s & 3),
-                  smem_desc_mn_sw128(base + kVOff + s * 2048, kPlane), umma_idesc(DH, true), s != 0);
-      umma_commit(bar_o);
-    }
-    __syncwarp();
-    // ---- O of the tile: out of tensor memory into the tile's (spent) query buffer, then out in whole rows
-    go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_o, parity));
-    if (!go) abort_s = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (go) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t r[2][32];
-        tmem_load_32(lane_addr + half * 64, r[0]);
-        tmem_load_32(lane_addr + half * 64 + 32, r[1]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float a = __uint_as_float(r[c][8 * i + 2 * k]), b = __uint_as_float(r[c][8 * i + 2 * k + 1]);
-              w[k] = kHeld ? pack_bf16x2(a, b) : pack_bf16x2(a * inv, b * inv);
-            }
-            // (64 columns are a plane of the buffer, laid out as the query rows were: a warp's rows stay inside the bytes
-            // that the warp itself fills again)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + half * kTcQPlane + row * 128 +
-                                                                           (((c * 4 + i) ^ (row & 7)) << 4)),
-                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
-                         : "memory");
-          }
-      }
-    }
-    __syncwarp();  // the warp's rows are staged
-    if (go) {
-#pragma unroll 4
-      for (int j = 0; j < 16; ++j) {
-        const int r = 2 * j + (lane >> 4);
-        const int32_t to = __shfl_sync(0xffffffffu, slot, r);
-        if (to < 0) continue;
-        uint4 piece;
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
-                     : "r"(buf + lane_at + r * 128 + (((chunk & 7) ^ (r & 7)) << 4)));
-        *reinterpret_cast<uint4 *>(p.part_out + (int64_t)to * DH + chunk * 8) = piece;
-      }
-    }
-    __syncwarp();  // and have been read out
-    if (tile + 2 < n_tiles) {
-      list_rows(tile + 2);
+  // One KV head after another: the segment, the bucket's members and the pairs are fetched once, three dependent rounds
+  // of loads that a CTA a head paid before each head's first product (131,072 tokens of 40 heads over 8: 35.3 -> 33.8 ms).
+  int n = 0;  // tiles this warpgroup has had
+  const int end_head = (blockIdx.y + 1) * p.heads_a_cta;
+  for (int h = blockIdx.y * p.heads_a_cta; h < end_head; ++h) {
+    stage_kv(h);
+    if (wg < n_tiles) {
+      list_rows(h, wg);
       gather_q();
     }
+    cp_async_wait<0>();
+    proxy_fence();
+    __syncthreads();  // K and V are in place (a warpgroup without tiles has copied its share too)
+    for (int tile = wg; tile < n_tiles; tile += 2, ++n) {
+      const uint32_t parity = n & 1;
+      if (tile > wg) {
+        cp_async_wait<0>();
+        proxy_fence();
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(bar_w);  // this thread's part of the tile's queries is in place, and it has read its row of the last O
+      if (quarter == 0 && my_turn(0) && lane == 0) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
+#pragma unroll
+        for (int plane = 0; plane < 2; ++plane)
+#pragma unroll
+          for (int s = 0; s < 4; ++s)
+            umma_bf16(tmem, smem_desc_sw128(buf + plane * kTcQPlane) + 2 * s,
+                      smem_desc_sw128(base + kKOff + plane * kPlane) + 2 * s, umma_idesc(n_keys), (plane | s) != 0);
+        umma_commit(bar_s);
+      }
+      __syncwarp();
+      // A group of 8 keys that lies inside the key range of every row of the warp needs no masks: most do.
+      const int hi_min = __reduce_min_sync(0xffffffffu, hi_key);
+      auto whole = [&](int c0) { return c0 >= lo_key && c0 + 8 <= hi_min && valid_byte(c0) == 0xFFu; };
+      // ---- softmax of the row: P is the A operand of the second product. (One decision a warp on a wait: the
+      // tensor-memory loads are warp-wide instructions.)
+      bool go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_s, parity));
+      if (!go) abort_s = 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      uint32_t sv[kHeld ? kWords : 1][32];
+      // keys 32 c .. 32 c + 31 of the row, the masked ones at -inf
+      auto load_keys = [&](int c, uint32_t (&v)[32]) {
+        if (go) tmem_load_32(lane_addr + 32 * c, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c0 = 32 * c + 8 * j;
+          if (c0 >= n_keys || whole(c0)) continue;
+          const uint32_t vb = valid_byte(c0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // (bitwise logic and selects: branches here would diverge lane by lane)
+            const bool ok = (c0 + i >= lo_key) & (c0 + i < hi_key) & (bool)((vb >> i) & 1u);
+            v[8 * j + i] = ok ? v[8 * j + i] : 0xFF800000u;
+          }
+        }
+      };
+      // (four running maxima, and four running sums below: one chain of 64 dependent operations is what a thread with few
+      // warps beside it waits on)
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < kWords; ++c) {
+        if (32 * c >= n_keys) continue;
+        uint32_t (&v)[32] = sv[kHeld ? c : 0];
+        load_keys(c, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (32 * c + 8 * j >= n_keys) continue;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[8 * j + i]));
+        }
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      const float m_row = mx == -INFINITY ? 0.0f : mx * p.scale_log2;  // (finite, so that a masked key gives exp2(-inf) = 0)
+      float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      auto exponentials = [&](int c, uint32_t (&v)[32]) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (32 * c + 8 * j >= n_keys) continue;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float e = fast_exp2(fmaf(__uint_as_float(v[8 * j + i]), p.scale_log2, -m_row));
+            l4[i & 3] += e;
+            v[8 * j + i] = __float_as_uint(e);
+          }
+        }
+      };
+      // 16-byte slot (key / 8 % 8) ^ (row % 8) of the row, in the plane of the key's 64
+      auto store_p = [&](int c, uint32_t (&v)[32], float by) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c8 = 4 * c + j;
+          if (8 * c8 >= n_keys) continue;
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float a = __uint_as_float(v[8 * j + 2 * i]), b = __uint_as_float(v[8 * j + 2 * i + 1]);
+            w[i] = kHeld ? pack_bf16x2(a * by, b * by) : pack_bf16x2(a, b);
+          }
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (c8 >> 3) * kTcQPlane + row * 128 +
+                                                                         (((c8 & 7) ^ (row & 7)) << 4)),
+                       "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                       : "memory");
+        }
+      };
+#pragma unroll
+      for (int c = 0; c < kWords; ++c) {
+        if (32 * c >= n_keys) continue;
+        uint32_t (&v)[32] = sv[kHeld ? c : 0];
+        if constexpr (!kHeld) load_keys(c, v);
+        exponentials(c, v);
+        if constexpr (!kHeld) store_p(c, v, 1.0f);
+      }
+      const float l_row = (l4[0] + l4[1]) + (l4[2] + l4[3]);
+      const float inv = l_row > 0.0f ? 1.0f / l_row : 0.0f;
+      if constexpr (kHeld) {
+#pragma unroll
+        for (int c = 0; c < kWords; ++c)
+          if (32 * c < n_keys) store_p(c, sv[c], inv);
+      }
+      if (go && slot >= 0) p.part_lse[slot] = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+      proxy_fence();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(bar_w);
+      if (quarter == 0 && my_turn(1) && lane == 0) {  // O = P V: 16 keys are 32 bytes along P's rows, 2,048 down V's planes
+        for (int s = 0; s < n_keys / 16; ++s)
+          umma_bf16(tmem, smem_desc_sw128(buf + (s >> 2) * kTcQPlane) + 2 * (s & 3),
+                    smem_desc_mn_sw128(base + kVOff + s * 2048, kPlane), umma_idesc(DH, true), s != 0);
+        umma_commit(bar_o);
+      }
+      __syncwarp();
+      // ---- O of the tile: out of tensor memory into the tile's (spent) query buffer, then out in whole rows
+      go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_o, parity));
+      if (!go) abort_s = 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (go) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t r[2][32];
+          tmem_load_32(lane_addr + half * 64, r[0]);
+          tmem_load_32(lane_addr + half * 64 + 32, r[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t w[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float a = __uint_as_float(r[c][8 * i + 2 * k]), b = __uint_as_float(r[c][8 * i + 2 * k + 1]);
+                w[k] = kHeld ? pack_bf16x2(a, b) : pack_bf16x2(a * inv, b * inv);
+              }
+              // (64 columns are a plane of the buffer, laid out as the query rows were: a warp's rows stay inside the bytes
+              // that the warp itself fills again)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + half * kTcQPlane + row * 128 +
+                                                                             (((c * 4 + i) ^ (row & 7)) << 4)),
+                           "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                           : "memory");
+            }
+        }
+      }
+      __syncwarp();  // the warp's rows are staged
+      if (go) {
+#pragma unroll 4
+        for (int j = 0; j < 16; ++j) {
+          const int r = 2 * j + (lane >> 4);
+          const int32_t to = __shfl_sync(0xffffffffu, slot, r);
+          if (to < 0) continue;
+          uint4 piece;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
+                       : "r"(buf + lane_at + r * 128 + (((chunk & 7) ^ (r & 7)) << 4)));
+          *reinterpret_cast<uint4 *>(p.part_out + (int64_t)to * DH + chunk * 8) = piece;
+        }
+      }
+      __syncwarp();  // and have been read out
+      if (tile + 2 < n_tiles) {
+        list_rows(h, tile + 2);
+        gather_q();
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();  // every product over this head's keys and values is over
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_s), "r"(kTcTmemCols));
@@ -382,13 +388,19 @@ static int launch_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t 
   auto kernel = bucket_attend_tc_kernel<128, KEYS>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem<KEYS>()) != cudaSuccess)
     return LSA_ERR_LAUNCH;
-  const dim3 grid((unsigned)segment_bound, (unsigned)p.Hkv);
+  const dim3 grid((unsigned)segment_bound, (unsigned)(p.Hkv / p.heads_a_cta));
   kernel<<<grid, kTcThreads, tc_smem<KEYS>(), stream>>>(p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }
 
-int launch_bucket_attend_tc(const BucketParams &p, int64_t segment_bound, cudaStream_t stream) {
+int launch_bucket_attend_tc(const BucketParams &params, int64_t segment_bound, cudaStream_t stream) {
+  BucketParams p = params;
+  // As many heads a CTA as leave eight waves of two CTAs an SM, counting the segments that full ones would make.
+  const int64_t segments = p.R * p.top_p / p.segment;
+  p.heads_a_cta = 1;
+  while (p.Hkv % (2 * p.heads_a_cta) == 0 && segments * (p.Hkv / (2 * p.heads_a_cta)) >= 16 * (int64_t)sm_count())
+    p.heads_a_cta *= 2;
   return p.cap <= 64 ? launch_tc<64>(p, segment_bound, stream) : launch_tc<128>(p, segment_bound, stream);
 }
 

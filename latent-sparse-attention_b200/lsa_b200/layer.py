@@ -433,10 +433,11 @@ class FlatLayer:
     def _reads_by_bucket(self) -> bool:
         """Whether reading the selected keys bucket by bucket is the faster read. It costs a partial output a (row, pick,
         query head), whatever the bucket holds; the gather costs the bytes of a pick's keys once a KV head. Measured on a
-        B200, bucket-major against gather, whole prefills: buckets of 8 keys under groups of 4, 8 and 5 heads 22.3 / 13.3,
-        35.1 / 13.6 and 82.7 / 39.8 ms (24,576 tokens); buckets of 32 keys under groups of 4, 5 and 8 heads 19.0 / 32.6,
-        69.7 / 137.5 and 29.7 / 34.0 ms (131,072 tokens): the two meet near four keys a query head of the group."""
-        return self.design.bucket_size >= 4 * (self.heads // self.kv_heads)
+        B200, bucket-major against gather, whole prefills: buckets of 8 keys under groups of 4, 8 and 5 heads 16.9 / 12.0,
+        26.8 / 12.3 and 62.5 / 35.9 ms (24,576 tokens); buckets of 32 keys under groups of 4, 5 and 8 heads 18.1 / 32.3,
+        62.3 / 144.8 and 27.4 / 34.7 ms (131,072 tokens); of 64 keys under groups of 4 1.9 / 3.3 ms (24,576 tokens): the two
+        meet near three keys a query head of the group."""
+        return self.design.bucket_size >= 3 * (self.heads // self.kv_heads)
 
     def prefill_rows(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, band: bool = True, bucket_major: bool = True) -> torch.Tensor:
