@@ -109,12 +109,12 @@ int lsa_pool_keys(const void *index_keys, int key_dtype, int64_t n_pools, int po
  *   labels     [blocks, P] int64 out - each pool's bucket, numbered by first pool
  *   reached    [blocks] uint8 out - 1 where the block got down to bucket_count
  *   rounds     [blocks] int32 out or NULL - merge rounds the block ran
- * Blocks of up to 512 pools are merged by one CTA out of shared memory (d % 4 == 0, d <= 1024, the block's
- * P * (d + 4) floats within 227 KB: 64 pools of the 512-dim latent space fit) and need no workspace. Larger blocks (up to 4,096 pools, d 16, 32 or 64: the node-bucket pairings of the tree,
- * src/lsa/core/hierarchy.py:73-98, cluster_node_buckets at src/lsa/core/kernels/ward.py:84-110) keep their state in
- * the caller's workspace and run two launches a round for max_rounds rounds without a host read; a block that is
- * finished returns at once. Costs are fp32 in the reference's evaluation order, the Gram dot added in ascending
- * dim order, so labels equal a CPU replay in that order.
+ * Blocks of up to 4,096 pools of 16, 32 or 64 dims are merged by a cluster of 1 to 8 CTAs in one launch; up to 512 pools
+ * they need no workspace, larger ones (the node-bucket pairings of the tree, src/lsa/core/hierarchy.py:73-98,
+ * cluster_node_buckets at src/lsa/core/kernels/ward.py:84-110) keep their key sums there. Other widths (d % 4 == 0,
+ * d <= 1024) take one CTA a block and up to 512 pools whose P * (d + 4) floats are within 227 KB: 64 pools of the 512-dim
+ * latent space fit. Costs are fp32 in the reference's evaluation order, the Gram dot added in ascending dim order, so
+ * labels equal a CPU replay in that order.
  * --------------------------------------------------------------------------------------------------------- */
 size_t lsa_ward_merge_workspace_bytes(int64_t blocks, int P, int d);
 int lsa_ward_merge(const float *pool_keys, const float *pool_sizes, float uniform_pool_size, int64_t blocks, int P,
@@ -492,7 +492,8 @@ int lsa_latent_attend(const uint16_t *q, int64_t R, int Hq, int dk, int dv, int6
  * Reference: expand_buckets + topk_attention (src/lsa/core/reference.py:268-289, src/lsa/core/attention.py:65-146).
  *   picked   [R, top_p] int32 bucket ids, best first, -1 = none (lsa_flat_select's picked_out)
  *   members  [m, bucket_cap] int32, ASCENDING within a bucket and -1 padded at the end (as lsa_bucket_table writes
- *            them); bucket_cap <= 64
+ *            them); bucket_cap <= 128 (<= 64 with LSA_BUCKET_WARP_MMA, or where R * top_p * Hq
+ *            does not fit 31 bits)
  *   row_top_p / row_top_k [R] or NULL: a row's own budgets (the early budget)
  *   init_out [R, Hq, dh] fp32 + init_lse [R, Hq], or both NULL
  *   out_bf16 [R, Hq, dh]; lse_out [R, Hq] or NULL

@@ -469,7 +469,11 @@ class FlatLayer:
         banded = band and self.design.sink_size <= 64 and k.shape[0] >= stop
         lse = self._buffer("lse", (n, self.heads), torch.float32, dev)
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
-        if banded and bucket_major and self._reads_by_bucket and \
+        # (Its partial outputs are a workspace by the pick: buckets of more than 64 members, which the gather serves too, take
+        # it up to 8 GiB.)
+        need = _lib.query("lsa_bucket_attend_workspace_bytes", n, self.design.top_p, self.heads, self.head_dim,
+                          index.buckets.bucket_members.shape[0])
+        if banded and bucket_major and self._reads_by_bucket and (self.design.bucket_cap <= 64 or need <= 8 << 30) and \
                 ops.bucket_attend_supported(rows, k, self.design.bucket_cap, self.design.top_p,
                                             not self.bucket_tensor_memory):
             # The band and the read of the selected keys meet only in the merge, and one waits on the tensor pipe
@@ -485,8 +489,6 @@ class FlatLayer:
             # (row, pick) pairs instead of once per pair.
             picked, positions, row_p, row_k = self.pick(index_queries, positions, index, reuse_buffers=True,
                                                         last_position=stop - 1)
-            need = _lib.query("lsa_bucket_attend_workspace_bytes", n, self.design.top_p, self.heads, self.head_dim,
-                              index.buckets.bucket_members.shape[0])
             with probe.region("attend"):
                 ops.bucket_attend(rows, k, v, picked, positions, index.buckets.bucket_members, self.design.top_k,
                                   self.design.sink_size, self.design.window_size, self.scale, init=init,
