@@ -280,7 +280,8 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
                forward_batch: Any) -> torch.Tensor | None:
     """A prefill batch with prompts that start in it: the rows that read every key up to their own take the dense causal
     read of the batch's own keys and values, the others their lists. None where no row does, or where the pool does not
-    hold what the batch hands over (another dtype)."""
+    hold what the batch hands over (another dtype). (As in `FlatLayer.prefill`'s band: a key after a row weighs zero in the
+    tile of 128 they share, so a value that is not finite reaches the rows of its tile before it too.)"""
     lengths = list(forward_batch.extend_seq_lens_cpu)
     whole = indexer.whole_rows(forward_batch)
     heads, head_dim = layer.tp_q_head_num, layer.head_dim
