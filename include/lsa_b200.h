@@ -497,8 +497,9 @@ int lsa_latent_attend(const uint16_t *q, int64_t R, int Hq, int dk, int dv, int6
  *   row_top_p / row_top_k [R] or NULL: a row's own budgets (the early budget)
  *   init_out [R, Hq, dh] fp32 + init_lse [R, Hq], or both NULL
  *   out_bf16 [R, Hq, dh]; lse_out [R, Hq] or NULL
- *   workspace: lsa_bucket_attend_workspace_bytes(); it holds a bf16 partial output per (row, pick, head), which is
- *            what trades the gather's repeated reads for one write and one read
+ *   workspace: lsa_bucket_attend_workspace_bytes() (with bucket_cap > 64 lsa_bucket_attend_wide_workspace_bytes()); it
+ *            holds a bf16 (fp32) partial output per (row, pick, head), which is what trades the gather's repeated reads
+ *            for one write and one read
  *   init_ready_event  a cudaEvent_t (as void*) or NULL: when init_out / init_lse are written on ANOTHER stream (the
  *            band kernel running beside this call's first passes) the event recorded after that work; only the
  *            merge pass waits for it
@@ -510,6 +511,7 @@ int lsa_latent_attend(const uint16_t *q, int64_t R, int Hq, int dk, int dv, int6
  * lsa_expand + lsa_sparse_attend. */
 #define LSA_BUCKET_WARP_MMA 1
 size_t lsa_bucket_attend_workspace_bytes(int64_t R, int top_p, int Hq, int dh, int64_t m);
+size_t lsa_bucket_attend_wide_workspace_bytes(int64_t R, int top_p, int Hq, int dh, int64_t m);
 int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride, int64_t q_head_stride,
                       const uint16_t *k, const uint16_t *v, int64_t slots, int Hkv, int64_t kv_row_stride,
                       int64_t kv_head_stride, const int32_t *picked, int top_p, const int64_t *positions,

@@ -9,8 +9,8 @@
 //   invert    the (row, pick) pairs are grouped by bucket: histogram, scan, scatter
 //   attend    a CTA owns (bucket, KV head, segment of 128 or 256 pairs): the bucket's K/V rows are staged ONCE in shared
 //             memory, each warp takes one query head of the group and runs its pairs through them in tiles of 16
-//             query rows (queries as the M side of mma.m16n8k16), writing a normalised bf16 partial output and a
-//             log-sum-exp per (pair, head)
+//             query rows (queries as the M side of mma.m16n8k16), writing a normalised partial output (bf16, or fp32
+//             where buckets may hold more than 64 members) and a log-sum-exp per (pair, head)
 //   merge     a warp per (row, head) merges the row's partials with the dense band's partial (window and sinks)
 //
 // A pair's keys are its bucket's members inside [sink, window_start(row)), cut where the row's running count
@@ -18,6 +18,8 @@
 #include "bucket_attend.cuh"
 #include "common.cuh"
 #include "mma.cuh"
+
+#include <type_traits>
 
 namespace lsa {
 
@@ -398,7 +400,7 @@ __global__ void __maxnreg__(96) bucket_attend_kernel(BucketParams p) {
       asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
                    : "r"(q_tile + row * ROW_BYTES + ((chunk ^ (row & 7)) << 4)));
-      *reinterpret_cast<uint4 *>(p.part_out + ((int64_t)pair * p.Hq + head) * DH + chunk * 8) = piece;
+      *reinterpret_cast<uint4 *>((uint16_t *)p.part_out + ((int64_t)pair * p.Hq + head) * DH + chunk * 8) = piece;
     }
   }
 }
@@ -407,10 +409,11 @@ __global__ void __maxnreg__(96) bucket_attend_kernel(BucketParams p) {
 
 // A warp per (row, head): the row's partials (one per pick that added keys) and the band's partial, merged by their
 // log-sum-exps. A lane holds DH / 32 consecutive dims.
-template <int DH>
+template <int DH, typename T>
 __global__ void __launch_bounds__(256) bucket_merge_kernel(BucketParams p) {
   constexpr int PER = DH / 32;
-  static_assert(PER == 4, "a lane reads four bf16 dims (8 bytes) of a partial");
+  static_assert(PER == 4, "a lane reads four dims (8 bytes of bf16, 16 of fp32) of a partial");
+  using Four = std::conditional_t<sizeof(T) == 2, uint2, float4>;
   const int lane = lane_id();
   const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (item >= p.R * p.Hq) return;
@@ -442,25 +445,30 @@ __global__ void __launch_bounds__(256) bucket_merge_kernel(BucketParams p) {
         w_mine = lse > -INFINITY ? expf(lse - m) : 0.0f;
       }
       // four partials at a time, their loads in flight together
-      unsigned left = __ballot_sync(0xffffffffu, w_mine > 0.0f);
+      unsigned left = __ballot_sync(0xffffffffu, w_mine != 0.0f);  // (a weight that is not a number is not left out)
       while (left) {
         float w[4];
-        uint2 v[4];
+        Four v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int src_lane = left ? __ffs(left) - 1 : 0;
           w[j] = left ? __shfl_sync(0xffffffffu, w_mine, src_lane) : 0.0f;
           left &= left - 1;
-          const uint16_t *src = p.part_out + ((r * p.top_p + i0 + src_lane) * p.Hq + head) * DH + lane * PER;
-          v[j] = w[j] > 0.0f ? *reinterpret_cast<const uint2 *>(src) : make_uint2(0u, 0u);
+          const T *src = (const T *)p.part_out + ((r * p.top_p + i0 + src_lane) * p.Hq + head) * DH + lane * PER;
+          v[j] = w[j] > 0.0f ? *reinterpret_cast<const Four *>(src) : Four{};
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           l += w[j];
-          acc[0] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].x & 0xFFFF)), acc[0]);
-          acc[1] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].x >> 16)), acc[1]);
-          acc[2] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].y & 0xFFFF)), acc[2]);
-          acc[3] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].y >> 16)), acc[3]);
+          if constexpr (sizeof(T) == 2) {
+            acc[0] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].x & 0xFFFF)), acc[0]);
+            acc[1] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].x >> 16)), acc[1]);
+            acc[2] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].y & 0xFFFF)), acc[2]);
+            acc[3] = fmaf(w[j], bf16_bits_to_float((uint16_t)(v[j].y >> 16)), acc[3]);
+          } else {
+            acc[0] = fmaf(w[j], v[j].x, acc[0]), acc[1] = fmaf(w[j], v[j].y, acc[1]);
+            acc[2] = fmaf(w[j], v[j].z, acc[2]), acc[3] = fmaf(w[j], v[j].w, acc[3]);
+          }
         }
       }
     }
@@ -482,7 +490,7 @@ static int64_t segment_bound(int64_t R, int top_p, int64_t m) {
   return pairs / kBktSegment + (m < pairs ? m : pairs) + 1;
 }
 
-static BucketWorkspace bucket_workspace(int64_t R, int top_p, int Hq, int dh, int64_t m) {
+static BucketWorkspace bucket_workspace(int64_t R, int top_p, int Hq, int dh, int64_t m, bool wide) {
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   BucketWorkspace w;
   size_t at = 0;
@@ -497,7 +505,7 @@ static BucketWorkspace bucket_workspace(int64_t R, int top_p, int Hq, int dh, in
   w.takes = at, at += up(pairs * 4);
   w.order_takes = at, at += up(pairs * 4);
   w.segments = at, at += up((size_t)segment_bound(R, top_p, m) * 16);
-  w.part_out = at, at += up(pairs * Hq * dh * 2);
+  w.part_out = at, at += up(pairs * Hq * dh * (wide ? 4 : 2));
   w.part_lse = at, at += up(pairs * Hq * 4);
   w.total = at;
   return w;
@@ -509,7 +517,12 @@ static BucketWorkspace bucket_workspace(int64_t R, int top_p, int Hq, int dh, in
 
 LSA_API size_t lsa_bucket_attend_workspace_bytes(int64_t R, int top_p, int Hq, int dh, int64_t m) {
   if (R <= 0 || top_p <= 0 || Hq <= 0 || dh <= 0 || m < 0) return 0;
-  return lsa::bucket_workspace(R, top_p, Hq, dh, m).total;
+  return lsa::bucket_workspace(R, top_p, Hq, dh, m, false).total;
+}
+
+LSA_API size_t lsa_bucket_attend_wide_workspace_bytes(int64_t R, int top_p, int Hq, int dh, int64_t m) {
+  if (R <= 0 || top_p <= 0 || Hq <= 0 || dh <= 0 || m < 0) return 0;
+  return lsa::bucket_workspace(R, top_p, Hq, dh, m, true).total;
 }
 
 LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride,
@@ -535,7 +548,8 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
                   ((uintptr_t)q % 16) == 0,
               LSA_ERR_ARGUMENT);
   if (R == 0) return LSA_OK;
-  const lsa::BucketWorkspace w = lsa::bucket_workspace(R, top_p, Hq, dh, m);
+  const bool wide = bucket_cap > lsa::kBktKeys;
+  const lsa::BucketWorkspace w = lsa::bucket_workspace(R, top_p, Hq, dh, m, wide);
   LSA_REQUIRE(workspace_bytes >= w.total, LSA_ERR_WORKSPACE);
   unsigned char *base = reinterpret_cast<unsigned char *>(workspace);
   lsa::BucketParams p = {};
@@ -554,7 +568,7 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
   p.takes = reinterpret_cast<int32_t *>(base + w.takes);
   p.order_takes = reinterpret_cast<int32_t *>(base + w.order_takes);
   p.segments = reinterpret_cast<int4 *>(base + w.segments);
-  p.part_out = reinterpret_cast<uint16_t *>(base + w.part_out);
+  p.part_out = base + w.part_out;
   p.part_lse = reinterpret_cast<float *>(base + w.part_lse);
   p.R = R, p.m = m, p.slots = slots;
   p.q_row_stride = q_row_stride, p.q_head_stride = q_head_stride;
@@ -594,7 +608,11 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
   // init_out / init_lse may be the work of another stream (the dense band running beside the passes above): only
   // the merge reads them, so only the merge waits.
   if (init_ready_event && cudaStreamWaitEvent(s, (cudaEvent_t)init_ready_event, 0) != cudaSuccess) return LSA_ERR_LAUNCH;
-  lsa::bucket_merge_kernel<128><<<(unsigned)((R * Hq + 7) / 8), 256, 0, s>>>(p);
+  const unsigned merge_grid = (unsigned)((R * Hq + 7) / 8);
+  if (wide)
+    lsa::bucket_merge_kernel<128, float><<<merge_grid, 256, 0, s>>>(p);
+  else
+    lsa::bucket_merge_kernel<128, uint16_t><<<merge_grid, 256, 0, s>>>(p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

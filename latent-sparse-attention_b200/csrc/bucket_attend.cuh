@@ -30,7 +30,7 @@ struct BucketParams {
   int32_t *takes;          // [R * top_p] keys of its bucket a pair reads (0 = none), by pair
   int32_t *order_takes;    // [R * top_p] the same beside `order`, so a CTA fetches both with one round of loads
   int4 *segments;          // [segment bound] bucket, first pair in `order`, pairs: what a CTA of the attend pass runs
-  uint16_t *part_out;      // [R * top_p, Hq, dh] bf16
+  void *part_out;          // [R * top_p, Hq, dh] bf16, or fp32 where a bucket may hold more than kBktKeys members
   float *part_lse;         // [R * top_p, Hq]
   int64_t R, m, slots, q_row_stride, q_head_stride, kv_row_stride, kv_head_stride;
   int top_p, cap, top_k, sink, window, Hq, Hkv, group;

@@ -20,8 +20,11 @@
 // copy - product - softmax - product - copy of a tile: 0.85 G warp instructions a launch of 8,192 rows x 64 picks x 40 heads,
 // issued on 41 % of the cycles. (With both warpgroups on ONE tile, two threads a row, swapping maxima and sums and waiting
 // for one another six times a tile, it was 1.2 G; a 131,072-token prompt spent 41.1 ms here, and 35.3 after that step.) Buckets of 65
-// to 128 members take twice the shared memory, so one CTA an SM, and a thread reads its row of S twice; against the gather
-// of every row's list a 16,384-token prompt of 64-key buckets reads in 0.78 ms instead of 1.8.
+// to 128 members take twice the shared memory, so one CTA an SM, and a thread reads its row of S twice.
+// Their partial outputs are fp32: the gather, which such buckets have too, holds a row's sums in fp32 from its first key to
+// its last, and rounded partials were further from the sums in 64 bits than it is (a 16,384-token prompt of 64-key buckets,
+// 2-norm of the bf16 output's error over the output's: gather 1.6619e-3, bf16 partials 1.6624e-3, fp32 partials 1.6587e-3; the
+// whole prefill 2.21, 1.23 and 1.40 ms).
 //
 // Shared-memory operands are written by ordinary and asynchronous copies (the generic proxy), so a proxy fence stands
 // before every hand-over to the tensor cores. Every wait on an mbarrier is bounded; a wait that gives up raises the
@@ -58,7 +61,7 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
   constexpr int kPlane = KEYS * 128;           // a plane of KEYS rows x 64 dims
   constexpr int kKOff = 0, kVOff = 2 * kPlane, kQOff = 4 * kPlane;
   constexpr int kWords = KEYS / 32;
-  constexpr bool kHeld = KEYS == 64;           // a thread holds its whole row of S
+  constexpr bool kHeld = KEYS == 64;           // a thread holds its whole row of S, and partials leave in bf16
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ int32_t ids_s[KEYS];
   __shared__ int32_t pairs_s[kBktSegmentTc];   // the segment's pairs, -1 past its end
@@ -305,13 +308,17 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
         if constexpr (!kHeld) store_p(c, v, 1.0f);
       }
       const float l_row = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-      const float inv = l_row > 0.0f ? 1.0f / l_row : 0.0f;
+      const float inv = (kHeld ? l_row > 0.0f : l_row != 0.0f) ? 1.0f / l_row : 0.0f;
       if constexpr (kHeld) {
 #pragma unroll
         for (int c = 0; c < kWords; ++c)
           if (32 * c < n_keys) store_p(c, sv[c], inv);
       }
-      if (go && slot >= 0) p.part_lse[slot] = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+      float lse = l_row > 0.0f ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+      // (a score that is not a number is carried out of a wide bucket, as the gather carries it: infinity is the
+      // log-sum-exp that the merge cannot leave out)
+      if (!kHeld && isnan(l_row)) lse = INFINITY;
+      if (go && slot >= 0) p.part_lse[slot] = lse;
       proxy_fence();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(bar_w);
@@ -326,34 +333,16 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
       go = __all_sync(0xffffffffu, !abort_s && mbar_wait(bar_o, parity));
       if (!go) abort_s = 1;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (go) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t r[2][32];
-          tmem_load_32(lane_addr + half * 64, r[0]);
-          tmem_load_32(lane_addr + half * 64 + 32, r[1]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w[4];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float a = __uint_as_float(r[c][8 * i + 2 * k]), b = __uint_as_float(r[c][8 * i + 2 * k + 1]);
-                w[k] = kHeld ? pack_bf16x2(a, b) : pack_bf16x2(a * inv, b * inv);
-              }
-              // (64 columns are a plane of the buffer, laid out as the query rows were: a warp's rows stay inside the bytes
-              // that the warp itself fills again)
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + half * kTcQPlane + row * 128 +
-                                                                             (((c * 4 + i) ^ (row & 7)) << 4)),
-                           "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
-                           : "memory");
-            }
-        }
-      }
-      __syncwarp();  // the warp's rows are staged
-      if (go) {
+      // 16-byte piece `at` (of 16) of the row: a plane of the buffer holds eight, laid out as the query rows were, so a
+      // warp's rows stay inside the bytes that the warp itself fills again
+      auto stage_piece = [&](int at, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (at >> 3) * kTcQPlane + row * 128 +
+                                                                       (((at & 7) ^ (row & 7)) << 4)),
+                     "r"(w0), "r"(w1), "r"(w2), "r"(w3)
+                     : "memory");
+      };
+      // The warp's staged rows, half a warp a row, to where its slots begin (16-byte pieces a slot: `pitch`).
+      auto write_out = [&](uint4 *to_slot_0, int pitch) {
 #pragma unroll 4
         for (int j = 0; j < 16; ++j) {
           const int r = 2 * j + (lane >> 4);
@@ -363,10 +352,42 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(piece.x), "=r"(piece.y), "=r"(piece.z), "=r"(piece.w)
                        : "r"(buf + lane_at + r * 128 + (((chunk & 7) ^ (r & 7)) << 4)));
-          *reinterpret_cast<uint4 *>(p.part_out + (int64_t)to * DH + chunk * 8) = piece;
+          to_slot_0[(int64_t)to * pitch + chunk] = piece;
         }
+      };
+      uint4 *parts = reinterpret_cast<uint4 *>(p.part_out);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {  // 64 columns: a plane of bf16, or both planes of fp32
+        if (go) {
+          uint32_t r[2][32];
+          tmem_load_32(lane_addr + half * 64, r[0]);
+          tmem_load_32(lane_addr + half * 64 + 32, r[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t (&v)[32] = r[c];
+              if constexpr (kHeld) {
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  w[k] = pack_bf16x2(__uint_as_float(v[8 * i + 2 * k]), __uint_as_float(v[8 * i + 2 * k + 1]));
+                stage_piece(half * 8 + c * 4 + i, w[0], w[1], w[2], w[3]);
+              } else {
+                uint32_t w[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) w[k] = __float_as_uint(__uint_as_float(v[8 * i + k]) * inv);
+                stage_piece(c * 8 + 2 * i, w[0], w[1], w[2], w[3]);
+                stage_piece(c * 8 + 2 * i + 1, w[4], w[5], w[6], w[7]);
+              }
+            }
+        }
+        if (kHeld && half == 0) continue;  // (both halves of a bf16 row leave together)
+        __syncwarp();  // the warp's rows are staged
+        if (go) write_out(kHeld ? parts : parts + half * 16, kHeld ? DH / 8 : DH / 4);
+        __syncwarp();  // and have been read out
       }
-      __syncwarp();  // and have been read out
       if (tile + 2 < n_tiles) {
         list_rows(h, tile + 2);
         gather_q();

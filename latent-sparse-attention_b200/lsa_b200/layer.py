@@ -471,8 +471,8 @@ class FlatLayer:
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
         # (Its partial outputs are a workspace by the pick: buckets of more than 64 members, which the gather serves too, take
         # it up to 8 GiB.)
-        need = _lib.query("lsa_bucket_attend_workspace_bytes", n, self.design.top_p, self.heads, self.head_dim,
-                          index.buckets.bucket_members.shape[0])
+        need = ops.bucket_attend_workspace(n, self.design.top_p, self.heads, self.head_dim,
+                                           *index.buckets.bucket_members.shape)
         if banded and bucket_major and self._reads_by_bucket and (self.design.bucket_cap <= 64 or need <= 8 << 30) and \
                 ops.bucket_attend_supported(rows, k, self.design.bucket_cap, self.design.top_p,
                                             not self.bucket_tensor_memory):

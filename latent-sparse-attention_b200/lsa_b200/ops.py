@@ -679,6 +679,13 @@ def bucket_attend_supported(q: torch.Tensor, k: torch.Tensor, bucket_cap: int, t
         and q.shape[1] // k.shape[1] <= 8
 
 
+def bucket_attend_workspace(R: int, top_p: int, heads: int, head_dim: int, buckets: int, bucket_cap: int) -> int:
+    """Bytes of `bucket_attend`'s workspace: a partial output a (row, pick, head), bf16 for buckets of up to 64 members and
+    fp32 for wider ones."""
+    return query("lsa_bucket_attend_workspace_bytes" if bucket_cap <= 64 else "lsa_bucket_attend_wide_workspace_bytes",
+                 R, top_p, heads, head_dim, buckets)
+
+
 def bucket_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, picked: torch.Tensor, positions: torch.Tensor,
                   members: torch.Tensor, top_k: int, sink: int, window: int, scale: float, init: tuple | None = None,
                   row_top_p: torch.Tensor | None = None, row_top_k: torch.Tensor | None = None,
@@ -701,7 +708,7 @@ def bucket_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, picked: tor
     if out.shape != (R, Hq, dh) or out.dtype != torch.bfloat16 or not out.is_contiguous():
         raise ValueError(f"out must be a contiguous bfloat16 [{R}, {Hq}, {dh}]")
     lse = torch.empty(R, Hq, device=q.device, dtype=torch.float32) if lse is None else lse
-    need = query("lsa_bucket_attend_workspace_bytes", R, top_p, Hq, dh, members.shape[0])
+    need = bucket_attend_workspace(R, top_p, Hq, dh, *members.shape)
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8)
     call("lsa_bucket_attend", ptr(q), R, Hq, dh, q.stride(0), q.stride(1), ptr(k), ptr(v), slots, Hkv, k.stride(0),

@@ -184,3 +184,46 @@ def test_bucket_major_read_of_wide_buckets(cap, Hq, Hkv):
             assert torch.equal(some, torch.isfinite(lse)) and (lse - want_lse)[some].abs().max() <= 2e-2
     with pytest.raises(ValueError):
         ops.bucket_attend(Q, K, V, pk, pos, mem, 100, sink, window, 128 ** -0.5, warp_mma=True)
+
+
+@pytest.mark.parametrize("cap", [65, 128])
+def test_wide_buckets_keep_their_sums_in_fp32(cap):
+    """Buckets whose means are near 100 and near -100, read with equal weights: the row's mean is a thousandth of its parts.
+    A part rounded to bf16 is up to 0.25 off; sums of 128 fp32 terms of 100 are within 128 * 2^-24 * 100 < 1e-3, and the
+    output is rounded once (2^-9 of itself)."""
+    from lsa_b200 import ops
+
+    m, R, Hq, Hkv = 6, 200, 8, 2
+    members = np.arange(m * cap, dtype=np.int32).reshape(m, cap)
+    gen = torch.Generator(device="cuda").manual_seed(cap)
+    Q = torch.randn(R, Hq, 128, generator=gen, device="cuda").bfloat16()
+    K = torch.zeros(m * cap + 64, Hkv, 128, device="cuda", dtype=torch.bfloat16)
+    V = torch.randn(m * cap + 64, Hkv, 128, generator=gen, device="cuda")
+    V += torch.where(torch.arange(len(V), device="cuda") // cap % 2 == 0, 100.0, -100.0)[:, None, None]
+    V = V.bfloat16()
+    rng = np.random.default_rng(cap)
+    picked = np.stack([np.r_[2 * rng.permutation(3)[:2], 1 + 2 * rng.permutation(3)[:2]] for _ in range(R)]).astype(np.int32)
+    positions = np.full(R, m * cap + 63)
+    out, _ = ops.bucket_attend(Q, K, V, cuda(picked), cuda(positions), cuda(members), 10000, 0, 64, 128 ** -0.5)
+    means = V[:m * cap].double().view(m, cap, Hkv, 128).mean(1)
+    want = means[cuda(picked).long()].mean(1).repeat_interleave(Hq // Hkv, dim=1)
+    assert ((out.double() - want).abs() <= 1e-3 + 2 ** -8 * want.abs()).all()
+
+
+def test_a_score_that_is_not_a_number_is_carried_out_of_a_wide_bucket():
+    """Keys that are not finite reach the rows that read them, and no others: the gather's rows, in the bucket-major read."""
+    from lsa_b200 import ops
+
+    cap, m, R, top_p, Hq, Hkv = 100, 30, 300, 5, 8, 2
+    members = np.arange(m * cap, dtype=np.int32).reshape(m, cap)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    Q = torch.randn(R, Hq, 128, generator=gen, device="cuda").bfloat16()
+    K, V = (torch.randn(m * cap, Hkv, 128, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    K[250, 1, 3], K[1717, 0, 0] = float("nan"), float("inf")
+    rng = np.random.default_rng(1)
+    picked = cuda(np.stack([rng.permutation(m)[:top_p] for _ in range(R)]).astype(np.int32))
+    positions, mem = cuda(np.sort(rng.integers(m * cap // 2, m * cap, R))), cuda(members)
+    lists, lens, _ = ops.expand(picked, positions, mem, 10000, 4, 64, local=False)
+    want, _ = ops.sparse_attend(Q, K, V, lists, lens, 128 ** -0.5)
+    out, _ = ops.bucket_attend(Q, K, V, picked, positions, mem, 10000, 4, 64, 128 ** -0.5)
+    assert want.isnan().any() and torch.equal(out.isnan(), want.isnan())
