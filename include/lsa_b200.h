@@ -444,9 +444,12 @@ int lsa_sparse_attend_static(const uint16_t *q, int64_t R, int Hq, int dh, int64
  *   flags  0: heads of 128 dims packed densely and at least 128 rows go to the tensor-memory form - 128 rows of one
  *          head a CTA, both products on tcgen05 (the rows as M), K/V tiles streamed by tensor-map copies, the band
  *          walked twice (row maxima, then the sums) so the accumulator in tensor memory is never rescaled;
- *          LSA_BAND_WARP_MMA: always the warp-level form
+ *          LSA_BAND_WARP_MMA: always the warp-level form;
+ *          LSA_BAND_TWO_TERM: the probabilities enter the second product as two bf16 terms (the value and what rounding
+ *          left of it), for a read that stands for lsa_sparse_attend over every key up to a row's own
  *   status (may be NULL) is raised if a bounded on-chip wait of the tensor-memory form gives up */
 #define LSA_BAND_WARP_MMA 1
+#define LSA_BAND_TWO_TERM 2
 int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride, int64_t q_head_stride,
                     const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride,
                     int64_t kv_head_stride, int64_t first_position, int window, int sink, float scale, float *out_f32,

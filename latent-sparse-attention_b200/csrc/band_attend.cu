@@ -24,7 +24,8 @@ struct BandParams {
 
 // grid (ceil(R / 16), Hkv, ceil(group / 8)); blockDim = min(group, 8) * 32. Row i of the call sits at position first_position + i and KV
 // row p holds position p.
-template <int DH>
+// TWO_TERM: the probabilities enter the second product as bf16 and what bf16 left of them.
+template <int DH, bool TWO_TERM>
 __global__ void band_attend_kernel(BandParams p) {
   constexpr int ROW_BYTES = DH * 2, CHUNKS = ROW_BYTES / 16, KSTEPS = DH / 16;
   constexpr int TILE_BYTES = kBandKeys * ROW_BYTES;
@@ -174,6 +175,13 @@ __global__ void band_attend_kernel(BandParams p) {
     for (int kk = 0; kk < kBandKeys / 16; ++kk) {
       const uint32_t a0 = pack_bf16x2(s[2 * kk][0], s[2 * kk][1]), a1 = pack_bf16x2(s[2 * kk][2], s[2 * kk][3]);
       const uint32_t a2 = pack_bf16x2(s[2 * kk + 1][0], s[2 * kk + 1][1]), a3 = pack_bf16x2(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+      auto left = [](const float *x, uint32_t w) {
+        return pack_bf16x2(x[0] - __uint_as_float(w << 16), x[1] - __uint_as_float(w & 0xFFFF0000u));
+      };
+      uint32_t b[4] = {0u, 0u, 0u, 0u};
+      if constexpr (TWO_TERM)
+        b[0] = left(s[2 * kk], a0), b[1] = left(s[2 * kk] + 2, a1), b[2] = left(s[2 * kk + 1], a2),
+        b[3] = left(s[2 * kk + 1] + 2, a3);
 #pragma unroll
       for (int np = 0; np < DH / 16; ++np) {
         const int row = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
@@ -182,6 +190,10 @@ __global__ void band_attend_kernel(BandParams p) {
         ldmatrix_x4_trans(v_src + row * ROW_BYTES + ((chunk ^ (row & 7)) << 4), b0, b1, b2, b3);
         mma_bf16(o[2 * np], a0, a1, a2, a3, b0, b1);
         mma_bf16(o[2 * np + 1], a0, a1, a2, a3, b2, b3);
+        if constexpr (TWO_TERM) {
+          mma_bf16(o[2 * np], b[0], b[1], b[2], b[3], b0, b1);
+          mma_bf16(o[2 * np + 1], b[0], b[1], b[2], b[3], b2, b3);
+        }
       }
     }
     __syncthreads();
@@ -206,7 +218,7 @@ __global__ void band_attend_kernel(BandParams p) {
 
 int launch_band_attend_tc(const uint16_t *q, int64_t R, int Hq, int64_t q_row_stride, const uint16_t *k,
                           const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride, int64_t first_position,
-                          int window, int sink, float scale, float *out, float *lse, int32_t *status,
+                          int window, int sink, float scale, float *out, float *lse, bool two_term, int32_t *status,
                           cudaStream_t stream);
 
 }  // namespace lsa
@@ -233,9 +245,10 @@ LSA_API int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   // dims packed densely (a row of heads is a row of the map) and 16-byte aligned rows; a chunk shorter than a tile
   // of rows gains nothing from it.
   const bool dense = q_head_stride == dh && kv_head_stride == dh && q_row_stride % 8 == 0 && ((uintptr_t)q % 16) == 0;
+  const bool two_term = flags & LSA_BAND_TWO_TERM;
   if (!(flags & LSA_BAND_WARP_MMA) && dh == 128 && dense && R >= 128 && n_keys < INT32_MAX)
     return lsa::launch_band_attend_tc(q, R, Hq, q_row_stride, k, v, n_keys, Hkv, kv_row_stride, first_position,
-                                      window, sink, scale, out_f32, lse, status, (cudaStream_t)stream);
+                                      window, sink, scale, out_f32, lse, two_term, status, (cudaStream_t)stream);
   lsa::BandParams p;
   p.q = q;
   p.k = k;
@@ -259,23 +272,14 @@ LSA_API int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   dim3 grid((unsigned)((R + lsa::kBandRows - 1) / lsa::kBandRows), (unsigned)Hkv, (unsigned)((group + 7) / 8));
   const int threads = (group < 8 ? group : 8) * 32;
   cudaStream_t s = (cudaStream_t)stream;
-  if (dh == 128) {
-    // 64 KB of tiles a CTA: ask for the largest shared-memory carve-out so that two or three CTAs share an SM
-    if (cudaFuncSetAttribute(lsa::band_attend_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(lsa::band_attend_kernel<128>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      return LSA_ERR_LAUNCH;
-    lsa::band_attend_kernel<128><<<grid, threads, smem, s>>>(p);
-  } else {
-    // 64 KB of tiles a CTA: ask for the largest shared-memory carve-out so that two or three CTAs share an SM
-    if (cudaFuncSetAttribute(lsa::band_attend_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(lsa::band_attend_kernel<64>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      return LSA_ERR_LAUNCH;
-    lsa::band_attend_kernel<64><<<grid, threads, smem, s>>>(p);
-  }
+  auto kernel = dh == 128 ? (two_term ? lsa::band_attend_kernel<128, true> : lsa::band_attend_kernel<128, false>)
+                          : (two_term ? lsa::band_attend_kernel<64, true> : lsa::band_attend_kernel<64, false>);
+  // 64 KB of tiles a CTA: ask for the largest shared-memory carve-out so that two or three CTAs share an SM
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
+          cudaSuccess)
+    return LSA_ERR_LAUNCH;
+  kernel<<<grid, threads, smem, s>>>(p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

@@ -435,7 +435,7 @@ class FlatLayer:
         query head), whatever the bucket holds; the gather costs the bytes of a pick's keys once a KV head. Measured on a
         B200, bucket-major against gather, whole prefills: buckets of 8 keys under groups of 4, 8 and 5 heads 16.9 / 12.0,
         26.8 / 12.3 and 62.5 / 35.9 ms (24,576 tokens); buckets of 32 keys under groups of 4, 5 and 8 heads 18.1 / 32.3,
-        62.3 / 144.8 and 27.4 / 34.7 ms (131,072 tokens); of 64 keys under groups of 4 1.9 / 3.3 ms (24,576 tokens): the two
+        62.3 / 144.8 and 27.4 / 34.7 ms (131,072 tokens); of 64 keys under groups of 4 2.2 / 3.3 ms (24,576 tokens): the two
         meet near three keys a query head of the group."""
         return self.design.bucket_size >= 3 * (self.heads // self.kv_heads)
 
@@ -446,15 +446,16 @@ class FlatLayer:
         n, dev = rows.shape[0], rows.device
         stop = start + n
         if band and self.design.sink_size <= 64 and k.shape[0] >= stop and start < self._whole_until(index):
-            # (a tensor-core row costs 1.4 ps a key and head here: 0.17 us for the 3,000 keys of a row of 40 heads, against
-            # 0.5 us for its window and 64 picked buckets)
+            # (a tensor-core row costs 1.5 ps a key and head here: 0.18 us for the 3,000 keys of a row of 40 heads, against
+            # 0.5 us for its window and 64 picked buckets. The probabilities go in as two bf16 terms, 1.25 ps with one: the
+            # lists' read, which this stands for, is closer to the sums in 64 bits than one rounded term a key.)
             whole = min(n, self._whole_until(index) - start)
             with probe.region("band"):
                 dense, _ = ops.band_attend(rows[:whole], k, v, start, start + whole, 0, self.scale,
                                            out=self._buffer("dense out", (whole, self.heads, self.head_dim),
                                                             torch.float32, dev),
                                            lse=self._buffer("dense lse", (whole, self.heads), torch.float32, dev),
-                                           status=self._attend_status)
+                                           status=self._attend_status, two_term=True)
                 out[:whole].copy_(dense)
             if whole == n:
                 return out
