@@ -131,6 +131,9 @@ class GroupedQueryIndexer:
         self.shard, self.heads, self.prefill_chunk, self.maps = shard or Shard(), heads, prefill_chunk, maps
         self.check_index, self.sum_heads = check_index, sum_heads
         self.index: LayerIndex | None = None
+        # Bounded on-chip waits of the dense reads that gave up: the device's count, and the host's pinned copy of it, which
+        # every forward that reads densely refreshes behind its reads
+        self._gave_up = self._gave_up_seen = None
 
     def request_table(self) -> torch.Tensor:
         return self.backend.req_to_token
@@ -169,8 +172,35 @@ class GroupedQueryIndexer:
             self.index.writes_pool = False  # `select_and_read` saves a forward's keys before it selects
         return self.index
 
+    def read_status(self, device) -> torch.Tensor:
+        """The word a dense read raises when one of its bounded waits gives up."""
+        if self._gave_up is None:
+            self._gave_up = torch.zeros(1, dtype=torch.int32, device=device)
+            self._gave_up_seen = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        return self._gave_up
+
+    def reads_done(self) -> None:
+        """A forward's dense reads are launched: their status follows them to the host."""
+        self._gave_up_seen.copy_(self._gave_up, non_blocking=True)
+
+    def check_reads(self) -> None:
+        """The deferred check of the dense reads, without a synchronisation: what has reached the host by now (after one, all
+        that was launched before it).
+
+        Raises:
+            RuntimeError: A bounded on-chip wait gave up; the outputs of the forwards since the last check are void.
+        """
+        if self._gave_up_seen is None or not int(self._gave_up_seen):
+            return
+        count = int(self._gave_up_seen)
+        self._gave_up.zero_()
+        self._gave_up_seen.zero_()
+        raise RuntimeError(f"{count} bounded on-chip waits gave up in the dense reads of layer {self.layer}: the outputs since "
+                           "the last check are void")
+
     def maintain(self, forward_batch: Any) -> None:
         """Bring each request's cache up to the tokens already in the KV pool, before every forward."""
+        self.check_reads()
         rows = forward_batch.lsa_rows
         self.ready().maintain(forward_batch.rids, rows, ends_of(forward_batch, len(rows)))
 
@@ -297,14 +327,15 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     q = q.contiguous().view(tokens, heads, head_dim)
     k, v = (x.contiguous().view(tokens, kv_heads, head_dim) for x in (k, v))
     out = torch.empty(tokens, heads, head_dim, device=q.device, dtype=q.dtype)
-    rest, first = [], 0
+    rest, first, status = [], 0, indexer.read_status(q.device)
     for count, dense in zip(lengths, whole, strict=True):
         if dense:
             piece = slice(first, first + dense)
-            out[piece] = ops.band_attend(q[piece], k[piece], v[piece], 0, dense, 0, layer.scaling, two_term=True)[0]
+            out[piece] = ops.band_attend(q[piece], k[piece], v[piece], 0, dense, 0, layer.scaling, status=status, two_term=True)[0]
         if dense < count:
             rest.append(slice(first + dense, first + count))
         first += count
+    indexer.reads_done()
     if rest:
         read = sparse_read(backend, torch.cat([q[piece] for piece in rest]), layer, lists).view(-1, heads, head_dim)
         at = 0

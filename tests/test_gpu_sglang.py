@@ -398,6 +398,15 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
     q, k, v = (cuda(x[:90], torch.bfloat16) for x in data[2])
     backend.maintain_all(engine, batch)
     got = backend.select_and_read(Engine.forward_extend, engine, q.view(90, HQ * DH), k, v, layer, batch)
+    band = backend.ops.band_attend
+    with monkeypatch.context() as patch:  # a read whose wait gives up (said on the host) is told by the next forward
+        patch.setattr(backend.ops, "band_attend", lambda *a, status, **kw: (status.add_(1), band(*a, status=status, **kw))[1])
+        batch.rids = ["again"]
+        backend.maintain_all(engine, batch)
+        backend.select_and_read(Engine.forward_extend, engine, q.view(90, HQ * DH), k, v, layer, batch)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="gave up in the dense reads"):
+        backend.maintain_all(engine, batch)
     k64, v64 = (x.double().repeat_interleave(HQ // HKV, dim=1) for x in (k, v))
     scores = torch.einsum("qhd,khd->hqk", q.double(), k64) * DH ** -0.5
     scores.masked_fill_(torch.ones(90, 90, device="cuda").triu(1).bool(), -float("inf"))

@@ -383,3 +383,23 @@ def test_decode_graphs_are_keyed_by_context_ranges(monkeypatch):
     assert plugin.context_graphs(registry, registry.HookType, targets)
     assert [(t, h.__name__, k) for t, h, k in registry.hooks] == [(targets[0], "capture_context_graphs",
                                                                    FakeRegistry.HookType.AROUND)]
+
+
+def test_a_dense_read_that_gave_up_is_told_before_the_next_forward(monkeypatch):
+    """What the kernels raised and the last forward brought to the host: the next maintenance raises, once."""
+    from lsa_b200.sglang import backend, index_space, settings
+
+    design = settings.parse({"indexer": {}, "serving": {}})
+    indexer = backend.GroupedQueryIndexer(7, index_space.Geometry(4, 2, 64, 32, (7,)), design, None)
+    indexer.index = types.SimpleNamespace(maintain=lambda rids, rows, ends: seen.append(rids))
+    mode = types.SimpleNamespace(is_extend=lambda: False)
+    batch = types.SimpleNamespace(forward_mode=mode, rids=["a"], lsa_rows=[0], seq_lens_cpu=torch.tensor([5]))
+    seen = []
+    indexer.maintain(batch)  # (no dense read so far)
+    indexer._gave_up, indexer._gave_up_seen = torch.tensor([2], dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+    indexer.maintain(batch)  # (raised on the device, not here yet)
+    indexer.reads_done()
+    with pytest.raises(RuntimeError, match="2 bounded on-chip waits .* layer 7"):
+        indexer.maintain(batch)
+    indexer.maintain(batch)
+    assert len(seen) == 3
