@@ -310,8 +310,9 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
                forward_batch: Any) -> torch.Tensor | None:
     """A prefill batch with prompts that start in it: the rows that read every key up to their own take the dense causal
     read of the batch's own keys and values (the probabilities as two bf16 terms: no further from the sums in 64 bits than the
-    lists' read), the others their lists. None where no row does, or where the pool does not
-    hold what the batch hands over (another dtype). (As in `FlatLayer.prefill`'s band: a key after a row weighs zero in the
+    lists' read), the others their lists. None where no row does, where the pool does not
+    hold what the batch hands over (another dtype), or where the lists' read takes what the dense one refuses (a scale that is
+    not positive). (As in `FlatLayer.prefill`'s band: a key after a row weighs zero in the
     tile of 128 they share, so a value that is not finite reaches the rows of its tile before it too.)"""
     lengths = list(forward_batch.extend_seq_lens_cpu)
     whole = indexer.whole_rows(forward_batch)
@@ -319,13 +320,15 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     keys, values = _pool(backend, layer)
     kv_heads = keys.shape[1]
     if not any(whole) or {t.dtype for t in (q, k, v, keys, values)} != {torch.bfloat16} or head_dim not in (64, 128) \
-            or heads // kv_heads > 16 or keys.shape[2] != head_dim or values.shape[1:] != keys.shape[1:] \
+            or heads // kv_heads > 16 or not layer.scaling > 0 or keys.shape[2] != head_dim or values.shape[1:] != keys.shape[1:] \
             or k[0].numel() != v[0].numel() or k[0].numel() != kv_heads * head_dim or sum(lengths) != q.shape[0]:
         return None
     tokens = q.shape[0]
     lists = indexer.select(q, k, forward_batch, whole)
-    q = q.contiguous().view(tokens, heads, head_dim)
-    k, v = (x.contiguous().view(tokens, kv_heads, head_dim) for x in (k, v))
+    # (the dense read copies rows 16 bytes at a time out of the batch's own tensors, which may start anywhere in a larger one;
+    # the lists' read takes keys and values from the pool)
+    q, k, v = (x.contiguous() if x.data_ptr() % 16 == 0 or not x.is_contiguous() else x.clone() for x in (q, k, v))
+    q, k, v = q.view(tokens, heads, head_dim), k.view(tokens, kv_heads, head_dim), v.view(tokens, kv_heads, head_dim)
     out = torch.empty(tokens, heads, head_dim, device=q.device, dtype=q.dtype)
     rest, first, status = [], 0, indexer.read_status(q.device)
     for count, dense in zip(lengths, whole, strict=True):

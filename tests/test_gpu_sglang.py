@@ -390,6 +390,21 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
         assert torch.equal(plain, want)
         gap = (got.float() - want.float()).abs()
         assert gap.max() <= 2e-2 and gap.mean() <= 2e-3, (gap.max(), gap.mean())
+    # what the lists' read takes and the dense one alone would refuse: tensors that start at an odd element, no positive scale
+    for scale, shift in ((DH ** -0.5, 1), (-0.1, 0), (0.0, 0)):
+        monkeypatch.setattr(backend, "ROWS", {})
+        engine = Engine(types.SimpleNamespace(pool=Pool(slots_total), req_to_token=cuda(table)))
+        engine.lsa_indexers = {0: backend.GroupedQueryIndexer(0, geometry, design, engine, maps=maps)}
+        batch = _batch(True, [rows[0]], ["odd"], np.arange(700), table[rows[0], :700], [700], [700])
+        q, k, v = (torch.empty(x[:700].size + shift, device="cuda", dtype=torch.bfloat16)[shift:].view(700, -1, DH).copy_(
+            cuda(x[:700], torch.bfloat16)) for x in data[0])
+        odd = types.SimpleNamespace(**{**vars(layer), "scaling": scale})
+        backend.maintain_all(engine, batch)
+        got = backend.select_and_read(Engine.forward_extend, engine, q.view(700, HQ * DH), k, v, odd, batch)
+        scores = torch.einsum("qhd,khd->hqk", q[:500].double(), k[:500].double().repeat_interleave(HQ // HKV, dim=1)) * scale
+        scores.masked_fill_(torch.ones(500, 500, device="cuda").triu(1).bool(), -float("inf"))
+        want = torch.einsum("hqk,khd->qhd", scores.softmax(-1), v[:500].double().repeat_interleave(HQ // HKV, dim=1))
+        assert (got[:500].double() - want.reshape(500, -1)).abs().max() <= 2e-2  # (these rows read everything)
     # the short prompt
     monkeypatch.setattr(backend, "ROWS", {})
     engine = Engine(types.SimpleNamespace(pool=Pool(slots_total), req_to_token=cuda(table)))
