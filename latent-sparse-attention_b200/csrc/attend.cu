@@ -398,9 +398,7 @@ static int launch_attend(const AttendParams &p, cudaStream_t s) {
   const int64_t spread = (items + sm_count() - 1) / sm_count();
   const int warps = (int)(spread < W ? spread : W);
   const size_t smem = (size_t)warps * WARP_BYTES;
-  if (cudaFuncSetAttribute(sparse_attend_kernel<DH, NT, W, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return LSA_ERR_LAUNCH;
+  if (!allow_shared(sparse_attend_kernel<DH, NT, W, STAGES>, (size_t)W * WARP_BYTES)) return LSA_ERR_LAUNCH;
   const int64_t grid = (items + warps - 1) / warps;
   if (grid > INT32_MAX) return LSA_ERR_ARGUMENT;
   launch(p.R <= kChainedRows, sparse_attend_kernel<DH, NT, W, STAGES>, dim3((unsigned)grid), dim3(warps * 32), smem, s, p);

@@ -593,10 +593,9 @@ LSA_API int lsa_bucket_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
     LSA_LAUNCH_CHECK();
     const int64_t bound = lsa::segment_bound(R, top_p, m);
     if (!tensor_memory) {
-      const size_t smem = 2 * (size_t)lsa::kBktKeys * dh * 2 + (size_t)p.group * lsa::kBktTile * dh * 2;
-      if (cudaFuncSetAttribute(lsa::bucket_attend_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem) != cudaSuccess)
-        return LSA_ERR_LAUNCH;
+      auto shared_of = [&](int group) { return (2 * lsa::kBktKeys + (size_t)group * lsa::kBktTile) * dh * 2; };
+      const size_t smem = shared_of(p.group);
+      if (!lsa::allow_shared(lsa::bucket_attend_kernel<128>, shared_of(8))) return LSA_ERR_LAUNCH;
       const dim3 grid((unsigned)bound, (unsigned)Hkv);
       lsa::bucket_attend_kernel<128><<<grid, p.group * 32, smem, s>>>(p);
       LSA_LAUNCH_CHECK();

@@ -352,8 +352,8 @@ LSA_API int lsa_ward_merge(const float *pool_keys, const float *pool_sizes, floa
   }
   const size_t smem = lsa::ward_smem_bytes(P, d);
   LSA_REQUIRE(P <= 512 && smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
-  if (cudaFuncSetAttribute(lsa::ward_any_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return LSA_ERR_LAUNCH;
+  // (two ints of the kernel's own beside it)
+  if (!lsa::allow_shared(lsa::ward_any_kernel, 227 * 1024 - 16)) return LSA_ERR_LAUNCH;
   lsa::ward_any_kernel<<<(unsigned)blocks, lsa::kWardAnyThreads, smem, s>>>(
       pool_keys, pool_sizes, uniform_pool_size, P, d, bucket_count, bucket_cap, max_rounds, labels, reached, rounds);
   LSA_LAUNCH_CHECK();
@@ -385,16 +385,12 @@ LSA_API int lsa_bucket_table(const void *index_keys, int key_dtype, const int64_
   LSA_REQUIRE(smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
   const dim3 grid((unsigned)blocks, (unsigned)((bucket_count + run - 1) / run));
   if (key_dtype == LSA_DTYPE_F32) {
-    if (cudaFuncSetAttribute(lsa::bucket_table_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    if (!lsa::allow_shared(lsa::bucket_table_kernel<float>, 227 * 1024)) return LSA_ERR_LAUNCH;
     lsa::bucket_table_kernel<float><<<grid, lsa::kTableThreads, smem, s>>>(
         (const float *)index_keys, labels, P, pool_size, d, bucket_count, run, bucket_cap, first_position, members, sizes,
         key_sums, centroids, centroids_bf16, status);
   } else {
-    if (cudaFuncSetAttribute(lsa::bucket_table_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    if (!lsa::allow_shared(lsa::bucket_table_kernel<uint16_t>, 227 * 1024)) return LSA_ERR_LAUNCH;
     lsa::bucket_table_kernel<uint16_t><<<grid, lsa::kTableThreads, smem, s>>>(
         (const uint16_t *)index_keys, labels, P, pool_size, d, bucket_count, run, bucket_cap, first_position, members,
         sizes, key_sums, centroids, centroids_bf16, status);

@@ -116,6 +116,15 @@ inline void launch(bool chained, void (*kernel)(Params...), dim3 grid, dim3 bloc
   (void)cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
+// The dynamic shared memory a kernel may be launched with is an attribute of the KERNEL on the device. Every call sets it to
+// the same `most` that any call of that kernel takes, whatever its own launch uses: a host thread that set less would have
+// another thread's launch refused between that thread's call of this and its launch.
+template <typename Kernel>
+inline bool allow_shared(Kernel *kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
+}
+constexpr size_t kSelectShared = 200 * 1024;  // what the kernels of the bucket search take at most
+
 inline int sm_count() {
   int dev = 0, n = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);

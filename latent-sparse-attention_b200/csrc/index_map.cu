@@ -242,8 +242,8 @@ static int launch_index_map(const void *x, int64_t rows, int heads, int group, i
   const int slices = (d_idx + kMapColSlice - 1) / kMapColSlice;
   const size_t smem =
       sizeof(float) * ((size_t)kMapRows * (kMapSlice + 1) + (size_t)kMapSlice * min(d_idx, kMapColSlice));
-  if (cudaFuncSetAttribute(index_map_kernel<TX, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  if (!allow_shared(index_map_kernel<TX, TW>,
+                    sizeof(float) * (kMapRows * (kMapSlice + 1) + (size_t)kMapSlice * kMapColSlice)))
     return LSA_ERR_LAUNCH;
   const dim3 grid((unsigned)((rows + kMapRows - 1) / kMapRows), (unsigned)slices);
   // One slice: the CTA holds whole rows and normalises them itself. More: fp32 rows first, then unit rows in place.
@@ -403,11 +403,11 @@ LSA_API int lsa_rows_linear(const uint16_t *x, int rows, int heads, int64_t x_ro
   LSA_REQUIRE(((uintptr_t)Wt % 16) == 0, LSA_ERR_ARGUMENT);
   LSA_REQUIRE(!(flags & LSA_ROWS_NORMALIZE) || out_f32, LSA_ERR_ARGUMENT);
   const size_t smem = (size_t)rows * d_in * 2;
-  LSA_REQUIRE(smem <= 160 * 1024, LSA_ERR_UNSUPPORTED);
+  constexpr size_t most = 160 * 1024;
+  LSA_REQUIRE(smem <= most, LSA_ERR_UNSUPPORTED);
   if (rows == 0) return LSA_OK;
   auto kernel = d_in <= 2048 ? lsa::rows_linear_kernel<8> : lsa::rows_linear_kernel<20>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return LSA_ERR_LAUNCH;
+  if (!lsa::allow_shared(kernel, most)) return LSA_ERR_LAUNCH;
   const unsigned grid = (unsigned)((d_out + lsa::kLinThreads / 32 - 1) / (lsa::kLinThreads / 32));
   const bool unit = flags & LSA_ROWS_NORMALIZE;
   lsa::launch(true, kernel, dim3(grid), dim3(lsa::kLinThreads), smem, (cudaStream_t)stream, x, rows,

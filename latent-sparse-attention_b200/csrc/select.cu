@@ -730,7 +730,7 @@ static int pow2_at_least(int n) {
 
 // Chunk of candidates a pass scores: as many as shared memory holds beside the held keys, at most 2048.
 static int select_chunk(int rb, int keep, int d, size_t *smem_out) {
-  const size_t budget = 200 * 1024;
+  const size_t budget = kSelectShared;
   const size_t tile = rb == 1 && select_stages(d) ? (size_t)kSelThreads * (d * 4 + 8) : 0;
   const size_t fixed = (size_t)rb * (pow2_at_least(keep) * 8 + d * 4 + kHistBins * 4) + tile;
   int chunk = 2048;
@@ -747,16 +747,12 @@ static int launch_select(SelectParams p, int splits, cudaStream_t s) {
   if (p.chunk == 0) return LSA_ERR_UNSUPPORTED;
   dim3 grid((unsigned)((p.R + RB - 1) / RB), (unsigned)splits);
   if (p.shape.floors) {
-    if (cudaFuncSetAttribute(select_kernel<RB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    if (!allow_shared(select_kernel<RB, true>, kSelectShared)) return LSA_ERR_LAUNCH;
     launch(p.R <= kChainedRows, select_kernel<RB, true>, grid, dim3(kSelThreads), smem, s, p);
     LSA_LAUNCH_CHECK();
     return LSA_OK;
   }
-  if (cudaFuncSetAttribute(select_kernel<RB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return LSA_ERR_LAUNCH;
+  if (!allow_shared(select_kernel<RB, false>, kSelectShared)) return LSA_ERR_LAUNCH;
   launch(p.R <= kChainedRows, select_kernel<RB, false>, grid, dim3(kSelThreads), smem, s, p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
@@ -909,19 +905,15 @@ static int launch_flat(FlatParams p, cudaStream_t s) {
   while (keep_room < p.keep) keep_room <<= 1;
   const size_t fixed = (size_t)kFlatRows * (keep_room * 8 + D * 4 + kHistBins * 4);
   p.chunk = 1024;
-  while (p.chunk > 256 && fixed + (size_t)kFlatRows * p.chunk * 8 > 200 * 1024) p.chunk -= 256;
+  while (p.chunk > 256 && fixed + (size_t)kFlatRows * p.chunk * 8 > kSelectShared) p.chunk -= 256;
   const size_t smem = fixed + (size_t)kFlatRows * p.chunk * 8;
-  if (smem > 200 * 1024) return LSA_ERR_UNSUPPORTED;
+  if (smem > kSelectShared) return LSA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)((p.R + kFlatRows - 1) / kFlatRows);
   if (p.shape.floors) {
-    if (cudaFuncSetAttribute(flat_select_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    if (!allow_shared(flat_select_kernel<D, true>, kSelectShared)) return LSA_ERR_LAUNCH;
     flat_select_kernel<D, true><<<grid, kFlatThreads, smem, s>>>(p);
   } else {
-    if (cudaFuncSetAttribute(flat_select_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    if (!allow_shared(flat_select_kernel<D, false>, kSelectShared)) return LSA_ERR_LAUNCH;
     flat_select_kernel<D, false><<<grid, kFlatThreads, smem, s>>>(p);
   }
   LSA_LAUNCH_CHECK();
@@ -1277,9 +1269,8 @@ LSA_API int lsa_scan_select(const float *queries, int64_t R, int d, const float 
     if (rc != LSA_OK) return rc;
     const int room = p.room;
     const size_t smem = (size_t)lsa::kSelWarps * ((size_t)room * 8 + lsa::kHistBins * 4);
-    LSA_REQUIRE(smem <= 200 * 1024, LSA_ERR_UNSUPPORTED);
-    if (cudaFuncSetAttribute(lsa::scan_pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return LSA_ERR_LAUNCH;
+    LSA_REQUIRE(smem <= lsa::kSelectShared, LSA_ERR_UNSUPPORTED);
+    if (!lsa::allow_shared(lsa::scan_pick_kernel, lsa::kSelectShared)) return LSA_ERR_LAUNCH;
     lsa::scan_pick_kernel<<<(unsigned)((R + lsa::kSelWarps - 1) / lsa::kSelWarps), lsa::kSelThreads, smem, s>>>(
         p, queries, centroids, flags, bucket_id_base, room, keys_out, picked_out);
     LSA_LAUNCH_CHECK();
@@ -1509,10 +1500,8 @@ static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, 
   // (the lists folded in registers pass through kSelWarps / 2 slots of 128 keys, whatever they hold themselves)
   const int room = max(pow2_at_least(parts * top_p), kSelWarps / 2 * kTopWarp);
   const size_t smem = (size_t)room * 8 + kHistBins * 4;
-  LSA_REQUIRE(smem <= 200 * 1024, LSA_ERR_UNSUPPORTED);
-  if (cudaFuncSetAttribute(merge_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return LSA_ERR_LAUNCH;
+  LSA_REQUIRE(smem <= kSelectShared, LSA_ERR_UNSUPPORTED);
+  if (!allow_shared(merge_candidates_kernel, kSelectShared)) return LSA_ERR_LAUNCH;
   launch(R <= kChainedRows, merge_candidates_kernel, dim3((unsigned)R), dim3(merge_threads(parts, top_p)), smem, stream,
          keys_in, parts, R, top_p, room, keys_out, picked_out, children, fanout, carried_out, sorted ? 1 : 0);
   LSA_LAUNCH_CHECK();

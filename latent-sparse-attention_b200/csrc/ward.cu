@@ -37,6 +37,7 @@ constexpr int kWardRows = 8, kWardFewRows = 2;
 __host__ __device__ constexpr int ward_threads(bool local) { return local ? 256 : 512; }
 __host__ __device__ constexpr int ward_tile(bool local) { return kWardRows * ward_threads(local) / 32; }
 constexpr int kWardMaxCtas = 8;      // a cluster's portable size
+constexpr int kWardMaxPools = 4096;  // pools of a block, at most
 constexpr int kWardLocalPools = 512;  // blocks up to this many pools keep their key sums in every CTA's shared memory
 
 enum : uint8_t { kAlive = 1, kOpen = 2, kChanged = 4, kMerged = 8 };
@@ -527,7 +528,7 @@ static int launch_ward(const WardParams &p, int64_t G, cudaStream_t s) {
   int ctas = (int)(most < 1 ? 1 : most < kWardMaxCtas ? most : kWardMaxCtas);
   WardShared<D, LOCAL> shared;
   const size_t smem = shared.carve(nullptr, p.P, ctas > 1);
-  if (cudaFuncSetAttribute(ward_kernel<D, LOCAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (!allow_shared(ward_kernel<D, LOCAL>, shared.carve(nullptr, LOCAL ? kWardLocalPools : kWardMaxPools, true))) {
     (void)cudaGetLastError();
     return LSA_ERR_LAUNCH;
   }

@@ -4,6 +4,8 @@ Integer results (labels, member tables, picked buckets, read lists) must be bit-
 2e-6 (fp32 sums in another order), attention within max-abs 2e-2 / mean-abs 2e-3 of the fp32 oracle on bf16 inputs.
 """
 
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -734,3 +736,58 @@ def test_few_row_paths_of_a_decode_step(ops, oracle):
             assert (out.double() - (weights[..., None] * parts.double()).sum(0)).abs().max() <= 1e-5
             assert (lse - torch.logsumexp(lses.double(), 0))[torch.isfinite(lse)].abs().max() <= 1e-5
             assert not torch.isfinite(lse[6]) and not out[6].any()
+
+
+@pytest.mark.parametrize("kernel", ["gather", "scan", "decode scan", "merge", "ward", "bucket table", "map", "row map"])
+def test_host_threads_that_launch_a_kernel_with_different_sizes(ops, kernel, monkeypatch):
+    """The library lets go of the interpreter's lock, so a decode step's small launch and a chunk's large one of the same
+    kernel meet: neither may have the other refused. (The outputs are those of a call alone.)"""
+    from lsa_b200 import _lib
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")
+    if kernel == "gather":
+        q, k = rand(2000, 8, 128).bfloat16(), rand(64, 2, 128).bfloat16()
+        ids = torch.arange(8, device="cuda", dtype=torch.int32).expand(2000, 8).contiguous()
+        run = lambda big: ops.sparse_attend(q if big else q[:1], k, k, ids if big else ids[:1], None, 0.1)[0]
+    elif kernel in ("scan", "decode scan"):
+        rows, cent, seen = rand(16, 64), rand(700, 64), torch.full((16,), 700, device="cuda", dtype=torch.int32)
+        scan = ops.flat_select if kernel == "scan" else lambda r, c, s, top: ops.flat_select_decode(r, c, None, s, top)
+        run = lambda big: scan(rows, cent, seen, 512 if big else 1)[0]
+    elif kernel == "merge":
+        keys = {n: torch.randint(0, 1 << 60, (n, 4, 256), generator=gen, device="cuda") for n in (2, 32)}
+        run = lambda big: ops.merge_candidates(keys[32 if big else 2])[0]
+    elif kernel == "ward":
+        pools = torch.nn.functional.normalize(rand(1, 512, 64), dim=2)
+        run = lambda big: ops.ward_rounds(pools if big else pools[:, :8].contiguous(), 1.0, 64 if big else 4, 16.0)[0]
+    elif kernel == "bucket table":
+        keys, labels = rand(600 * 32, 64), torch.arange(600 * 32, device="cuda").view(600, 32) % 16
+        run = lambda big: ops.bucket_table(keys if big else keys[:32], labels if big else labels[:1], 1, 16, 4)[2]
+    elif kernel == "map":
+        x, w = rand(100, 2, 64), {n: rand(128, n) for n in (8, 64)}
+        run = lambda big: ops.index_map(x, w[64 if big else 8], group=1)
+    else:
+        x, w = rand(8, 2, 512).bfloat16(), rand(64, 1024).bfloat16()
+        run = lambda big: ops.rows_linear(x if big else x[:1], w)
+    entries = {}  # the entry point and the arguments of each call, to be made again with nothing in between
+
+    def recorded(name, *args, launches=1):
+        entries[len(entries)] = getattr(_lib.load(), name), args
+        return _lib.call(name, *args, launches=launches)
+
+    monkeypatch.setattr(ops, "call", recorded)
+    outs = [run(False), run(True)]
+    torch.cuda.synchronize()
+    want, wrong = [out.clone() for out in outs], []
+
+    def work(which):
+        entry, args = entries[which]
+        wrong.extend(code for code in (entry(*args) for _ in range(4000)) if code != 0)
+
+    threads = [threading.Thread(target=work, args=(which,)) for which in (0, 1, 0, 1)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert len(entries) == 2 and not wrong, (len(entries), wrong[:3])
+    assert all(torch.equal(out, same) for out, same in zip(outs, want))
