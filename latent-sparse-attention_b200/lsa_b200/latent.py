@@ -67,7 +67,7 @@ class LatentLayer(FlatLayer):
         if not self.two_layer:
             return ops.index_map_tc(rows, weights, out=out, status=self._map_status)
         piece = min(n, self.map_piece)
-        hidden = self._buffer("hidden", (piece, weights[0].shape[0]), torch.bfloat16, rows.device)
+        hidden = self._room("hidden", (piece, weights[0].shape[0]), torch.bfloat16, rows.device)
         for start in range(0, n, piece):
             m = min(piece, n - start)
             ops.mlp_map(rows[start:start + m], weights[0], weights[1], hidden=hidden[:m], out=out[start:start + m])
@@ -122,9 +122,9 @@ class LatentLayer(FlatLayer):
         n, dev = rows.shape[0], rows.device
         positions = torch.arange(start, start + n, device=dev)
         with probe.region("index map"):
-            index_queries = self.index_queries(rows, out=self._buffer("index queries", (n, self.index_dim),
-                                                                      torch.float32, dev))
-        lists, lengths = self.select(index_queries, positions, index, reuse_buffers=True, last_position=start + n - 1)
+            index_queries = self.index_queries(rows, out=self._room("index queries", (n, self.index_dim),
+                                                                    torch.float32, dev))
+        lists, lengths = self._select(index_queries, positions, index, self._room, True, start + n - 1)
         with probe.region("attend"):
             ops.latent_attend(rows, latent, lists, lengths, self.scale, value_dim=self.value_dim, out=out,
                               warp_mma=warp_mma, status=self._attend_status)
@@ -147,8 +147,8 @@ class LatentLayer(FlatLayer):
         while len(self._copy_events) < 2 * len(spans) + 1:
             self._copy_events.append(torch.cuda.Event())
         rows_in, arrived, done = self._copy_events[0], self._copy_events[1::2], self._copy_events[2::2]
-        q = self._buffer("q from host", tuple(q_host.shape), q_host.dtype, dev)
-        out = self._buffer("out to host", tuple(out_host.shape), out_host.dtype, dev)
+        q = self._room("q from host", tuple(q_host.shape), q_host.dtype, dev)
+        out = self._room("out to host", tuple(out_host.shape), out_host.dtype, dev)
         self._copy_in.wait_stream(main)   # the last call's reads of these buffers are over
         self._copy_out.wait_stream(main)
         with torch.cuda.stream(self._copy_in):

@@ -144,15 +144,31 @@ class FlatLayer:
     # ---- buffers
 
     def _buffer(self, name: str, shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
-        """A tensor that lives as long as the layer: a step allocates nothing once every shape has been seen. (Fewer rows
-        than a buffer of that name has are its leading ones: a ragged chunk allocates nothing beside a whole one.)"""
-        key = (name, tuple(shape[1:]), dtype, str(device))
-        held = self._buffers.setdefault(key, [])  # ascending: a call that outgrows them adds one, and none moves
+        """A tensor that lives as long as the layer, one a shape: what a call hands out stays until the next call of that
+        shape, and a step allocates nothing once every shape has been seen."""
+        key = (name, tuple(shape), dtype, str(device))
+        held = self._buffers.get(key)
+        if held is None:
+            held = self._buffers[key] = torch.empty(shape, device=device, dtype=dtype)
+        return held
+
+    def _room(self, name: str, shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
+        """The same for what no call hands out: the leading rows of a buffer of that name, so that a ragged chunk allocates
+        nothing beside a whole one. A buffer that is outgrown stays (a captured graph may hold its address) and the next has
+        half as many rows again, where there is memory for that: all of a name's are less than five times the largest asked
+        for."""
+        held = self._buffers.setdefault((name, "rows", tuple(shape[1:]), dtype, str(device)), [])
         for buffer in held:
             if buffer.shape[0] >= shape[0]:
                 return buffer[:shape[0]]
-        held.append(torch.empty(shape, device=device, dtype=dtype))
-        return held[-1]
+        rows = max(shape[0], held[-1].shape[0] * 3 // 2) if held else shape[0]
+        try:
+            held.append(torch.empty(rows, *shape[1:], device=device, dtype=dtype))
+        except torch.OutOfMemoryError:
+            if rows == shape[0]:
+                raise
+            held.append(torch.empty(shape, device=device, dtype=dtype))
+        return held[-1][:shape[0]]
 
     def _takes_tensor_cores(self, x: torch.Tensor) -> bool:
         """Heads packed densely in bf16 with a 16-byte aligned row pitch: the layout a TMA descriptor can walk."""
@@ -198,7 +214,7 @@ class FlatLayer:
         d, d_idx = self.design, self.index_dim
         blocks = T // d.cluster_block_size
         P, rows = d.cluster_block_size // d.pool_size, blocks * d.block_bucket_count
-        make = (lambda name, shape, dtype: self._buffer(f"{name} of {T}", shape, dtype, dev)) if reuse_buffers else \
+        make = (lambda name, shape, dtype: self._buffer(name, shape, dtype, dev)) if reuse_buffers else \
             (lambda name, shape, dtype: torch.empty(shape, device=dev, dtype=dtype))
         bufs = {"keys": make("index keys", (T, d_idx), torch.float32),
                 "pools": make("pools", (blocks, P, d_idx), torch.float32),
@@ -278,6 +294,10 @@ class FlatLayer:
         """The top-p buckets of every row, best first: (picked [R, top_p] int32, positions int64, and the rows' own
         budgets under an early budget, else None). `last_position` is the host's bound on `positions`, if it has
         one (it places the samples of the tensor-core scan; the result does not depend on it)."""
+        return self._pick(index_queries, positions, index, self._buffer if reuse_buffers else None, last_position)
+
+    def _pick(self, index_queries: torch.Tensor, positions: torch.Tensor, index: FlatIndex, held, last_position: int | None):
+        """`pick` into what `held` (`_buffer` or `_room`) gives, or into fresh tensors."""
         d, b, dev = self.design, index.buckets, index_queries.device
         R = index_queries.shape[0]
         positions = positions.to(torch.int64)
@@ -288,9 +308,9 @@ class FlatLayer:
             row_p = torch.where(early, d.early_budget.top_p, d.top_p).to(torch.int32)
             row_k = torch.where(early, d.early_budget.top_k, d.top_k).to(torch.int32)
         keys = picked = None
-        if reuse_buffers:
-            keys = self._buffer("keys", (R, d.top_p), torch.int64, dev)
-            picked = self._buffer("picked", (R, d.top_p), torch.int32, dev)
+        if held is not None:
+            keys = held("keys", (R, d.top_p), torch.int64, dev)
+            picked = held("picked", (R, d.top_p), torch.int32, dev)
         with probe.region("select"):
             bound = 0 if last_position is None else last_position // d.cluster_block_size * d.block_bucket_count
             bound = min(bound or b.bucket_centroids.shape[0], b.bucket_centroids.shape[0])
@@ -302,7 +322,7 @@ class FlatLayer:
             elif index.centroids_bf16 is not None and R >= self.scan_rows and d.top_p <= 512 and bound >= 1024 \
                     and 3 * d.top_p * 512 >= 8 * bound:
                 need = ops.query("lsa_scan_select_workspace_bytes", R, d.top_p, b.bucket_centroids.shape[0])
-                work = self._buffer("scan", (need,), torch.uint8, dev)
+                work = self._room("scan", (need,), torch.uint8, dev)
                 _, picked = ops.scan_select(index_queries, b.bucket_centroids, index.centroids_bf16, visible, d.top_p,
                                             row_p, max_visible=bound, keys=keys, picked=picked,
                                             status=self._scan_status, workspace=work, lengths=index.lengths,
@@ -322,12 +342,16 @@ class FlatLayer:
                reuse_buffers: bool = False, local: bool = True, last_position: int | None = None):
         """Read lists [R, top_k + window + sink] int32 and their lengths for queries at `positions`; with
         `local=False` the lists hold the expansion alone (a band kernel reads the window and the sinks)."""
+        return self._select(index_queries, positions, index, self._buffer if reuse_buffers else None, local, last_position)
+
+    def _select(self, index_queries: torch.Tensor, positions: torch.Tensor, index: FlatIndex, held, local: bool,
+                last_position: int | None):
+        """`select` into what `held` gives, or into fresh tensors."""
         d, b, dev = self.design, index.buckets, index_queries.device
         R = index_queries.shape[0]
-        picked, positions, row_p, row_k = self.pick(index_queries, positions, index, reuse_buffers, last_position)
-        if reuse_buffers:
-            lists, lengths = (self._buffer("lists", (R, d.list_width), torch.int32, dev),
-                              self._buffer("lengths", (R,), torch.int32, dev))
+        picked, positions, row_p, row_k = self._pick(index_queries, positions, index, held, last_position)
+        if held is not None:
+            lists, lengths = held("lists", (R, d.list_width), torch.int32, dev), held("lengths", (R,), torch.int32, dev)
         else:
             lists = torch.empty(R, d.list_width, device=dev, dtype=torch.int32)
             lengths = torch.empty(R, device=dev, dtype=torch.int32)
@@ -335,7 +359,7 @@ class FlatLayer:
             # (the layer's own buffers are read by their lengths: nothing is padded there)
             lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
                                            row_p, row_k, outs=(lists, lengths, self._expand_status), local=local,
-                                           pad=not reuse_buffers)
+                                           pad=held is None)
         return lists, lengths
 
     def attend(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, lists: torch.Tensor, lengths: torch.Tensor,
@@ -346,12 +370,18 @@ class FlatLayer:
 
     def band(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_position: int):
         """The window and sinks of consecutive rows as one dense banded read: a partial (out fp32, lse)."""
-        R, dev = q.shape[0], q.device
+        return self._band(q, k, v, first_position, *self._partial(self._buffer, "band", q.shape[0], q.device))
+
+    def _partial(self, held, name: str, rows: int, device) -> tuple:
+        """A partial read's tensors: out fp32 and lse."""
+        return (held(f"{name} out", (rows, self.heads, self.head_dim), torch.float32, device),
+                held(f"{name} lse", (rows, self.heads), torch.float32, device))
+
+    def _band(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_position: int, out: torch.Tensor,
+              lse: torch.Tensor):
         with probe.region("band"):
             return ops.band_attend(q, k, v, first_position, self.design.window_size, self.design.sink_size, self.scale,
-                                   out=self._buffer("band out", (R, self.heads, self.head_dim), torch.float32, dev),
-                                   lse=self._buffer("band lse", (R, self.heads), torch.float32, dev),
-                                   status=self._attend_status)
+                                   out=out, lse=lse, status=self._attend_status)
 
     # ---- the layer
 
@@ -395,10 +425,10 @@ class FlatLayer:
         while len(self._copy_events) < 3 * len(chunks):
             self._copy_events.append(torch.cuda.Event())
         arrived, done, built = self._copy_events[0::3], self._copy_events[1::3], self._copy_events[2::3]
-        q = self._buffer("q from host", tuple(q_host.shape), q_host.dtype, dev)
-        k = self._buffer("k from host", tuple(k_host.shape), k_host.dtype, dev)
-        v = self._buffer("v from host", tuple(v_host.shape), v_host.dtype, dev)
-        out = self._buffer("out to host", tuple(q_host.shape), torch.bfloat16, dev)
+        q = self._room("q from host", tuple(q_host.shape), q_host.dtype, dev)
+        k = self._room("k from host", tuple(k_host.shape), k_host.dtype, dev)
+        v = self._room("v from host", tuple(v_host.shape), v_host.dtype, dev)
+        out = self._room("out to host", tuple(q_host.shape), torch.bfloat16, dev)
         self._copy_in.wait_stream(main)   # the last call's reads of these buffers are over
         self._copy_out.wait_stream(main)
         with torch.cuda.stream(self._copy_in):
@@ -451,11 +481,9 @@ class FlatLayer:
             # lists' read, which this stands for, is closer to the sums in 64 bits than one rounded term a key.)
             whole = min(n, self._whole_until(index) - start)
             with probe.region("band"):
-                dense, _ = ops.band_attend(rows[:whole], k, v, start, start + whole, 0, self.scale,
-                                           out=self._buffer("dense out", (whole, self.heads, self.head_dim),
-                                                            torch.float32, dev),
-                                           lse=self._buffer("dense lse", (whole, self.heads), torch.float32, dev),
-                                           status=self._attend_status, two_term=True)
+                dense, dense_lse = self._partial(self._room, "dense", whole, dev)
+                ops.band_attend(rows[:whole], k, v, start, start + whole, 0, self.scale, out=dense, lse=dense_lse,
+                                status=self._attend_status, two_term=True)
                 out[:whole].copy_(dense)
             if whole == n:
                 return out
@@ -463,12 +491,13 @@ class FlatLayer:
             return out
         positions = torch.arange(start, stop, device=dev)
         with probe.region("index map"):
-            index_queries = self.index_queries(rows, out=self._buffer("index queries", (n, self.index_dim),
-                                                                      torch.float32, dev))
+            index_queries = self.index_queries(rows, out=self._room("index queries", (n, self.index_dim),
+                                                                    torch.float32, dev))
         # The window and the sinks are the same keys for neighbouring rows: one dense band serves them, and the
         # read of the selected keys starts from its partial result.
         banded = band and self.design.sink_size <= 64 and k.shape[0] >= stop
-        lse = self._buffer("lse", (n, self.heads), torch.float32, dev)
+        lse = self._room("lse", (n, self.heads), torch.float32, dev)
+        partial = self._partial(self._room, "band", n, dev) if banded else None
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
         # (Its partial outputs are a workspace by the pick: buckets of more than 64 members, which the gather serves too, take
         # it up to 8 GiB.)
@@ -484,12 +513,11 @@ class FlatLayer:
                 self._band_stream, self._band_done = torch.cuda.Stream(dev), torch.cuda.Event()
             self._band_stream.wait_stream(main)  # the inputs are ready; the last chunk's merge has read the buffers
             with torch.cuda.stream(self._band_stream):
-                init = self.band(rows, k, v, start)
+                init = self._band(rows, k, v, start, *partial)
                 self._band_done.record(self._band_stream)
             # The rows of a chunk pick the same buckets over and over: read each bucket's keys once per 128
             # (row, pick) pairs instead of once per pair.
-            picked, positions, row_p, row_k = self.pick(index_queries, positions, index, reuse_buffers=True,
-                                                        last_position=stop - 1)
+            picked, positions, row_p, row_k = self._pick(index_queries, positions, index, self._room, stop - 1)
             with probe.region("attend"):
                 ops.bucket_attend(rows, k, v, picked, positions, index.buckets.bucket_members, self.design.top_k,
                                   self.design.sink_size, self.design.window_size, self.scale, init=init,
@@ -498,9 +526,8 @@ class FlatLayer:
                                   status=self._attend_status,
                                   workspace=self._buffer("bucket workspace", (need,), torch.uint8, dev))
             return out
-        init = self.band(rows, k, v, start) if banded else None
-        lists, lengths = self.select(index_queries, positions, index, reuse_buffers=True, local=not banded,
-                                     last_position=stop - 1)
+        init = self._band(rows, k, v, start, *partial) if banded else None
+        lists, lengths = self._select(index_queries, positions, index, self._room, not banded, stop - 1)
         self.attend(rows, k, v, lists, lengths, out=out, lse=lse, init=init)
         return out
 

@@ -514,9 +514,9 @@ class ShardedLatentLayer:
         while len(layer._copy_events) < 2 * pieces + 1:
             layer._copy_events.append(torch.cuda.Event())
         rows_in, arrived, done = layer._copy_events[0], layer._copy_events[1::2], layer._copy_events[2::2]
-        q_own = layer._buffer("q share from host", tuple(q_host.shape), q_host.dtype, dev)
-        q_all = layer._buffer("q pieces", (pieces, piece, *q_host.shape[1:]), q_host.dtype, dev)
-        out = layer._buffer("out share to host", tuple(out_host.shape), out_host.dtype, dev)
+        q_own = layer._room("q share from host", tuple(q_host.shape), q_host.dtype, dev)
+        q_all = layer._room("q pieces", (pieces, piece, *q_host.shape[1:]), q_host.dtype, dev)
+        out = layer._room("out share to host", tuple(out_host.shape), out_host.dtype, dev)
         copy_in.wait_stream(main)   # the last call's reads of these buffers are over
         copy_out.wait_stream(main)
         with torch.cuda.stream(copy_in):

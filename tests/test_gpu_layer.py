@@ -129,3 +129,29 @@ def test_rows_that_read_everything_are_read_densely(oracle, T, Hq, Hkv, dh, chun
     else:
         assert everything[:until].all() and (until >= T or not everything[until:].all())
     layer.check()
+
+
+def test_a_selection_outlives_a_shorter_one():
+    """Lists and picks handed out in the layer's own buffers are those of their shape: a call with fewer rows, and a prefill
+    between, leave them as they were."""
+    from lsa_b200.layer import FlatDesign
+
+    T, Hq, Hkv = 3000, 8, 2
+    design = FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200, sink_size=4,
+                        window_size=128)
+    layer, _ = _layer(Hq, Hkv, 128, 64, design, 1)
+    Q, K, V = (cuda(a, torch.bfloat16) for a in layer_inputs(T, Hq, Hkv, 128, 16, 1))
+    index = layer.build_index(K)
+    index_q, positions = layer.index_queries(Q), torch.arange(T, device="cuda")
+    lists, lengths = layer.select(index_q[1000:], positions[1000:], index, reuse_buffers=True)
+    picked = layer.pick(index_q[1000:], positions[1000:], index, reuse_buffers=True)[0]
+    band = layer.band(Q[1000:], K, V, 1000)
+    held = (lists, lengths, picked, *band)
+    kept = [x.clone() for x in held]
+    layer.select(index_q[500:900], positions[500:900], index, reuse_buffers=True)
+    layer.pick(index_q[500:900], positions[500:900], index, reuse_buffers=True)
+    layer.band(Q[500:900], K, V, 500)
+    layer.prefill(Q[:1100], K[:1100], V[:1100], chunk=400)
+    inside = torch.arange(lists.shape[1], device="cuda") < lengths[:, None].long()
+    assert torch.equal(lists[inside], kept[0][inside])
+    assert all(torch.equal(x, y) for x, y in zip(held[1:], kept[1:]))

@@ -246,3 +246,21 @@ def test_prefix_reuse_shares_full_pages_by_fingerprint_and_keeps_a_finished_pref
         cache.fingerprint(0, page, object())
     plain = BucketCache(design, 32, pages=2, page_buckets=4, max_requests=2, max_request_pages=2, device="cpu")
     assert plain.adopt(0, 4 * page, object()) == 0 and plain.fingerprint(0, page, object()) is None
+
+
+def test_a_layers_buffers_are_one_a_shape_and_its_own_rooms_grow_by_halves():
+    """What a call hands out is not written over by a call of another shape; what stays inside is the leading rows of one
+    buffer, and lengths that go on growing hold less than five times the longest."""
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    layer = FlatLayer(FlatDesign(), torch.zeros(128, 64), torch.zeros(128, 64), 2, 1, 128)
+    longer = layer._buffer("lists", (8, 3), torch.int32, "cpu").fill_(7)
+    layer._buffer("lists", (5, 3), torch.int32, "cpu").fill_(1)
+    assert (longer == 7).all() and layer._buffer("lists", (8, 3), torch.int32, "cpu") is longer
+    whole = layer._room("lse", (100, 4), torch.float32, "cpu")
+    assert layer._room("lse", (37, 4), torch.float32, "cpu").data_ptr() == whole.data_ptr()
+    assert layer._room("lse", (37, 5), torch.float32, "cpu").shape == (37, 5)
+    for rows in range(101, 3000):
+        assert layer._room("lse", (rows, 4), torch.float32, "cpu").shape == (rows, 4)
+    held = layer._buffers["lse", "rows", (4,), torch.float32, "cpu"]
+    assert held[0].data_ptr() == whole.data_ptr() and sum(len(b) for b in held) < 5 * 3000
