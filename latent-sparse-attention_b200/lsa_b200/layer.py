@@ -390,8 +390,8 @@ class FlatLayer:
                 bucket_major: bool = True):
         """Causal prefill from position 0: q [T,Hq,dh], k/v [T,Hkv,dh] bf16 -> out [T,Hq,dh] bf16.
 
-        Every intermediate lives in buffers the layer keeps, so after the first call a step allocates nothing but
-        its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
+        Every intermediate but the bucket-major read's workspace (the allocator's again after each chunk) lives in buffers the
+        layer keeps, so after the first call a step allocates nothing beside it but its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
         `band` reads the window and the sinks as dense tiles; `bucket_major` reads the selected keys bucket by bucket
         where the shapes allow and it is the faster read (both off: every row gathers its whole list).
         """
@@ -469,6 +469,26 @@ class FlatLayer:
         meet near three keys a query head of the group."""
         return self.design.bucket_size >= 3 * (self.heads // self.kv_heads)
 
+    def _bucket_workspace(self, rows: int, index: FlatIndex, device) -> torch.Tensor | None:
+        """The bucket-major read's workspace, a partial output a (row, pick, head): gigabytes that the layer does not keep. It
+        goes back to the allocator with the chunk and serves the next, and the other layers of a model. Sizes are cut to 32
+        steps an octave, so that an index with a few buckets more asks for the same bytes. Buckets of more than 64 members,
+        which the gather served alone before there was a pass for them, go to the gather again where the workspace is over
+        8 GiB or there is no memory for it. (24,576 tokens of 40 heads, 48 picks of 64 keys: 14.4 ms with 8.1 GB, in shorter
+        chunks 14.9 with 4.0 and 18.0 with 1.0; the gather 25.6 to 28.3. The line keeps a chunk from a tenth of the GPU.)"""
+        members = index.buckets.bucket_members
+        need = ops.bucket_attend_workspace(rows, self.design.top_p, self.heads, self.head_dim, *members.shape)
+        wide = members.shape[1] > 64
+        if wide and need > 8 << 30:
+            return None
+        step = max(1 << 21, 1 << max(0, need.bit_length() - 6))
+        try:
+            return torch.empty(-(-need // step) * step, device=device, dtype=torch.uint8)
+        except torch.OutOfMemoryError:
+            if wide:
+                return None
+            raise
+
     def prefill_rows(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, band: bool = True, bucket_major: bool = True) -> torch.Tensor:
         """The read of consecutive query rows [n, Hq, dh] at positions start.. over a cache whose index is built,
@@ -499,13 +519,12 @@ class FlatLayer:
         lse = self._room("lse", (n, self.heads), torch.float32, dev)
         partial = self._partial(self._room, "band", n, dev) if banded else None
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
-        # (Its partial outputs are a workspace by the pick: buckets of more than 64 members, which the gather serves too, take
-        # it up to 8 GiB.)
-        need = ops.bucket_attend_workspace(n, self.design.top_p, self.heads, self.head_dim,
-                                           *index.buckets.bucket_members.shape)
-        if banded and bucket_major and self._reads_by_bucket and (self.design.bucket_cap <= 64 or need <= 8 << 30) and \
+        workspace = None
+        if banded and bucket_major and self._reads_by_bucket and \
                 ops.bucket_attend_supported(rows, k, self.design.bucket_cap, self.design.top_p,
                                             not self.bucket_tensor_memory):
+            workspace = self._bucket_workspace(n, index, dev)
+        if workspace is not None:
             # The band and the read of the selected keys meet only in the merge, and one waits on the tensor pipe
             # while the other is bound by instruction issue: the band runs on a stream of its own beside them.
             main = torch.cuda.current_stream(dev)
@@ -524,7 +543,7 @@ class FlatLayer:
                                   row_top_p=row_p, row_top_k=row_k, out=out, lse=lse,
                                   warp_mma=not self.bucket_tensor_memory, init_ready=self._band_done,
                                   status=self._attend_status,
-                                  workspace=self._buffer("bucket workspace", (need,), torch.uint8, dev))
+                                  workspace=workspace)
             return out
         init = self._band(rows, k, v, start, *partial) if banded else None
         lists, lengths = self._select(index_queries, positions, index, self._room, not banded, stop - 1)

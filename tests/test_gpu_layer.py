@@ -155,3 +155,48 @@ def test_a_selection_outlives_a_shorter_one():
     inside = torch.arange(lists.shape[1], device="cuda") < lengths[:, None].long()
     assert torch.equal(lists[inside], kept[0][inside])
     assert all(torch.equal(x, y) for x, y in zip(held[1:], kept[1:]))
+
+
+@pytest.mark.parametrize("sizes,d_idx", [
+    (dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=1024, sink_size=4,
+          window_size=128), 64),
+    (dict(pool_size=16, bucket_size=64, bucket_cap=128, cluster_block_size=512, top_p=16, top_k=1024, sink_size=4,
+          window_size=128), 32)])
+def test_prompts_that_grow_hold_no_workspace_more(sizes, d_idx, monkeypatch):
+    """Layers over prompts that get longer share the bucket-major read's workspace, and none is held after a prefill; wide
+    buckets without memory for one are gathered."""
+    from lsa_b200 import ops
+    from lsa_b200.layer import FlatDesign
+
+    design, Hq, Hkv, chunk = FlatDesign(**sizes), 16, 4, 2048
+    k, v = (torch.randn(9000, Hkv, 128, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(9000, Hq, 128, device="cuda").bfloat16()
+    layers = [_layer(Hq, Hkv, 128, d_idx, design, 1)[0] for _ in range(2)]
+    need = ops.bucket_attend_workspace(chunk, design.top_p, Hq, 128, 9000 // design.bucket_size, design.bucket_cap)
+    torch.cuda.empty_cache()
+    base, reserved = torch.cuda.memory_allocated(), torch.cuda.memory_reserved()
+    out = torch.empty(9000, Hq, 128, device="cuda", dtype=torch.bfloat16)
+    for T in range(5000, 9001, 500):
+        for layer in layers:
+            layer.prefill(q[:T], k[:T], v[:T], chunk=chunk, out=out[:T])
+    own = sum(b.numel() * b.element_size() for layer in layers for held in layer._buffers.values()
+              for b in (held if isinstance(held, list) else [held]))
+    grown = torch.cuda.memory_allocated() - base - out.numel() * 2
+    assert grown <= own + (1 << 21) * 8, (grown, own)   # (a layer's buffers, rounded up a little each)
+    assert own < 18 * need // 2, (own, need)            # (eighteen prefills; no workspace is among the buffers)
+    assert torch.cuda.memory_reserved() - reserved < own + out.numel() * 2 + 3 * need
+    want = layers[0].prefill(q, k, v, chunk=chunk, bucket_major=False)
+    empty = torch.empty
+
+    def without(*shape, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("said on the host")
+        return empty(*shape, **kw)
+
+    with monkeypatch.context() as patch:
+        patch.setattr(torch, "empty", without)
+        if design.bucket_cap > 64:
+            assert torch.equal(layers[0].prefill(q, k, v, chunk=chunk, out=out), want)
+        else:
+            with pytest.raises(torch.OutOfMemoryError):
+                layers[0].prefill(q, k, v, chunk=chunk, out=out)
