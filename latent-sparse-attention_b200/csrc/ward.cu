@@ -197,9 +197,10 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
           is_merged = f & kMerged;
         }
       }
+      static_assert(kThreads < 1024, "three sums of up to kThreads in a word");
       const unsigned vd = __ballot_sync(0xffffffffu, is_dirty), vs = __ballot_sync(0xffffffffu, is_steady);
       const unsigned vm = __ballot_sync(0xffffffffu, is_merged);
-      if (lane == 0) warp_count[warp] = __popc(vd) | __popc(vs) << 10 | __popc(vm) << 20;  // (each sums to 256 at most)
+      if (lane == 0) warp_count[warp] = __popc(vd) | __popc(vs) << 10 | __popc(vm) << 20;  // (ten bits a sum: the threads of the CTA at most)
       __syncthreads();
       int before = 0, all = 0;
 #pragma unroll
@@ -238,6 +239,12 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
     for (int i = tid; i < P; i += kThreads) s.sq[i] = __ldcg(sq_g + i), s.al[i] = __ldcg(al_g + i);
     __syncthreads();
   }
+
+  // A merged row's norm is at most the block's norms together: 4,096 of up to 1e15 keep `both` under 1e19, whose square is in
+  // range. (Norms that are not numbers count as greater; an infinite slack leaves `most` infinitely below zero, or no number.)
+  bool great = false;
+  for (int i = tid; i < P; i += kThreads) great = great || !(s.al[i] <= 1e15f);
+  const float slack = __syncthreads_or(great) ? INFINITY : 9.5367431640625e-7f;
 
   for (; rounds < p.max_rounds && n_alive > p.bucket_count; ++rounds) {
     // ---- the cheapest partners: tiles of (dirty x open) and (steady x merged), dealt to the CTAs in runs
@@ -320,8 +327,10 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
             // Most pairs are far from the cheapest so far, and a product says so without the root: with
             // most = both - best - both / 2^20 positive and m2 <= most^2 (1 - 2^-20), the root is under `most` by more
             // than the roundings of all of these (a few 2^-24 of `both`), so the cost is above the best, and not a tie.
-            const float most = (both - best_c[i]) - both * 9.5367431640625e-7f;
-            if (most > 0.0f && m2 <= most * most * 0.99999904632568359375f) continue;
+            // (That takes squares that are normal numbers: `most` is above 1e-15, and `slack` lets no pair through here in a
+            // block whose norms may leave their range.)
+            const float most = (both - best_c[i]) - both * slack;
+            if (most > 1e-15f && m2 <= most * most * 0.99999904632568359375f) continue;
             if (id_j[j] < 0 || id_i == id_j[j] || __fadd_rn(sz_i, sz_j[j]) > p.bucket_cap) continue;
             const float whole = sqrtf(m2 > 0.0f ? m2 : 0.0f);
             const float cost = __fsub_rn(both, whole);

@@ -159,6 +159,21 @@ def test_ward_blocks_over_one_to_eight_ctas_are_bit_exact(ops, oracle, G, P, d, 
         assert np.array_equal(rounds.cpu().numpy(), want_rounds)
 
 
+@pytest.mark.parametrize("scale", [1e-30, 1e-22, 1e-19, 3e-17, 1e-10, 1e14, 1e15, 4e18, 1.2e19])
+@pytest.mark.parametrize("P", [96, 600])
+def test_ward_of_keys_whose_squares_leave_fp32s_range_is_bit_exact(ops, oracle, scale, P):
+    """Norms whose squares are denormal, zero or infinite, in both forms: the costs are the replay's, so the labels are."""
+    rng = np.random.default_rng(P)
+    with np.errstate(all="ignore"):
+        keys = (unit_rows(mixture(2 * P, 64, 12, 0.4, P)) * rng.uniform(0.3, 2.0, (2 * P, 1)) * scale).astype(np.float32)
+        keys = keys.reshape(2, P, 64)
+        sizes = np.full((2, P), 4.0, np.float32)
+        want, want_reached, want_rounds = oracle.ward_rounds(keys, sizes, P // 8, 64.0, return_rounds=True)
+    got, reached, rounds = ops.ward_rounds(cuda(keys), cuda(sizes), P // 8, 64.0, return_rounds=True)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(reached.cpu().numpy(), want_reached) and np.array_equal(rounds.cpu().numpy(), want_rounds)
+
+
 def test_ward_golden_and_adversarial_cases(ops, oracle):
     g = golden("ward")
     for tag in "abcde":
