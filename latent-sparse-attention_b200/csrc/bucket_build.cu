@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kTableThreads)
   int *pools_of = reinterpret_cast<int *>(smem_raw);  // [run] pools of a bucket so far
   int *place = pools_of + run;                        // [step] a pool's bucket of this run, or -1
   int *before = place + kTablePools;                  // [step] and the bucket's pools before it
-  float *sums = reinterpret_cast<float *>(before + kTablePools);  // [run][d]
+  float *sums = reinterpret_cast<float *>(smem_raw);  // [run][d], where the places were once they are used up
   for (int b = threadIdx.x; b < buckets; b += blockDim.x) pools_of[b] = 0;
   for (int from = 0; from < P; from += kTablePools) {
     const int pools = min(kTablePools, P - from);
@@ -374,14 +374,19 @@ LSA_API int lsa_bucket_table(const void *index_keys, int key_dtype, const int64_
   // (a block's sums and norms beside one another in one CTA's shared memory: the size this call has always taken)
   LSA_REQUIRE(!sums || sizeof(float) * ((size_t)bucket_count * d + bucket_count) <= 227 * 1024, LSA_ERR_UNSUPPORTED);
   cudaStream_t s = (cudaStream_t)stream;
-  // CTAs a block: enough to give every SM four, and no fewer than a run's sums fit shared memory with the pools' places.
+  // CTAs a block: enough to give every SM four, and no fewer than a run's sums (or, before them, its pools' places) fit
+  // shared memory.
   const int sms = lsa::sm_count();
-  const size_t fixed = sizeof(int) * 2 * lsa::kTablePools, a_bucket = sizeof(int) + (sums ? sizeof(float) * ((size_t)d + 1) : 0);
+  auto shared_of = [&](int buckets) {
+    const size_t places = sizeof(int) * ((size_t)buckets + 2 * lsa::kTablePools);
+    const size_t keys = sums ? sizeof(float) * buckets * ((size_t)d + 1) : 0;
+    return places > keys ? places : keys;
+  };
   int64_t runs = (4 * (int64_t)sms + blocks - 1) / blocks;
   runs = runs < bucket_count ? runs : bucket_count;
   int run = (int)((bucket_count + runs - 1) / runs);
-  while (run > 1 && fixed + run * a_bucket > 200 * 1024) run = (run + 1) / 2;
-  const size_t smem = fixed + run * a_bucket;
+  while (run > 1 && shared_of(run) > 200 * 1024) run = (run + 1) / 2;
+  const size_t smem = shared_of(run);
   LSA_REQUIRE(smem <= 227 * 1024, LSA_ERR_UNSUPPORTED);
   const dim3 grid((unsigned)blocks, (unsigned)((bucket_count + run - 1) / run));
   if (key_dtype == LSA_DTYPE_F32) {

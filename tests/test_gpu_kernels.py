@@ -316,6 +316,18 @@ def test_bucket_table_of_ragged_blocks(ops, G, P, pool, count, cap):
         assert np.array_equal(sums.cpu().numpy()[row], acc)
 
 
+def test_bucket_table_of_the_widest_keys(ops):
+    """One bucket whose sums and norm are all of a CTA's shared memory, as this call has always taken: 58,111 dims."""
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    keys = torch.randn(3, 58111, generator=gen, device="cuda")
+    members, sizes, sums, cent, _, status = ops.bucket_table(keys, torch.zeros(1, 3, device="cuda", dtype=torch.int64), 1, 1, 4)
+    assert members.tolist() == [[0, 1, 2, -1]] and sizes.tolist() == [3] and not int(status)
+    assert torch.equal(sums[0], (keys[0] + keys[1]) + keys[2])
+    assert (cent[0].norm() - 1).abs() <= 1e-3  # (58,111 squares added one by one: 58,111 * 2^-24 of the sum at most)
+    with pytest.raises(ValueError):
+        ops.bucket_table(torch.zeros(3, 58112, device="cuda"), torch.zeros(1, 3, device="cuda", dtype=torch.int64), 1, 1, 4)
+
+
 def test_bucket_table_is_bit_exact(ops, oracle):
     for name, (pool, bucket, cap, block) in {"flat_small": (4, 8, 16, 64), "flat_c1like": (16, 64, 128, 512)}.items():
         g = golden(name)
