@@ -29,6 +29,11 @@ struct ExpandParams {
   bool keeps_all;        // no owner range and no dealt granules: every id is kept
 };
 
+// A row's own budget, or the call's. (A row with less than nothing to spend, or before position 0, has an empty list.)
+__device__ __forceinline__ int budget(const int32_t *rows, int64_t r, int most) {
+  return rows ? max(0, min(rows[r], most)) : most;
+}
+
 // Whether this caller keeps an id: inside its contiguous range and, when the cache is dealt out in granules of
 // positions round-robin over `world` ranks, in one of its granules.
 __device__ __forceinline__ bool owned(const ExpandParams &p, int64_t id) {
@@ -70,8 +75,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) expand_kernel(ExpandParams 
   const int64_t pos = p.positions[r];
   const int64_t request = p.row_request ? p.row_request[r] : 0;
   const int32_t *table = p.page_table ? p.page_table + request * p.page_table_stride : nullptr;
-  const int row_p = p.row_top_p ? min(p.row_top_p[r], p.top_p) : p.top_p;
-  const int row_k = p.row_top_k ? min(p.row_top_k[r], p.top_k) : p.top_k;
+  const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
   const unsigned below = (1u << lane) - 1;
@@ -190,8 +194,7 @@ __global__ void __launch_bounds__(kRunThreads) expand_run_kernel(ExpandParams p)
   const int64_t pos = p.positions[r];
   const int64_t request = p.row_request ? p.row_request[r] : 0;
   const int32_t *table = p.page_table ? p.page_table + request * p.page_table_stride : nullptr;
-  const int row_p = p.row_top_p ? min(p.row_top_p[r], p.top_p) : p.top_p;
-  const int row_k = p.row_top_k ? min(p.row_top_k[r], p.top_k) : p.top_k;
+  const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
   int all = 0, bad = 0;
@@ -260,10 +263,10 @@ __global__ void __launch_bounds__(kRunThreads) expand_run_kernel(ExpandParams p)
   }
   int total = min(all, row_k);
   if (!(p.flags & LSA_EXPAND_NO_LOCAL)) {
-    const int in_window = (int)(pos + 1 - window_start);
+    const int in_window = (int)max((int64_t)0, pos + 1 - window_start);
     for (int i = tid; i < in_window; i += kRunThreads) out[total + i] = stored_id(p, table, window_start + i);
     total += in_window;
-    const int sinks = (int)min((int64_t)p.sink, min(window_start, pos + 1));
+    const int sinks = (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
     for (int i = tid; i < sinks; i += kRunThreads) out[total + i] = stored_id(p, table, i);
     total += sinks;
   }
@@ -294,8 +297,7 @@ __global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams 
   const int64_t pos = p.positions[r];
   const int64_t request = p.row_request ? p.row_request[r] : 0;
   const int32_t *table = p.page_table ? p.page_table + request * p.page_table_stride : nullptr;
-  const int row_p = p.row_top_p ? min(p.row_top_p[r], p.top_p) : p.top_p;
-  const int row_k = p.row_top_k ? min(p.row_top_k[r], p.top_k) : p.top_k;
+  const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
   const unsigned below = (1u << lane) - 1;
@@ -371,10 +373,10 @@ __global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams 
   }
   int total = min(start_s[row_p], row_k);
   if (!(p.flags & LSA_EXPAND_NO_LOCAL)) {
-    const int in_window = (int)(pos + 1 - window_start);
+    const int in_window = (int)max((int64_t)0, pos + 1 - window_start);
     for (int i = tid; i < in_window; i += kWideThreads) out[total + i] = stored_id(p, table, window_start + i);
     total += in_window;
-    const int sinks = (int)min((int64_t)p.sink, min(window_start, pos + 1));
+    const int sinks = (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
     for (int i = tid; i < sinks; i += kWideThreads) out[total + i] = stored_id(p, table, i);
     total += sinks;
   }
@@ -410,8 +412,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
   const int64_t pos = p.positions[r];
   const int64_t request = p.row_request ? p.row_request[r] : 0;
   const int32_t *table = p.page_table ? p.page_table + request * p.page_table_stride : nullptr;
-  const int row_p = p.row_top_p ? min(p.row_top_p[r], p.top_p) : p.top_p;
-  const int row_k = p.row_top_k ? min(p.row_top_k[r], p.top_k) : p.top_k;
+  const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
   const unsigned below = (1u << lane) - 1;
@@ -526,10 +527,10 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
   int total = min(all, row_k);
   const int gtid = cta * kClusterThreads + tid, gthreads = kClusterCtas * kClusterThreads;
   if (!(p.flags & LSA_EXPAND_NO_LOCAL)) {
-    const int in_window = (int)(pos + 1 - window_start);
+    const int in_window = (int)max((int64_t)0, pos + 1 - window_start);
     for (int i = gtid; i < in_window; i += gthreads) out[total + i] = stored_id(p, table, window_start + i);
     total += in_window;
-    const int sinks = (int)min((int64_t)p.sink, min(window_start, pos + 1));
+    const int sinks = (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
     for (int i = gtid; i < sinks; i += gthreads) out[total + i] = stored_id(p, table, i);
     total += sinks;
   }

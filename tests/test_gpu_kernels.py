@@ -236,6 +236,25 @@ def test_lists_over_narrow_and_wide_buckets_are_the_oracles(ops, oracle, cap, m,
             assert np.array_equal(lists[r].cpu().numpy()[:int(lengths[r])], ids[mine])
 
 
+@pytest.mark.parametrize("rows,cap,top_p", [(70, 16, 40), (70, 65, 20), (70, 100, 90), (5, 64, 40), (5, 1280, 40)])
+def test_rows_before_the_first_position_and_empty_budgets_have_empty_lists(ops, rows, cap, top_p):
+    """Every form of the expansion (a warp, a CTA or a cluster a row): nothing is listed, and nothing written outside the row."""
+    m, top_k, sink, window = 100, 500, 4, 32
+    members = cuda(np.arange(m * cap, dtype=np.int32).reshape(m, cap))
+    picked = cuda(np.stack([np.random.default_rng(r).permutation(m)[:top_p] for r in range(rows)]).astype(np.int32))
+    width = top_k + window + sink
+    for position, p_row, k_row in ((-1, 9, 9), (-5, 9, 9), (-1000, 9, 9), (3000, 9, -5), (3000, -3, 9), (3000, 0, 0)):
+        positions = torch.full((rows,), position, device="cuda", dtype=torch.int64)
+        budgets = [torch.full((rows,), x, device="cuda", dtype=torch.int32) for x in (p_row, k_row)]
+        room = torch.full((rows + 8, width), 123, device="cuda", dtype=torch.int32)
+        lengths, status = (torch.zeros(n, device="cuda", dtype=torch.int32) for n in (rows, 1))
+        ops.expand(picked, positions, members, top_k, sink, window, *budgets, outs=(room[4:-4], lengths, status))
+        local = min(max(position + 1, 0), window + sink)
+        assert (lengths == local).all() and (room[:4] == 123).all() and (room[-4:] == 123).all()
+        want = [*range(position + 1 - window, position + 1), *range(sink)][:local]
+        assert all(row == want + [-1] * (width - local) for row in room[4:-4].tolist())
+
+
 def test_linear_layers_over_a_few_rows(ops):
     """The decode-row maps: heads summed or read side by side, GELU or not, unit rows or not, against fp32 torch on
     the same bf16 values (the hidden layer of the two-layer map is rounded to bf16, as the batched map rounds it)."""
