@@ -455,6 +455,16 @@ int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_
                     int64_t kv_head_stride, int64_t first_position, int window, int sink, float scale, float *out_f32,
                     float *lse, int flags, int32_t *status, void *stream);
 
+/* The output `in` of an lsa_band_attend call whose window reaches back to position 0 (a dense causal read), rounded to bf16 and / or
+ * as it is.
+ * In a tile of rows a later key weighs zero, which a value that is not finite turns into NaN: rows that are not finite are
+ * read again, key by key, over the keys up to their own, so that such a value reaches the rows that read it and no others.
+ * out_bf16, out_f32 [R, Hq, dh], one of them may be NULL (out_f32 may be `in`); the other arguments are that call's. */
+int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride,
+                   int64_t q_head_stride, const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv,
+                   int64_t kv_row_stride, int64_t kv_head_stride, int64_t first_position, float scale,
+                   uint16_t *out_bf16, float *out_f32, void *stream);
+
 /* Gather-sparse attention over a shared latent cache (the MLA form): all Hq heads of a row attend over the SAME
  * listed latent rows; a key is the whole row (dk dims, rope part last), a value its first dv dims, and q holds the
  * absorbed queries (the key up-projection folded into them), so no per-head key is ever materialised.

@@ -216,6 +216,70 @@ __global__ void band_attend_kernel(BandParams p) {
   }
 }
 
+struct RoundParams {
+  const float *in;
+  const uint16_t *q, *k, *v;
+  uint16_t *out_bf16;
+  float *out_f32;
+  int64_t R, n_keys, first_position, q_row_stride, q_head_stride, kv_row_stride, kv_head_stride;
+  int Hq, group;
+  float scale_log2;
+};
+
+// A dense causal read on its way out (rounded to bf16, or as it is), a warp a (row, head). In a tile of 128 rows a key after a row weighs zero, and zero
+// times a value that is not finite is not a number: a row of the tile that holds one is read again here, key by key, over the
+// keys up to its own alone (what a list would name). Memory bounds the rows that are finite, all of them as a rule (six
+// bytes a dim, what the copy to bf16 in its place moved).
+template <int DH>
+__global__ void __launch_bounds__(256) band_round_kernel(RoundParams p) {
+  constexpr int PER = DH / 32;  // dims a lane holds
+  const int lane = lane_id();
+  const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (item >= p.R * p.Hq) return;
+  float x[PER];
+  bool finite = true;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) x[c] = p.in[item * DH + lane * PER + c], finite = finite && isfinite(x[c]);
+  if (!__all_sync(0xffffffffu, finite)) {
+    const int64_t r = item / p.Hq;
+    const int head = (int)(item - r * p.Hq), h = head / p.group;
+    const uint16_t *q = p.q + r * p.q_row_stride + (int64_t)head * p.q_head_stride + lane * PER;
+    const uint16_t *k = p.k + (int64_t)h * p.kv_head_stride + lane * PER, *v = p.v + (int64_t)h * p.kv_head_stride + lane * PER;
+    float m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int c = 0; c < PER; ++c) x[c] = 0.0f;
+    const int64_t end = min(p.n_keys, p.first_position + r + 1);
+    for (int64_t j = 0; j < end; ++j) {
+      float s = 0.0f;
+#pragma unroll
+      for (int c = 0; c < PER; ++c)
+        s = fmaf(bf16_bits_to_float(q[c]), bf16_bits_to_float(k[j * p.kv_row_stride + c]), s);
+      s = warp_sum(s) * p.scale_log2;
+      const float m_new = fmaxf(m, s), m_safe = m_new == -INFINITY ? 0.0f : m_new;
+      const float alpha = exp2f(m - m_safe), e = exp2f(s - m_safe);
+      m = m_new;
+      l = fmaf(l, alpha, e);
+#pragma unroll
+      for (int c = 0; c < PER; ++c) x[c] = fmaf(e, bf16_bits_to_float(v[j * p.kv_row_stride + c]), x[c] * alpha);
+    }
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+    for (int c = 0; c < PER; ++c) x[c] *= inv;
+  }
+  const int64_t at = item * DH + lane * PER;
+  if (p.out_f32) {
+#pragma unroll
+    for (int c = 0; c < PER; ++c) p.out_f32[at + c] = x[c];
+  }
+  if (p.out_bf16 && ((uintptr_t)p.out_bf16 & 3) == 0) {
+#pragma unroll
+    for (int c = 0; c < PER; c += 2) *reinterpret_cast<uint32_t *>(p.out_bf16 + at + c) = pack_bf16x2(x[c], x[c + 1]);
+  } else if (p.out_bf16) {
+#pragma unroll
+    for (int c = 0; c < PER; ++c) p.out_bf16[at + c] = float_to_bf16_bits(x[c]);
+  }
+}
+
 int launch_band_attend_tc(const uint16_t *q, int64_t R, int Hq, int64_t q_row_stride, const uint16_t *k,
                           const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride, int64_t first_position,
                           int window, int sink, float scale, float *out, float *lse, bool two_term, int32_t *status,
@@ -280,6 +344,32 @@ LSA_API int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_
           cudaSuccess)
     return LSA_ERR_LAUNCH;
   kernel<<<grid, threads, smem, s>>>(p);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
+LSA_API int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride,
+                           int64_t q_head_stride, const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv,
+                           int64_t kv_row_stride, int64_t kv_head_stride, int64_t first_position, float scale,
+                           uint16_t *out_bf16, float *out_f32, void *stream) {
+  LSA_REQUIRE(in && q && k && v && (out_bf16 || out_f32), LSA_ERR_NULL);
+  LSA_REQUIRE(R >= 0 && Hq >= 1 && Hkv >= 1 && Hq % Hkv == 0 && n_keys >= 0 && first_position >= 0 && scale > 0.0f,
+              LSA_ERR_ARGUMENT);
+  LSA_REQUIRE(dh == 64 || dh == 128, LSA_ERR_UNSUPPORTED);
+  LSA_REQUIRE((R * Hq + 7) / 8 <= INT32_MAX, LSA_ERR_ARGUMENT);
+  if (R == 0) return LSA_OK;
+  lsa::RoundParams p;
+  p.in = in, p.q = q, p.k = k, p.v = v, p.out_bf16 = out_bf16, p.out_f32 = out_f32;
+  p.R = R, p.n_keys = n_keys, p.first_position = first_position;
+  p.q_row_stride = q_row_stride, p.q_head_stride = q_head_stride;
+  p.kv_row_stride = kv_row_stride, p.kv_head_stride = kv_head_stride;
+  p.Hq = Hq, p.group = Hq / Hkv;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  const unsigned grid = (unsigned)((R * Hq + 7) / 8);
+  if (dh == 128)
+    lsa::band_round_kernel<128><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+  else
+    lsa::band_round_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

@@ -63,6 +63,7 @@ SIGNATURES = {
     "lsa_sparse_attend_workspace_bytes": (_Z, [_L, _I, _I, _I]),
     "lsa_sparse_attend": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _L, _I, _L, _L, _P, _L, _P, _P, _P, _F, _I, _P, _P,
                                _P, _P, _Z, _P]),
+    "lsa_band_round": (_I, [_P, _P, _L, _I, _I, _L, _L, _P, _P, _L, _I, _L, _L, _L, _F, _P, _P, _P]),
     "lsa_band_attend": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _I, _L, _L, _L, _I, _I, _F, _P, _P, _I, _P, _P]),
     "lsa_sparse_attend_static_scratch_bytes": (_Z, []),
     "lsa_sparse_attend_static": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _L, _I, _L, _L, _P, _L, _P, _F, _I, _P, _P,

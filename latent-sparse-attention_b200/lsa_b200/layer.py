@@ -501,10 +501,13 @@ class FlatLayer:
             # lists' read, which this stands for, is closer to the sums in 64 bits than one rounded term a key.)
             whole = min(n, self._whole_until(index) - start)
             with probe.region("band"):
-                dense, dense_lse = self._partial(self._room, "dense", whole, dev)
-                ops.band_attend(rows[:whole], k, v, start, start + whole, 0, self.scale, out=dense, lse=dense_lse,
-                                status=self._attend_status, two_term=True)
-                out[:whole].copy_(dense)
+                partial, into = self._partial(self._room, "dense", whole, dev), out[:whole]
+                if not into.is_contiguous() or into.dtype not in (torch.bfloat16, torch.float32):
+                    into = partial[0]
+                ops.causal_attend(rows[:whole], k, v, start, self.scale, out=into, partial=partial,
+                                  status=self._attend_status)
+                if into is partial[0]:
+                    out[:whole].copy_(into)
             if whole == n:
                 return out
             self.prefill_rows(rows[whole:], start + whole, k, v, index, out[whole:], band, bucket_major)

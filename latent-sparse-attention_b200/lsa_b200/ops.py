@@ -741,6 +741,26 @@ def band_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_positio
     return out, lse
 
 
+def causal_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_position: int, scale: float,
+                  out: torch.Tensor | None = None, partial: tuple | None = None,
+                  status: torch.Tensor | None = None) -> torch.Tensor:
+    """The dense read of every key up to a row's own, for rows whose list would name them all: q [R, Hq, dh] at positions
+    first_position.., out [R, Hq, dh] bf16 (or fp32, where `out` is). As close to the sums in 64 bits as a list's read (the probabilities are two bf16
+    terms), and a value that is not finite reaches the rows that read it alone. `partial`: (fp32 [R, Hq, dh], [R, Hq]) to work
+    in."""
+    R, Hq, dh = q.shape
+    out = torch.empty(R, Hq, dh, device=q.device, dtype=torch.bfloat16) if out is None else out
+    if out.shape != (R, Hq, dh) or out.dtype not in (torch.bfloat16, torch.float32) or not out.is_contiguous():
+        raise ValueError(f"out must be a contiguous bfloat16 or float32 [{R}, {Hq}, {dh}]")
+    dense, lse = partial if partial is not None else (None, None)
+    dense, _ = band_attend(q, k, v, first_position, first_position + R, 0, scale, out=dense, lse=lse, status=status,
+                           two_term=True)
+    call("lsa_band_round", ptr(dense), ptr(q), R, Hq, dh, q.stride(0), q.stride(1), ptr(k), ptr(v), k.shape[0], k.shape[1],
+         k.stride(0), k.stride(1), first_position, float(scale), ptr(out) if out.dtype == torch.bfloat16 else None,
+         ptr(out) if out.dtype == torch.float32 else None, stream())
+    return out
+
+
 def lse_merge(parts: torch.Tensor, lses: torch.Tensor, out_dtype=torch.float32):
     """Merge [n, rows..., dh] partial outputs (fp32, or bf16 for fewer than 16 parts) by their [n, rows...]
     log-sum-exps."""

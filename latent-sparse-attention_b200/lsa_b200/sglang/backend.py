@@ -309,11 +309,9 @@ def save(backend: Any, layer: Any, k: torch.Tensor, v: torch.Tensor, forward_bat
 def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, layer: Any, indexer: Any,
                forward_batch: Any) -> torch.Tensor | None:
     """A prefill batch with prompts that start in it: the rows that read every key up to their own take the dense causal
-    read of the batch's own keys and values (the probabilities as two bf16 terms: no further from the sums in 64 bits than the
-    lists' read), the others their lists. None where no row does, where the pool does not
-    hold what the batch hands over (another dtype), or where the lists' read takes what the dense one refuses (a scale that is
-    not positive). (As in `FlatLayer.prefill`'s band: a key after a row weighs zero in the
-    tile of 128 they share, so a value that is not finite reaches the rows of its tile before it too.)"""
+    read of the batch's own keys and values, the others their lists. None where no row does, where the pool does not hold
+    what the batch hands over (another dtype), or where the lists' read takes what the dense one refuses (a scale that is not
+    positive)."""
     lengths = list(forward_batch.extend_seq_lens_cpu)
     whole = indexer.whole_rows(forward_batch)
     heads, head_dim = layer.tp_q_head_num, layer.head_dim
@@ -334,7 +332,7 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     for count, dense in zip(lengths, whole, strict=True):
         if dense:
             piece = slice(first, first + dense)
-            out[piece] = ops.band_attend(q[piece], k[piece], v[piece], 0, dense, 0, layer.scaling, status=status, two_term=True)[0]
+            ops.causal_attend(q[piece], k[piece], v[piece], 0, layer.scaling, out=out[piece], status=status)
         if dense < count:
             rest.append(slice(first + dense, first + count))
         first += count

@@ -641,6 +641,31 @@ def test_sparse_attention_within_bf16_tolerance(ops, oracle, T, Hq, Hkv, dh, R, 
     assert np.abs(out16.float().cpu().numpy() - want).max() <= 2e-2
 
 
+@pytest.mark.parametrize("T,Hq,Hkv,dh,first", [(40, 4, 2, 64, 0), (300, 8, 1, 128, 0), (131, 6, 2, 128, 260)])
+def test_a_value_that_is_not_finite_reaches_the_rows_that_read_it(ops, T, Hq, Hkv, dh, first):
+    """Dense causal rows of both forms, in bf16 and fp32, to tensors that start anywhere: the gather's rows are not numbers, and
+    the rows before it are what they are without the value."""
+    n = first + T
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(n, Hq, Hkv, dh, 16, n))
+    q = q[first:]
+    ids = torch.arange(n, device="cuda", dtype=torch.int32).expand(T, n).contiguous()
+    lengths = first + 1 + torch.arange(T, device="cuda", dtype=torch.int32)
+    clean = ops.causal_attend(q, k, v, first, dh ** -0.5, out=torch.empty(T, Hq, dh, device="cuda"))
+    for x, at, what in ((v, first + 20, float("nan")), (v, n - 1, float("inf")), (k, first + 9, float("nan")), (k, n - 2, float("-inf"))):
+        kept = x[at, 0, 3].clone()
+        x[at, 0, 3] = what
+        want, _ = ops.sparse_attend(q, k, v, ids, lengths, dh ** -0.5)
+        room = torch.empty(q.numel() + 1, device="cuda", dtype=torch.bfloat16)
+        for out in (room[1:].view(T, Hq, dh), room[:-1].view(T, Hq, dh), torch.empty(T, Hq, dh, device="cuda")):
+            got = ops.causal_attend(q, k, v, first, dh ** -0.5, out=out)
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+            same = want.isfinite()
+            assert (got.float() - want.float())[same].abs().max() <= 2e-2 and not same.all()
+            before = clean[:at - first]  # (read again in fp32 where the tile holds the value: one rounding to bf16 apart)
+            assert ((got[:at - first].float() - before).abs() <= 2 ** -8 * before.abs() + 2 ** -13).all()
+        x[at, 0, 3] = kept
+
+
 @pytest.mark.parametrize("T,Hq,Hkv,dh", [(90, 8, 2, 64), (127, 16, 1, 128), (128, 8, 2, 128), (300, 5, 1, 64), (1153, 16, 2, 128)])
 def test_a_dense_read_is_as_close_to_64_bits_as_the_gather_of_every_key(ops, T, Hq, Hkv, dh):
     """Causal rows over clustered keys, probabilities as two bf16 terms, both forms. Two terms leave 2^-17 of a probability;

@@ -390,6 +390,13 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
         assert torch.equal(plain, want)
         gap = (got.float() - want.float()).abs()
         assert gap.max() <= 2e-2 and gap.mean() <= 2e-3, (gap.max(), gap.mean())
+    # values that are not finite reach the rows that read them, as through the lists
+    for at, what in (((200, 0, 5), np.nan), ((130, HKV - 1, 0), np.inf)):
+        kept = data[0][2][at]
+        data[0][2][at] = what
+        outs = [~served(how)[0][0].isfinite() for how in (True, False)]
+        data[0][2][at] = kept
+        assert torch.equal(*outs) and outs[0].any() and not outs[0][:at[0]].any()
     # what the lists' read takes and the dense one alone would refuse: tensors that start at an odd element, no positive scale
     for scale, shift in ((DH ** -0.5, 1), (-0.1, 0), (0.0, 0)):
         monkeypatch.setattr(backend, "ROWS", {})
