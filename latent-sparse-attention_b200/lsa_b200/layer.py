@@ -469,6 +469,12 @@ class FlatLayer:
         meet near three keys a query head of the group."""
         return self.design.bucket_size >= 3 * (self.heads // self.kv_heads)
 
+    def _bucket_takes(self, rows: torch.Tensor, out: torch.Tensor) -> bool:
+        """Whether wide buckets may be read bucket by bucket here: the gather, which serves them too, also writes fp32 and
+        takes query rows that are not 16-byte aligned."""
+        return self.design.bucket_cap <= 64 or (out.dtype == torch.bfloat16 and rows.stride(0) % 8 == 0
+                                                and rows.stride(1) % 8 == 0 and rows.data_ptr() % 16 == 0)
+
     def _bucket_workspace(self, rows: int, index: FlatIndex, device) -> torch.Tensor | None:
         """The bucket-major read's workspace, a partial output a (row, pick, head): gigabytes that the layer does not keep. It
         goes back to the allocator with the chunk and serves the next, and the other layers of a model. Sizes are cut to 32
@@ -523,7 +529,7 @@ class FlatLayer:
         partial = self._partial(self._room, "band", n, dev) if banded else None
         # (without the band the window and the sinks are in the lists, which only the gather path reads)
         workspace = None
-        if banded and bucket_major and self._reads_by_bucket and \
+        if banded and bucket_major and self._reads_by_bucket and self._bucket_takes(rows, out) and \
                 ops.bucket_attend_supported(rows, k, self.design.bucket_cap, self.design.top_p,
                                             not self.bucket_tensor_memory):
             workspace = self._bucket_workspace(n, index, dev)

@@ -200,3 +200,26 @@ def test_prompts_that_grow_hold_no_workspace_more(sizes, d_idx, monkeypatch):
         else:
             with pytest.raises(torch.OutOfMemoryError):
                 layers[0].prefill(q, k, v, chunk=chunk, out=out)
+
+
+def test_wide_buckets_write_fp32_and_take_queries_that_start_anywhere():
+    """What the gather of wide buckets takes, though the bucket-major read does not: an fp32 output, and query rows at an odd
+    pair of elements; the same read as the aligned bf16 call."""
+    from lsa_b200.layer import FlatDesign
+
+    T, Hq, Hkv = 3000, 8, 2
+    design = FlatDesign(pool_size=16, bucket_size=64, bucket_cap=128, cluster_block_size=512, top_p=4, top_k=512, sink_size=4,
+                        window_size=512)
+    layer, _ = _layer(Hq, Hkv, 128, 32, design, 2)
+    Q, K, V = (cuda(a, torch.bfloat16) for a in layer_inputs(T, Hq, Hkv, 128, 16, 2))
+    want = layer.prefill(Q, K, V, chunk=1024)
+    exact = torch.empty(T, Hq, 128, device="cuda")
+    layer.prefill(Q, K, V, chunk=1024, out=exact)
+    odd = torch.empty(Q.numel() + 2, device="cuda", dtype=torch.bfloat16)[2:].view(T, Hq, 128).copy_(Q)
+    shifted = layer.prefill(odd, K, V, chunk=1024)
+    err = (exact - want.float()).abs()
+    assert err.max() <= 2e-2 and err.mean() <= 2e-3 and not torch.equal(exact, exact.bfloat16().float())
+    # (rows that no tensor map can walk are mapped in fp32: another order of sums, another bucket where two scores nearly tie)
+    near = (shifted.float() - want.float()).abs().amax(dim=(1, 2)) <= 2e-2
+    assert near.float().mean() >= 0.98, near.float().mean()
+    layer.check()

@@ -264,3 +264,18 @@ def test_a_layers_buffers_are_one_a_shape_and_its_own_rooms_grow_by_halves():
         assert layer._room("lse", (rows, 4), torch.float32, "cpu").shape == (rows, 4)
     held = layer._buffers["lse", "rows", (4,), torch.float32, "cpu"]
     assert held[0].data_ptr() == whole.data_ptr() and sum(len(b) for b in held) < 5 * 3000
+
+
+def test_wide_buckets_go_to_the_gather_where_it_alone_takes_the_call():
+    """An fp32 output or query rows off 16 bytes: the gather's, for buckets of more than 64 members; narrow ones as ever."""
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    sizes = dict(pool_size=16, bucket_size=32, cluster_block_size=512, top_p=16, top_k=512, window_size=512)
+    takes = lambda cap: FlatLayer(FlatDesign(bucket_cap=cap, **sizes), torch.zeros(256, 32), torch.zeros(256, 32), 4, 2,
+                                  128)._bucket_takes
+    room = torch.zeros(3 * 4 * 128 + 16, dtype=torch.bfloat16)
+    start = (-room.data_ptr() // 2) % 8  # (the first element on a 16-byte boundary)
+    rows, odd = (room[start + at:start + at + 3 * 512].view(3, 4, 128) for at in (0, 2))
+    out = torch.zeros(3, 4, 128, dtype=torch.bfloat16)
+    assert takes(128)(rows, out) and not takes(128)(odd, out) and not takes(128)(rows, out.float())
+    assert takes(64)(odd, out.float())
