@@ -97,37 +97,51 @@ def test_prefill_from_pinned_host_memory_is_the_resident_prefill():
         assert torch.equal(out, want.cpu())
 
 
-@pytest.mark.parametrize("T,Hq,Hkv,dh,chunk,sizes", [
-    (1500, 8, 2, 128, 512, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=600,
-                                sink_size=4, window_size=150)),   # the key budget runs out first, inside a chunk
-    (1500, 8, 2, 128, 2048, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=640,
-                                 sink_size=0, window_size=128)),  # the picks run out first
-    (777, 5, 1, 64, 300, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=4096,
-                              sink_size=4, window_size=256)),     # every row reads everything
-    (700, 8, 2, 128, 256, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=256, top_p=64, top_k=600,
-                               sink_size=4, window_size=100)),    # a window short of a block: no row is read densely
+@pytest.mark.parametrize("T,Hq,Hkv,dh,chunk,until,sizes", [
+    (1500, 8, 2, 128, 512, 640, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=600,
+                                     sink_size=4, window_size=150)),  # the picks run out first, at 64 buckets of 16 a block
+    (1500, 8, 2, 128, 2048, 384, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=640,
+                                      sink_size=0, window_size=128)),  # and at 40, inside a chunk
+    (1500, 8, 2, 128, 300, 384, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=300,
+                                     sink_size=4, window_size=150)),  # the key budget first: 454 keys
+    (777, 5, 1, 64, 300, 1024, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=4096,
+                                    sink_size=4, window_size=256)),   # every row reads everything
+    (700, 8, 2, 128, 256, 0, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=256, top_p=64, top_k=600,
+                                  sink_size=4, window_size=100)),     # a window short of a block: no row is read densely
 ])
-def test_rows_that_read_everything_are_read_densely(oracle, T, Hq, Hkv, dh, chunk, sizes):
-    """Rows before a design leaves anything out take the dense causal read; from there on the lists: both equal the gather
-    of every row's whole list, and the boundary lies where the oracle's lists first leave a key out."""
+def test_rows_that_read_everything_are_read_densely(oracle, T, Hq, Hkv, dh, chunk, until, sizes, monkeypatch):
+    """Rows before a design leaves anything out take the dense causal read, and no others; from there on the lists: both equal
+    the gather of every row's whole list, and the boundary is the whole tile of 128 rows at or before the first row whose list,
+    the oracle's, leaves a key out."""
+    from lsa_b200 import ops
     from lsa_b200.layer import FlatDesign
 
     design = FlatDesign(**sizes)
     layer, _ = _layer(Hq, Hkv, dh, 64, design, T)
     q, k, v = layer_inputs(T, Hq, Hkv, dh, 16, T + 2)
     Q, K, V = (cuda(a, torch.bfloat16) for a in (q, k, v))
+    dense, read = [], ops.causal_attend
+
+    def recorded(rows, keys, values, first, *args, **kw):
+        dense.extend(range(first, first + rows.shape[0]))
+        return read(rows, keys, values, first, *args, **kw)
+
+    monkeypatch.setattr(ops, "causal_attend", recorded)
     out, index = layer.prefill(Q, K, V, chunk=chunk, return_index=True)
+    assert dense == list(range(min(T, until))) and layer._whole_until(index) == until
     gathered = layer.prefill(Q, K, V, chunk=chunk, band=False, bucket_major=False)
+    assert len(dense) == min(T, until)
     err = (out.float() - gathered.float()).abs()
     assert err.max() <= 2e-2 and err.mean() <= 2e-3, (err.max(), err.mean())
-    positions = np.arange(T)
-    _, lengths = layer.select(layer.index_queries(Q), cuda(positions), index)
-    everything = lengths.cpu().numpy() == positions + 1
-    until = layer._whole_until(index)
-    if design.window_size < design.cluster_block_size:
-        assert until == 0
-    else:
-        assert everything[:until].all() and (until >= T or not everything[until:].all())
+    index_q, index_k = layer.index_queries(Q).cpu().numpy(), index.index_keys.cpu().numpy()
+    buckets = oracle.build_buckets(index_k, design.pool_size, design.bucket_size, design.bucket_cap,
+                                   design.cluster_block_size)
+    _, lengths = oracle.read(index_q, np.arange(T), buckets, design.top_p, design.top_k, design.sink_size, design.window_size)
+    short = np.flatnonzero(lengths != np.arange(T) + 1)
+    first = int(short[0]) if len(short) else T
+    assert min(T, until) <= first
+    if until and until < T:  # (a window that reaches past the last block's start hides the boundary for a while)
+        assert first < until + design.window_size + design.cluster_block_size
     layer.check()
 
 
