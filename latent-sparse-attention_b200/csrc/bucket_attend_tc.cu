@@ -14,7 +14,7 @@
 //
 // Two warpgroups, each with tiles of its own (every other tile of the segment), its own query buffer and its own 128
 // columns of tensor memory (O takes the columns of S, which has been read by then). A warp copies, multiplies and writes
-// out ITS 32 rows, so between the hand-overs to the tensor cores nothing waits for another warp; lane 0 of a
+// out ITS 32 rows, so between the hand-overs to the tensor cores nothing waits for another warp; a
 // warpgroup's first warp issues its products. Two CTAs share an SM (buckets of up to 64 keys), so four tiles are under
 // way on it and fill one another's waits. What bounds it is the instruction stream around the products and the chain
 // copy - product - softmax - product - copy of a tile: 0.85 G warp instructions a launch of 8,192 rows x 64 picks x 40 heads,
@@ -216,13 +216,14 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(bar_w);  // this thread's part of the tile's queries is in place, and it has read its row of the last O
-      if (quarter == 0 && my_turn(0) && lane == 0) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
+      if (quarter == 0 && my_turn(0) && elect_one()) {  // S = Q K^T: 16 dims are 32 bytes further inside the swizzle atom
+        const uint64_t q_desc = smem_desc_sw128(buf), k_desc = smem_desc_sw128(base + kKOff);
 #pragma unroll
         for (int plane = 0; plane < 2; ++plane)
 #pragma unroll
           for (int s = 0; s < 4; ++s)
-            umma_bf16(tmem, smem_desc_sw128(buf + plane * kTcQPlane) + 2 * s,
-                      smem_desc_sw128(base + kKOff + plane * kPlane) + 2 * s, umma_idesc(n_keys), (plane | s) != 0);
+            umma_bf16(tmem, q_desc + (plane * kTcQPlane >> 4) + 2 * s, k_desc + (plane * kPlane >> 4) + 2 * s,
+                      umma_idesc(n_keys), (plane | s) != 0);
         umma_commit(bar_s);
       }
       __syncwarp();
@@ -322,10 +323,13 @@ __global__ void __launch_bounds__(kTcThreads, KEYS == 64 ? 2 : 1) bucket_attend_
       proxy_fence();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(bar_w);
-      if (quarter == 0 && my_turn(1) && lane == 0) {  // O = P V: 16 keys are 32 bytes along P's rows, 2,048 down V's planes
-        for (int s = 0; s < n_keys / 16; ++s)
-          umma_bf16(tmem, smem_desc_sw128(buf + (s >> 2) * kTcQPlane) + 2 * (s & 3),
-                    smem_desc_mn_sw128(base + kVOff + s * 2048, kPlane), umma_idesc(DH, true), s != 0);
+      if (quarter == 0 && my_turn(1) && elect_one()) {  // O = P V: 16 keys are 32 bytes along P's rows, 2,048 down V's planes
+        const uint64_t p_desc = smem_desc_sw128(buf), v_desc = smem_desc_mn_sw128(base + kVOff, kPlane);
+#pragma unroll
+        for (int s = 0; s < KEYS / 16; ++s)
+          if (16 * s < n_keys)
+            umma_bf16(tmem, p_desc + ((s >> 2) * kTcQPlane >> 4) + 2 * (s & 3), v_desc + (s * 2048 >> 4), umma_idesc(DH, true),
+                      s != 0);
         umma_commit(bar_o);
       }
       __syncwarp();

@@ -17,14 +17,16 @@
 //
 //   warps 0-3   a thread a head (lanes 0-15 of a warp; lanes 16-31 own the upper half of O): S out of tensor memory,
 //               masks, P into shared memory, the rare rescale of O, the normalised output
-//   warp 4      tensor-memory allocation; one lane issues S = Q K^T of every tile
-//   warp 9      one lane issues O += P V of every tile (a lane of its own: the two products belong to tiles in
-//               different stages, and one lane for both makes each wait for the other's loads)
+//   warp 4      tensor-memory allocation; issues S = Q K^T of every tile
+//   warp 9      issues O += P V of every tile (a warp of its own: the two products belong to tiles in
+//               different stages, and one warp for both makes each wait for the other's loads)
 //   warps 5-8   staging: a tile is up to 64 listed rows. 64 consecutive rows of the cache - what a bucket's pools
 //               and a window are made of - are ONE box of a tensor-map copy per plane, wherever they start;
 //               anything else is gathered with 16-byte asynchronous copies into the same swizzled planes
 //
-// The two stages run as two chains (load, S, softmax, O) that fill one another's waits. Every wait on an mbarrier is bounded; a wait that gives up raises the CTA's
+// The two stages run as two chains (load, S, softmax, O) that fill one another's waits. A tile is 36 first products of 32 cycles
+// and 8 second ones of 128. (8,192 rows at the end of 10M positions: 103.5 ms when a lane issued the products from a branch of its
+// own, 47 cycles a first one, and 96.0 since a warp does; 777 rows at 1M 13.7 and 12.9.) Every wait on an mbarrier is bounded; a wait that gives up raises the CTA's
 // abort flag and the status word, the roles drain, the tensor memory is freed and the CTA leaves.
 #include "latent_attend.cuh"
 #include "mma.cuh"
@@ -187,14 +189,8 @@ __global__ void __launch_bounds__(kLtThreads, 1)
   const uint32_t tmem_base = tmem_base_s;
   LT_TRACE(tid == 0, 10, 1);
 
-  // A wait of one thread: false (and the abort flag) when it gives up or the CTA has already given up elsewhere.
-  auto wait_one = [&](uint32_t b, uint32_t parity) {
-    bool done = false;
-    for (uint32_t spin = 0; spin < kLtSpinLimit && !done && !abort_s; ++spin) done = mbar_try(b, parity);
-    if (!done) abort_s = 1;
-    return done;
-  };
-  // The same for a warp whose lanes go on together.
+  // A wait of a warp whose lanes go on together: false (and the abort flag) when it gives up or the CTA has already given up
+  // elsewhere.
   auto wait = [&](uint32_t b, uint32_t parity) {
     bool done = false;
     for (uint32_t spin = 0; spin < kLtSpinLimit && !done && !abort_s; ++spin) done = mbar_try(b, parity);
@@ -202,10 +198,11 @@ __global__ void __launch_bounds__(kLtThreads, 1)
     if (!ok) abort_s = 1;
     return ok;
   };
-  // An issuing lane leaves only when its products are complete (bounded, but not cut short by the abort flag: the
+  // An issuing warp leaves only when its products are complete (bounded, but not cut short by the abort flag: the
   // tensor memory must not be freed under a running product).
   auto drain = [&](uint32_t b) {
-    umma_commit(b);
+    if (elect_one()) umma_commit(b);
+    __syncwarp();
     bool done = false;
     for (uint32_t spin = 0; spin < kLtSpinLimit && !done; ++spin) done = mbar_try(b, 0);
   };
@@ -344,58 +341,67 @@ __global__ void __launch_bounds__(kLtThreads, 1)
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------------------------------ S = Q K^T
-    if (lane == 0) {
-      bool alive = true;
-      for (int i = 0; alive; ++i) {
-        const int sb = i & 1;
-        alive = wait_one(bar(kFull, sb), (i >> 1) & 1);
-        if (!alive) break;
-        const bool last = info_s[sb][2] != 0, nothing = info_s[sb][3] != 0;
-        if (i >= 2) alive = wait_one(bar(kSEmpty, sb), ((i >> 1) - 1) & 1);
-        if (!alive) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        LT_TRACE(true, 3, i);
-        const uint32_t k_s = base + kLtKOff + sb * kLtStage;
+    // (the whole warp walks the tiles and one lane of it issues: descriptors stay in uniform registers)
+    const uint32_t s_col = __shfl_sync(0xffffffffu, tmem_base, 0) + kLtSCol;
+    const uint64_t q_desc = smem_desc_sw128(base), k_desc = smem_desc_sw128(base + kLtKOff);
+    bool alive = true;
+    for (int i = 0; alive; ++i) {
+      const int sb = i & 1;
+      alive = wait(bar(kFull, sb), (i >> 1) & 1);
+      if (!alive) break;
+      const bool last = __any_sync(0xffffffffu, info_s[sb][2] != 0), nothing = __any_sync(0xffffffffu, info_s[sb][3] != 0);
+      if (i >= 2) alive = wait(bar(kSEmpty, sb), ((i >> 1) - 1) & 1);
+      if (!alive) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      LT_TRACE(lane == 0, 3, i);
+      const uint64_t k_tile = k_desc + sb * (kLtStage >> 4);
+      if (elect_one()) {
+        if (!nothing) {
 #pragma unroll
-        for (int plane = 0; plane < kLtPlanes; ++plane)
+          for (int plane = 0; plane < kLtPlanes; ++plane)
 #pragma unroll
-          for (int s = 0; s < 4; ++s)
-            if (!nothing)
-              umma_bf16(tmem_base + kLtSCol + sb * kLtKeys, smem_desc_sw128(base + plane * kLtPlane) + 2 * s,
-                      smem_desc_sw128(k_s + plane * kLtPlane) + 2 * s, lt_idesc(kLtKeys, false), (plane | s) != 0);
+            for (int s = 0; s < 4; ++s)
+              umma_bf16(s_col + sb * kLtKeys, q_desc + (plane * kLtPlane >> 4) + 2 * s, k_tile + (plane * kLtPlane >> 4) + 2 * s,
+                        lt_idesc(kLtKeys, false), (plane | s) != 0);
+        }
         umma_commit(bar(kSFull, sb));
-        LT_TRACE(true, 4, i);
-        if (last) break;
       }
-      drain(drained_s);
+      __syncwarp();
+      LT_TRACE(lane == 0, 4, i);
+      if (last) break;
     }
+    drain(drained_s);
   } else if (warp == 9) {
     // ------------------------------------------------------------------------------------------ O += P V
-    if (lane == 0) {
-      bool alive = true;
-      for (int t = 0; alive; ++t) {
-        alive = wait_one(p_full, t & 1);
-        if (!alive) break;
-        const bool last = info_s[t & 1][2] != 0, nothing = info_s[t & 1][3] != 0;  // (read before the stage is given back)
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        LT_TRACE(true, 5, t);
-        const uint32_t v_s = base + kLtKOff + (t & 1) * kLtStage;
+    const uint32_t o_col = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint64_t p_desc = smem_desc_sw128(base + kLtPOff), v_desc = smem_desc_mn_sw128(base + kLtKOff, kLtPlane);
+    bool alive = true;
+    for (int t = 0; alive; ++t) {
+      alive = wait(p_full, t & 1);
+      if (!alive) break;
+      const int sb = t & 1;  // (read before the stage is given back)
+      const bool last = __any_sync(0xffffffffu, info_s[sb][2] != 0), nothing = __any_sync(0xffffffffu, info_s[sb][3] != 0);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      LT_TRACE(lane == 0, 5, t);
+      const uint64_t v_tile = v_desc + sb * (kLtStage >> 4);
+      if (elect_one()) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
+          if (!nothing) {
 #pragma unroll
-          for (int ks = 0; ks < kLtKeys / 16; ++ks)
-            if (!nothing)
-              umma_bf16(tmem_base + ((uint32_t)(h * 16) << 16), smem_desc_sw128(base + kLtPOff) + 2 * ks,
-                      smem_desc_mn_sw128(v_s + h * 4 * kLtPlane + ks * 2048, kLtPlane), lt_idesc(256, true),
-                      (t | ks) != 0);
-          umma_commit(bar(h == 0 ? kEmpty : kEmptyB, t & 1));
+            for (int ks = 0; ks < kLtKeys / 16; ++ks)
+              umma_bf16(o_col + ((uint32_t)(h * 16) << 16), p_desc + 2 * ks, v_tile + ((h * 4 * kLtPlane + ks * 2048) >> 4),
+                        lt_idesc(256, true), (t | ks) != 0);
+          }
+          umma_commit(bar(h == 0 ? kEmpty : kEmptyB, sb));
         }
         umma_commit(pv_done);
-        LT_TRACE(true, 6, t);
-        if (last) break;
       }
-      drain(drained_o);
+      __syncwarp();
+      LT_TRACE(lane == 0, 6, t);
+      if (last) break;
     }
+    drain(drained_o);
   } else {
     // ------------------------------------------------------------------------------------------ softmax and output
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);

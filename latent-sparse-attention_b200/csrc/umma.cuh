@@ -37,6 +37,15 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// One lane of a warp that is here whole. Products are issued by a whole warp with this around them, and not from a branch on
+// the lane: descriptors and addresses then stay in uniform registers, where a lane's own would be moved there for every
+// product (M = 64, N = 64, K = 16 issued back to back: 32 cycles a product this way, the tensor pipe's own, and 47 from a
+// lane's branch, measured alone; a warp that shares its scheduler with softmax warps took 100).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
