@@ -4,6 +4,7 @@
 // with fp32 accumulation in ascending input-dim order. This is the exact-arithmetic form; rows are read once and
 // the head sum never reaches memory.
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace lsa {
 
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(kMapThreads)
   }
 }
 
-// A few rows (a decode step): one CTA a row, its threads splitting the input dims, so the map of a single query
+// A few rows under a map that is not bf16 of 32, 64 or 128 columns: one CTA a row, its threads splitting the input dims, so the map of a single query
 // is not one thread block walking the whole contraction alone.
 constexpr int kRowThreads = 256;
 
@@ -115,32 +116,12 @@ __global__ void __launch_bounds__(kRowThreads)
   float acc[COLS];
 #pragma unroll
   for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
-  // A dim's weights are a row of W: taken 16 bytes at a time where they are whole bf16 rows (a thread's 64 loads of two
-  // bytes each, every one of a warp's lanes in a line of its own, were 30 of this kernel's 39 us for a row of 5,120 dims).
-  const bool runs = sizeof(TW) == 2 && W && d_idx == COLS && ((uintptr_t)W % 16) == 0;
   for (int k = tid; k < d_in; k += kRowThreads) {
-    uint4 w[COLS / 8];
-    if (runs) {
-#pragma unroll
-      for (int j = 0; j < COLS / 8; ++j) w[j] = reinterpret_cast<const uint4 *>(W + (int64_t)k * COLS)[j];
-    }
     const int kv = k / dh_used, c = k - kv * dh_used;
     const TX *src = x + row * x_row_stride + (int64_t)kv * group * x_head_stride + dh_off + c;
     float xs = 0.0f;
 #pragma unroll 8
     for (int g = 0; g < group; ++g) xs = __fadd_rn(xs, load_as_float<TX>(src, (int64_t)g * x_head_stride));
-    if (runs) {
-#pragma unroll
-      for (int j = 0; j < COLS / 8; ++j) {
-        const uint32_t w2[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc[8 * j + 2 * i] = fmaf(xs, __uint_as_float(w2[i] << 16), acc[8 * j + 2 * i]);
-          acc[8 * j + 2 * i + 1] = fmaf(xs, __uint_as_float(w2[i] & 0xFFFF0000u), acc[8 * j + 2 * i + 1]);
-        }
-      }
-      continue;
-    }
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
       if (j < d_idx) acc[j] = fmaf(xs, W ? load_as_float<TW>(W, (int64_t)k * d_idx + j) : (k == j ? 1.0f : 0.0f), acc[j]);
@@ -177,6 +158,96 @@ __global__ void __launch_bounds__(kRowThreads)
     const float v = total[tid] / norm_s;
     if (out_f32) out_f32[row * d_idx + tid] = v;
     if (out_bf16) out_bf16[row * d_idx + tid] = float_to_bf16_bits(v);
+  }
+}
+
+// The same for a bf16 map of 32, 64 or 128 columns: a CTA of 1,024 threads a row, so that the row's heads are one
+// round of loads and the map's 128 KB another, both on their way at once. COLS / 8 neighbouring lanes take a row of the map,
+// sixteen bytes each (a warp's load is 512 bytes in a run, where a lane that took a whole row of it touched a line a load),
+// against the head sums in shared memory. What bounds it is the latency of those two rounds and of three barriers: a row of
+// 5,120 dims to 64 takes 5.0 us (8.9 with a lane a row of the map), and 128 rows 5.4 (26.8 as one tile of the tensor-core map,
+// whose CTA walks the 5,120 dims alone).
+constexpr int kFewThreads = 1024, kFewHeld = 8, kFewRows = 128, kFewDims = 32 * 1024;
+
+template <typename TX, int COLS>
+__global__ void __launch_bounds__(kFewThreads, 1)
+    index_map_few_kernel(const TX *__restrict__ x, int group, int dh_off, int dh_used, int64_t x_row_stride,
+                         int64_t x_head_stride, const uint16_t *__restrict__ W, int d_in, int normalize,
+                         float *__restrict__ out_f32, uint16_t *__restrict__ out_bf16) {
+  constexpr int LANES = COLS / 8, DIMS = 32 / LANES, WARPS = kFewThreads / 32;  // lanes a map row, map rows a warp's load
+  extern __shared__ __align__(16) float sums_s[];  // [d_in] the row's heads added up
+  __shared__ float partial_s[WARPS][COLS];
+  const int64_t row = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int first = warp * DIMS + lane / LANES, cols = lane % LANES * 8;
+  const bool runs = ((uintptr_t)W % 16) == 0;
+  auto run = [&](int k) {
+    const uint16_t *w = W + (int64_t)k * COLS + cols;
+    if (runs) return *reinterpret_cast<const uint4 *>(w);
+    uint32_t w2[4];  // (a map that starts anywhere)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w2[j] = (uint32_t)w[2 * j] | (uint32_t)w[2 * j + 1] << 16;
+    return make_uint4(w2[0], w2[1], w2[2], w2[3]);
+  };
+  uint4 held[kFewHeld];
+#pragma unroll
+  for (int i = 0; i < kFewHeld; ++i) {
+    const int k = first + i * WARPS * DIMS;
+    held[i] = k < d_in ? run(k) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  for (int k = tid; k < d_in; k += kFewThreads) {
+    const int kv = k / dh_used, c = k - kv * dh_used;
+    const TX *src = x + row * x_row_stride + (int64_t)kv * group * x_head_stride + dh_off + c;
+    float sum = 0.0f;
+#pragma unroll 8
+    for (int g = 0; g < group; ++g) sum = __fadd_rn(sum, load_as_float<TX>(src, (int64_t)g * x_head_stride));
+    sums_s[k] = sum;
+  }
+  __syncthreads();
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  auto fold = [&](const uint4 w, float by) {
+    const uint32_t w2[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[2 * j] = fmaf(by, __uint_as_float(w2[j] << 16), acc[2 * j]);
+      acc[2 * j + 1] = fmaf(by, __uint_as_float(w2[j] & 0xFFFF0000u), acc[2 * j + 1]);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < kFewHeld; ++i) {
+    const int k = first + i * WARPS * DIMS;
+    if (k < d_in) fold(held[i], sums_s[k]);
+  }
+#pragma unroll 4
+  for (int k = first + kFewHeld * WARPS * DIMS; k < d_in; k += WARPS * DIMS) fold(run(k), sums_s[k]);
+#pragma unroll
+  for (int o = LANES; o < 32; o <<= 1)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  if (lane < LANES) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) partial_s[warp][cols + j] = acc[j];
+  }
+  __syncthreads();
+  if (warp > 0) return;
+  float v[COLS / 32], ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < COLS / 32; ++i) {
+    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) part[w & 3] += partial_s[w][lane + 32 * i];
+    v[i] = (part[0] + part[1]) + (part[2] + part[3]);
+    ss = fmaf(v[i], v[i], ss);
+  }
+  const float den = normalize ? fmaxf(sqrtf(warp_sum(ss)), 1e-12f) : 1.0f;
+#pragma unroll
+  for (int i = 0; i < COLS / 32; ++i) {
+    const int64_t at = row * COLS + lane + 32 * i;
+    const float unit = v[i] / den;
+    if (out_f32) out_f32[at] = unit;
+    if (out_bf16) out_bf16[at] = float_to_bf16_bits(unit);
   }
 }
 
@@ -227,6 +298,16 @@ static int launch_index_map(const void *x, int64_t rows, int heads, int group, i
     LSA_LAUNCH_CHECK();
     return LSA_OK;
   }
+  const int d_in = heads / group * dh_used;
+  if (rows <= kFewRows && sizeof(TW) == 2 && W && (d_idx == 32 || d_idx == 64 || d_idx == 128) && d_in <= kFewDims) {
+    auto few = d_idx == 32 ? index_map_few_kernel<TX, 32> : d_idx == 64 ? index_map_few_kernel<TX, 64> : index_map_few_kernel<TX, 128>;
+    if (!allow_shared(few, kFewDims * sizeof(float))) return LSA_ERR_LAUNCH;
+    few<<<(unsigned)rows, kFewThreads, (size_t)d_in * sizeof(float), s>>>(
+        (const TX *)x, group, dh_off, dh_used, x_row_stride, x_head_stride, (const uint16_t *)W, d_in, normalize, out_f32,
+        out_bf16);
+    LSA_LAUNCH_CHECK();
+    return LSA_OK;
+  }
   if (rows <= 32 && d_idx <= 128) {
     if (d_idx <= 64)
       index_map_rows_kernel<TX, TW, 64><<<(unsigned)rows, kRowThreads, 0, s>>>(
@@ -261,16 +342,20 @@ static int launch_index_map(const void *x, int64_t rows, int heads, int group, i
 // A linear layer over a FEW rows (a decode step's queries): out[r, n] = act(sum_k xs[r, k] Wt[n, k]), xs = the row's
 // heads summed (fp32, rounded once to bf16) or the row itself. A warp owns an output column and walks its weights once
 // for all rows; eight columns a CTA, so even a single row's map spreads over N / 8 CTAs instead of one.
-constexpr int kLinThreads = 256;
 constexpr int kLinMaxRows = 8;
+constexpr size_t kLinStaged = 96 * 1024;  // a row's heads are staged whole where they take no more than this
 // 16-byte runs of a column's weights a lane takes before anything else: 8 (2,048 weights a column), or 20 (5,120) for
 // the widest maps - the kernel is built for both, so that a narrow map does not carry the registers of a wide one.
 
-template <int kLinHeld>
-__global__ void __launch_bounds__(kLinThreads)
+// STAGED: a row's heads come into shared memory in one round of asynchronous copies and are added from there, in head order
+// (sixteen warps a CTA then: every CTA sums the heads for itself, 73 KB of them for 64 heads of 576 dims into 2,048 columns:
+// 7.8 us with two dependent rounds of a thread's own loads, 4.4 this way; 8 rows 30.6 and 21.7).
+template <int kLinHeld, bool STAGED>
+__global__ void __launch_bounds__(STAGED ? 512 : 256)
     rows_linear_kernel(const uint16_t *__restrict__ x, int rows, int heads, int64_t x_row_stride, int64_t x_head_stride,
                        int K, const uint16_t *__restrict__ Wt, int N, int gelu, float *__restrict__ out_f32,
                        uint16_t *__restrict__ out_bf16) {
+  constexpr int kLinThreads = STAGED ? 512 : 256;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint16_t *xs = reinterpret_cast<uint16_t *>(smem_raw);  // [rows][K] bf16
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -287,7 +372,31 @@ __global__ void __launch_bounds__(kLinThreads)
   wait_for_earlier_grids();
   // the head sum: a thread a pair of dims, 32 heads' loads in flight at a time, added in head order
   const bool pairs = (K % 2 == 0) && (x_row_stride % 2 == 0) && (x_head_stride % 2 == 0) && ((uintptr_t)x % 4 == 0);
-  if (heads == 1 && x_row_stride % 8 == 0 && ((uintptr_t)x % 16) == 0) {
+  if constexpr (STAGED) {
+    const int per_head = K / 8;
+    const uint32_t staged = smem_u32(xs + rows * K);
+    const uint32_t *staged_pairs = reinterpret_cast<const uint32_t *>(xs + rows * K);
+    for (int r = 0; r < rows; ++r) {
+      if (r > 0) __syncthreads();  // (the last row's heads have been added)
+      for (int e = tid; e < heads * per_head; e += kLinThreads) {
+        const int h = e / per_head;
+        cp_async_16(staged + e * 16, x + (int64_t)r * x_row_stride + (int64_t)h * x_head_stride + (e - h * per_head) * 8, 16);
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+      for (int k = tid; k < K / 2; k += kLinThreads) {
+        float lo = 0.0f, hi = 0.0f;
+#pragma unroll 16
+        for (int h = 0; h < heads; ++h) {
+          const uint32_t v = staged_pairs[h * (K / 2) + k];
+          lo = __fadd_rn(lo, __uint_as_float(v << 16));
+          hi = __fadd_rn(hi, __uint_as_float(v & 0xFFFF0000u));
+        }
+        reinterpret_cast<uint32_t *>(xs + r * K)[k] = pack_bf16x2(lo, hi);
+      }
+    }
+  } else if (heads == 1 && x_row_stride % 8 == 0 && ((uintptr_t)x % 16) == 0) {
     // nothing to sum: the rows are copied 16 bytes a thread, four loads in flight (K is a multiple of 8)
     const int per_row = K / 8, total = rows * per_row;
     for (int e0 = tid; e0 < total; e0 += 4 * kLinThreads) {
@@ -402,15 +511,20 @@ LSA_API int lsa_rows_linear(const uint16_t *x, int rows, int heads, int64_t x_ro
               LSA_ERR_ARGUMENT);
   LSA_REQUIRE(((uintptr_t)Wt % 16) == 0, LSA_ERR_ARGUMENT);
   LSA_REQUIRE(!(flags & LSA_ROWS_NORMALIZE) || out_f32, LSA_ERR_ARGUMENT);
-  const size_t smem = (size_t)rows * d_in * 2;
+  size_t smem = (size_t)rows * d_in * 2;
   constexpr size_t most = 160 * 1024;
   LSA_REQUIRE(smem <= most, LSA_ERR_UNSUPPORTED);
   if (rows == 0) return LSA_OK;
-  auto kernel = d_in <= 2048 ? lsa::rows_linear_kernel<8> : lsa::rows_linear_kernel<20>;
+  const size_t heads_bytes = (size_t)heads * d_in * 2;
+  const bool staged = heads > 1 && d_in <= 2048 && heads_bytes <= lsa::kLinStaged && smem + heads_bytes <= most &&
+                      x_row_stride % 8 == 0 && x_head_stride % 8 == 0 && ((uintptr_t)x % 16) == 0;
+  if (staged) smem += heads_bytes;
+  auto kernel = staged ? lsa::rows_linear_kernel<8, true>
+                       : d_in <= 2048 ? lsa::rows_linear_kernel<8, false> : lsa::rows_linear_kernel<20, false>;
   if (!lsa::allow_shared(kernel, most)) return LSA_ERR_LAUNCH;
-  const unsigned grid = (unsigned)((d_out + lsa::kLinThreads / 32 - 1) / (lsa::kLinThreads / 32));
+  const unsigned threads = staged ? 512 : 256, grid = (unsigned)((d_out + threads / 32 - 1) / (threads / 32));
   const bool unit = flags & LSA_ROWS_NORMALIZE;
-  lsa::launch(true, kernel, dim3(grid), dim3(lsa::kLinThreads), smem, (cudaStream_t)stream, x, rows,
+  lsa::launch(true, kernel, dim3(grid), dim3(threads), smem, (cudaStream_t)stream, x, rows,
               heads, x_row_stride, x_head_stride, d_in, Wt, d_out, flags & LSA_ROWS_GELU ? 1 : 0, out_f32,
               unit ? nullptr : out_bf16);
   LSA_LAUNCH_CHECK();
