@@ -1,7 +1,5 @@
 // Expansion: a row's picked buckets become its read list - members best bucket first, then the window, then
 // the sinks. Pure integer work, one warp a row, ballot-compacted so the order is the table's order.
-#include <cooperative_groups.h>
-
 #include "common.cuh"
 
 namespace lsa {
@@ -277,21 +275,28 @@ __global__ void __launch_bounds__(kRunThreads) expand_run_kernel(ExpandParams p)
   if (lane == 0 && bad && p.status) atomicAdd(p.status, bad);
 }
 
-// A few rows with long lists (a decode step): a whole CTA a row. The warps count every pick's ids at once, one warp
-// scans the counts into write offsets, and the warps write their picks' ids in place - the list is the same as the
-// one-warp kernel's, id for id. Only for callers that keep every id (no owner range, no dealt granules), so the ids
-// that count toward top_k are the ids written.
-constexpr int kWideThreads = 1024;
-constexpr int kWideMaxPicks = 1024;
+// A few rows with long lists (a decode step): `gridDim.x` CTAs a row. Members ascend, so how many of a pick count is found
+// without reading its row: a warp looks at 32 places spread over it and then at the places between two of them, two rounds of
+// loads for every pick at once. Every CTA finds all picks' counts and scans them - the same few loads, and nothing to exchange
+// - and writes its share of the list, a thread an id: the pick that owns it by bisection of the scanned counts. Only for
+// callers that keep every id, so the ids that count toward top_k are the ids written. What bounds it is four dependent rounds
+// of loads (positions and picks, the two of the counts, the ids). (A row of 83,000 ids from 128 picks of up to 1,280: 10.5 us in a
+// cluster of eight CTAs whose warps read a whole bucket each to count it, 9.6 this way, and in a decode step, where the members
+// come out of HBM, 15.6 and 9.6; 3,100 ids from 64 picks of 64 5.9 and 5.7, 64 rows of 9,200 from 32 picks of 512 7.6 and 6.9 in
+// a CTA a row that did the same.)
+constexpr int kSpreadThreads = 1024;
+constexpr int kSpreadMaxPicks = 1024;
+constexpr int kSpreadMaxCtas = 32;
+constexpr int kSpreadPicks = 4;  // picks a warp looks at side by side
 
-__global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams p) {
-  __shared__ int64_t bucket_s[kWideMaxPicks];
-  __shared__ int count_s[kWideMaxPicks];
-  __shared__ int start_s[kWideMaxPicks + 1];
+__global__ void __launch_bounds__(kSpreadThreads) expand_spread_kernel(ExpandParams p) {
+  __shared__ int64_t from_s[kSpreadMaxPicks];  // where the pick's run starts in the member table
+  __shared__ int count_s[kSpreadMaxPicks];
+  __shared__ int start_s[kSpreadMaxPicks + 1];  // and in the list
   __shared__ int bad_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int kWarps = kWideThreads / 32;
-  const int64_t r = blockIdx.x;
+  constexpr int kWarps = kSpreadThreads / 32;
+  const int64_t r = blockIdx.y;
   dependents_may_launch();
   wait_for_earlier_grids();
   const int64_t pos = p.positions[r];
@@ -300,10 +305,9 @@ __global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams 
   const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
-  const unsigned below = (1u << lane) - 1;
   if (tid == 0) bad_s = 0;
   __syncthreads();
-  for (int i = tid; i < row_p; i += kWideThreads) {
+  for (int i = tid; i < row_p; i += kSpreadThreads) {
     int64_t bucket = p.picked[r * p.top_p + i];
     if (bucket >= 0 && p.bucket_pages) {
       const int64_t slot = bucket / p.bucket_page_rows;
@@ -314,24 +318,47 @@ __global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams 
       bucket = -1;
       atomicAdd(&bad_s, 1);
     }
-    bucket_s[i] = bucket;
+    from_s[i] = bucket >= 0 ? bucket * p.cap : -1;
   }
   __syncthreads();
-  for (int pick = warp; pick < row_p; pick += kWarps) {
-    const int64_t bucket = bucket_s[pick];
-    int n = 0;
-    if (bucket >= 0)
-      for (int at0 = 0; at0 < p.cap; at0 += 128) {  // four loads in flight
-        int32_t ids[4];
+  const int step = (p.cap + 31) / 32;
+  auto before_window = [&](int32_t id) { return id >= 0 && id < window_start; };
+  for (int i0 = warp * kSpreadPicks; i0 < row_p; i0 += kWarps * kSpreadPicks) {
+    int64_t at[kSpreadPicks];
+    int32_t sample[kSpreadPicks], head[kSpreadPicks];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int at = at0 + 32 * j + lane;
-          ids[j] = at < p.cap ? p.members[bucket * p.cap + at] : LSA_PAD;
-        }
+    for (int j = 0; j < kSpreadPicks; ++j) {
+      at[j] = i0 + j < row_p ? from_s[i0 + j] : -1;
+      // the last place of each 32nd of the row, and the row's first 32 places
+      const int place = min(p.cap, (lane + 1) * step) - 1;
+      sample[j] = at[j] >= 0 && lane * step < p.cap ? p.members[at[j] + place] : LSA_PAD;
+      head[j] = at[j] >= 0 && lane < p.cap ? p.members[at[j] + lane] : LSA_PAD;
+    }
+    int whole[kSpreadPicks];  // 32nds that lie before the window
+    int32_t inner[kSpreadPicks];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) n += __popc(__ballot_sync(0xffffffffu, ids[j] >= p.sink && ids[j] < window_start));
+    for (int j = 0; j < kSpreadPicks; ++j) {
+      whole[j] = __popc(__ballot_sync(0xffffffffu, before_window(sample[j])));
+      const int place = whole[j] * step + lane;
+      inner[j] = at[j] >= 0 && lane < step && place < p.cap ? p.members[at[j] + place] : LSA_PAD;
+    }
+#pragma unroll
+    for (int j = 0; j < kSpreadPicks; ++j) {
+      int end = min(p.cap, whole[j] * step) + __popc(__ballot_sync(0xffffffffu, before_window(inner[j])));
+      for (int l0 = 32; l0 < step; l0 += 32) {  // (rows of more than 1,024 places)
+        const int place = whole[j] * step + l0 + lane;
+        const int32_t id = at[j] >= 0 && l0 + lane < step && place < p.cap ? p.members[at[j] + place] : LSA_PAD;
+        end += __popc(__ballot_sync(0xffffffffu, before_window(id)));
       }
-    if (lane == 0) count_s[pick] = n;
+      int first = __popc(__ballot_sync(0xffffffffu, head[j] >= 0 && head[j] < p.sink));
+      if (first == 32)  // (more sinks in the bucket than that: one after another)
+        while (first < end && p.members[at[j] + first] < p.sink) ++first;
+      first = min(first, end);
+      if (lane == 0 && i0 + j < row_p) {
+        count_s[i0 + j] = end - first;
+        if (at[j] >= 0) from_s[i0 + j] = at[j] + first;
+      }
+    }
   }
   __syncthreads();
   if (warp == 0) {
@@ -350,197 +377,41 @@ __global__ void __launch_bounds__(kWideThreads) expand_wide_kernel(ExpandParams 
     if (lane == 0) start_s[row_p] = carry;
   }
   __syncthreads();
-  for (int pick = warp; pick < row_p; pick += kWarps) {
-    const int64_t bucket = bucket_s[pick];
-    int written = start_s[pick];
-    if (bucket < 0) continue;
-    for (int at0 = 0; at0 < p.cap && written < row_k; at0 += 128) {
-      int32_t ids[4];
+  const int listed = min(start_s[row_p], row_k);
+  const int in_window = p.flags & LSA_EXPAND_NO_LOCAL ? 0 : (int)max((int64_t)0, pos + 1 - window_start);
+  const int sinks = p.flags & LSA_EXPAND_NO_LOCAL ? 0 : (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
+  const int total = listed + in_window + sinks;
+  const int gtid = blockIdx.x * kSpreadThreads + tid, gthreads = gridDim.x * kSpreadThreads;
+  constexpr int kAhead = 4;
+  for (int e0 = gtid; e0 < listed; e0 += kAhead * gthreads) {
+    int32_t ids[kAhead];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int at = at0 + 32 * j + lane;
-        ids[j] = at < p.cap ? p.members[bucket * p.cap + at] : LSA_PAD;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool counts = ids[j] >= p.sink && ids[j] < window_start;
-        const unsigned votes = __ballot_sync(0xffffffffu, counts);
-        const int at = written + __popc(votes & below);
-        if (counts && at < row_k) out[at] = stored_id(p, table, ids[j]);
-        written += __popc(votes);
+    for (int j = 0; j < kAhead; ++j) {
+      const int e = e0 + j * gthreads;
+      ids[j] = LSA_PAD;
+      if (e < listed) {
+        int lo = 0, hi = row_p;  // the last pick whose run starts at or before e
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (start_s[mid] <= e) lo = mid; else hi = mid;
+        }
+        ids[j] = p.members[from_s[lo] + (e - start_s[lo])];
       }
     }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int e = e0 + j * gthreads;
+      if (e < listed) out[e] = stored_id(p, table, ids[j]);
+    }
   }
-  int total = min(start_s[row_p], row_k);
-  if (!(p.flags & LSA_EXPAND_NO_LOCAL)) {
-    const int in_window = (int)max((int64_t)0, pos + 1 - window_start);
-    for (int i = tid; i < in_window; i += kWideThreads) out[total + i] = stored_id(p, table, window_start + i);
-    total += in_window;
-    const int sinks = (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
-    for (int i = tid; i < sinks; i += kWideThreads) out[total + i] = stored_id(p, table, i);
-    total += sinks;
-  }
+  for (int i = gtid; i < in_window; i += gthreads) out[listed + i] = stored_id(p, table, window_start + i);
+  for (int i = gtid; i < sinks; i += gthreads) out[listed + in_window + i] = stored_id(p, table, i);
   if (!(p.flags & LSA_EXPAND_NO_PAD))
-    for (int j = total + tid; j < p.width; j += kWideThreads) out[j] = LSA_PAD;
-  if (tid == 0) {
+    for (int j = total + gtid; j < p.width; j += gthreads) out[j] = LSA_PAD;
+  if (tid == 0 && blockIdx.x == 0) {
     p.lengths[r] = total;
     if (bad_s && p.status) atomicAdd(p.status, bad_s);
   }
-}
-
-// The same list from a CLUSTER of eight CTAs a row: a decode row of a long context lists hundreds of kilobytes of ids,
-// more than one SM moves in the time the rest of the step takes. Each CTA counts and writes an eighth of the picks;
-// the CTAs' totals cross through distributed shared memory, which is all the exchange a prefix sum over picks needs.
-constexpr int kClusterCtas = 8;
-constexpr int kClusterThreads = 512;
-
-__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
-    expand_cluster_kernel(ExpandParams p) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  constexpr int kMine = kWideMaxPicks / kClusterCtas;  // picks a CTA takes, at most
-  __shared__ int64_t bucket_s[kMine];
-  __shared__ int count_s[kMine];
-  __shared__ int start_s[kMine];
-  __shared__ int total_s, bad_s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int kWarps = kClusterThreads / 32;
-  const int cta = (int)cluster.block_rank();
-  const int64_t r = blockIdx.y;
-  dependents_may_launch();
-  wait_for_earlier_grids();
-  const int64_t pos = p.positions[r];
-  const int64_t request = p.row_request ? p.row_request[r] : 0;
-  const int32_t *table = p.page_table ? p.page_table + request * p.page_table_stride : nullptr;
-  const int row_p = budget(p.row_top_p, r, p.top_p), row_k = budget(p.row_top_k, r, p.top_k);
-  const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
-  int32_t *out = p.selected + r * p.width;
-  const unsigned below = (1u << lane) - 1;
-  const int share = (row_p + kClusterCtas - 1) / kClusterCtas;
-  const int first_pick = cta * share;
-  const int picks = max(0, min(share, row_p - first_pick));
-  if (tid == 0) bad_s = 0;
-  __syncthreads();
-  for (int i = tid; i < picks; i += kClusterThreads) {
-    int64_t bucket = p.picked[r * p.top_p + first_pick + i];
-    if (bucket >= 0 && p.bucket_pages) {
-      const int64_t slot = bucket / p.bucket_page_rows;
-      const int page = slot < p.bucket_max_pages ? p.bucket_pages[request * p.bucket_pages_stride + slot] : -1;
-      bucket = page >= 0 ? (int64_t)page * p.bucket_page_rows + bucket % p.bucket_page_rows : p.m;
-    }
-    if (bucket >= p.m) {
-      bucket = -1;
-      atomicAdd(&bad_s, 1);
-    }
-    bucket_s[i] = bucket;
-  }
-  __syncthreads();
-  // A warp's first pick stays in its registers between the count and the write (a row of up to 1,280 members: forty
-  // loads a lane, all in flight at once), so the step waits for memory once a pass instead of once a group of four.
-  constexpr int kHeld = 40;
-  const bool holds = p.cap <= 32 * kHeld && warp < picks;
-  int32_t held[kHeld];
-  if (holds) {
-    const int64_t bucket = bucket_s[warp];
-    int n = 0;
-#pragma unroll
-    for (int j = 0; j < kHeld; ++j) {
-      const int at = 32 * j + lane;
-      held[j] = bucket >= 0 && at < p.cap ? p.members[bucket * p.cap + at] : LSA_PAD;
-    }
-#pragma unroll
-    for (int j = 0; j < kHeld; ++j) n += __popc(__ballot_sync(0xffffffffu, held[j] >= p.sink && held[j] < window_start));
-    if (lane == 0) count_s[warp] = n;
-  }
-  for (int pick = holds ? warp + kWarps : warp; pick < picks; pick += kWarps) {
-    const int64_t bucket = bucket_s[pick];
-    int n = 0;
-    if (bucket >= 0)
-      for (int at0 = 0; at0 < p.cap; at0 += 128) {  // four loads in flight
-        int32_t ids[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int at = at0 + 32 * j + lane;
-          ids[j] = at < p.cap ? p.members[bucket * p.cap + at] : LSA_PAD;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) n += __popc(__ballot_sync(0xffffffffu, ids[j] >= p.sink && ids[j] < window_start));
-      }
-    if (lane == 0) count_s[pick] = n;
-  }
-  __syncthreads();
-  if (warp == 0) {  // this CTA's picks, scanned; its total for the others
-    int carry = 0;
-    for (int base = 0; base < picks; base += 32) {
-      const int v = base + lane < picks ? count_s[base + lane] : 0;
-      int incl = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      if (base + lane < picks) start_s[base + lane] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) total_s = carry;
-  }
-  cluster.sync();
-  int before = 0, all = 0;  // ids of the CTAs before this one, and of all of them
-  for (int c = 0; c < kClusterCtas; ++c) {
-    const int t = *cluster.map_shared_rank(&total_s, c);
-    if (c < cta) before += t;
-    all += t;
-  }
-  if (holds) {
-    int written = before + start_s[warp];
-#pragma unroll
-    for (int j = 0; j < kHeld; ++j) {
-      const bool counts = held[j] >= p.sink && held[j] < window_start;
-      const unsigned votes = __ballot_sync(0xffffffffu, counts);
-      const int at = written + __popc(votes & below);
-      if (counts && at < row_k) out[at] = stored_id(p, table, held[j]);
-      written += __popc(votes);
-    }
-  }
-  for (int pick = holds ? warp + kWarps : warp; pick < picks; pick += kWarps) {
-    const int64_t bucket = bucket_s[pick];
-    int written = before + start_s[pick];
-    if (bucket < 0) continue;
-    for (int at0 = 0; at0 < p.cap && written < row_k; at0 += 128) {
-      int32_t ids[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int at = at0 + 32 * j + lane;
-        ids[j] = at < p.cap ? p.members[bucket * p.cap + at] : LSA_PAD;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool counts = ids[j] >= p.sink && ids[j] < window_start;
-        const unsigned votes = __ballot_sync(0xffffffffu, counts);
-        const int at = written + __popc(votes & below);
-        if (counts && at < row_k) out[at] = stored_id(p, table, ids[j]);
-        written += __popc(votes);
-      }
-    }
-  }
-  // the window, the sinks and the padding: an eighth of each a CTA
-  int total = min(all, row_k);
-  const int gtid = cta * kClusterThreads + tid, gthreads = kClusterCtas * kClusterThreads;
-  if (!(p.flags & LSA_EXPAND_NO_LOCAL)) {
-    const int in_window = (int)max((int64_t)0, pos + 1 - window_start);
-    for (int i = gtid; i < in_window; i += gthreads) out[total + i] = stored_id(p, table, window_start + i);
-    total += in_window;
-    const int sinks = (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
-    for (int i = gtid; i < sinks; i += gthreads) out[total + i] = stored_id(p, table, i);
-    total += sinks;
-  }
-  if (!(p.flags & LSA_EXPAND_NO_PAD))
-    for (int j = total + gtid; j < p.width; j += gthreads) out[j] = LSA_PAD;
-  if (tid == 0) {
-    if (cta == 0) p.lengths[r] = total;
-    if (bad_s && p.status) atomicAdd(p.status, bad_s);
-  }
-  cluster.sync();  // nobody leaves while its total may still be read
 }
 
 }  // namespace lsa
@@ -597,18 +468,14 @@ LSA_API int lsa_expand_batched(const int32_t *picked, int64_t R, int top_p, cons
   const bool keeps_all = owner_world <= 1 && owner_first <= 0 && owner_end == INT64_MAX;
   p.keeps_all = keeps_all;
   p.cap_inverse = ((1u << 21) + (uint32_t)bucket_cap - 1) / (uint32_t)bucket_cap;
-  if (R <= 8 && keeps_all && top_p <= lsa::kWideMaxPicks && (int64_t)top_p * bucket_cap >= 32768) {
-    // a few rows with very long lists: a cluster of CTAs a row
-    const dim3 grid(lsa::kClusterCtas, (unsigned)R);
-    lsa::launch(true, lsa::expand_cluster_kernel, grid, dim3(lsa::kClusterThreads), 0, (cudaStream_t)stream, p);
-    LSA_LAUNCH_CHECK();
-    return LSA_OK;
-  }
-  if (keeps_all && top_p <= lsa::kWideMaxPicks &&
+  if (keeps_all && top_p <= lsa::kSpreadMaxPicks &&
       (int64_t)top_p * bucket_cap + window >= (R <= 8 ? 1024 : (R <= 64 ? 4096 : INT64_MAX))) {
-    // a decode step's long lists: one CTA a row
-    lsa::launch(R <= lsa::kChainedRows, lsa::expand_wide_kernel, dim3((unsigned)R), dim3(lsa::kWideThreads), 0,
-                (cudaStream_t)stream, p);
+    // a decode step's long lists: as many CTAs a row as give a thread two ids of half-full buckets, a wave of them at most
+    const int64_t wanted = ((int64_t)top_p * bucket_cap / 2 + window) / (2 * lsa::kSpreadThreads);
+    const int64_t most = lsa::sm_count() / R < lsa::kSpreadMaxCtas ? lsa::sm_count() / R : lsa::kSpreadMaxCtas;
+    const int64_t ctas = wanted < most ? wanted : most;
+    const dim3 grid((unsigned)(ctas < 1 ? 1 : ctas), (unsigned)R);
+    lsa::launch(R <= lsa::kChainedRows, lsa::expand_spread_kernel, grid, dim3(lsa::kSpreadThreads), 0, (cudaStream_t)stream, p);
     LSA_LAUNCH_CHECK();
     return LSA_OK;
   }

@@ -38,3 +38,33 @@ def test_heads_summed_in_shared_memory_are_the_heads_summed(rows, heads, d_in, d
     apart = torch.zeros(rows, heads, d_in + 2, device="cuda", dtype=torch.bfloat16)[..., :d_in].copy_(x)
     assert apart.stride(1) % 8
     assert torch.equal(ops.rows_linear(x, w, sum_heads=True), ops.rows_linear(apart, w, sum_heads=True))
+
+
+@pytest.mark.parametrize("cap,top_p,top_k,sink,window", [(1, 1024, 300, 4, 30), (31, 64, 4096, 40, 100), (33, 64, 500, 4, 64),
+                                                         (256, 16, 1 << 14, 4, 700), (1030, 40, 1 << 15, 50, 64), (1280, 128, 163840, 4, 5120)])
+def test_a_few_rows_list_what_many_rows_do(cap, top_p, top_k, sink, window):
+    """Rows expanded a few at a time (found by samples, spread over CTAs) against the same rows among many, id for id: windows that
+    cut buckets, buckets of sinks, empty and full ones, picks outside the table, budgets; positions and pages of slots."""
+    from lsa_b200 import ops
+
+    rng = np.random.default_rng(cap)
+    T, m, R = 40000, 1100 if cap < 64 else 150, 5
+    members = np.full((m, cap), -1, dtype=np.int32)
+    for b in range(m):
+        count = (0, cap, int(rng.integers(1, cap + 1)))[b % 3] if b > 4 else min(cap, 60)
+        members[b, :count] = np.sort(rng.choice(T, count, replace=False)) if b > 4 else np.arange(b, 5 * count, 5)[:count]
+    positions = np.array([0, 700, 20000, T - 1, 39000])
+    picked = np.stack([rng.permutation(m)[:top_p] for _ in range(R)]).astype(np.int32)
+    picked[:, :3] = np.array([0, 1, m + 3])[:min(3, top_p)]
+    row_p, row_k = rng.integers(0, top_p + 1, R).astype(np.int32), rng.integers(0, top_k + 1, R).astype(np.int32)
+    many = lambda x: None if x is None else cuda(np.concatenate([x] * 14))  # 70 rows: the other forms
+    table = rng.permutation(-(-(T + 64) // 64)).astype(np.int32)
+    for budgets in ((None, None), (row_p, row_k)):
+        for pages in (dict(), dict(page_table=cuda(table), page_size=64)):
+            for local in (True, False):
+                got = ops.expand(cuda(picked), cuda(positions), cuda(members), top_k, sink, window,
+                                 *(None if b is None else cuda(b) for b in budgets), local=local, **pages)
+                want = ops.expand(many(picked), many(positions), cuda(members), top_k, sink, window, *(many(b) for b in budgets),
+                                  local=local, **pages)
+                assert torch.equal(got[0], want[0][:R]) and torch.equal(got[1], want[1][:R])
+                assert 14 * int(got[2]) == int(want[2])
