@@ -116,6 +116,26 @@ inline void launch(bool chained, void (*kernel)(Params...), dim3 grid, dim3 bloc
   (void)cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
+// The same for a kernel of one parameter block, in clusters of `cluster` CTAs along y.
+template <typename P>
+inline void launch_clusters(bool chained, void (*kernel)(P), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                            const P &p, int cluster) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem, config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  config.attrs = attributes;
+  if (chained && chained_launches()) {
+    attributes[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attributes[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attributes[config.numAttrs].val.clusterDim.x = 1, attributes[config.numAttrs].val.clusterDim.z = 1;
+    attributes[config.numAttrs++].val.clusterDim.y = (unsigned)cluster;
+  }
+  (void)cudaLaunchKernelEx(&config, kernel, p);
+}
+
 // The dynamic shared memory a kernel may be launched with is an attribute of the KERNEL on the device. Every call sets it to
 // the same `most` that any call of that kernel takes, whatever its own launch uses: a host thread that set less would have
 // another thread's launch refused between that thread's call of this and its launch.

@@ -4,11 +4,15 @@
 // scan (one row, its buckets split over CTAs, lists merged afterwards) and a beam step of the tree (one row,
 // carried children beside a run of open rows). Selection is exact: a streaming top-k over 64-bit keys whose low
 // word breaks a score tie toward the lower id, so the result does not depend on the order keys were produced in.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "scan_select.cuh"
 #include "shape.cuh"
 
 namespace lsa {
+
+namespace cg = cooperative_groups;
 
 #ifdef LSA_SELECT_TRACE
 // Clock stamps of thread 0 of one CTA of a decode row's scan (row 0) and of its merge (row 1), for a build that asks.
@@ -361,6 +365,7 @@ struct SelectParams {
   const int32_t *pages;         // [R, max_pages] page of every page_rows ids of a row (-1 = none), or NULL
   int d, n_carried, keep, fanout, id_base, chunk, run_limit, max_pages, page_rows;
   ShapeTable shape;             // the vectors' shapes, row for row (floors NULL: none)
+  bool fold;                    // a row's splits are one cluster, whose first CTA folds their lists and writes the row
 };
 
 // RB rows a CTA. Shared memory: queries [RB][d], per-row key buffers [RB][keep_pow2 + chunk], histograms.
@@ -593,6 +598,50 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
     __syncthreads();
   }
 
+  if constexpr (RB == 1) {
+    if (p.fold) {
+      // The lists of a row's CTAs meet in the first one's registers, through distributed shared memory.
+      cg::cluster_group cluster = cg::this_cluster();
+      if (warp == 0) {
+        if (!sorted) warp_sort_descending(bufs, held);
+        for (int i = held + lane; i < kTopWarp; i += 32) bufs[i] = kEmptyKey;
+      }
+      cluster.sync();
+      if (split == 0) {
+        int64_t k[kTopLane];
+        const int64_t *theirs = cluster.map_shared_rank(bufs, warp < splits ? warp : 0);
+#pragma unroll
+        for (int j = 0; j < kTopLane; ++j) k[j] = warp < splits ? theirs[j * 32 + lane] : kEmptyKey;
+        block_top128(k, bufs + kTopWarp, kSelWarps, warp, lane);
+        if (warp == 0) {
+          int valid = 0;
+#pragma unroll
+          for (int j = 0; j < kTopLane; ++j) {
+            bufs[j * 32 + lane] = k[j];
+            valid += k[j] != kEmptyKey;
+          }
+          valid = min(warp_sum_int(valid), my_keep_all);
+          if (lane == 0) block_counter = valid;
+        }
+        __syncthreads();
+        held = block_counter;
+        for (int i = tid; i < p.keep; i += kSelThreads) {
+          const int64_t key = i < held ? bufs[i] : kEmptyKey;
+          if (p.keys_out) p.keys_out[row0 * p.keep + i] = key;
+          if (p.ids_out) p.ids_out[row0 * p.keep + i] = key == kEmptyKey ? LSA_PAD : key_id(key);
+        }
+        if (p.carried_out) {
+          for (int e = tid; e < p.keep * p.fanout; e += kSelThreads) {
+            const int i = e / p.fanout, c = e - i * p.fanout;
+            p.carried_out[row0 * p.keep * p.fanout + e] =
+                i < held ? (int32_t)p.children[(int64_t)(key_id(bufs[i]) - p.id_base) * p.fanout + c] : LSA_PAD;
+          }
+        }
+      }
+      cluster.sync();  // nobody leaves while its list may still be read
+      return;
+    }
+  }
   if (warp < RB && my_row < p.R) {
     int64_t *buf = bufs + (size_t)warp * row_room;
     if (!sorted) warp_sort_descending(buf, held);
@@ -746,18 +795,12 @@ static int launch_select(SelectParams p, int splits, cudaStream_t s) {
   p.chunk = select_chunk(RB, p.keep, p.d, &smem);
   if (p.chunk == 0) return LSA_ERR_UNSUPPORTED;
   dim3 grid((unsigned)((p.R + RB - 1) / RB), (unsigned)splits);
-  if (p.shape.floors) {
-    if (!allow_shared(select_kernel<RB, true>, kSelectShared)) return LSA_ERR_LAUNCH;
-    launch(p.R <= kChainedRows, select_kernel<RB, true>, grid, dim3(kSelThreads), smem, s, p);
-    LSA_LAUNCH_CHECK();
-    return LSA_OK;
-  }
-  if (!allow_shared(select_kernel<RB, false>, kSelectShared)) return LSA_ERR_LAUNCH;
-  launch(p.R <= kChainedRows, select_kernel<RB, false>, grid, dim3(kSelThreads), smem, s, p);
+  auto kernel = p.shape.floors ? select_kernel<RB, true> : select_kernel<RB, false>;
+  if (!allow_shared(kernel, kSelectShared)) return LSA_ERR_LAUNCH;
+  launch_clusters(p.R <= kChainedRows, kernel, grid, dim3(kSelThreads), smem, s, p, p.fold ? splits : 1);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }
-
 
 // ---------------------------------------------------------------------------------------- flat prefill scan
 
@@ -1507,6 +1550,31 @@ static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, 
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }
+
+// Splits of a row that are folded in a cluster, at most: a warp a list; and only for a few rows. (One row's 1,024 buckets over 8
+// CTAs, top 128: 13.3 us with the merge a launch of its own, 11.6 folded; a beam level of 1,024 nodes with 32 times 64 children
+// 18.2 and 13.3. The clusters of 64 rows wait for SMs that are free together: 4 CTAs a row took 22.5 and 26.7; and clusters of
+// 16, beyond the portable size, took a batch of 8 rows from 14.9 to 25.7.)
+constexpr int kFoldSplits = kSelWarps;
+
+// The best p.keep of each row's candidates, the row's split over `splits` CTAs: folded by a cluster where its registers take
+// the lists, else written to the workspace and merged by a launch of their own.
+static int select_split(SelectParams p, int splits, int64_t *keys_out, int32_t *ids_out, void *workspace, cudaStream_t s) {
+  size_t smem = 0;
+  p.fold = splits > 1 && splits <= kFoldSplits && p.R <= kChainedRows && p.keep <= kTopWarp &&
+           select_chunk(1, p.keep, p.d, &smem) >= (1 + kSelWarps / 2) * kTopWarp;
+  if (splits == 1 || p.fold) {
+    p.keys_out = keys_out, p.ids_out = ids_out;
+    return launch_select<1>(p, splits, s);
+  }
+  const int64_t *children = p.children;
+  int32_t *carried_out = p.carried_out;
+  p.children = nullptr, p.carried_out = nullptr;
+  p.keys_out = (int64_t *)workspace, p.ids_out = nullptr;
+  const int rc = launch_select<1>(p, splits, s);
+  if (rc != LSA_OK) return rc;
+  return merge_lists((const int64_t *)workspace, splits, p.R, p.keep, keys_out, ids_out, children, p.fanout, carried_out, true, s);
+}
 }  // namespace lsa
 
 LSA_API int lsa_merge_candidates(const int64_t *keys_in, int parts, int64_t R, int top_p, int64_t *keys_out,
@@ -1539,16 +1607,7 @@ LSA_API int lsa_flat_select_decode(const float *queries, int64_t R, int d, const
   p.d = d;
   p.keep = top_p;
   p.run_limit = INT32_MAX;
-  if (splits == 1) {
-    p.keys_out = keys_out;
-    p.ids_out = picked_out;
-    return lsa::launch_select<1>(p, 1, (cudaStream_t)stream);
-  }
-  p.keys_out = (int64_t *)workspace;
-  int rc = lsa::launch_select<1>(p, splits, (cudaStream_t)stream);
-  if (rc != LSA_OK) return rc;
-  return lsa::merge_lists((const int64_t *)workspace, splits, R, top_p, keys_out, picked_out, nullptr, 0, nullptr, true,
-                          (cudaStream_t)stream);
+  return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 
 LSA_API int lsa_shaped_select_decode(const float *queries, int64_t R, int d, const float *centroids,
@@ -1569,15 +1628,7 @@ LSA_API int lsa_shaped_select_decode(const float *queries, int64_t R, int d, con
   p.queries = queries, p.vectors = centroids, p.vector_base = request_first, p.run_end = visible;
   p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = INT32_MAX;
   p.shape = table;
-  if (splits == 1) {
-    p.keys_out = keys_out, p.ids_out = picked_out;
-    return lsa::launch_select<1>(p, 1, (cudaStream_t)stream);
-  }
-  p.keys_out = (int64_t *)workspace;
-  int rc = lsa::launch_select<1>(p, splits, (cudaStream_t)stream);
-  if (rc != LSA_OK) return rc;
-  return lsa::merge_lists((const int64_t *)workspace, splits, R, top_p, keys_out, picked_out, nullptr, 0, nullptr, true,
-                          (cudaStream_t)stream);
+  return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 
 LSA_API int lsa_beam_step(const float *queries, int64_t R, int d, const float *vectors, int64_t N,
@@ -1637,16 +1688,7 @@ LSA_API int lsa_flat_select_paged(const float *queries, int64_t R, int d, const 
   p.d = d;
   p.keep = top_p;
   p.run_limit = INT32_MAX;
-  if (splits == 1) {
-    p.keys_out = keys_out;
-    p.ids_out = picked_out;
-    return lsa::launch_select<1>(p, 1, (cudaStream_t)stream);
-  }
-  p.keys_out = (int64_t *)workspace;
-  int rc = lsa::launch_select<1>(p, splits, (cudaStream_t)stream);
-  if (rc != LSA_OK) return rc;
-  return lsa::merge_lists((const int64_t *)workspace, splits, R, top_p, keys_out, picked_out, nullptr, 0, nullptr, true,
-                          (cudaStream_t)stream);
+  return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 
 LSA_API int lsa_shaped_select_paged(const float *queries, int64_t R, int d, const float *centroids, int64_t rows,
@@ -1669,15 +1711,7 @@ LSA_API int lsa_shaped_select_paged(const float *queries, int64_t R, int d, cons
   p.pages = pages, p.max_pages = max_pages, p.page_rows = page_rows;
   p.R = R, p.N = rows, p.d = d, p.keep = top_p, p.run_limit = INT32_MAX;
   p.shape = table;
-  if (splits == 1) {
-    p.keys_out = keys_out, p.ids_out = picked_out;
-    return lsa::launch_select<1>(p, 1, (cudaStream_t)stream);
-  }
-  p.keys_out = (int64_t *)workspace;
-  int rc = lsa::launch_select<1>(p, splits, (cudaStream_t)stream);
-  if (rc != LSA_OK) return rc;
-  return lsa::merge_lists((const int64_t *)workspace, splits, R, top_p, keys_out, picked_out, nullptr, 0, nullptr, true,
-                          (cudaStream_t)stream);
+  return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 
 LSA_API size_t lsa_beam_step_workspace_bytes(int64_t R, int keep, int splits) {
@@ -1708,15 +1742,14 @@ LSA_API int lsa_beam_step_split(const float *queries, int64_t R, int d, const fl
   p.run_first = open_first;
   p.run_end = open_end;
   p.carried = carried;
-  p.keys_out = (int64_t *)workspace;
+  p.children = children;
+  p.carried_out = carried_out;
   p.R = R;
   p.N = N;
   p.d = d;
   p.n_carried = n_carried;
   p.keep = keep;
+  p.fanout = fanout;
   p.run_limit = (int)N;
-  int rc = lsa::launch_select<1>(p, splits, (cudaStream_t)stream);
-  if (rc != LSA_OK) return rc;
-  return lsa::merge_lists((const int64_t *)workspace, splits, R, keep, keys_out, kept_out, children, fanout, carried_out,
-                          true, (cudaStream_t)stream);
+  return lsa::select_split(p, splits, keys_out, kept_out, workspace, (cudaStream_t)stream);
 }

@@ -330,11 +330,8 @@ class FlatLayer:
                                             status=self._scan_status, workspace=work, lengths=index.lengths,
                                             radius=index.radius)
             elif R <= 8 and row_p is None and d.top_p <= 128 and keys is None and b.bucket_centroids.shape[1] in (32, 64):
-                # A decode step: a CTA sorts a thousand candidates of one row in registers, and more are split over CTAs
-                # and merged (one row over 1,024 buckets: 32.1 us in the kernel whose CTA holds 16 rows, 16.7 in this one).
-                m = b.bucket_centroids.shape[0]
                 _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p,
-                                                   splits=1 if m <= 1024 else min(32, -(-m // 512)))
+                                                   splits=self._decode_splits(R, b.bucket_centroids.shape[0]))
             else:
                 _, picked = ops.flat_select(index_queries, b.bucket_centroids, visible, d.top_p, row_p, keys=keys,
                                             picked=picked)
@@ -560,6 +557,14 @@ class FlatLayer:
         lists, lengths = self._select(index_queries, positions, index, self._room, not banded, stop - 1)
         self.attend(rows, k, v, lists, lengths, out=out, lse=lse, init=init)
         return out
+
+    @staticmethod
+    def _decode_splits(rows: int, buckets: int) -> int:
+        """CTAs that a decode row's buckets are split over. A CTA sorts up to a thousand candidates of a row in registers; up to
+        4,096 go to the eight CTAs of a cluster, which fold their lists (one row over 1,024: 15.3 us in one CTA, 11.6 in eight;
+        over 4,096: 16.3 in 32 CTAs and a merge, 14.0 in eight), more to 32 CTAs and a merge, or 16 where there are several rows
+        (16,384 buckets: one row 18.8 us in 32; 8 rows 29.2 in 32, 20.5 in 16)."""
+        return 1 if buckets <= 512 else 8 if buckets <= 4096 else 32 if rows == 1 else 16
 
     def decode(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                splits: int = 8):

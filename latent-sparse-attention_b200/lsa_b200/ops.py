@@ -333,6 +333,12 @@ def _scan_samples(m: int, top_p: int, max_visible: int) -> bool:
     return m >= 1024 and factor * top_p * 512 >= 8 * widest
 
 
+def _split_launches(rows: int, splits: int, keep: int) -> int:
+    """Launches of a scan whose rows are split: the lists of up to 8 CTAs of 128 keys of a few rows are folded by a cluster,
+    others merged by a launch of their own."""
+    return 1 if splits <= 1 or (rows <= 8 and splits <= 8 and keep <= 128) else 2
+
+
 def flat_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, request_first: torch.Tensor | None,
                        visible: torch.Tensor, top_p: int, splits: int = 1, workspace: torch.Tensor | None = None):
     """Decode-form flat scan (src/lsa/sglang/index/selector.py:603-660): few rows, their buckets split over CTAs."""
@@ -346,7 +352,7 @@ def flat_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, req
     call("lsa_flat_select_decode", ptr(q), R, d, ptr(c), ptr(request_first), ptr(_as(visible, torch.int32)),
          top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
-         launches=1 if splits == 1 else 2)
+         launches=_split_launches(R, splits, top_p))
     return keys, picked
 
 
@@ -366,7 +372,7 @@ def flat_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, page
     call("lsa_flat_select_paged", ptr(q), R, d, ptr(c), c.shape[0], ptr(pages), pages.shape[1], page_rows,
          ptr(_as(counts, torch.int32)), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
-         launches=1 if splits == 1 else 2)
+         launches=_split_launches(R, splits, top_p))
     return keys, picked
 
 
@@ -449,7 +455,7 @@ def shaped_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, s
     call("lsa_shaped_select_decode", ptr(q), R, d, ptr(c), ptr(basis), ptr(variances), ptr(floor), basis.shape[1],
          float(shapes.deviations), ptr(request_first), ptr(_as(visible, torch.int32)), top_p, splits, ptr(keys),
          ptr(picked), ptr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0,
-         stream(), launches=1 if splits == 1 else 2)
+         stream(), launches=_split_launches(R, splits, top_p))
     return keys, picked
 
 
@@ -471,7 +477,7 @@ def shaped_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, sh
          basis.shape[1], float(shapes.deviations), ptr(pages), pages.shape[1], page_rows,
          ptr(_as(counts, torch.int32)), top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
-         launches=1 if splits == 1 else 2)
+         launches=_split_launches(R, splits, top_p))
     return keys, picked
 
 
@@ -547,7 +553,7 @@ def beam_step(index_queries: torch.Tensor, vectors: torch.Tensor, carried: torch
     call("lsa_beam_step_split", ptr(q), R, d, ptr(v), v.shape[0], ptr(carried), n_carried,
          ptr(_as(open_first, torch.int32)), ptr(_as(open_end, torch.int32)), keep, ptr(children),
          fanout, splits, ptr(kept), ptr(keys), ptr(carried_out), ptr(workspace) if need else None, need, stream(),
-         launches=1 if splits <= 1 else 2)
+         launches=_split_launches(R, splits, keep))
     return carried_out if children is not None else (kept, keys)
 
 

@@ -68,3 +68,31 @@ def test_a_few_rows_list_what_many_rows_do(cap, top_p, top_k, sink, window):
                                   local=local, **pages)
                 assert torch.equal(got[0], want[0][:R]) and torch.equal(got[1], want[1][:R])
                 assert 14 * int(got[2]) == int(want[2])
+
+
+@pytest.mark.parametrize("m,d,keep", [(3, 64, 1), (130, 32, 128), (1024, 64, 128), (5000, 64, 33), (9001, 128, 100)])
+def test_lists_folded_in_a_cluster_are_the_scan_s(m, d, keep):
+    """A row's candidates split over 2 to 8 CTAs against one CTA, key for key; rows that see few or none; and a level of a tree."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    q = torch.randn(5, d, device="cuda", generator=gen)
+    c = torch.randn(m, d, device="cuda", generator=gen).mul(8).round().div(8)
+    c[m // 2:] = c[:m - m // 2].clone()  # (ties)
+    visible = torch.tensor([m, m // 2, 1, 0, max(0, m - 1)], device="cuda", dtype=torch.int32)
+    want = ops.flat_select_decode(q, c, None, visible, keep, splits=1)
+    for splits in (2, 3, 7, 8):
+        got = ops.flat_select_decode(q, c, None, visible, keep, splits=splits)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    children = torch.randint(0, 1 << 20, (m, 5), device="cuda", generator=gen)
+    first, end = torch.zeros_like(visible), visible
+    for kids in (None, children):
+        want = ops.beam_step(q, c, None, first, end, keep, children=kids, splits=1)
+        for splits in (2, 8):
+            got = ops.beam_step(q, c, None, first, end, keep, children=kids, splits=splits)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) if kids is None else torch.equal(got, want)
+    distinct = torch.stack([torch.randperm(m, device="cuda", generator=gen)[:min(m, 40)] for _ in range(5)]).to(torch.int32)
+    none = torch.zeros_like(visible)
+    want = ops.beam_step(q, c, distinct, none, none, keep, splits=1)
+    got = ops.beam_step(q, c, distinct, none, none, keep, splits=8)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
