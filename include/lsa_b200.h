@@ -441,12 +441,12 @@ int lsa_sparse_attend_static(const uint16_t *q, int64_t R, int Hq, int dh, int64
  * The result is partial - normalised fp32 output and log-sum-exp - and is meant as lsa_sparse_attend's
  * init_out / init_lse, whose lists then hold only the selected keys (lsa_expand with LSA_EXPAND_NO_LOCAL).
  * Reference: the window and sink terms of keep_set (src/lsa/core/attention.py:49-58). sink <= 64.
- *   flags  0: heads of 128 dims packed densely and at least 128 rows go to the tensor-memory form - 128 rows of one
- *          head a CTA, both products on tcgen05 (the rows as M), K/V tiles streamed by tensor-map copies, the band
- *          walked twice (row maxima, then the sums) so the accumulator in tensor memory is never rescaled;
+ *   flags  0: heads of 128 dims packed densely and at least 128 rows go to the tensor-memory form - two tiles of 128 rows of
+ *          one head a CTA, both products on tcgen05 (the rows as M), K/V tiles streamed by tensor-map copies, and the
+ *          probabilities in tensor memory as two bf16 terms;
  *          LSA_BAND_WARP_MMA: always the warp-level form;
- *          LSA_BAND_TWO_TERM: the probabilities enter the second product as two bf16 terms (the value and what rounding
- *          left of it), for a read that stands for lsa_sparse_attend over every key up to a row's own
+ *          LSA_BAND_TWO_TERM: in the warp-level form too the probabilities enter the second product as two bf16 terms (the
+ *          value and what rounding left of it)
  *   status (may be NULL) is raised if a bounded on-chip wait of the tensor-memory form gives up */
 #define LSA_BAND_WARP_MMA 1
 #define LSA_BAND_TWO_TERM 2
@@ -464,6 +464,20 @@ int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq, int dh
                    int64_t q_head_stride, const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv,
                    int64_t kv_row_stride, int64_t kv_head_stride, int64_t first_position, float scale,
                    uint16_t *out_bf16, float *out_f32, void *stream);
+
+/* Dense attention of consecutive rows (row i at first_position + i, KV row p at position p) over every key up to a row's own,
+ * or, with `mask`, over those of them that its list names: what lsa_sparse_attend gives for such lists, on the tensor cores.
+ * Heads of 128 dims packed densely, 16-byte aligned rows and outputs (else LSA_ERR_UNSUPPORTED).
+ * Rows whose output is not finite are read again, key by key, so that a value that is not finite reaches the rows that read
+ * it and no others.
+ *   mask        [key tiles of 128][R][4] uint32, a bit a key (every tile up to the last row's position), or NULL
+ *   out_bf16, out_f32  [R, Hq, 128], one of them may be NULL
+ *   not_finite  one int32 of workspace
+ *   status      (may be NULL) is raised if a bounded on-chip wait gives up */
+int lsa_dense_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride, int64_t q_head_stride,
+                     const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride,
+                     int64_t kv_head_stride, int64_t first_position, const uint32_t *mask, float scale, uint16_t *out_bf16,
+                     float *out_f32, int32_t *not_finite, int32_t *status, void *stream);
 
 /* Gather-sparse attention over a shared latent cache (the MLA form): all Hq heads of a row attend over the SAME
  * listed latent rows; a key is the whole row (dk dims, rope part last), a value its first dv dims, and q holds the

@@ -6,6 +6,7 @@
 // on mma.m16n8k16 with the queries as M; softmax is online in fp32. The result is a PARTIAL read: normalised output
 // and log-sum-exp per (row, head), which lsa_sparse_attend takes as its starting state and extends with the
 // gathered keys.
+#include "band_attend.cuh"
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -226,6 +227,61 @@ struct RoundParams {
   float scale_log2;
 };
 
+// A (row, head) read key by key by a warp, a lane DH / 32 of its dims: the keys up to the row's own, or those of them that
+// `mask` (a bit a key, in tiles of 128 keys a row) names.
+template <int DH>
+__device__ __noinline__ void read_again(const RoundParams &p, int64_t item, const uint32_t *mask, float (&x)[DH / 32]) {
+  constexpr int PER = DH / 32;
+  const int lane = lane_id();
+  const int64_t r = item / p.Hq;
+  const int head = (int)(item - r * p.Hq), h = head / p.group;
+  const uint16_t *q = p.q + r * p.q_row_stride + (int64_t)head * p.q_head_stride + lane * PER;
+  const uint16_t *k = p.k + (int64_t)h * p.kv_head_stride + lane * PER, *v = p.v + (int64_t)h * p.kv_head_stride + lane * PER;
+  float m = -INFINITY, l = 0.0f;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) x[c] = 0.0f;
+  const int64_t end = min(p.n_keys, p.first_position + r + 1);
+  for (int64_t j = 0; j < end; ++j) {
+    if (mask && !((mask[((j >> 7) * p.R + r) * 4 + ((j >> 5) & 3)] >> (j & 31)) & 1u)) continue;
+    float s = 0.0f;
+#pragma unroll
+    for (int c = 0; c < PER; ++c)
+      s = fmaf(bf16_bits_to_float(q[c]), bf16_bits_to_float(k[j * p.kv_row_stride + c]), s);
+    s = warp_sum(s) * p.scale_log2;
+    const float m_new = fmaxf(m, s), m_safe = m_new == -INFINITY ? 0.0f : m_new;
+    const float alpha = exp2f(m - m_safe), e = exp2f(s - m_safe);
+    m = m_new;
+    l = fmaf(l, alpha, e);
+#pragma unroll
+    for (int c = 0; c < PER; ++c) x[c] = fmaf(e, bf16_bits_to_float(v[j * p.kv_row_stride + c]), x[c] * alpha);
+  }
+  const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) x[c] *= inv;
+}
+
+// The rows of a dense read whose output is not finite, read again: nothing but a look at a word where there are none. A key
+// that a row does not read weighs zero in its tile, and zero times a value that is not finite is not a number.
+__global__ void __launch_bounds__(256) dense_repair_kernel(RoundParams p, const uint32_t *mask, const int32_t *not_finite) {
+  if (*not_finite == 0) return;
+  const int lane = lane_id();
+  for (int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); item < p.R * p.Hq; item += (int64_t)gridDim.x * 8) {
+    const int64_t at = item * 128 + lane * 4;
+    bool finite = true;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      finite = finite && isfinite(p.out_bf16 ? bf16_bits_to_float(p.out_bf16[at + c]) : p.out_f32[at + c]);
+    if (__all_sync(0xffffffffu, finite)) continue;
+    float x[4];
+    read_again<128>(p, item, mask, x);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (p.out_bf16) p.out_bf16[at + c] = float_to_bf16_bits(x[c]);
+      if (p.out_f32) p.out_f32[at + c] = x[c];
+    }
+  }
+}
+
 // A dense causal read on its way out (rounded to bf16, or as it is), a warp a (row, head). In a tile of 128 rows a key after a row weighs zero, and zero
 // times a value that is not finite is not a number: a row of the tile that holds one is read again here, key by key, over the
 // keys up to its own alone (what a list would name). Memory bounds the rows that are finite, all of them as a rule (six
@@ -241,30 +297,7 @@ __global__ void __launch_bounds__(256) band_round_kernel(RoundParams p) {
 #pragma unroll
   for (int c = 0; c < PER; ++c) x[c] = p.in[item * DH + lane * PER + c], finite = finite && isfinite(x[c]);
   if (!__all_sync(0xffffffffu, finite)) {
-    const int64_t r = item / p.Hq;
-    const int head = (int)(item - r * p.Hq), h = head / p.group;
-    const uint16_t *q = p.q + r * p.q_row_stride + (int64_t)head * p.q_head_stride + lane * PER;
-    const uint16_t *k = p.k + (int64_t)h * p.kv_head_stride + lane * PER, *v = p.v + (int64_t)h * p.kv_head_stride + lane * PER;
-    float m = -INFINITY, l = 0.0f;
-#pragma unroll
-    for (int c = 0; c < PER; ++c) x[c] = 0.0f;
-    const int64_t end = min(p.n_keys, p.first_position + r + 1);
-    for (int64_t j = 0; j < end; ++j) {
-      float s = 0.0f;
-#pragma unroll
-      for (int c = 0; c < PER; ++c)
-        s = fmaf(bf16_bits_to_float(q[c]), bf16_bits_to_float(k[j * p.kv_row_stride + c]), s);
-      s = warp_sum(s) * p.scale_log2;
-      const float m_new = fmaxf(m, s), m_safe = m_new == -INFINITY ? 0.0f : m_new;
-      const float alpha = exp2f(m - m_safe), e = exp2f(s - m_safe);
-      m = m_new;
-      l = fmaf(l, alpha, e);
-#pragma unroll
-      for (int c = 0; c < PER; ++c) x[c] = fmaf(e, bf16_bits_to_float(v[j * p.kv_row_stride + c]), x[c] * alpha);
-    }
-    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-#pragma unroll
-    for (int c = 0; c < PER; ++c) x[c] *= inv;
+    read_again<DH>(p, item, nullptr, x);
   }
   const int64_t at = item * DH + lane * PER;
   if (p.out_f32) {
@@ -280,10 +313,13 @@ __global__ void __launch_bounds__(256) band_round_kernel(RoundParams p) {
   }
 }
 
-int launch_band_attend_tc(const uint16_t *q, int64_t R, int Hq, int64_t q_row_stride, const uint16_t *k,
-                          const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride, int64_t first_position,
-                          int window, int sink, float scale, float *out, float *lse, bool two_term, int32_t *status,
-                          cudaStream_t stream);
+// Whether the tensor-memory form takes these tensors: heads of 128 dims packed densely (a row of heads is a row of the
+// tensor map) and 16-byte aligned rows.
+static bool tensor_maps_take(const void *q, int dh, int64_t q_row_stride, int64_t q_head_stride, const void *k, const void *v,
+                             int64_t n_keys, int64_t kv_row_stride, int64_t kv_head_stride) {
+  return dh == 128 && q_head_stride == dh && kv_head_stride == dh && q_row_stride % 8 == 0 && kv_row_stride % 8 == 0 &&
+         ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 && n_keys >= 1 && n_keys < INT32_MAX;
+}
 
 }  // namespace lsa
 
@@ -305,14 +341,17 @@ LSA_API int lsa_band_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_
                   ((uintptr_t)q % 4) == 0,
               LSA_ERR_ARGUMENT);
   if (R == 0) return LSA_OK;
-  // The tensor-memory form: a head's 128 rows a CTA, operands fetched through tensor maps. It wants heads of 128
-  // dims packed densely (a row of heads is a row of the map) and 16-byte aligned rows; a chunk shorter than a tile
-  // of rows gains nothing from it.
-  const bool dense = q_head_stride == dh && kv_head_stride == dh && q_row_stride % 8 == 0 && ((uintptr_t)q % 16) == 0;
+  // (a chunk shorter than a tile of rows gains nothing from the tensor-memory form)
   const bool two_term = flags & LSA_BAND_TWO_TERM;
-  if (!(flags & LSA_BAND_WARP_MMA) && dh == 128 && dense && R >= 128 && n_keys < INT32_MAX)
-    return lsa::launch_band_attend_tc(q, R, Hq, q_row_stride, k, v, n_keys, Hkv, kv_row_stride, first_position,
-                                      window, sink, scale, out_f32, lse, two_term, status, (cudaStream_t)stream);
+  if (!(flags & LSA_BAND_WARP_MMA) && R >= 128 && first_position + R < INT32_MAX - 256 && ((uintptr_t)out_f32 % 16) == 0 &&
+      lsa::tensor_maps_take(q, dh, q_row_stride, q_head_stride, k, v, n_keys, kv_row_stride, kv_head_stride)) {
+    lsa::BandTcCall call = {q, k, v, q_row_stride, kv_row_stride, Hkv, {}};
+    call.p.out = out_f32, call.p.lse = lse, call.p.status = status;
+    call.p.R = (int)R, call.p.n_keys = (int)n_keys, call.p.first_position = (int)first_position;
+    call.p.Hq = Hq, call.p.group = group, call.p.window = window, call.p.sink = sink;
+    call.p.scale_log2 = scale * 1.4426950408889634f;
+    return lsa::launch_band_attend_tc(call, (cudaStream_t)stream);
+  }
   lsa::BandParams p;
   p.q = q;
   p.k = k;
@@ -370,6 +409,41 @@ LSA_API int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq
     lsa::band_round_kernel<128><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
   else
     lsa::band_round_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
+LSA_API int lsa_dense_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride, int64_t q_head_stride,
+                             const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride,
+                             int64_t kv_head_stride, int64_t first_position, const uint32_t *mask, float scale,
+                             uint16_t *out_bf16, float *out_f32, int32_t *not_finite, int32_t *status, void *stream) {
+  LSA_REQUIRE(q && k && v && (out_bf16 || out_f32) && not_finite, LSA_ERR_NULL);
+  LSA_REQUIRE(R >= 0 && Hq >= 1 && Hkv >= 1 && Hq % Hkv == 0 && n_keys >= 0 && first_position >= 0 && scale > 0.0f,
+              LSA_ERR_ARGUMENT);
+  LSA_REQUIRE(R < INT32_MAX / 2 && first_position < INT32_MAX - 256 - R, LSA_ERR_ARGUMENT);
+  LSA_REQUIRE(lsa::tensor_maps_take(q, dh, q_row_stride, q_head_stride, k, v, n_keys, kv_row_stride, kv_head_stride) &&
+                  ((uintptr_t)out_bf16 % 16) == 0 && ((uintptr_t)out_f32 % 16) == 0 && ((uintptr_t)mask % 16) == 0,
+              LSA_ERR_UNSUPPORTED);
+  if (R == 0) return LSA_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (cudaMemsetAsync(not_finite, 0, 4, s) != cudaSuccess) return LSA_ERR_LAUNCH;
+  lsa::BandTcCall call = {q, k, v, q_row_stride, kv_row_stride, Hkv, {}};
+  call.p.out = out_f32, call.p.out_bf16 = out_bf16, call.p.not_finite = not_finite, call.p.status = status;
+  call.p.mask = reinterpret_cast<const uint4 *>(mask);
+  call.p.R = (int)R, call.p.n_keys = (int)n_keys, call.p.first_position = (int)first_position;
+  call.p.Hq = Hq, call.p.group = Hq / Hkv, call.p.window = (int)(first_position + R), call.p.sink = 0;
+  call.p.scale_log2 = scale * 1.4426950408889634f;
+  const int rc = lsa::launch_band_attend_tc(call, s);
+  if (rc != LSA_OK) return rc;
+  lsa::RoundParams p = {};
+  p.q = q, p.k = k, p.v = v, p.out_bf16 = out_bf16, p.out_f32 = out_f32;
+  p.R = R, p.n_keys = n_keys, p.first_position = first_position;
+  p.q_row_stride = q_row_stride, p.q_head_stride = q_head_stride;
+  p.kv_row_stride = kv_row_stride, p.kv_head_stride = kv_head_stride;
+  p.Hq = Hq, p.group = Hq / Hkv;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  const int64_t items = (R * Hq + 7) / 8, most = 4 * (int64_t)lsa::sm_count();
+  lsa::dense_repair_kernel<<<(unsigned)(items < most ? items : most), 256, 0, s>>>(p, mask, not_finite);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }

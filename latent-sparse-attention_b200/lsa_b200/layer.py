@@ -501,17 +501,19 @@ class FlatLayer:
         n, dev = rows.shape[0], rows.device
         stop = start + n
         if band and self.design.sink_size <= 64 and k.shape[0] >= stop and start < self._whole_until(index):
-            # (a tensor-core row costs 1.5 ps a key and head here: 0.18 us for the 3,000 keys of a row of 40 heads, against
-            # 0.5 us for its window and 64 picked buckets. The probabilities go in as two bf16 terms, 1.25 ps with one: the
-            # lists' read, which this stands for, is closer to the sums in 64 bits than one rounded term a key.)
+            # (a tensor-core row costs 0.6 ps a key and head here: 0.07 us for the 3,000 keys of a row of 40 heads, against
+            # 0.5 us for its window and 64 picked buckets. The probabilities go in as two bf16 terms: the lists' read, which this
+            # stands for, is closer to the sums in 64 bits than one rounded term a key.)
             whole = min(n, self._whole_until(index) - start)
             with probe.region("band"):
-                partial, into = self._partial(self._room, "dense", whole, dev), out[:whole]
-                if not into.is_contiguous() or into.dtype not in (torch.bfloat16, torch.float32):
-                    into = partial[0]
+                partial, into = None, out[:whole]
+                if whole < 128 or not ops.dense_attend_supported(rows[:whole], k, v, into):
+                    partial = self._partial(self._room, "dense", whole, dev)
+                    if not into.is_contiguous() or into.dtype not in (torch.bfloat16, torch.float32):
+                        into = partial[0]
                 ops.causal_attend(rows[:whole], k, v, start, self.scale, out=into, partial=partial,
                                   status=self._attend_status)
-                if into is partial[0]:
+                if partial is not None and into is partial[0]:
                     out[:whole].copy_(into)
             if whole == n:
                 return out

@@ -732,8 +732,8 @@ def band_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_positio
     """The window and sinks of consecutive query rows as dense banded attention: q [R, Hq, dh] at positions
     first_position.., k/v [n_keys, Hkv, dh] by position. Returns the PARTIAL read (out fp32 [R, Hq, dh], lse [R, Hq])
     that `sparse_attend(..., init=(out, lse))` extends with the selected keys. Dense heads of 128 dims and 128 rows
-    or more run on tcgen05 with tensor-memory accumulators unless `warp_mma` asks for the warp-level kernel. `two_term`
-    takes the probabilities into the second product as two bf16 terms: a read that stands for a list of every key."""
+    or more run on tcgen05 with tensor-memory accumulators, the probabilities as two bf16 terms, unless `warp_mma` asks for
+    the warp-level kernel; `two_term` has that one take two terms as well: a read that stands for a list of every key."""
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
         raise ValueError("q, k and v must be bfloat16")
     if q.stride(2) != 1 or k.stride(2) != 1 or v.stride(2) != 1 or k.stride() != v.stride():
@@ -747,17 +747,39 @@ def band_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_positio
     return out, lse
 
 
+def dense_attend_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the tensor-memory dense read takes these tensors: heads of 128 dims packed densely, 16-byte aligned rows."""
+    dh = q.shape[2]
+    return dh == 128 and q.stride(1) == dh and k.stride(1) == dh and q.stride(2) == 1 and k.stride(2) == 1 \
+        and v.stride() == k.stride() and q.stride(0) % 8 == 0 and k.stride(0) % 8 == 0 and k.shape[0] > 0 \
+        and not any(t.data_ptr() % 16 for t in (q, k, v, out)) \
+        and all(t.dtype == torch.bfloat16 for t in (q, k, v)) and out.is_contiguous() \
+        and out.dtype in (torch.bfloat16, torch.float32)
+
+
+def _dense_attend(q, k, v, first_position: int, scale: float, out: torch.Tensor, mask: torch.Tensor | None,
+                  status: torch.Tensor | None) -> torch.Tensor:
+    R, Hq, dh = q.shape
+    not_finite = torch.empty(1, device=q.device, dtype=torch.int32)
+    call("lsa_dense_attend", ptr(q), R, Hq, dh, q.stride(0), q.stride(1), ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0),
+         k.stride(1), first_position, ptr(mask), float(scale), ptr(out) if out.dtype == torch.bfloat16 else None,
+         ptr(out) if out.dtype == torch.float32 else None, ptr(not_finite), ptr(status), stream(), launches=2)
+    return out
+
+
 def causal_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_position: int, scale: float,
                   out: torch.Tensor | None = None, partial: tuple | None = None,
                   status: torch.Tensor | None = None) -> torch.Tensor:
     """The dense read of every key up to a row's own, for rows whose list would name them all: q [R, Hq, dh] at positions
     first_position.., out [R, Hq, dh] bf16 (or fp32, where `out` is). As close to the sums in 64 bits as a list's read (the probabilities are two bf16
     terms), and a value that is not finite reaches the rows that read it alone. `partial`: (fp32 [R, Hq, dh], [R, Hq]) to work
-    in."""
+    in, for the forms that need it."""
     R, Hq, dh = q.shape
     out = torch.empty(R, Hq, dh, device=q.device, dtype=torch.bfloat16) if out is None else out
     if out.shape != (R, Hq, dh) or out.dtype not in (torch.bfloat16, torch.float32) or not out.is_contiguous():
         raise ValueError(f"out must be a contiguous bfloat16 or float32 [{R}, {Hq}, {dh}]")
+    if R >= 128 and dense_attend_supported(q, k, v, out):
+        return _dense_attend(q, k, v, first_position, scale, out, None, status)
     dense, lse = partial if partial is not None else (None, None)
     dense, _ = band_attend(q, k, v, first_position, first_position + R, 0, scale, out=dense, lse=lse, status=status,
                            two_term=True)
