@@ -470,7 +470,7 @@ int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq, int dh
  * Heads of 128 dims packed densely, 16-byte aligned rows and outputs (else LSA_ERR_UNSUPPORTED).
  * Rows whose output is not finite are read again, key by key, so that a value that is not finite reaches the rows that read
  * it and no others.
- *   mask        [key tiles of 128][R][4] uint32, a bit a key (every tile up to the last row's position), or NULL
+ *   mask        [key tiles of 128][R][4] uint32 as lsa_list_bits writes it (every tile up to the last row's position), or NULL
  *   out_bf16, out_f32  [R, Hq, 128], one of them may be NULL
  *   not_finite  one int32 of workspace
  *   status      (may be NULL) is raised if a bounded on-chip wait gives up */
@@ -478,6 +478,15 @@ int lsa_dense_attend(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row
                      const uint16_t *k, const uint16_t *v, int64_t n_keys, int Hkv, int64_t kv_row_stride,
                      int64_t kv_head_stride, int64_t first_position, const uint32_t *mask, float scale, uint16_t *out_bf16,
                      float *out_f32, int32_t *not_finite, int32_t *status, void *stream);
+
+/* The lists of lsa_expand as one bit a key, for lsa_dense_attend: picked, positions, members, the row budgets, top_k, sink and
+ * window as there. `tiles` key tiles of 128 positions are written; ids at or past n_keys count toward top_k and are left out.
+ *   mask        [tiles][R][4] uint32, 16-byte aligned
+ *   status      raised by every picked bucket id outside [0, m), or NULL
+ * LSA_ERR_UNSUPPORTED where eight rows' bits do not fit a CTA's shared memory (tiles > 1,600). */
+int lsa_list_bits(const int32_t *picked, int64_t R, int top_p, const int64_t *positions, const int32_t *members, int64_t m,
+                  int cap, const int32_t *row_top_p, const int32_t *row_top_k, int top_k, int sink, int window,
+                  int64_t n_keys, int tiles, uint32_t *mask, int32_t *status, void *stream);
 
 /* Gather-sparse attention over a shared latent cache (the MLA form): all Hq heads of a row attend over the SAME
  * listed latent rows; a key is the whole row (dk dims, rope part last), a value its first dv dims, and q holds the

@@ -398,9 +398,13 @@ class FlatLayer:
         index = self.build_index(k, reuse_buffers=not return_index)
         out = torch.empty_like(q) if out is None else out
         whole = min(T, self._whole_until(index)) if band else 0  # (rows that read everything make chunks of their own)
-        for first, end in ((0, whole), (whole, T)):
-            for start in range(first, end, chunk):
-                stop = min(end, start + chunk)
+        listed = max(whole, min(T, self._listed_until())) if band and bucket_major else whole
+        # (a CTA of the masked read has 256 rows of a head: chunks of fewer than two waves leave part of the GPU idle, 24,576
+        # tokens of 8 heads in chunks of 2,048 rows 7.1 ms and 4.8 this way)
+        waves = -(-2 * 148 * 256 // self.heads // 128) * 128
+        for first, end, step in ((0, whole, chunk), (whole, listed, max(chunk, waves)), (listed, T, chunk)):
+            for start in range(first, end, step):
+                stop = min(end, start + step)
                 self.prefill_rows(q[start:stop], start, k, v, index, out[start:stop], band, bucket_major)
         return (out, index) if return_index else out
 
@@ -494,6 +498,38 @@ class FlatLayer:
                 return None
             raise
 
+    def _listed_until(self) -> int:
+        """The position up to which a row's list is read as a mask over every key before it (`ops.listed_attend`): where that
+        costs what the other reads do. Measured on a B200, in ps a row and query head: a key of the masked read 0.68, so a
+        row's cost grows with its position; a pick read bucket by bucket 140 (partials in bf16; 420 where buckets hold more
+        than 64 members and they are fp32) and a key of the band beside it 1.2; a key of a gathered list 48 a KV head, and 10
+        for its place in the list. Whole prefills, the other reads against this one up to the line: 20,011 tokens of 32 heads
+        over 8, 64 picks of 32 keys 6.2 / 4.8 ms; 16,384 of 8 over 2, 16 picks of 64 keys 1.33 / 1.05; 24,576 of 8 over 2,
+        4,096 keys of 1,024 picks 12.1 / 4.8."""
+        d, group = self.design, self.heads // self.kv_heads
+        cost = 1.2 * (d.window_size + d.sink_size)
+        if self._reads_by_bucket:
+            cost += d.top_p * (140 if d.bucket_cap <= 64 else 420)
+        else:
+            cost += d.top_k * (48 + 10 / self.kv_heads) / group
+        return min(int(cost / 0.68), self.most_listed) // 128 * 128
+
+    most_listed = 1600 * 128  # positions whose bits `ops.list_bits` holds in a CTA's shared memory, eight rows of them
+
+    def _list_masks(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor):
+        """Memory for the masks of a chunk that is read through them ([key tiles, rows, 4] int32, the allocator's again after the
+        chunk); None for one that is not: rows past `_listed_until`, tensors the dense read does not take, too few rows for its
+        tiles, or no memory."""
+        n = rows.shape[0]
+        stop = start + n
+        if n < 128 or start >= self._listed_until() or stop > self.most_listed or k.shape[0] < stop or \
+                not ops.dense_attend_supported(rows, k, v, out):
+            return None
+        try:
+            return torch.empty(-(-stop // 128) * n * 16, device=rows.device, dtype=torch.uint8).view(torch.int32).view(-1, n, 4)
+        except torch.OutOfMemoryError:
+            return None
+
     def prefill_rows(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, band: bool = True, bucket_major: bool = True) -> torch.Tensor:
         """The read of consecutive query rows [n, Hq, dh] at positions start.. over a cache whose index is built,
@@ -519,10 +555,24 @@ class FlatLayer:
                 return out
             self.prefill_rows(rows[whole:], start + whole, k, v, index, out[whole:], band, bucket_major)
             return out
+        listed = self._listed_until() - start
+        if band and bucket_major and 0 < listed < n:  # (a row's read depends on its position, not on the chunk it is in)
+            self.prefill_rows(rows[:listed], start, k, v, index, out[:listed], band, bucket_major)
+            self.prefill_rows(rows[listed:], start + listed, k, v, index, out[listed:], band, bucket_major)
+            return out
         positions = torch.arange(start, stop, device=dev)
         with probe.region("index map"):
             index_queries = self.index_queries(rows, out=self._room("index queries", (n, self.index_dim),
                                                                     torch.float32, dev))
+        mask = self._list_masks(rows, start, k, v, out) if band and bucket_major else None
+        if mask is not None:
+            picked, positions, row_p, row_k = self._pick(index_queries, positions, index, self._room, stop - 1)
+            d = self.design
+            with probe.region("expand"):
+                ops.list_bits(picked, positions, index.buckets.bucket_members, d.top_k, d.sink_size, d.window_size, k.shape[0],
+                              mask.shape[0], row_p, row_k, self._expand_status, out=mask)
+            with probe.region("attend"):
+                return ops.listed_attend(rows, k, v, start, mask, self.scale, out, self._attend_status)
         # The window and the sinks are the same keys for neighbouring rows: one dense band serves them, and the
         # read of the selected keys starts from its partial result.
         banded = band and self.design.sink_size <= 64 and k.shape[0] >= stop

@@ -789,6 +789,28 @@ def causal_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_posit
     return out
 
 
+def list_bits(picked: torch.Tensor, positions: torch.Tensor, members: torch.Tensor, top_k: int, sink: int, window: int,
+              keys: int, tiles: int, row_top_p: torch.Tensor | None = None, row_top_k: torch.Tensor | None = None,
+              status: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+    """The lists of `expand` as one bit a key, [tiles, R, 4] int32: bit i of word w of a row is key 128 tile + 32 w + i. Ids at or
+    past `keys` are left out."""
+    picked, members = _contig(picked), _contig(members)
+    R, top_p = picked.shape
+    mask = torch.empty(tiles, R, 4, device=picked.device, dtype=torch.int32) if out is None else out
+    if mask.shape != (tiles, R, 4) or mask.dtype != torch.int32 or not mask.is_contiguous():
+        raise ValueError(f"out must be a contiguous int32 [{tiles}, {R}, 4]")
+    call("lsa_list_bits", ptr(picked), R, top_p, ptr(_as(positions, torch.int64)), ptr(members), members.shape[0],
+         members.shape[1], ptr(row_top_p), ptr(row_top_k), top_k, sink, window, keys, tiles, ptr(mask), ptr(status), stream())
+    return mask
+
+
+def listed_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_position: int, mask: torch.Tensor, scale: float,
+                  out: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
+    """`causal_attend` over the keys alone that `mask` (`list_bits`, every tile up to the last row) names: what
+    `sparse_attend` gives for the lists, by walking every key on the tensor cores."""
+    return _dense_attend(q, k, v, first_position, scale, out, mask, status)
+
+
 def lse_merge(parts: torch.Tensor, lses: torch.Tensor, out_dtype=torch.float32):
     """Merge [n, rows..., dh] partial outputs (fp32, or bf16 for fewer than 16 parts) by their [n, rows...]
     log-sum-exps."""

@@ -51,3 +51,120 @@ def test_a_running_maximum_that_grows_keeps_the_sums():
     got = ops.causal_attend(q, k, v, 0, 128 ** -0.5, out=torch.empty(n, 2, 128, device="cuda"))
     # (scores of up to 600 in log2: an fp32 product is off by 2^-24 of it, 2^-14 of a probability, and rounds in sums of 128)
     assert (got.double() - want).norm() <= 2 ** -12 * want.norm()
+
+
+def _bits(keep):
+    """keep [R, n] bool as words [tiles, R, 4] int32."""
+    R, n = keep.shape
+    tiles = -(-n // 128)
+    bits = torch.zeros(R, tiles * 128, dtype=torch.int64, device=keep.device)
+    bits[:, :n] = keep
+    words = (bits.view(R, tiles, 4, 32) << torch.arange(32, device=keep.device)).sum(-1)
+    return torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32).permute(1, 0, 2).contiguous()
+
+
+@pytest.mark.parametrize("R,first,Hq,Hkv", [(1, 0, 1, 1), (127, 1, 2, 1), (128, 0, 5, 1), (129, 127, 4, 2), (255, 0, 2, 2),
+                                            (256, 640, 8, 1), (257, 129, 3, 3), (640, 77, 6, 2)])
+def test_masked_rows_read_the_keys_they_list(R, first, Hq, Hkv):
+    """Random lists, rows that list nothing, one key or every key; and a value and a key that are not finite reach the rows that
+    list them alone. 2^-16 as above."""
+    from lsa_b200 import ops
+
+    n = first + R
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(n, Hq, Hkv, 128, 16, n))
+    q = q[first:]
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    keep = torch.rand(R, n, device="cuda", generator=gen) < torch.rand(R, 1, device="cuda", generator=gen)
+    keep &= torch.arange(n, device="cuda") <= first + torch.arange(R, device="cuda")[:, None]
+    keep[0] = False
+    if R > 2:
+        keep[1] = False
+        keep[1, first] = True
+        keep[2] = torch.arange(n, device="cuda") <= first + 2
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    read = lambda dtype: ops.listed_attend(q, k, v, first, _bits(keep), 128 ** -0.5,
+                                           torch.empty(R, Hq, 128, device="cuda", dtype=dtype), status)
+    want, _ = _read(q, k, v, keep)
+    got = read(torch.float32)
+    assert (got.double() - want).norm() <= 2 ** -16 * want.norm() and not got[0].any()
+    assert (read(torch.bfloat16).double() - want).abs().max() <= 2 ** -8 * want.abs().max() and int(status) == 0
+    for x, at, what in ((v, first, float("inf")), (k, first, float("nan"))):
+        kept = x[at, 0, 5].clone()
+        x[at, 0, 5] = what
+        odd = ~read(torch.float32).isfinite().all(-1)
+        x[at, 0, 5] = kept
+        heads = torch.arange(Hq, device="cuda") < Hq // Hkv
+        assert torch.equal(odd, keep[:, first, None] & heads)
+
+
+@pytest.mark.parametrize("cap,top_p,top_k,sink,window,sizes", [
+    (16, 40, 200, 4, 100, (0, 16)), (16, 64, 10000, 0, 1, (8, 16)), (1, 33, 20, 2, 64, (1, 1)), (24, 17, 100, 70, 200, (0, 24)),
+    (30, 10, 77, 4, 128, (3, 30)), (64, 16, 300, 4, 256, (20, 64)), (128, 8, 500, 4, 300, (0, 128)), (600, 3, 1000, 4, 64, (1, 600))])
+def test_lists_as_bits_are_the_lists(cap, top_p, top_k, sink, window, sizes):
+    """The bits of every row against the ids `expand` writes for it: cuts at top-k inside a bucket, empty buckets, rows before
+    the first block, picks outside the table, row budgets, ids past the cache."""
+    from lsa_b200 import ops
+
+    rng = np.random.default_rng(cap)
+    T, m = 1500, 60
+    deal, members = rng.permutation(T), np.full((m, cap), -1, dtype=np.int32)
+    at = 0
+    for b in range(m):
+        count = min(int(rng.integers(sizes[0], sizes[1] + 1)), T - at)
+        members[b, :count] = np.sort(deal[at:at + count])
+        at += count
+    positions = np.concatenate([[-1, 0, 1, 5], rng.integers(0, T, 60), [T - 1]])
+    R = len(positions)
+    picked = np.stack([rng.permutation(m)[:top_p] if top_p <= m else rng.permutation(top_p) for _ in range(R)]).astype(np.int32)
+    picked[picked >= m] = -1
+    picked[3, 0] = m + 7
+    row_p = rng.integers(-1, top_p + 1, R).astype(np.int32)
+    row_k = rng.integers(-1, top_k + 1, R).astype(np.int32)
+    args = (cuda(picked), cuda(positions), cuda(members), top_k, sink, window)
+    for budgets in ((None, None), (cuda(row_p), cuda(row_k))):
+        lists, lengths, bad = ops.expand(*args, *budgets)
+        for keys in (T, 1111):
+            status = torch.zeros(1, dtype=torch.int32, device="cuda")
+            words = ops.list_bits(*args, keys, -(-T // 128), *budgets, status=status).cpu().numpy().view(np.uint32)
+            bits = np.unpackbits(words.transpose(1, 0, 2).copy().view(np.uint8), axis=-1, bitorder="little").reshape(R, -1)
+            for r in range(R):
+                ids = lists[r, :lengths[r]].cpu().numpy()
+                assert np.array_equal(np.flatnonzero(bits[r]), np.sort(ids[ids < keys])), (r, positions[r])
+            assert int(status) == int(bad)
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,chunk,sizes", [
+    (2500, 8, 2, 512, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=300, sink_size=4,
+                           window_size=128)),   # gathered else
+    (3000, 5, 1, 1024, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=512, top_p=16, top_k=300,
+                            sink_size=4, window_size=300)),  # read by bucket else
+    (2000, 4, 2, 2048, dict(pool_size=16, bucket_size=64, bucket_cap=128, cluster_block_size=512, top_p=4, top_k=200,
+                            sink_size=0, window_size=100))])
+def test_a_prefill_read_through_masks_is_the_one_read_by_lists(T, Hq, Hkv, chunk, sizes, monkeypatch):
+    """Whole prefills with the masked read for every row, up to a row inside a chunk, and for none: the same rows within the
+    rounding to bf16, and no further from the gather of whole lists than that."""
+    from lsa_b200 import ops
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    rng = np.random.default_rng(T)
+    w = [cuda(rng.standard_normal((Hkv * 128, 64), dtype=np.float32) / 16, torch.bfloat16) for _ in range(2)]
+    layer = FlatLayer(FlatDesign(**sizes), *w, Hq, Hkv, 128)
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(T, Hq, Hkv, 128, 16, T))
+    listed, read = [], ops.listed_attend
+    monkeypatch.setattr(ops, "listed_attend", lambda q, *a, **kw: (listed.append(q.shape[0]), read(q, *a, **kw))[1])
+    gathered = layer.prefill(q, k, v, chunk=chunk, band=False, bucket_major=False).float()
+    assert not listed
+    for until in (0, T // 256 * 128, 128 * 1024):
+        monkeypatch.setattr(FlatLayer, "_listed_until", lambda self: until)
+        got = layer.prefill(q, k, v, chunk=chunk).float()
+        assert bool(listed) == bool(until)
+        assert (got - gathered).abs().max() <= 2e-2 and (got - gathered).abs().mean() <= 2e-3
+    assert sum(listed) > T // 2
+    layer.check()
+    # tensors the dense read does not take go the way they went
+    listed.clear()
+    odd = torch.empty(T * Hq * 128 + 2, device="cuda", dtype=torch.bfloat16)[2:].view(T, Hq, 128).copy_(q)
+    if sizes["bucket_cap"] <= 16:
+        got = layer.prefill(odd, k, v, chunk=chunk).float()
+        # (rows that no tensor map can walk are mapped in fp32: another bucket where two scores nearly tie)
+        assert not listed and ((got - gathered).abs().amax((1, 2)) <= 2e-2).float().mean() >= 0.98
