@@ -488,6 +488,19 @@ int lsa_list_bits(const int32_t *picked, int64_t R, int top_p, const int64_t *po
                   int cap, const int32_t *row_top_p, const int32_t *row_top_k, int top_k, int sink, int window,
                   int64_t n_keys, int tiles, uint32_t *mask, int32_t *status, void *stream);
 
+/* One decode step of a few rows over a flat index, in one call: lsa_index_map (group Hq / Hkv, unit rows), lsa_visible_buckets,
+ * lsa_flat_select_decode, lsa_expand (no padding) and lsa_sparse_attend over KV rows at their positions, with the arguments of
+ * those calls (map [Hkv * dh_used, d_idx] of map_dtype; a bucket's block holds `block` keys in `block_buckets` buckets). Their
+ * intermediates live in the workspace; width = top_k + window + sink. */
+size_t lsa_flat_decode_workspace_bytes(int64_t R, int Hq, int dh, int d_idx, int top_p, int64_t width, int select_splits,
+                                       int splits);
+int lsa_flat_decode(const uint16_t *q, int64_t R, int Hq, int dh, int64_t q_row_stride, int64_t q_head_stride, const void *map,
+                    int map_dtype, int dh_off, int dh_used, int d_idx, const int64_t *positions, const float *centroids, int64_t m,
+                    const int32_t *members, int bucket_cap, int64_t block, int64_t block_buckets, int top_p, int top_k, int sink,
+                    int window, int select_splits, const uint16_t *k, const uint16_t *v, int64_t slots, int Hkv,
+                    int64_t kv_row_stride, int64_t kv_head_stride, float scale, int splits, uint16_t *out_bf16,
+                    int32_t *expand_status, void *workspace, size_t workspace_bytes, void *stream);
+
 /* Gather-sparse attention over a shared latent cache (the MLA form): all Hq heads of a row attend over the SAME
  * listed latent rows; a key is the whole row (dk dims, rope part last), a value its first dv dims, and q holds the
  * absorbed queries (the key up-projection folded into them), so no per-head key is ever materialised.

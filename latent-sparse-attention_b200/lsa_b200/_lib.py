@@ -13,7 +13,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblsa_b200.so")
-ABI_VERSION = 22
+ABI_VERSION = 23
 
 DTYPE_F32, DTYPE_BF16 = 0, 1
 PAD = -1
@@ -67,6 +67,9 @@ SIGNATURES = {
     "lsa_band_attend": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _I, _L, _L, _L, _I, _I, _F, _P, _P, _I, _P, _P]),
     "lsa_dense_attend": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _I, _L, _L, _L, _P, _F, _P, _P, _P, _P, _P]),
     "lsa_list_bits": (_I, [_P, _L, _I, _P, _P, _L, _I, _P, _P, _I, _I, _I, _L, _I, _P, _P, _P]),
+    "lsa_flat_decode_workspace_bytes": (_Z, [_L, _I, _I, _I, _I, _L, _I, _I]),
+    "lsa_flat_decode": (_I, [_P, _L, _I, _I, _L, _L, _P, _I, _I, _I, _I, _P, _P, _L, _P, _I, _L, _L, _I, _I, _I, _I, _I, _P, _P, _L,
+                             _I, _L, _L, _F, _I, _P, _P, _P, _Z, _P]),
     "lsa_sparse_attend_static_scratch_bytes": (_Z, []),
     "lsa_sparse_attend_static": (_I, [_P, _L, _I, _I, _L, _L, _P, _P, _L, _L, _I, _L, _L, _P, _L, _P, _F, _I, _P, _P,
                                       _P, _P]),

@@ -618,9 +618,27 @@ class FlatLayer:
         (16,384 buckets: one row 18.8 us in 32; 8 rows 29.2 in 32, 20.5 in 16)."""
         return 1 if buckets <= 512 else 8 if buckets <= 4096 else 32 if rows == 1 else 16
 
+    def _decodes_in_one_call(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
+                             index: FlatIndex) -> bool:
+        """Whether a step may go to the GPU as one call: where the calls it is made of would take these tensors as they are."""
+        d, b = self.design, index.buckets
+        return q.dim() == 3 and 0 < q.shape[0] <= 8 and q.shape[1:] == (self.heads, self.head_dim) and d.early_budget is None \
+            and index.shapes is None and d.top_p <= 128 and self.index_dim in (32, 64) and not probe.listening() \
+            and positions.dtype == torch.int64 and positions.shape == q.shape[:1] and q.stride(2) == k.stride(2) == v.stride(2) == 1 \
+            and k.stride() == v.stride() and k.shape[1:] == v.shape[1:] == (self.kv_heads, self.head_dim) \
+            and q.dtype == k.dtype == v.dtype == torch.bfloat16 and positions.is_contiguous() \
+            and b.bucket_centroids.dtype == torch.float32 and b.bucket_members.dtype == torch.int32 \
+            and b.bucket_centroids.is_contiguous() and b.bucket_members.is_contiguous()
+
     def decode(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                splits: int = 8):
         """One step for rows at `positions` over a cache whose index is built: out [R,Hq,dh] bf16."""
+        if self._decodes_in_one_call(q, positions, k, v, index):
+            d, b = self.design, index.buckets
+            return ops.flat_decode(q, self.query_map, self.dh_off, self.dh_used, positions, b.bucket_centroids, b.bucket_members,
+                                   d.cluster_block_size, d.block_bucket_count, d.top_p, d.top_k, d.sink_size, d.window_size,
+                                   self._decode_splits(q.shape[0], b.bucket_centroids.shape[0]), k, v, self.scale, splits,
+                                   self._expand_status)
         lists, lengths = self.select(self.index_queries(q), positions, index)
         out, _ = self.attend(q, k, v, lists, lengths, splits=splits)
         return out

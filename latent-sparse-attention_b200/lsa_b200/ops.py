@@ -642,6 +642,25 @@ def sparse_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ids: torch.
     return (out_bf16 if out_bf16 is not None else out_f32), lse
 
 
+def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh_used: int, positions: torch.Tensor,
+                centroids: torch.Tensor, members: torch.Tensor, block_size: int, block_buckets: int, top_p: int, top_k: int,
+                sink: int, window: int, select_splits: int, k: torch.Tensor, v: torch.Tensor, scale: float, splits: int,
+                expand_status: torch.Tensor | None = None) -> torch.Tensor:
+    """`index_map`, `visible_buckets`, `flat_select_decode`, `expand` and `sparse_attend` of a decode step's few rows in one call:
+    out [R, Hq, dh] bf16. All of the tensors as those take them without a copy (bf16 q, k, v; int64 positions, fp32 centroids)."""
+    R, Hq, dh = q.shape
+    d_idx, width = centroids.shape[1], top_k + window + sink
+    out = torch.empty(R, Hq, dh, device=q.device, dtype=torch.bfloat16)
+    need = query("lsa_flat_decode_workspace_bytes", R, Hq, dh, d_idx, top_p, width, select_splits, splits)
+    workspace = torch.empty(need, device=q.device, dtype=torch.uint8)
+    call("lsa_flat_decode", ptr(q), R, Hq, dh, q.stride(0), q.stride(1), ptr(index_map_weight), _lib.dtype_code(index_map_weight),
+         dh_off, dh_used, d_idx, ptr(positions), ptr(centroids), centroids.shape[0], ptr(members), members.shape[1], block_size,
+         block_buckets, top_p, top_k, sink, window, select_splits, ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0), k.stride(1),
+         float(scale), splits, ptr(out), ptr(expand_status), ptr(workspace), need, stream(),
+         launches=3 + _split_launches(R, select_splits, top_p) + (1 if splits == 1 else 2))
+    return out
+
+
 def latent_attend(q: torch.Tensor, latent: torch.Tensor, ids: torch.Tensor, lengths: torch.Tensor | None,
                   scale: float, value_dim: int = 512, splits: int = 1, out_dtype=torch.bfloat16,
                   workspace: torch.Tensor | None = None, warp_mma: bool = False,

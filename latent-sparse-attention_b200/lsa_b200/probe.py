@@ -24,6 +24,11 @@ def uninstall() -> None:
     install(None)
 
 
+def listening() -> bool:
+    """Whether a recorder is installed: what one call would do is then done region by region."""
+    return _recorder is not None
+
+
 def region(name: str):
     if _recorder is None:
         return contextlib.nullcontext()

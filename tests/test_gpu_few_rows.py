@@ -96,3 +96,31 @@ def test_lists_folded_in_a_cluster_are_the_scan_s(m, d, keep):
     want = ops.beam_step(q, c, distinct, none, none, keep, splits=1)
     got = ops.beam_step(q, c, distinct, none, none, keep, splits=8)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("T,R,splits,sizes", [
+    (700, 1, 8, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200, sink_size=4, window_size=128)),
+    (9000, 8, 1, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=700, sink_size=0, window_size=100))])
+def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monkeypatch):
+    """The same rows bit for bit, at the end, in the middle and before the first block; strided queries; a status that is raised."""
+    from helpers import layer_inputs
+    from lsa_b200 import ops
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    rng = np.random.default_rng(T)
+    w = [cuda(rng.standard_normal((256, 64), dtype=np.float32) / 16, torch.bfloat16) for _ in range(2)]
+    layer = FlatLayer(FlatDesign(**sizes), *w, 8, 2, 128)
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(T, 8, 2, 128, 16, T))
+    index = layer.build_index(k)
+    positions = cuda(np.array([T - 1, T // 2, 5, 0, 130, T - 2, 256, 90])[:R])
+    once, calls = ops.flat_decode, []
+    monkeypatch.setattr(ops, "flat_decode", lambda *a: (calls.append(1), once(*a))[1])
+    for rows in (q[positions], q.repeat(1, 2, 1)[positions][:, :8]):
+        got = layer.decode(rows, positions, k, v, index, splits=splits)
+        with monkeypatch.context() as patch:
+            patch.setattr(FlatLayer, "_decodes_in_one_call", lambda *a: False)
+            assert torch.equal(got, layer.decode(rows, positions, k, v, index, splits=splits))
+    assert len(calls) == 2
+    layer.decode(q[positions], positions.int(), k, v, index)  # (positions that would be converted: the calls one by one)
+    assert len(calls) == 2
+    layer.check()
