@@ -9,43 +9,51 @@
 namespace lsa {
 
 constexpr int kMapThreads = 256;
-constexpr int kMapRows = 64;    // rows a CTA maps, two a thread
+constexpr int kMapRows = 64;    // rows a CTA maps, two a thread (half of them, one a thread, where 64 leave SMs without a second CTA)
 constexpr int kMapSlice = 64;   // input dims staged at a time
 constexpr int kMapMaxCols = 16; // output dims a thread holds: a CTA writes a slice of up to 128 output dims
 constexpr int kMapColSlice = 8 * kMapMaxCols;
 
-template <typename TX, typename TW>
+// COLS: output dims a thread holds. What bounds it is the chain of a slice: staging, 64 multiply-adds on one sum, and back. A
+// slice whose columns are all there is unrolled, so that the shared-memory loads run ahead of the chain (7,613 rows of 256 dims
+// to 64 121.8 -> 42.1 us, 200 of them 120 -> 34; 100,000 of 1,024 dims to 128 2.77 -> 1.48 ms).
+template <typename TX, typename TW, int ROWS, int COLS>
 __global__ void __launch_bounds__(kMapThreads)
     index_map_kernel(const TX *__restrict__ x, int64_t rows, int heads, int group, int dh_off, int dh_used,
                      int64_t x_row_stride, int64_t x_head_stride, const TW *__restrict__ W, int d_idx, int normalize,
                      float *__restrict__ out_f32, uint16_t *__restrict__ out_bf16) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float *xs = reinterpret_cast<float *>(smem_raw);       // [kMapRows][kMapSlice + 1]
-  float *ws = xs + kMapRows * (kMapSlice + 1);           // [kMapSlice][d_idx]
+  float *xs = reinterpret_cast<float *>(smem_raw);       // [ROWS][kMapSlice + 1]
+  float *ws = xs + ROWS * (kMapSlice + 1);           // [kMapSlice][d_idx]
   const int tid = threadIdx.x;
   const int row_a = tid >> 3, row_b = row_a + 32, cg = tid & 7;
-  const int64_t row0 = (int64_t)blockIdx.x * kMapRows;
+  const int64_t row0 = (int64_t)blockIdx.x * ROWS;
+  constexpr bool kTwo = ROWS == 64;  // whether a thread has a second row
   const int d_in = heads / group * dh_used;
   // blockIdx.y picks the slice of output dims; a map wider than one slice is normalised by a second kernel
   const int col0 = blockIdx.y * kMapColSlice, width = min(kMapColSlice, d_idx - col0);
   const int cols = (width + 7) / 8;
-  float acc_a[kMapMaxCols], acc_b[kMapMaxCols];
+  float acc_a[COLS], acc_b[COLS];
 #pragma unroll
-  for (int i = 0; i < kMapMaxCols; ++i) acc_a[i] = acc_b[i] = 0.0f;
+  for (int i = 0; i < COLS; ++i) acc_a[i] = acc_b[i] = 0.0f;
 
   for (int k0 = 0; k0 < d_in; k0 += kMapSlice) {
     const int kn = min(kMapSlice, d_in - k0);
-    for (int e = tid; e < kMapRows * kMapSlice; e += kMapThreads) {
+    // (loads of several elements in flight: one after another, each a round trip of the heads, they were most of the kernel)
+#pragma unroll 4
+    for (int e = tid; e < ROWS * kMapSlice; e += kMapThreads) {
       const int rr = e / kMapSlice, kk = e - rr * kMapSlice;
       float sum = 0.0f;
       const int64_t r = row0 + rr;
       if (r < rows && kk < kn) {
         const int k = k0 + kk, kv = k / dh_used, c = k - kv * dh_used;
         const TX *src = x + r * x_row_stride + (int64_t)kv * group * x_head_stride + dh_off + c;
+#pragma unroll 8
         for (int g = 0; g < group; ++g) sum = __fadd_rn(sum, load_as_float<TX>(src, (int64_t)g * x_head_stride));
       }
       xs[rr * (kMapSlice + 1) + kk] = sum;
     }
+#pragma unroll 8
     for (int e = tid; e < kMapSlice * width; e += kMapThreads) {
       const int kk = e / width, j = col0 + e - kk * width;
       float w = 0.0f;
@@ -53,15 +61,29 @@ __global__ void __launch_bounds__(kMapThreads)
       ws[e] = w;
     }
     __syncthreads();
+    if (width == 8 * COLS && kn == kMapSlice) {
+#pragma unroll 8
+      for (int kk = 0; kk < kMapSlice; ++kk) {
+        const float xa = xs[row_a * (kMapSlice + 1) + kk], xb = kTwo ? xs[row_b * (kMapSlice + 1) + kk] : 0.0f;
+        const float *wrow = ws + kk * 8 * COLS + cg;
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) {
+          acc_a[i] = fmaf(xa, wrow[8 * i], acc_a[i]);
+          if (kTwo) acc_b[i] = fmaf(xb, wrow[8 * i], acc_b[i]);
+        }
+      }
+      __syncthreads();
+      continue;
+    }
     for (int kk = 0; kk < kn; ++kk) {
-      const float xa = xs[row_a * (kMapSlice + 1) + kk], xb = xs[row_b * (kMapSlice + 1) + kk];
+      const float xa = xs[row_a * (kMapSlice + 1) + kk], xb = kTwo ? xs[row_b * (kMapSlice + 1) + kk] : 0.0f;
       const float *wrow = ws + kk * width + cg;
 #pragma unroll
-      for (int i = 0; i < kMapMaxCols; ++i) {
+      for (int i = 0; i < COLS; ++i) {
         if (i < cols) {
           const float w = (cg + 8 * i) < width ? wrow[8 * i] : 0.0f;
           acc_a[i] = fmaf(xa, w, acc_a[i]);
-          acc_b[i] = fmaf(xb, w, acc_b[i]);
+          if (kTwo) acc_b[i] = fmaf(xb, w, acc_b[i]);
         }
       }
     }
@@ -70,7 +92,7 @@ __global__ void __launch_bounds__(kMapThreads)
 
   float ss_a = 0.0f, ss_b = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kMapMaxCols; ++i) {
+  for (int i = 0; i < COLS; ++i) {
     ss_a = fmaf(acc_a[i], acc_a[i], ss_a);
     ss_b = fmaf(acc_b[i], acc_b[i], ss_b);
   }
@@ -82,7 +104,7 @@ __global__ void __launch_bounds__(kMapThreads)
   const float den_a = normalize ? fmaxf(sqrtf(ss_a), 1e-12f) : 1.0f;
   const float den_b = normalize ? fmaxf(sqrtf(ss_b), 1e-12f) : 1.0f;
 #pragma unroll
-  for (int i = 0; i < kMapMaxCols; ++i) {
+  for (int i = 0; i < COLS; ++i) {
     const int j = col0 + cg + 8 * i;
     if (i >= cols || cg + 8 * i >= width) continue;
     if (row0 + row_a < rows) {
@@ -90,7 +112,7 @@ __global__ void __launch_bounds__(kMapThreads)
       if (out_f32) out_f32[(row0 + row_a) * d_idx + j] = v;
       if (out_bf16) out_bf16[(row0 + row_a) * d_idx + j] = float_to_bf16_bits(v);
     }
-    if (row0 + row_b < rows) {
+    if (kTwo && row0 + row_b < rows) {
       const float v = acc_b[i] / den_b;
       if (out_f32) out_f32[(row0 + row_b) * d_idx + j] = v;
       if (out_bf16) out_bf16[(row0 + row_b) * d_idx + j] = float_to_bf16_bits(v);
@@ -321,14 +343,19 @@ static int launch_index_map(const void *x, int64_t rows, int heads, int group, i
     return LSA_OK;
   }
   const int slices = (d_idx + kMapColSlice - 1) / kMapColSlice;
+  const bool half = (rows + kMapRows - 1) / kMapRows * slices < 2 * sm_count();
+  const int cta_rows = half ? kMapRows / 2 : kMapRows;
   const size_t smem =
-      sizeof(float) * ((size_t)kMapRows * (kMapSlice + 1) + (size_t)kMapSlice * min(d_idx, kMapColSlice));
-  if (!allow_shared(index_map_kernel<TX, TW>,
-                    sizeof(float) * (kMapRows * (kMapSlice + 1) + (size_t)kMapSlice * kMapColSlice)))
+      sizeof(float) * ((size_t)cta_rows * (kMapSlice + 1) + (size_t)kMapSlice * min(d_idx, kMapColSlice));
+  auto of = [&](auto whole, auto halves) { return half ? halves : whole; };
+  auto kernel = d_idx <= 32   ? of(index_map_kernel<TX, TW, kMapRows, 4>, index_map_kernel<TX, TW, kMapRows / 2, 4>)
+                : d_idx <= 64 ? of(index_map_kernel<TX, TW, kMapRows, 8>, index_map_kernel<TX, TW, kMapRows / 2, 8>)
+                              : of(index_map_kernel<TX, TW, kMapRows, kMapMaxCols>, index_map_kernel<TX, TW, kMapRows / 2, kMapMaxCols>);
+  if (!allow_shared(kernel, sizeof(float) * (kMapRows * (kMapSlice + 1) + (size_t)kMapSlice * kMapColSlice)))
     return LSA_ERR_LAUNCH;
-  const dim3 grid((unsigned)((rows + kMapRows - 1) / kMapRows), (unsigned)slices);
+  const dim3 grid((unsigned)((rows + cta_rows - 1) / cta_rows), (unsigned)slices);
   // One slice: the CTA holds whole rows and normalises them itself. More: fp32 rows first, then unit rows in place.
-  index_map_kernel<TX, TW><<<grid, kMapThreads, smem, s>>>(
+  kernel<<<grid, kMapThreads, smem, s>>>(
       (const TX *)x, rows, heads, group, dh_off, dh_used, x_row_stride, x_head_stride, (const TW *)W, d_idx,
       slices == 1 ? normalize : 0, out_f32, slices == 1 || !normalize ? out_bf16 : nullptr);
   LSA_LAUNCH_CHECK();

@@ -124,3 +124,20 @@ def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monk
     layer.decode(q[positions], positions.int(), k, v, index)  # (positions that would be converted: the calls one by one)
     assert len(calls) == 2
     layer.check()
+
+
+@pytest.mark.parametrize("rows", [129, 700, 19000])  # (32 rows a CTA, and 64)
+@pytest.mark.parametrize("d_in,d_idx", [(256, 32), (192, 64), (130, 64), (64, 60), (256, 128), (100, 100)])
+def test_the_exact_map_keeps_the_oracle_s_bits(oracle, rows, d_in, d_idx):
+    """Whole slices of input and output dims and ragged ones, against the oracle's product in its own order, bit for bit."""
+    from lsa_b200 import ops
+
+    rng = np.random.default_rng(d_in + d_idx)
+    x, w = rng.standard_normal((rows, d_in), dtype=np.float32), rng.standard_normal((d_in, d_idx), dtype=np.float32)
+    got = ops.index_map(cuda(x)[:, None], cuda(w), normalize=False).cpu().numpy()
+    some = np.unique(np.concatenate([np.arange(40), rng.integers(0, rows, 60), np.arange(rows - 40, rows)]))
+    want = np.zeros((len(some), d_idx), dtype=np.float32)
+    for k in range(d_in):  # (a multiply-add in 64 bits rounds to the fp32 one: 48 bits of product beside 24)
+        want = (x[some, k, None].astype(np.float64) * w[k].astype(np.float64) + want.astype(np.float64)).astype(np.float32)
+    off = got[some].view(np.int32).astype(np.int64) - want.view(np.int32)
+    assert (off == 0).mean() >= 0.999 and np.abs(got[some] - want).max() <= 1e-4  # (a double rounding in a million)
