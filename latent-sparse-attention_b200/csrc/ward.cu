@@ -1,11 +1,13 @@
 // Capped Ward bucketing of cluster blocks of up to 4,096 pools with 16, 32 or 64 index dims: the buckets of a cache,
 // and the node-bucket pairings of the tree over them.
 //
-// A cluster of 1 to 8 CTAs merges one block from its first round to its last. Every CTA keeps the block's per-row state
-// (sizes, norms, cheapest partner, who is alive) in its own shared memory and takes every decision itself, so only two
-// things cross between the CTAs of a round: the cheapest partners (64-bit minima, the greater word the cost and the
-// lower the partner, so that a tie goes to the lower row whatever the order of arrival; every CTA keeps the minima of
-// the pairs it looked at, and reads the others' through distributed shared memory) and, where the key sums do not fit beside the rest, the merged rows, which then live in the workspace.
+// A block of up to 512 pools is merged from its first round to its last by a cluster of 1 to 8 CTAs, a larger one by a cluster
+// or by up to as many CTAs as there are SMs. Every CTA keeps the block's per-row state (sizes, norms, cheapest partner, who is
+// alive) in its own shared memory and takes every decision itself, so only two things cross between the CTAs of a round: the
+// cheapest partners (64-bit minima, the greater word the cost and the lower the partner, so that a tie goes to the lower row
+// whatever the order of arrival) and the merged rows. In the smaller blocks every CTA keeps the minima of the pairs it looked
+// at, reads the others' through distributed shared memory and merges every row itself; in the larger ones the key sums do not
+// fit beside the rest, and both live in the workspace.
 //
 // A round looks only at what the round before changed. A pair's cost depends on nothing but its two rows, so a row whose
 // cheapest partner neither merged nor went keeps it, unless a row that just merged is cheaper:
@@ -15,7 +17,7 @@
 // bounds it is fp32 multiply-adds in the first round and barriers in the last ones, where a handful of rows is dirty (a
 // round of a block of 80 pools takes 7 us, of which the tiles are 2).
 // Measured on a B200, against every row searching all of its partners every round (one CTA a block up to 512 pools, two
-// launches a round, 256 rounds, above): the pairings of 16 blocks of 4,096, 2,048 and 1,024 buckets 26.0 -> 6.0 ms; 1,024
+// launches a round, 256 rounds, above): the pairings of 16 blocks of 4,096, 2,048 and 1,024 buckets 26.0 -> 4.4 ms; 1,024
 // blocks of 256 pools with the pairings of 512, 256 and 128 buckets 7.2 -> 2.4 ms; 9 blocks of 128 pools 165 -> 57 us; one
 // block of 80 pools, sixteen rounds, 190 -> 119 us.
 //
@@ -38,6 +40,8 @@ __host__ __device__ constexpr int ward_threads(bool local) { return local ? 256 
 __host__ __device__ constexpr int ward_tile(bool local) { return kWardRows * ward_threads(local) / 32; }
 constexpr int kWardMaxCtas = 8;      // a cluster's portable size
 constexpr int kWardMaxPools = 4096;  // pools of a block, at most
+constexpr int kWardApart = 64;       // ints from one block's counter of arrivals to the next (nothing else in its cache lines)
+constexpr int kWardPatience = 1 << 24;  // looks at the counter before a wait gives up (seconds)
 constexpr int kWardLocalPools = 512;  // blocks up to this many pools keep their key sums in every CTA's shared memory
 
 enum : uint8_t { kAlive = 1, kOpen = 2, kChanged = 4, kMerged = 8 };
@@ -50,9 +54,12 @@ struct WardParams {
   int64_t *labels;    // [G, P]
   uint8_t *reached;   // [G]
   int32_t *rounds;    // [G] or NULL
-  // the workspace of larger blocks: key sums [G, P, D], squared norms and norms [G, P], cheapest partners [2, G, P]
+  // the workspace of larger blocks: key sums [G, P, D], squared norms and norms [G, P], cheapest partners [2, G, P], and where
+  // a block's CTAs are no cluster how many of them arrived at its barriers [G, kWardApart] (zero at launch; else NULL)
   float *sums, *sq, *al;
   unsigned long long *cheapest;
+  int *arrived;
+  int ctas;  // CTAs a block
 };
 
 // A CTA's shared memory, carved from the dynamic part.
@@ -116,7 +123,7 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int kThreads = ward_threads(LOCAL), TILE = ward_tile(LOCAL), LD = D + 4, COLS = TILE / 32;
-  const int ctas = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int ctas = p.ctas, rank = (int)(blockIdx.x % ctas);
   const int64_t g = blockIdx.x / ctas;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, P = p.P;
   const unsigned below = (1u << lane) - 1;
@@ -127,11 +134,29 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   const int64_t apart = LOCAL ? (ctas > 1 ? P : 0) : (int64_t)(gridDim.x / ctas) * P;
   unsigned long long *mine = LOCAL ? s.cheapest : p.cheapest + g * P;
   __shared__ int warp_count[kThreads / 32], n_merge_s, smallest_s;
-  auto everyone = [&] {  // what a CTA wrote before is seen by the whole cluster after
-    if (ctas > 1)
-      cluster.sync();
-    else
+  // What a CTA wrote before is seen by all of the block's after. (CTAs that are no cluster are launched as a cooperative grid,
+  // so that all of them run: a wait that gives up all the same ends the block as one that did not reach its count.)
+  bool gave_up = false;
+  int due = 0;
+  auto everyone = [&] {
+    if (ctas == 1) {
       __syncthreads();
+    } else if (LOCAL || !p.arrived) {
+      cluster.sync();
+    } else {
+      __syncthreads();
+      due += ctas;
+      int late = 0;
+      if (tid == 0) {
+        volatile int *arrived = p.arrived + g * kWardApart;
+        __threadfence();
+        atomicAdd((int *)arrived, 1);
+        late = 1;
+        for (int look = 0; late && look < kWardPatience; ++look) late = *arrived < due;
+        __threadfence();
+      }
+      gave_up = __syncthreads_or(late);
+    }
   };
   const float *src = p.pool_keys + g * (int64_t)P * D;
   float *sums_g = LOCAL ? nullptr : p.sums + g * (int64_t)P * D;
@@ -246,7 +271,7 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   for (int i = tid; i < P; i += kThreads) great = great || !(s.al[i] <= 1e15f);
   const float slack = __syncthreads_or(great) ? INFINITY : 9.5367431640625e-7f;
 
-  for (; rounds < p.max_rounds && n_alive > p.bucket_count; ++rounds) {
+  for (; rounds < p.max_rounds && n_alive > p.bucket_count && !gave_up; ++rounds) {
     // ---- the cheapest partners: tiles of (dirty x open) and (steady x merged), dealt to the CTAs in runs
     auto stage = [&](float *tile, const uint16_t *list, int from, int n) {
       for (int e = tid; e < TILE * (D / 4); e += kThreads) {
@@ -389,6 +414,7 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
     search_all(s.dirty, n_dirty, false, s.dirty, n_dirty, s.steady, n_steady);
     search_all(s.steady, n_steady, true, s.merged, n_merged, nullptr, 0);
     everyone();
+    if (gave_up) break;
 
     // ---- mutual cheapest pairs, held by their lower row; the cheapest of them merge, a tie to the lower row
     for (int i = tid; i < P; i += kThreads) {
@@ -509,10 +535,10 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
     p.labels[g * P + i] = number[r];
   }
   if (rank == 0 && tid == 0) {
-    p.reached[g] = n_alive <= p.bucket_count;
+    p.reached[g] = n_alive <= p.bucket_count && !gave_up;
     if (p.rounds) p.rounds[g] = rounds;
   }
-  if (ctas > 1) cluster.sync();  // (nobody's shared memory goes while another may still read it)
+  if (LOCAL && ctas > 1) cluster.sync();  // (nobody's shared memory goes while another may still read it)
 }
 
 static size_t align_up(size_t n) { return (n + 255) & ~(size_t)255; }
@@ -524,17 +550,20 @@ bool ward_cluster_takes(int d) { return d == 16 || d == 32 || d == 64; }
 size_t ward_cluster_workspace_bytes(int64_t G, int P, int d) {
   if (ward_is_local(P, d)) return 0;
   const size_t rows = (size_t)G * P;
-  return align_up(rows * d * 4) + 2 * align_up(rows * 4) + align_up(2 * rows * 8);
+  return align_up(rows * d * 4) + 2 * align_up(rows * 4) + align_up(2 * rows * 8) + (size_t)G * kWardApart * 4;
 }
 
 template <int D, bool LOCAL>
-static int launch_ward(const WardParams &p, int64_t G, cudaStream_t s) {
+static int launch_ward(WardParams &p, int64_t G, cudaStream_t s) {
   // CTAs a block: as many as leave every block an SM a CTA, and two of the small tiles or more a CTA in the first round
-  // (one block of 80 pools: 164 us with one CTA, 120 with five; 3 blocks of 256: 92 with four, 69 with eight).
+  // (one block of 80 pools: 164 us with one CTA, 120 with five; 3 blocks of 256: 92 with four, 69 with eight). A local block
+  // reads its cluster's shared memory, so it takes eight at most; a larger one has its rows and minima in the workspace, and
+  // any number of CTAs can share it.
   constexpr int TILE = ward_tile(LOCAL), SMALL = TILE / kWardRows * kWardFewRows;
   const int64_t tiles = (int64_t)((p.P + TILE - 1) / TILE) * ((p.P + SMALL - 1) / SMALL);
   const int64_t most = tiles / 2 < sm_count() / G ? tiles / 2 : sm_count() / G;
-  int ctas = (int)(most < 1 ? 1 : most < kWardMaxCtas ? most : kWardMaxCtas);
+  const int wanted = (int)(most < 1 ? 1 : most);
+  int ctas = wanted < kWardMaxCtas ? wanted : kWardMaxCtas;
   WardShared<D, LOCAL> shared;
   const size_t smem = shared.carve(nullptr, p.P, ctas > 1);
   if (!allow_shared(ward_kernel<D, LOCAL>, shared.carve(nullptr, LOCAL ? kWardLocalPools : kWardMaxPools, true))) {
@@ -545,9 +574,9 @@ static int launch_ward(const WardParams &p, int64_t G, cudaStream_t s) {
   config.gridDim = dim3((unsigned)(G * ctas)), config.blockDim = dim3(ward_threads(LOCAL));
   config.dynamicSmemBytes = smem, config.stream = s;
   cudaLaunchAttribute attribute[1];
+  config.attrs = attribute, config.numAttrs = ctas > 1;
   attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = (unsigned)ctas, attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
-  config.attrs = attribute, config.numAttrs = 1;
+  attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
   // (a cluster lives inside a GPC, and 148 SMs hold fewer clusters of eight than 18: one CTA less a block where a second
   // wave would follow)
   for (int fit = 0; ctas > 1; --ctas) {
@@ -555,7 +584,22 @@ static int launch_ward(const WardParams &p, int64_t G, cudaStream_t s) {
     if (cudaOccupancyMaxActiveClusters(&fit, ward_kernel<D, LOCAL>, &config) != cudaSuccess) (void)cudaGetLastError();
     if (fit >= G) break;
   }
-  config.gridDim = dim3((unsigned)(G * ctas)), attribute[0].val.clusterDim.x = (unsigned)ctas;
+  attribute[0].val.clusterDim.x = (unsigned)ctas;
+  // A larger block whose clusters leave SMs idle (16 blocks: six CTAs each, 96 of 148 SMs) takes a cooperative grid and a
+  // counter in memory as its barrier. Pairings, one cluster a block -> the grid: one block of 4,096 buckets 2,322 -> 455 us, of
+  // 1,024 253 -> 159; 16 blocks of 4,096 3,124 -> 2,166, of 640 no change. Of as many CTAs the cluster is the faster (its barrier
+  // is: 32 blocks of 640 256 us, 268 as a grid), so it stays where it has them.
+  if (LOCAL || wanted <= ctas) {
+    p.arrived = nullptr;
+  } else {
+    ctas = wanted;
+    config.numAttrs = 1;
+    attribute[0].id = cudaLaunchAttributeCooperative;
+    attribute[0].val.cooperative = 1;
+    if (cudaMemsetAsync(p.arrived, 0, (size_t)G * kWardApart * 4, s) != cudaSuccess) return LSA_ERR_LAUNCH;
+  }
+  p.ctas = ctas;
+  config.gridDim = dim3((unsigned)(G * ctas));
   (void)cudaLaunchKernelEx(&config, ward_kernel<D, LOCAL>, p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
@@ -575,7 +619,8 @@ int ward_cluster_run(const float *pool_keys, const float *pool_sizes, float unif
     p.sums = (float *)at, at += align_up(rows * d * 4);
     p.sq = (float *)at, at += align_up(rows * 4);
     p.al = (float *)at, at += align_up(rows * 4);
-    p.cheapest = (unsigned long long *)at;
+    p.cheapest = (unsigned long long *)at, at += align_up(2 * rows * 8);
+    p.arrived = (int *)at;
   }
   if (d == 64) return local ? launch_ward<64, true>(p, G, s) : launch_ward<64, false>(p, G, s);
   if (d == 32) return local ? launch_ward<32, true>(p, G, s) : launch_ward<32, false>(p, G, s);

@@ -165,8 +165,7 @@ def ward_rounds(pools: torch.Tensor, pool_sizes: torch.Tensor | float, bucket_co
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, device=pools.device, dtype=torch.uint8)
     call("lsa_ward_merge", ptr(pools), ptr(sizes), uniform, G, P, d, bucket_count, float(bucket_cap), max_rounds,
-         ptr(labels), ptr(raw_reached), ptr(rounds), ptr(workspace) if need else None, need, stream(),
-         launches=1 if not need else 2 + 2 * max_rounds)
+         ptr(labels), ptr(raw_reached), ptr(rounds), ptr(workspace) if need else None, need, stream())
     if reached is not None:
         return labels, raw_reached
     if return_rounds:

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import cuda
+from helpers import cuda, mixture, unit_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -128,7 +128,7 @@ def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monk
 
 @pytest.mark.parametrize("rows", [129, 700, 19000])  # (32 rows a CTA, and 64)
 @pytest.mark.parametrize("d_in,d_idx", [(256, 32), (192, 64), (130, 64), (64, 60), (256, 128), (100, 100)])
-def test_the_exact_map_keeps_the_oracle_s_bits(oracle, rows, d_in, d_idx):
+def test_the_exact_map_keeps_the_oracle_s_bits(rows, d_in, d_idx):
     """Whole slices of input and output dims and ragged ones, against the oracle's product in its own order, bit for bit."""
     from lsa_b200 import ops
 
@@ -141,3 +141,27 @@ def test_the_exact_map_keeps_the_oracle_s_bits(oracle, rows, d_in, d_idx):
         want = (x[some, k, None].astype(np.float64) * w[k].astype(np.float64) + want.astype(np.float64)).astype(np.float32)
     off = got[some].view(np.int32).astype(np.int64) - want.view(np.int32)
     assert (off == 0).mean() >= 0.999 and np.abs(got[some] - want).max() <= 1e-4  # (a double rounding in a million)
+
+
+@pytest.mark.parametrize("G,P,d", [(1, 1025, 64), (16, 640, 32), (20, 520, 64), (32, 640, 16), (5, 4096, 16)])
+def test_ward_over_clusters_and_over_a_grid_keeps_the_oracle_s_labels(oracle, G, P, d):
+    """Blocks past one CTA's shared memory as grids of 148, 9, 7 and 29 CTAs a block and as clusters of four, in turn on the same
+    workspace (the counters of arrivals are set up by every call), and replayed from a graph."""
+    from lsa_b200 import ops
+
+    keys = unit_rows(mixture(G * P, d, 24, 0.4, G + P)).reshape(G, P, d)
+    count = (P + 1) // 2  # (pairs, and the one left over)
+    want, want_reached, want_rounds = oracle.ward_rounds(keys, np.ones((G, P), dtype=np.float32), count, 2.0, return_rounds=True)
+    pools, workspace = cuda(keys), torch.full((64 << 20,), 255, device="cuda", dtype=torch.uint8)
+    for _ in range(2):
+        got, reached, rounds = ops.ward_rounds(pools, 1.0, count, 2.0, return_rounds=True, workspace=workspace)
+        assert np.array_equal(got.cpu().numpy(), want) and np.array_equal(rounds.cpu().numpy(), want_rounds)
+        assert np.array_equal(reached.cpu().numpy(), want_reached)
+    labels, flags = torch.empty_like(got), torch.empty(G, device="cuda", dtype=torch.uint8)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.ward_rounds(pools, 1.0, count, 2.0, labels=labels, reached=flags, workspace=workspace)
+    for _ in range(2):
+        labels.fill_(-1)
+        graph.replay()
+        assert np.array_equal(labels.cpu().numpy(), want) and np.array_equal(flags.bool().cpu().numpy(), want_reached)
