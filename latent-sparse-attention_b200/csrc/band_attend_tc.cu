@@ -17,7 +17,8 @@
 //
 // A row's exponents are taken against a running maximum that follows the true one lazily: it moves, and O and the sum so far
 // are scaled, only when a tile holds a score 2^8 times as heavy. (O is complete then: the issuing warp's commit of S covers
-// every product before it.) Probabilities are 2^8 at most, and their two terms hold them to 2^-17 of themselves, so what the
+// every product before it. And a product adds to all 128 columns of O, of which a row's two threads scale 64 each: none is
+// issued until the threads of BOTH halves have arrived with their P, and with it their columns scaled.) Probabilities are 2^8 at most, and their two terms hold them to 2^-17 of themselves, so what the
 // reference point is does not show.
 //
 // What bounds it is the tensor pipe: a step of a tile is 1,536 cycles of products (the two terms of P cost a second product),
@@ -76,8 +77,8 @@ __global__ void __launch_bounds__(kBtThreads, 1)
                           const __grid_constant__ CUtensorMap map_bf16, BandTcParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // full / empty: a ring slot has landed / may be overwritten; s_ready: S of a tile is there (and every product issued
-  // before it is over); p_ready: the P of 64 keys is; o_done: a tile's last product is over; q_full, drained once.
-  enum { kFull = 0, kEmpty = kBtStages, kSReady = 2 * kBtStages, kPReady = kSReady + 2, kODone = kPReady + 4,
+  // before it is over); p_ready: P of a tile is, and O scaled; o_done: a tile's last product is over; q_full, drained once.
+  enum { kFull = 0, kEmpty = kBtStages, kSReady = 2 * kBtStages, kPReady = kSReady + 2, kODone = kPReady + 2,
          kQFull = kODone + 2, kDrained = kQFull + 1, kBars = kDrained + 1 };
   __shared__ __align__(8) uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(kBtThreads, 1)
   };
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kBars; ++i) mbar_init(bar(i), i >= kPReady && i < kODone ? kBtRows : 1);
+    for (int i = 0; i < kBars; ++i) mbar_init(bar(i), i >= kPReady && i < kODone ? 2 * kBtRows : 1);
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -190,22 +191,21 @@ __global__ void __launch_bounds__(kBtThreads, 1)
         for (int t = 0; t < kBtTiles; ++t) {
           const uint32_t s_col = tmem + t * kBtKeys, o_col = tmem + kBtOCol + t * 128;
           if (pending >> t & 1) {
+            ok = ok && wait(kPReady + t, p_phase >> t & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-              ok = ok && wait(kPReady + 2 * t + half, p_phase >> t & 1);
-              if (!ok) break;
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              if (elect_one()) {
+              for (int half = 0; half < 2; ++half)
 #pragma unroll
                 for (int term = 0; term < 2; ++term)
 #pragma unroll
                   for (int k = 0; k < 4; ++k)  // 16 keys: 8 columns of P, 2,048 bytes down a plane of V
                     umma_bf16_ts(o_col, s_col + 64 * half + 32 * (k >> 1) + 16 * term + 8 * (k & 1),
                                  v_tile + (4 * half + k) * (2048 >> 4), idesc_o, (half | term | k) != 0 || started[t]);
-                if (half == 1 && n > lasts[t]) umma_commit(bars_at + 8 * (kODone + t));
-              }
-              __syncwarp();
+              if (n > lasts[t]) umma_commit(bars_at + 8 * (kODone + t));
             }
+            __syncwarp();
             p_phase ^= 1u << t, started[t] = true;
           }
           if (ok && n < tiles && (seen >> t & 1)) {
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kBtThreads, 1)
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(kPReady + 2 * t + half)) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(kPReady + t)) : "memory");
       ++steps;
     }
     float a, b, c, d;

@@ -53,6 +53,37 @@ def test_a_running_maximum_that_grows_keeps_the_sums():
     assert (got.double() - want).norm() <= 2 ** -12 * want.norm()
 
 
+@pytest.mark.parametrize("listed", [False, True])
+def test_a_maximum_that_moves_at_every_tile_scales_whole_rows_of_o(listed):
+    """Scores that climb by 9 to 20 in log2 a key tile, so that nearly every product finds an O that two threads a row have just
+    scaled: more CTAs than SMs, again and again, against 64 bits and bit for bit against the first time. Exponents of up to 700 in
+    fp32 are off by 2^-24 of it and the 128 terms of a product by some bits more: 2^-12 of a probability."""
+    from lsa_b200 import ops
+
+    R, n, Hq, Hkv = 1024, 4096, 40, 8
+    gen = torch.Generator(device="cuda").manual_seed(int(listed))
+    towards = torch.nn.functional.normalize(torch.randn(Hkv, 128, device="cuda", generator=gen), dim=-1)
+    tile = torch.arange(n, device="cuda")[:, None, None] // 128
+    k = (towards * tile + 0.3 * torch.randn(n, Hkv, 128, device="cuda", generator=gen)).bfloat16()
+    steep = torch.empty(R, Hq, 1, device="cuda").uniform_(9.0, 20.0, generator=gen) * 128 ** 0.5 * 0.6931471805599453
+    q = (steep * towards.repeat_interleave(Hq // Hkv, dim=0)).bfloat16()
+    v = torch.randn(n, Hkv, 128, device="cuda", generator=gen).bfloat16()
+    keep = torch.arange(n, device="cuda") <= n - R + torch.arange(R, device="cuda")[:, None]
+    if listed:
+        keep &= torch.rand(R, n, device="cuda", generator=gen) < 0.5
+        mask = _bits(keep)
+    out = torch.empty(R, Hq, 128, device="cuda")
+    read = lambda: ops.listed_attend(q, k, v, n - R, mask, 128 ** -0.5, out) if listed else \
+        ops.causal_attend(q, k, v, n - R, 128 ** -0.5, out=out)
+    first = read().clone()
+    for h in range(Hkv):
+        heads = slice(h * Hq // Hkv, (h + 1) * Hq // Hkv)
+        want, _ = _read(q[:, heads], k[:, h:h + 1], v[:, h:h + 1], keep)
+        assert (first[:, heads].double() - want).norm() <= 2 ** -12 * want.norm()
+    for _ in range(40):
+        assert torch.equal(read(), first)
+
+
 def _bits(keep):
     """keep [R, n] bool as words [tiles, R, 4] int32."""
     R, n = keep.shape
