@@ -22,11 +22,11 @@
 // reference point is does not show.
 //
 // What bounds it is the tensor pipe: a step of a tile is 1,536 cycles of products (the two terms of P cost a second product),
-// beside some 1,900 of softmax that four warps a scheduler share. 16,384 causal rows of 40 heads over 8: 3.30 ms, 834 TFLOP/s of
-// useful work and 1,250 with the second term counted (5.61 ms when the keys were walked twice, maxima then sums, with P in shared
-// memory and one tile a CTA); a masked read of the same rows a tenth more. 8,192 rows of a band of 1,024 keys 0.40 ms (0.53):
-// a CTA's ten steps stand beside its start and its end. Tried: S in two buffers of 64 keys a tile (products of two widths are not
-// kept in order, and drain the pipe), a thread a row (a softmax of 3,400 cycles a step).
+// beside some 1,900 of softmax that four warps a scheduler share, and the wait between a tile's P V and the S that is written over
+// its P. 16,384 causal rows of 40 heads over 8: 3.39 ms, 811 TFLOP/s of useful work and 1,217 with the second term counted (3.24
+// without the wait; 5.61 when the keys were walked twice, maxima then sums, with P in shared memory and one tile a CTA); a masked
+// read of the same rows 3.65. 8,192 rows of a band of 1,024 keys 0.40 ms (0.53): a CTA's ten steps stand beside its start and its
+// end. Tried: S in two buffers of 64 keys a tile (drains the pipe), a thread a row (a softmax of 3,400 cycles a step).
 //
 // Every wait on an mbarrier is bounded; a wait that gives up raises the CTA's abort flag and the status word, the
 // roles drain, the tensor memory is freed and the CTA leaves.
@@ -77,9 +77,10 @@ __global__ void __launch_bounds__(kBtThreads, 1)
                           const __grid_constant__ CUtensorMap map_bf16, BandTcParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // full / empty: a ring slot has landed / may be overwritten; s_ready: S of a tile is there (and every product issued
-  // before it is over); p_ready: P of a tile is, and O scaled; o_done: a tile's last product is over; q_full, drained once.
+  // before it is over); p_ready: P of a tile is, and O scaled; pv_done: P V of a tile is over,
+  // o_done: the last one of it; q_full, drained once.
   enum { kFull = 0, kEmpty = kBtStages, kSReady = 2 * kBtStages, kPReady = kSReady + 2, kODone = kPReady + 2,
-         kQFull = kODone + 2, kDrained = kQFull + 1, kBars = kDrained + 1 };
+         kPvDone = kODone + 2, kQFull = kPvDone + 2, kDrained = kQFull + 1, kBars = kDrained + 1 };
   __shared__ __align__(8) uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
@@ -203,9 +204,12 @@ __global__ void __launch_bounds__(kBtThreads, 1)
                   for (int k = 0; k < 4; ++k)  // 16 keys: 8 columns of P, 2,048 bytes down a plane of V
                     umma_bf16_ts(o_col, s_col + 64 * half + 32 * (k >> 1) + 16 * term + 8 * (k & 1),
                                  v_tile + (4 * half + k) * (2048 >> 4), idesc_o, (half | term | k) != 0 || started[t]);
-              if (n > lasts[t]) umma_commit(bars_at + 8 * (kODone + t));
+              umma_commit(bars_at + 8 * ((n > lasts[t] ? kODone : kPvDone) + t));
             }
             __syncwarp();
+            // S of the next keys is written over the P that these products read: they have to be over. (Products are kept in
+            // order by themselves only where they have one accumulator and one shape.)
+            if (n <= lasts[t]) ok = wait(kPvDone + t, p_phase >> t & 1);
             p_phase ^= 1u << t, started[t] = true;
           }
           if (ok && n < tiles && (seen >> t & 1)) {
