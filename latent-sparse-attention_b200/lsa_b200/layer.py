@@ -393,19 +393,35 @@ class FlatLayer:
         layer keeps, so after the first call a step allocates nothing beside it but its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
         `band` reads the window and the sinks as dense tiles; `bucket_major` reads the selected keys bucket by bucket
         where the shapes allow and it is the faster read (both off: every row gathers its whole list).
+
+        `chunk` is how many rows are worked on at a time, and with that how large the buffers get. Rows that are read through
+        masks (`_listed_until`) are taken two waves of the GPU at a time where that is more, their tensors are what the masked
+        read takes and there is memory for it; else, as all others, `chunk` at a time.
         """
         T = q.shape[0]
         index = self.build_index(k, reuse_buffers=not return_index)
         out = torch.empty_like(q) if out is None else out
         whole = min(T, self._whole_until(index)) if band else 0  # (rows that read everything make chunks of their own)
-        listed = max(whole, min(T, self._listed_until())) if band and bucket_major else whole
-        # (a CTA of the masked read has 256 rows of a head: chunks of fewer than two waves leave part of the GPU idle, 24,576
-        # tokens of 8 heads in chunks of 2,048 rows 7.1 ms and 4.8 this way)
-        waves = -(-2 * 148 * 256 // self.heads // 128) * 128
-        for first, end, step in ((0, whole, chunk), (whole, listed, max(chunk, waves)), (listed, T, chunk)):
-            for start in range(first, end, step):
-                stop = min(end, start + step)
+
+        def read(first: int, end: int) -> None:
+            for start in range(first, end, chunk):
+                stop = min(end, start + chunk)
                 self.prefill_rows(q[start:stop], start, k, v, index, out[start:stop], band, bucket_major)
+
+        read(0, whole)
+        first = whole
+        if band and bucket_major and ops.dense_attend_supported(q, k, v, out) and whole < min(T, self._listed_until()):
+            # (a CTA of the masked read has 256 rows of a head: chunks of fewer than two waves leave part of the GPU idle, 24,576
+            # tokens of 8 heads in chunks of 2,048 rows 7.1 ms and 4.8 this way)
+            sms = torch.cuda.get_device_properties(q.device).multi_processor_count
+            step = max(chunk, -(-2 * sms * 256 // self.heads // 128) * 128)
+            listed = min(T, self._listed_until())
+            for first in range(whole, listed, step):
+                stop = min(listed, first + step)
+                if stop - first <= chunk or not self._reads_wide(q[first:stop], first, k, v, index, out[first:stop]):
+                    read(first, stop)
+            first = listed
+        read(first, T)
         return (out, index) if return_index else out
 
     def prefill_from_host(self, q_host: torch.Tensor, k_host: torch.Tensor, v_host: torch.Tensor,
@@ -516,19 +532,49 @@ class FlatLayer:
 
     most_listed = 1600 * 128  # positions whose bits `ops.list_bits` holds in a CTA's shared memory, eight rows of them
 
-    def _list_masks(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor):
+    def _list_masks(self, rows: torch.Tensor, start: int, k: torch.Tensor):
         """Memory for the masks of a chunk that is read through them ([key tiles, rows, 4] int32, the allocator's again after the
-        chunk); None for one that is not: rows past `_listed_until`, tensors the dense read does not take, too few rows for its
-        tiles, or no memory."""
+        chunk); None for one that is not: rows past `_listed_until`, too few of them for its tiles, or no memory. (The caller has
+        asked whether the dense read takes the tensors.)"""
         n = rows.shape[0]
         stop = start + n
-        if n < 128 or start >= self._listed_until() or stop > self.most_listed or k.shape[0] < stop or \
-                not ops.dense_attend_supported(rows, k, v, out):
+        if n < 128 or start >= self._listed_until() or stop > self.most_listed or k.shape[0] < stop:
             return None
         try:
             return torch.empty(-(-stop // 128) * n * 16, device=rows.device, dtype=torch.uint8).view(torch.int32).view(-1, n, 4)
         except torch.OutOfMemoryError:
             return None
+
+    def _read_listed(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
+                     out: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
+        """The masked read of rows that `_list_masks` gave `mask` for."""
+        d = self.design
+        index_queries, positions = self._query_rows(rows, start)
+        picked, positions, row_p, row_k = self._pick(index_queries, positions, index, self._room, start + rows.shape[0] - 1)
+        with probe.region("expand"):
+            ops.list_bits(picked, positions, index.buckets.bucket_members, d.top_k, d.sink_size, d.window_size, k.shape[0],
+                          mask.shape[0], row_p, row_k, self._expand_status, out=mask)
+        with probe.region("attend"):
+            return ops.listed_attend(rows, k, v, start, mask, self.scale, out, self._attend_status)
+
+    def _reads_wide(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
+                    out: torch.Tensor) -> bool:
+        """A chunk of more rows than the caller asked for, read through masks; False where there is no memory for it."""
+        mask = self._list_masks(rows, start, k)
+        if mask is None:
+            return False
+        try:
+            self._read_listed(rows, start, k, v, index, out, mask)
+        except torch.OutOfMemoryError:
+            return False
+        return True
+
+    def _query_rows(self, rows: torch.Tensor, start: int) -> tuple:
+        """Index queries and positions of consecutive rows at positions start.."""
+        n, dev = rows.shape[0], rows.device
+        positions = torch.arange(start, start + n, device=dev)
+        with probe.region("index map"):
+            return self.index_queries(rows, out=self._room("index queries", (n, self.index_dim), torch.float32, dev)), positions
 
     def prefill_rows(self, rows: torch.Tensor, start: int, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, band: bool = True, bucket_major: bool = True) -> torch.Tensor:
@@ -555,24 +601,16 @@ class FlatLayer:
                 return out
             self.prefill_rows(rows[whole:], start + whole, k, v, index, out[whole:], band, bucket_major)
             return out
+        masked = band and bucket_major and ops.dense_attend_supported(rows, k, v, out)
         listed = self._listed_until() - start
-        if band and bucket_major and 0 < listed < n:  # (a row's read depends on its position, not on the chunk it is in)
+        if masked and 0 < listed < n:  # (a row's read depends on its position, not on the chunk it is in)
             self.prefill_rows(rows[:listed], start, k, v, index, out[:listed], band, bucket_major)
             self.prefill_rows(rows[listed:], start + listed, k, v, index, out[listed:], band, bucket_major)
             return out
-        positions = torch.arange(start, stop, device=dev)
-        with probe.region("index map"):
-            index_queries = self.index_queries(rows, out=self._room("index queries", (n, self.index_dim),
-                                                                    torch.float32, dev))
-        mask = self._list_masks(rows, start, k, v, out) if band and bucket_major else None
+        mask = self._list_masks(rows, start, k) if masked else None
         if mask is not None:
-            picked, positions, row_p, row_k = self._pick(index_queries, positions, index, self._room, stop - 1)
-            d = self.design
-            with probe.region("expand"):
-                ops.list_bits(picked, positions, index.buckets.bucket_members, d.top_k, d.sink_size, d.window_size, k.shape[0],
-                              mask.shape[0], row_p, row_k, self._expand_status, out=mask)
-            with probe.region("attend"):
-                return ops.listed_attend(rows, k, v, start, mask, self.scale, out, self._attend_status)
+            return self._read_listed(rows, start, k, v, index, out, mask)
+        index_queries, positions = self._query_rows(rows, start)
         # The window and the sinks are the same keys for neighbouring rows: one dense band serves them, and the
         # read of the selected keys starts from its partial result.
         banded = band and self.design.sink_size <= 64 and k.shape[0] >= stop

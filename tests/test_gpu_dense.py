@@ -199,3 +199,35 @@ def test_a_prefill_read_through_masks_is_the_one_read_by_lists(T, Hq, Hkv, chunk
         got = layer.prefill(odd, k, v, chunk=chunk).float()
         # (rows that no tensor map can walk are mapped in fp32: another bucket where two scores nearly tie)
         assert not listed and ((got - gathered).abs().amax((1, 2)) <= 2e-2).float().mean() >= 0.98
+
+
+@pytest.mark.parametrize("short", ["masks", "picks"])
+def test_a_prefill_without_memory_for_wide_masks_keeps_to_its_chunk(short, monkeypatch):
+    """Where a chunk of more rows than were asked for finds no memory, for its masks or later, the rows go `chunk` at a time, and
+    are the rows that they are then."""
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    T, Hq, Hkv, chunk = 5000, 8, 2, 1024
+    rng = np.random.default_rng(T)
+    w = [cuda(rng.standard_normal((Hkv * 128, 64), dtype=np.float32) / 16, torch.bfloat16) for _ in range(2)]
+    layer = FlatLayer(FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=300,
+                                 sink_size=4, window_size=128), *w, Hq, Hkv, 128)
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(T, Hq, Hkv, 128, 16, T))
+    wide = layer.prefill(q, k, v, chunk=chunk).float()
+    asked = []
+    name = "_list_masks" if short == "masks" else "_pick"
+    given = getattr(FlatLayer, name)
+
+    def refuse(self, rows, *args):
+        asked.append(rows.shape[0])
+        if rows.shape[0] > chunk:
+            if short == "picks":
+                raise torch.OutOfMemoryError("no memory")
+            return None
+        return given(self, rows, *args)
+
+    monkeypatch.setattr(FlatLayer, name, refuse)
+    got = layer.prefill(q, k, v, chunk=chunk)
+    assert asked[0] > chunk and max(asked[1:]) <= chunk and len(asked) > 2
+    assert (got.float() - wide).abs().max() <= 2e-2 and (got.float() - wide).abs().mean() <= 2e-3
+    layer.check()

@@ -279,3 +279,25 @@ def test_wide_buckets_go_to_the_gather_where_it_alone_takes_the_call():
     out = torch.zeros(3, 4, 128, dtype=torch.bfloat16)
     assert takes(128)(rows, out) and not takes(128)(odd, out) and not takes(128)(rows, out.float())
     assert takes(64)(odd, out.float())
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (2, 1, 64)])
+def test_a_prefill_that_no_mask_serves_keeps_to_its_chunk(heads, kv_heads, head_dim, monkeypatch):
+    """Heads that the masked read does not take go `chunk` rows at a time, before its line as past it."""
+    from types import SimpleNamespace
+
+    from lsa_b200.core import Buckets
+    from lsa_b200.layer import FlatLayer
+
+    layer = FlatLayer(FlatDesign(), torch.zeros(kv_heads * head_dim, 64), torch.zeros(kv_heads * head_dim, 64), heads, kv_heads,
+                      head_dim)
+    T, chunk, pieces = 9000, 2048, []
+    assert layer._listed_until() > T
+    index = SimpleNamespace(buckets=Buckets(torch.zeros(1000, 64), None, None, 32, 256))
+    monkeypatch.setattr(FlatLayer, "build_index", lambda self, k, reuse_buffers: index)
+    monkeypatch.setattr(FlatLayer, "prefill_rows", lambda self, rows, start, *a: pieces.append((start, rows.shape[0])))
+    q, k = torch.zeros(T, heads, head_dim, dtype=torch.bfloat16), torch.zeros(T, kv_heads, head_dim, dtype=torch.bfloat16)
+    layer.prefill(q, k, k, chunk=chunk)
+    assert max(n for _, n in pieces) <= chunk
+    assert [start for start, _ in pieces] == [0, *torch.tensor([n for _, n in pieces]).cumsum(0)[:-1].tolist()]
+    assert sum(n for _, n in pieces) == T
