@@ -366,6 +366,7 @@ int lsa_beam_step_split(const float *queries, int64_t R, int d, const float *vec
  *              their lengths, as the attention entry points do, saves the write of the padding)
  *   selected   [R, top_k + window + sink] int32 out - expansion, window ascending, sinks ascending, -1 padded
  *   lengths    [R] int32 out
+ *   status     raised by every picked bucket id outside [0, m) up to where a row's top_k is reached (a few rows: by every one)
  * --------------------------------------------------------------------------------------------------------- */
 int lsa_expand(const int32_t *picked, int64_t R, int top_p, const int64_t *positions, const int32_t *members,
                int64_t m, int bucket_cap, const int32_t *row_top_p, const int32_t *row_top_k, int top_k,

@@ -41,7 +41,8 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
     const int64_t key_end = min(p.n_keys, (int64_t)p.tiles * 128);
     int counted = 0, bad = 0;
     const int in_step = 32 / p.lanes, first = lane % p.lanes * p.places, places = min(p.places, p.cap - first);
-    for (int i0 = 0; i0 < row_p && counted < row_k; i0 += in_step) {
+    int i0 = 0;
+    for (; i0 < row_p && counted < row_k; i0 += in_step) {
       const int i = i0 + lane / p.lanes;
       int64_t bucket = i < row_p ? p.picked[r * p.top_p + i] : -1;
       if (bucket >= p.m) {
@@ -93,6 +94,8 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
       }
       counted += __shfl_sync(0xffffffffu, incl, 31);
     }
+    // (picks past the cut add no key, but those outside the table are told of as well)
+    for (int i = i0 + lane; i < row_p; i += 32) bad += p.picked[r * p.top_p + i] >= p.m;
     __syncwarp();
     // the window, and the sinks that lie before it
     const int64_t end = min(pos + 1, key_end), sinks = min((int64_t)p.sink, min(window_start, end));

@@ -149,11 +149,12 @@ def test_lists_as_bits_are_the_lists(cap, top_p, top_k, sink, window, sizes):
     picked = np.stack([rng.permutation(m)[:top_p] if top_p <= m else rng.permutation(top_p) for _ in range(R)]).astype(np.int32)
     picked[picked >= m] = -1
     picked[3, 0] = m + 7
+    picked[4:, -1] = np.where(rng.random(R - 4) < 0.5, m + 1, picked[4:, -1])  # (most of them past the cut at top-k)
     row_p = rng.integers(-1, top_p + 1, R).astype(np.int32)
     row_k = rng.integers(-1, top_k + 1, R).astype(np.int32)
     args = (cuda(picked), cuda(positions), cuda(members), top_k, sink, window)
     for budgets in ((None, None), (cuda(row_p), cuda(row_k))):
-        lists, lengths, bad = ops.expand(*args, *budgets)
+        lists, lengths, _ = ops.expand(*args, *budgets)
         for keys in (T, 1111):
             status = torch.zeros(1, dtype=torch.int32, device="cuda")
             words = ops.list_bits(*args, keys, -(-T // 128), *budgets, status=status).cpu().numpy().view(np.uint32)
@@ -161,7 +162,8 @@ def test_lists_as_bits_are_the_lists(cap, top_p, top_k, sink, window, sizes):
             for r in range(R):
                 ids = lists[r, :lengths[r]].cpu().numpy()
                 assert np.array_equal(np.flatnonzero(bits[r]), np.sort(ids[ids < keys])), (r, positions[r])
-            assert int(status) == int(bad)
+            within = np.arange(top_p) < (np.full(R, top_p) if budgets[0] is None else row_p.clip(0))[:, None]
+            assert int(status) == ((picked >= m) & within).sum()  # (every one, where `expand` may stop at the cut)
 
 
 @pytest.mark.parametrize("T,Hq,Hkv,chunk,sizes", [
