@@ -7,6 +7,7 @@ for a single request whose KV rows sit at their positions.
 
 from __future__ import annotations
 
+import operator
 from dataclasses import dataclass
 
 import torch
@@ -658,15 +659,19 @@ class FlatLayer:
 
     def _decodes_in_one_call(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                              index: FlatIndex) -> bool:
-        """Whether a step may go to the GPU as one call: where the calls it is made of would take these tensors as they are."""
+        """Whether a step may go to the GPU as one call: where the calls it is made of would take these tensors as they are, and
+        the methods that make them are this class's own."""
         d, b = self.design, index.buckets
+        if _stages_of(type(self)) != _DECODE_STAGES or not _STAGE_NAMES.isdisjoint(self.__dict__):
+            return False
         return q.dim() == 3 and 0 < q.shape[0] <= 8 and q.shape[1:] == (self.heads, self.head_dim) and d.early_budget is None \
             and index.shapes is None and d.top_p <= 128 and self.index_dim in (32, 64) and not probe.listening() \
             and positions.dtype == torch.int64 and positions.shape == q.shape[:1] and q.stride(2) == k.stride(2) == v.stride(2) == 1 \
             and k.stride() == v.stride() and k.shape[1:] == v.shape[1:] == (self.kv_heads, self.head_dim) \
             and q.dtype == k.dtype == v.dtype == torch.bfloat16 and positions.is_contiguous() \
             and b.bucket_centroids.dtype == torch.float32 and b.bucket_members.dtype == torch.int32 \
-            and b.bucket_centroids.is_contiguous() and b.bucket_members.is_contiguous()
+            and b.bucket_centroids.is_contiguous() and b.bucket_members.is_contiguous() \
+            and b.bucket_centroids.shape[1] == self.index_dim and b.bucket_members.shape[0] == b.bucket_centroids.shape[0]
 
     def decode(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor, index: FlatIndex,
                splits: int = 8):
@@ -680,3 +685,9 @@ class FlatLayer:
         lists, lengths = self.select(self.index_queries(q), positions, index)
         out, _ = self.attend(q, k, v, lists, lengths, splits=splits)
         return out
+
+
+# What `FlatLayer.decode` is made of: a layer that has another of these has it called.
+_STAGE_NAMES = frozenset(("index_queries", "select", "_select", "_pick", "attend"))
+_stages_of = operator.attrgetter(*_STAGE_NAMES)
+_DECODE_STAGES = _stages_of(FlatLayer)

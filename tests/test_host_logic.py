@@ -301,3 +301,39 @@ def test_a_prefill_that_no_mask_serves_keeps_to_its_chunk(heads, kv_heads, head_
     assert max(n for _, n in pieces) <= chunk
     assert [start for start, _ in pieces] == [0, *torch.tensor([n for _, n in pieces]).cumsum(0)[:-1].tolist()]
     assert sum(n for _, n in pieces) == T
+
+
+def test_a_decode_step_in_one_call_calls_no_method_that_another_layer_has_of_its_own(monkeypatch):
+    """A subclass or a layer with a stage of its own, or tables that are not of the layer's sizes: the stages one by one."""
+    from types import SimpleNamespace
+
+    from lsa_b200.core import Buckets
+    from lsa_b200.layer import FlatLayer
+
+    sizes = FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=64, top_p=8, top_k=64, sink_size=4,
+                       window_size=64)
+    make = lambda kind: kind(sizes, torch.zeros(256, 64), torch.zeros(256, 64), 4, 2, 128)
+    buckets = lambda m, rows, d: SimpleNamespace(buckets=Buckets(torch.zeros(m, d), torch.zeros(rows, 16, dtype=torch.int32), None,
+                                                                 8, 64), shapes=None)
+    index = buckets(64, 64, 64)
+    q, k = torch.zeros(2, 4, 128, dtype=torch.bfloat16), torch.zeros(600, 2, 128, dtype=torch.bfloat16)
+    args = (q, torch.tensor([500, 599]), k, k)
+    assert make(FlatLayer)._decodes_in_one_call(*args, index)
+    for other in (buckets(64, 63, 64), buckets(64, 64, 32)):
+        assert not make(FlatLayer)._decodes_in_one_call(*args, other)
+    for stage in ("index_queries", "select", "_pick", "attend"):
+        own = type("Own", (FlatLayer,), {stage: lambda self, *a, **kw: None})
+        assert not make(own)._decodes_in_one_call(*args, index)
+        layer = make(FlatLayer)
+        setattr(layer, stage, lambda *a, **kw: None)
+        assert not layer._decodes_in_one_call(*args, index)
+        with monkeypatch.context() as patch:
+            patch.setattr(FlatLayer, stage, lambda self, *a, **kw: None)
+            assert not make(FlatLayer)._decodes_in_one_call(*args, index)
+    # `decode` calls them
+    called = []
+    layer = make(type("Own", (FlatLayer,), {"select": lambda self, *a: (None, None),
+                                            "index_queries": lambda self, q: called.append("map"),
+                                            "attend": lambda self, *a, **kw: (called.append("attend"), None)}))
+    layer.decode(*args, index)
+    assert called == ["map", "attend"]
