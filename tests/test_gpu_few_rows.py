@@ -126,6 +126,23 @@ def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monk
     layer.check()
 
 
+def test_a_step_before_the_first_block_has_closed_is_refused_either_way(monkeypatch):
+    """An index without a bucket (a cache shorter than a cluster block): the scan of a few rows takes no empty table, in one call
+    or one by one."""
+    from helpers import layer_inputs
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    w = [cuda(np.zeros((256, 64), dtype=np.float32), torch.bfloat16) for _ in range(2)]
+    layer = FlatLayer(FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200,
+                                 sink_size=4, window_size=32), *w, 8, 2, 128)
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(100, 8, 2, 128, 16, 100))
+    index, positions = layer.build_index(k), cuda(np.array([99, 50]))
+    for once in (True, False):
+        monkeypatch.setattr(FlatLayer, "_decodes_in_one_call", lambda *a: once)
+        with pytest.raises(ValueError, match="NULL"):
+            layer.decode(q[positions], positions, k, v, index)
+
+
 @pytest.mark.parametrize("rows", [129, 700, 19000])  # (32 rows a CTA, and 64)
 @pytest.mark.parametrize("d_in,d_idx", [(256, 32), (192, 64), (130, 64), (64, 60), (256, 128), (100, 100)])
 def test_the_exact_map_keeps_the_oracle_s_bits(rows, d_in, d_idx):
