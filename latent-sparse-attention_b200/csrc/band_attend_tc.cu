@@ -51,25 +51,6 @@ constexpr float kBtLazy = 8.0f;                      // the running maximum move
 static_assert(kBtRows == kBtKeys, "query and key tiles share a plane's size");
 static_assert(16 * 8192 <= kBtStages * kBtSlot, "the softmax warps' finished rows leave through the ring");
 
-__device__ __forceinline__ uint64_t pair_of(float a, float b) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ void split_pair(uint64_t d, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
-}
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 template <bool LISTED>
 __global__ void __launch_bounds__(kBtThreads, 1)
     band_attend_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,

@@ -128,6 +128,36 @@ def test_masked_rows_read_the_keys_they_list(R, first, Hq, Hkv):
         assert torch.equal(odd, keep[:, first, None] & heads)
 
 
+@pytest.mark.parametrize("share,most", [(1.0, 100), (0.25, 40)])
+def test_a_value_that_is_not_finite_costs_a_bounded_time(share, most):
+    """An infinity in a value that most rows walk over (all of a KV head's rows are read again): 40 and 12 times the clean read
+    here, where a key at a time took 223 and 95."""
+    from lsa_b200 import ops
+
+    R, Hq, Hkv = 4096, 16, 2
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v = (torch.randn(R, h, 128, device="cuda", generator=gen).bfloat16() for h in (Hq, Hkv, Hkv))
+    keep = (torch.rand(R, R, device="cuda", generator=gen) < share).tril()
+    mask, out = _bits(keep), torch.empty_like(q)
+
+    def shortest(times):
+        took = []
+        for _ in range(times):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            ops.listed_attend(q, k, v, 0, mask, 128 ** -0.5, out)
+            end.record()
+            end.synchronize()
+            took.append(begin.elapsed_time(end))
+        return min(took)
+
+    clean = shortest(6)
+    v[5, :, 3] = float("inf")
+    assert shortest(3) <= most * clean
+    odd = ~out.isfinite()
+    assert torch.equal(odd[..., 3], keep[:, 5, None].expand(R, Hq)) and not odd[..., :3].any() and not odd[..., 4:].any()
+
+
 @pytest.mark.parametrize("cap,top_p,top_k,sink,window,sizes", [
     (16, 40, 200, 4, 100, (0, 16)), (16, 64, 10000, 0, 1, (8, 16)), (1, 33, 20, 2, 64, (1, 1)), (24, 17, 100, 70, 200, (0, 24)),
     (30, 10, 77, 4, 128, (3, 30)), (64, 16, 300, 4, 256, (20, 64)), (128, 8, 500, 4, 300, (0, 128)), (600, 3, 1000, 4, 64, (1, 600))])
