@@ -826,6 +826,13 @@ def listed_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, first_posit
                   out: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
     """`causal_attend` over the keys alone that `mask` (`list_bits`, every tile up to the last row) names: what
     `sparse_attend` gives for the lists, by walking every key on the tensor cores."""
+    R, Hq, dh = q.shape
+    if not dense_attend_supported(q, k, v, out) or v.shape != k.shape or out.shape != (R, Hq, dh):
+        raise ValueError("q, k, v must be bfloat16 heads of 128 dims packed densely, k and v alike, and out a contiguous bfloat16 or "
+                         f"float32 [{R}, {Hq}, {dh}], all 16-byte aligned")
+    if mask.dim() != 3 or mask.shape[0] < -(-(first_position + R) // 128) or mask.shape[1:] != (R, 4) \
+            or mask.dtype != torch.int32 or not mask.is_contiguous():
+        raise ValueError(f"mask must be a contiguous int32 [{-(-(first_position + R) // 128)} key tiles, {R}, 4]")
     return _dense_attend(q, k, v, first_position, scale, out, mask, status)
 
 

@@ -337,3 +337,28 @@ def test_a_decode_step_in_one_call_calls_no_method_that_another_layer_has_of_its
                                             "attend": lambda self, *a, **kw: (called.append("attend"), None)}))
     layer.decode(*args, index)
     assert called == ["map", "attend"]
+
+
+def test_a_masked_read_refuses_masks_and_outputs_that_are_not_its_own(monkeypatch):
+    """What the kernel takes on trust - as many key tiles as the last row walks, a word for every row, an output of the queries'
+    shape - is asked of the tensors before it is launched."""
+    from lsa_b200 import ops
+
+    R, first = 200, 300
+    q, k = torch.zeros(R, 4, 128, dtype=torch.bfloat16), torch.zeros(first + R, 2, 128, dtype=torch.bfloat16)
+    mask, out = torch.zeros(4, R, 4, dtype=torch.int32), torch.zeros(R, 4, 128, dtype=torch.bfloat16)
+    launched = []
+    monkeypatch.setattr(ops, "_dense_attend", lambda *a: launched.append(a))
+    read = lambda m=mask, o=out, v=k: ops.listed_attend(q, k, v, first, m, 1.0, o)
+    read()
+    assert len(launched) == 1
+    for bad in (mask[:3], mask[:, :199].contiguous(), mask[..., :3].contiguous(), mask.long(), mask.transpose(0, 1).contiguous(),
+                torch.zeros(4, R, 8, dtype=torch.int32)[..., ::2]):
+        with pytest.raises(ValueError, match="mask must be"):
+            read(bad)
+    for bad in (out.half(), out[:199], torch.zeros(R, 8, 128, dtype=torch.bfloat16)[:, ::2], out.view(R, 2, 256)):
+        with pytest.raises(ValueError, match="packed densely"):
+            read(o=bad)
+    with pytest.raises(ValueError, match="alike"):
+        read(v=k[:-1])
+    assert len(launched) == 1
