@@ -109,7 +109,8 @@ int lsa_pool_keys(const void *index_keys, int key_dtype, int64_t n_pools, int po
  *   labels     [blocks, P] int64 out - each pool's bucket, numbered by first pool
  *   reached    [blocks] uint8 out - 1 where the block got down to bucket_count
  *   rounds     [blocks] int32 out or NULL - merge rounds the block ran
- * Blocks of up to 4,096 pools of 16, 32 or 64 dims are merged by a cluster of 1 to 8 CTAs in one launch; up to 512 pools
+ * Blocks of up to 4,096 pools of 16, 32 or 64 dims are merged in one launch, by a cluster of 1 to 8 CTAs or, past 512 pools where
+ * clusters would leave SMs idle, by a cooperative grid that gives every block its share of them; up to 512 pools
  * they need no workspace, larger ones (the node-bucket pairings of the tree, src/lsa/core/hierarchy.py:73-98,
  * cluster_node_buckets at src/lsa/core/kernels/ward.py:84-110) keep their key sums there. Other widths (d % 4 == 0,
  * d <= 1024) take one CTA a block and up to 512 pools whose P * (d + 4) floats are within 227 KB: 64 pools of the 512-dim
@@ -224,7 +225,8 @@ int lsa_dense_scores(const float *queries, int64_t R, int d, const float *centro
                      float *scores_out, int64_t *keys_out, void *stream);
 
 /* Flat search, decode form: few rows, many buckets. The buckets of a row are split over `splits` CTAs whose
- * local top_p lists are merged by a second kernel. Reference: Selector.decode_flat
+ * local top_p lists are merged: by the row's cluster of CTAs for up to 8 rows of up to 8 splits and 128 keys, else by a second
+ * kernel. Reference: Selector.decode_flat
  * (src/lsa/sglang/index/selector.py:603-660), scan_paged (src/lsa/core/kernels/triton/paged.py:61-101),
  * DecodeSelect.listed (src/lsa/core/kernels/cutedsl/decode.py:1035-1068).
  *   request_first [R] int64 - first row of centroids of each request (requests hold their buckets contiguously)
@@ -337,7 +339,7 @@ int lsa_beam_step(const float *queries, int64_t R, int d, const float *vectors, 
                   const int64_t *children, int fanout, int32_t *kept_out, int64_t *keys_out, int32_t *carried_out,
                   void *stream);
 
-/* The same step with a row's candidates split over `splits` CTAs and merged by a second launch - the decode form,
+/* The same step with a row's candidates split over `splits` CTAs and merged as lsa_flat_select_decode's are - the decode form,
  * where one query would otherwise keep one CTA busy. workspace: lsa_beam_step_workspace_bytes(R, keep, splits). */
 size_t lsa_beam_step_workspace_bytes(int64_t R, int keep, int splits);
 int lsa_beam_step_split(const float *queries, int64_t R, int d, const float *vectors, int64_t N,

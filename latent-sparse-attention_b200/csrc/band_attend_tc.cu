@@ -21,9 +21,9 @@
 // issued until the threads of BOTH halves have arrived with their P, and with it their columns scaled.) Probabilities are 2^8 at most, and their two terms hold them to 2^-17 of themselves, so what the
 // reference point is does not show.
 //
-// What bounds it is the tensor pipe: a step of a tile is 1,536 cycles of products (the two terms of P cost a second product),
-// beside some 1,900 of softmax that four warps a scheduler share, and the wait between a tile's P V and the S that is written over
-// its P. 16,384 causal rows of 40 heads over 8: 3.39 ms, 811 TFLOP/s of useful work and 1,217 with the second term counted (3.24
+// What bounds it is the chain of a step, some 2,600 cycles a tile: 1,536 of products (the two terms of P cost a second one) that
+// alternate with the other tile's, 1,900 of softmax that four warps a scheduler share, and the hand-overs, the wait between a
+// tile's P V and the S that is written over its P among them. The tensor pipe is active 59 % of the time. 16,384 causal rows of 40 heads over 8: 3.39 ms, 811 TFLOP/s of useful work and 1,217 with the second term counted (3.24
 // without the wait; 5.61 when the keys were walked twice, maxima then sums, with P in shared memory and one tile a CTA); a masked
 // read of the same rows 3.65. 8,192 rows of a band of 1,024 keys 0.40 ms (0.53): a CTA's ten steps stand beside its start and its
 // end. Tried: S in two buffers of 64 keys a tile (drains the pipe), a thread a row (a softmax of 3,400 cycles a step).

@@ -1,8 +1,8 @@
 // Index space: grouped-query head sum, learned linear map and row normalisation in one pass over the heads.
 //
 // out[s] = normalize( sum_kv (sum_{g < group} x[s, kv*group + g, off : off + dh_used]) @ W[kv*dh_used : (kv+1)*dh_used] )
-// with fp32 accumulation in ascending input-dim order. This is the exact-arithmetic form; rows are read once and
-// the head sum never reaches memory.
+// with fp32 accumulation, in ascending input-dim order except for a few rows (up to 32, or 128 under a bf16 map), whose threads
+// share a row's dims. This is the exact-arithmetic form; rows are read once and the head sum never reaches memory.
 #include "common.cuh"
 #include "mma.cuh"
 

@@ -397,7 +397,9 @@ class FlatLayer:
 
         `chunk` is how many rows are worked on at a time, and with that how large the buffers get. Rows that are read through
         masks (`_listed_until`) are taken two waves of the GPU at a time where that is more, their tensors are what the masked
-        read takes and there is memory for it; else, as all others, `chunk` at a time.
+        read takes and there is memory for it; else, as all others, `chunk` at a time. Which keys a row lists depends on its
+        position and not on the chunk it is in, but for buckets whose scores nearly tie: a last piece of up to 128 rows is mapped in
+        fp32, larger ones on the tensor cores (and a piece of fewer than 128 rows is not read through masks).
         """
         T = q.shape[0]
         index = self.build_index(k, reuse_buffers=not return_index)
@@ -604,7 +606,7 @@ class FlatLayer:
             return out
         masked = band and bucket_major and ops.dense_attend_supported(rows, k, v, out)
         listed = self._listed_until() - start
-        if masked and 0 < listed < n:  # (a row's read depends on its position, not on the chunk it is in)
+        if masked and 0 < listed < n:  # (the rows past the line have the other reads)
             self.prefill_rows(rows[:listed], start, k, v, index, out[:listed], band, bucket_major)
             self.prefill_rows(rows[listed:], start + listed, k, v, index, out[listed:], band, bucket_major)
             return out

@@ -263,3 +263,28 @@ def test_a_prefill_without_memory_for_wide_masks_keeps_to_its_chunk(short, monke
     assert asked[0] > chunk and max(asked[1:]) <= chunk and len(asked) > 2
     assert (got.float() - wide).abs().max() <= 2e-2 and (got.float() - wide).abs().mean() <= 2e-3
     layer.check()
+
+
+@pytest.mark.parametrize("knobs", [dict(early_budget=dict(position=1500, top_k=90, top_p=20)), dict(bucket_shape=dict(rank=2, deviations=2.0)),
+                                   dict(early_budget=dict(position=700, top_k=40, top_p=64), bucket_shape=dict(rank=0, deviations=1.0))])
+def test_a_masked_prefill_under_an_early_budget_and_over_shaped_buckets(knobs, monkeypatch):
+    """The rows' own budgets and the shaped scan in front of the masked read, against the gather of the same lists."""
+    from lsa_b200 import ops
+    from lsa_b200.budget import EarlyBudget
+    from lsa_b200.layer import FlatDesign, FlatLayer
+
+    T, Hq, Hkv = 2500, 8, 2
+    if "early_budget" in knobs:
+        knobs = dict(knobs, early_budget=EarlyBudget(**knobs["early_budget"]))
+    rng = np.random.default_rng(T)
+    w = [cuda(rng.standard_normal((Hkv * 128, 64), dtype=np.float32) / 16, torch.bfloat16) for _ in range(2)]
+    layer = FlatLayer(FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=300,
+                                 sink_size=4, window_size=128, **knobs), *w, Hq, Hkv, 128)
+    q, k, v = (cuda(x, torch.bfloat16) for x in layer_inputs(T, Hq, Hkv, 128, 16, T))
+    gathered = layer.prefill(q, k, v, chunk=512, band=False, bucket_major=False).float()
+    listed, read = [], ops.listed_attend
+    monkeypatch.setattr(ops, "listed_attend", lambda q, *a, **kw: (listed.append(q.shape[0]), read(q, *a, **kw))[1])
+    got = layer.prefill(q, k, v, chunk=512).float()
+    assert sum(listed) > T // 2
+    assert (got - gathered).abs().max() <= 2e-2 and (got - gathered).abs().mean() <= 2e-3
+    layer.check()
