@@ -586,8 +586,9 @@ static int launch_ward(WardParams &p, int64_t G, cudaStream_t s) {
   }
   attribute[0].val.clusterDim.x = (unsigned)ctas;
   // A larger block whose clusters leave SMs idle (16 blocks: six CTAs each, 96 of 148 SMs) takes a cooperative grid and a
-  // counter in memory as its barrier. Pairings, one cluster a block -> the grid: one block of 4,096 buckets 2,322 -> 455 us, of
-  // 1,024 253 -> 159; 16 blocks of 4,096 3,124 -> 2,166, of 640 no change. Of as many CTAs the cluster is the faster (its barrier
+  // counter in memory as its barrier. Pairings of clustered unit rows, one cluster a block -> the grid: one block of 4,096
+  // buckets 2,322 -> 455 us, of 1,024 253 -> 159; 16 blocks of 4,096 3,124 -> 2,166 (those of an index of 1M tokens, which take
+  // more rounds, 4,396 -> 3,066), of 640 no change. Of as many CTAs the cluster is the faster (its barrier
   // is: 32 blocks of 640 256 us, 268 as a grid), so it stays where it has them.
   if (LOCAL || wanted <= ctas) {
     p.arrived = nullptr;
