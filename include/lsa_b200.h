@@ -471,8 +471,8 @@ int lsa_band_round(const float *in, const uint16_t *q, int64_t R, int Hq, int dh
 /* Dense attention of consecutive rows (row i at first_position + i, KV row p at position p) over every key up to a row's own,
  * or, with `mask`, over those of them that its list names: what lsa_sparse_attend gives for such lists, on the tensor cores.
  * Heads of 128 dims packed densely, 16-byte aligned rows and outputs (else LSA_ERR_UNSUPPORTED).
- * Rows whose output is not finite are read again, key by key, so that a value that is not finite reaches the rows that read
- * it and no others.
+ * Rows whose output is not finite are read again, over their own keys alone, so that a value that is not finite reaches the rows
+ * that read it and no others.
  *   mask        [key tiles of 128][R][4] uint32 as lsa_list_bits writes it (every tile up to the last row's position), or NULL
  *   out_bf16, out_f32  [R, Hq, 128], one of them may be NULL
  *   not_finite  one int32 of workspace

@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(kAgainWarps * 32, 4)
 }
 
 // A dense causal read on its way out (rounded to bf16, or as it is), a warp a (row, head). In a tile of 128 rows a key after a row weighs zero, and zero
-// times a value that is not finite is not a number: a row of the tile that holds one is read again here, key by key, over the
-// keys up to its own alone (what a list would name). Memory bounds the rows that are finite, all of them as a rule (six
+// times a value that is not finite is not a number: a row of the tile that holds one is read again here, over the keys up to
+// its own alone (what a list would name). Memory bounds the rows that are finite, all of them as a rule (six
 // bytes a dim, what the copy to bf16 in its place moved).
 template <int DH>
 __global__ void __launch_bounds__(256) band_round_kernel(RoundParams p) {
