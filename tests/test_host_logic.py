@@ -281,9 +281,10 @@ def test_wide_buckets_go_to_the_gather_where_it_alone_takes_the_call():
     assert takes(64)(odd, out.float())
 
 
-@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (2, 1, 64)])
-def test_a_prefill_that_no_mask_serves_keeps_to_its_chunk(heads, kv_heads, head_dim, monkeypatch):
-    """Heads that the masked read does not take go `chunk` rows at a time, before its line as past it."""
+@pytest.mark.parametrize("heads,kv_heads,head_dim,off", [(8, 2, 64, 0), (2, 1, 64, 0), (8, 2, 128, 1)])
+def test_a_prefill_that_no_mask_serves_keeps_to_its_chunk(heads, kv_heads, head_dim, off, monkeypatch):
+    """Heads that the masked read does not take, and rows that are not 16-byte aligned, go `chunk` rows at a time, before its line
+    as past it."""
     from types import SimpleNamespace
 
     from lsa_b200.core import Buckets
@@ -296,7 +297,8 @@ def test_a_prefill_that_no_mask_serves_keeps_to_its_chunk(heads, kv_heads, head_
     index = SimpleNamespace(buckets=Buckets(torch.zeros(1000, 64), None, None, 32, 256))
     monkeypatch.setattr(FlatLayer, "build_index", lambda self, k, reuse_buffers: index)
     monkeypatch.setattr(FlatLayer, "prefill_rows", lambda self, rows, start, *a: pieces.append((start, rows.shape[0])))
-    q, k = torch.zeros(T, heads, head_dim, dtype=torch.bfloat16), torch.zeros(T, kv_heads, head_dim, dtype=torch.bfloat16)
+    q = torch.zeros(T * heads * head_dim + off, dtype=torch.bfloat16)[off:].view(T, heads, head_dim)
+    k = torch.zeros(T, kv_heads, head_dim, dtype=torch.bfloat16)
     layer.prefill(q, k, k, chunk=chunk)
     assert max(n for _, n in pieces) <= chunk
     assert [start for start, _ in pieces] == [0, *torch.tensor([n for _, n in pieces]).cumsum(0)[:-1].tolist()]
