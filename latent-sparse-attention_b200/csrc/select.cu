@@ -1,8 +1,8 @@
 // Bucket search: score candidates with a fixed-order fp32 dot, keep each row's best as packed int64 keys.
 //
-// One kernel serves the flat prefill scan (eight rows a CTA share every centroid they load), the flat decode
-// scan (one row, its buckets split over CTAs, lists merged afterwards) and a beam step of the tree (one row,
-// carried children beside a run of open rows). Selection is exact: a streaming top-k over 64-bit keys whose low
+// One kernel serves prefill scans (eight rows a CTA share every centroid they load), another the flat decode scan
+// (one row, its buckets split over CTAs whose lists become one) and a beam step of the tree (one row, carried
+// children beside a run of open rows). Selection is exact: a top-k over 64-bit keys whose low
 // word breaks a score tie toward the lower id, so the result does not depend on the order keys were produced in.
 #include <cooperative_groups.h>
 
@@ -13,19 +13,6 @@
 namespace lsa {
 
 namespace cg = cooperative_groups;
-
-#ifdef LSA_SELECT_TRACE
-// Clock stamps of thread 0 of one CTA of a decode row's scan (row 0) and of its merge (row 1), for a build that asks.
-__device__ long long lsa_select_trace[2][16];
-#define LSA_STAMP(row, at)                                                         \
-  do {                                                                             \
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) lsa_select_trace[row][at] = clock64(); \
-  } while (0)
-#else
-#define LSA_STAMP(row, at) \
-  do {                     \
-  } while (0)
-#endif
 
 constexpr int kSelThreads = 256;
 constexpr int kSelWarps = kSelThreads / 32;
@@ -365,7 +352,7 @@ struct SelectParams {
   const int32_t *pages;         // [R, max_pages] page of every page_rows ids of a row (-1 = none), or NULL
   int d, n_carried, keep, fanout, id_base, chunk, run_limit, max_pages, page_rows;
   ShapeTable shape;             // the vectors' shapes, row for row (floors NULL: none)
-  bool fold;                    // a row's splits are one cluster, whose first CTA folds their lists and writes the row
+  int cluster;                  // CTAs a cluster, whose lists become one (row_select_kernel)
 };
 
 // RB rows a CTA. Shared memory: queries [RB][d], per-row key buffers [RB][keep_pow2 + chunk], histograms.
@@ -389,7 +376,6 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
   const int splits = gridDim.y, split = blockIdx.y;
   dependents_may_launch();
   wait_for_earlier_grids();
-  LSA_STAMP(0, 0);
 
   for (int e = tid; e < RB * p.d; e += kSelThreads) {
     const int64_t r = row0 + e / p.d;
@@ -409,7 +395,6 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
     total_s[tid] = r < p.R ? p.n_carried + (end - first) : 0;
   }
   __syncthreads();
-  LSA_STAMP(0, 1);
   int max_total = 0;
 #pragma unroll
   for (int i = 0; i < RB; ++i) max_total = max(max_total, total_s[i]);
@@ -426,11 +411,6 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
   // (a single row: every thread of the CTA carries the row's state, which stays the same in all of them)
   const int my_keep_all = (RB == 1 && row0 < p.R) ? (p.row_keep ? min(p.row_keep[row0], p.keep) : p.keep) : 0;
   __shared__ int block_counter, block_pick[3];
-  // A single row whose share of the candidates is one chunk of at most 1,024, cut to at most 128: sorted in registers.
-  const bool in_registers = RB == 1 && cand_end - cand_begin <= kSelWarps * kTopWarp && cand_end > cand_begin &&
-                            cand_end - cand_begin <= p.chunk && p.keep <= kTopWarp &&
-                            p.chunk >= kSelWarps / 2 * kTopWarp;  // (the chunk's room holds the lists being folded)
-  bool sorted = false;
 
   for (int chunk_base = cand_begin; chunk_base < cand_end; chunk_base += p.chunk) {
     const int chunk_n = min(p.chunk, cand_end - chunk_base);
@@ -534,35 +514,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
       for (int i = 0; i < RB; ++i)
         bufs[(size_t)i * row_room + keep_room + t] = ids[i] >= 0 ? pack_key(acc[i], ids[i] + p.id_base) : kEmptyKey;
     }
-    LSA_STAMP(0, 2);
     __syncthreads();
-    LSA_STAMP(0, 3);
-    if (RB == 1 && in_registers) {
-      // ---- select: every warp sorts 128 of the chunk's keys, the warps' lists are folded into warp 0's
-      int64_t *chunk = bufs + keep_room;
-      int64_t k[kTopLane];
-#pragma unroll
-      for (int j = 0; j < kTopLane; ++j) {
-        const int at = warp * kTopWarp + j * 32 + lane;
-        k[j] = at < chunk_n ? chunk[at] : kEmptyKey;
-      }
-      warp_sort128(k, lane);
-      LSA_STAMP(0, 4);
-      block_top128(k, chunk, kSelWarps, warp, lane);
-      LSA_STAMP(0, 5);
-      if (warp == 0) {
-        int valid = 0;
-#pragma unroll
-        for (int j = 0; j < kTopLane; ++j) {
-          bufs[j * 32 + lane] = k[j];
-          valid += k[j] != kEmptyKey;
-        }
-        held = min(warp_sum_int(valid), my_keep_all);
-        __syncwarp();
-      }
-      sorted = true;
-      continue;
-    }
     // ---- select: a row that has the CTA to itself is folded by all of its threads (the keys are distinct and the
     // final sort orders them, so the order they are kept in does not matter)
     if (RB == 1 && row_room <= kBlockCompactPerThread * kSelThreads) {
@@ -598,53 +550,9 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
     __syncthreads();
   }
 
-  if constexpr (RB == 1) {
-    if (p.fold) {
-      // The lists of a row's CTAs meet in the first one's registers, through distributed shared memory.
-      cg::cluster_group cluster = cg::this_cluster();
-      if (warp == 0) {
-        if (!sorted) warp_sort_descending(bufs, held);
-        for (int i = held + lane; i < kTopWarp; i += 32) bufs[i] = kEmptyKey;
-      }
-      cluster.sync();
-      if (split == 0) {
-        int64_t k[kTopLane];
-        const int64_t *theirs = cluster.map_shared_rank(bufs, warp < splits ? warp : 0);
-#pragma unroll
-        for (int j = 0; j < kTopLane; ++j) k[j] = warp < splits ? theirs[j * 32 + lane] : kEmptyKey;
-        block_top128(k, bufs + kTopWarp, kSelWarps, warp, lane);
-        if (warp == 0) {
-          int valid = 0;
-#pragma unroll
-          for (int j = 0; j < kTopLane; ++j) {
-            bufs[j * 32 + lane] = k[j];
-            valid += k[j] != kEmptyKey;
-          }
-          valid = min(warp_sum_int(valid), my_keep_all);
-          if (lane == 0) block_counter = valid;
-        }
-        __syncthreads();
-        held = block_counter;
-        for (int i = tid; i < p.keep; i += kSelThreads) {
-          const int64_t key = i < held ? bufs[i] : kEmptyKey;
-          if (p.keys_out) p.keys_out[row0 * p.keep + i] = key;
-          if (p.ids_out) p.ids_out[row0 * p.keep + i] = key == kEmptyKey ? LSA_PAD : key_id(key);
-        }
-        if (p.carried_out) {
-          for (int e = tid; e < p.keep * p.fanout; e += kSelThreads) {
-            const int i = e / p.fanout, c = e - i * p.fanout;
-            p.carried_out[row0 * p.keep * p.fanout + e] =
-                i < held ? (int32_t)p.children[(int64_t)(key_id(bufs[i]) - p.id_base) * p.fanout + c] : LSA_PAD;
-          }
-        }
-      }
-      cluster.sync();  // nobody leaves while its list may still be read
-      return;
-    }
-  }
   if (warp < RB && my_row < p.R) {
     int64_t *buf = bufs + (size_t)warp * row_room;
-    if (!sorted) warp_sort_descending(buf, held);
+    warp_sort_descending(buf, held);
     const int64_t out_row = ((int64_t)split * p.R + my_row) * p.keep;
     for (int i = lane; i < p.keep; i += 32) {
       const int64_t key = i < held ? buf[i] : kEmptyKey;
@@ -661,7 +569,6 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectParams p) {
       }
     }
   }
-  LSA_STAMP(0, 6);
 }
 
 // Global top-k of `parts` lists of packed keys, a warp a row.
@@ -678,7 +585,6 @@ __global__ void __launch_bounds__(kSelThreads) merge_candidates_kernel(const int
   const int64_t r = blockIdx.x;
   dependents_may_launch();
   wait_for_earlier_grids();
-  LSA_STAMP(1, 0);
   int n = 0;
   bool sorted = false;
   if (keep <= kTopWarp && parts > 1) {
@@ -696,15 +602,12 @@ __global__ void __launch_bounds__(kSelThreads) merge_candidates_kernel(const int
       if (!lists_sorted) warp_sort128(into, lane);
     };
     take(k, warp);
-    LSA_STAMP(1, 1);
     for (int part = warp + warps; part < parts; part += warps) {  // (the same trips for every lane of a warp)
       int64_t t[kTopLane];
       take(t, part);
       warp_fold128(k, t, lane);
     }
-    LSA_STAMP(1, 2);
     block_top128(k, buf, warps, warp, lane);
-    LSA_STAMP(1, 3);
     if (warp > 0) return;
 #pragma unroll
     for (int j = 0; j < kTopLane; ++j) {
@@ -757,7 +660,6 @@ __global__ void __launch_bounds__(kSelThreads) merge_candidates_kernel(const int
       carried_out[r * keep * fanout + e] = i < n ? (int32_t)children[(int64_t)key_id(buf[i]) * fanout + c] : LSA_PAD;
     }
   }
-  LSA_STAMP(1, 4);
 }
 
 // Threads of a candidate merge: a warp for a few hundred candidates, the whole CTA for what its registers can hold.
@@ -797,9 +699,332 @@ static int launch_select(SelectParams p, int splits, cudaStream_t s) {
   dim3 grid((unsigned)((p.R + RB - 1) / RB), (unsigned)splits);
   auto kernel = p.shape.floors ? select_kernel<RB, true> : select_kernel<RB, false>;
   if (!allow_shared(kernel, kSelectShared)) return LSA_ERR_LAUNCH;
-  launch_clusters(p.R <= kChainedRows, kernel, grid, dim3(kSelThreads), smem, s, p, p.fold ? splits : 1);
+  launch(p.R <= kChainedRows, kernel, grid, dim3(kSelThreads), smem, s, p);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
+}
+
+// ---------------------------------------------------------------------------------------- a few rows, at most 128 kept
+
+// The scan of a decode row: its candidates are split over CTAs, each CTA ranks its share a tile of 256 at a time (a thread a
+// candidate), and the CTAs of a cluster rank their lists against one another, so a row of up to eight CTAs is one launch.
+//
+// What bounds it is a chain of latencies, so nothing is sorted that can be counted: a warp sorts its 32 keys with shuffles,
+// and a key's place in a longer list is its place in its own run plus how many keys of each other run come before it - binary
+// searches in shared memory that do not wait for one another. In a cluster every CTA writes its list into all of the others'
+// shared memory before one barrier; after it each CTA places its own keys and writes them where they belong.
+constexpr int kRowTile = kSelThreads;
+constexpr int kRowKeep = 128;
+constexpr int kRowCluster = 8;
+
+// How many of list[0..size) (descending, size a power of two) come before `key`: those greater, and equal ones too if `ties`.
+__device__ __forceinline__ int keys_before(const int64_t *list, int size, int64_t key, bool ties) {
+  int at = 0;
+  for (int step = size >> 1; step; step >>= 1) {
+    const int64_t other = list[at + step - 1];
+    at += other > key || (ties && other == key) ? step : 0;
+  }
+  const int64_t other = list[at];
+  return at + (other > key || (ties && other == key) ? 1 : 0);
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// NV: 16-byte columns of a vector (8 or 16: tiles of vectors staged through shared memory, a half warp on a vector's bytes), or
+// 0: any width, every thread reading its own candidate's vector.
+template <int NV, bool SHAPED>
+__global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p) {
+  constexpr int kColumns = NV > 0 ? NV : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4 *tile_s = reinterpret_cast<float4 *>(smem_raw);                  // [256][NV], columns swizzled
+  float *qs = reinterpret_cast<float *>(tile_s + (size_t)kRowTile * NV);  // [d]
+  __shared__ int64_t rowof_s[2][kRowTile], runs_s[kRowTile], top_s[kRowKeep], held_s[2][kRowKeep], all_s[kRowCluster][kRowKeep];
+  __shared__ int64_t waits_s[kRowKeep + kRowTile];
+  __shared__ int count_s[kRowCluster], kept_rank_s[kRowKeep], kept_id_s[kRowKeep], kept_s, waiting_s;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t row = blockIdx.x;
+  const int split = blockIdx.y, splits = gridDim.y, mine = split % p.cluster;
+  if (p.cluster > 1) cluster_arrive();  // (waited for before the first write into another CTA)
+  dependents_may_launch();
+  wait_for_earlier_grids();
+
+  const int first = p.run_first ? p.run_first[row] : 0;
+  int end = p.run_end ? p.run_end[row] : 0;
+  const int my_keep = p.row_keep ? max(0, min(p.row_keep[row], p.keep)) : p.keep;
+  const int64_t vector_base = p.vector_base ? p.vector_base[row] : 0;
+  for (int e = tid; e < p.d; e += kSelThreads) qs[e] = p.queries[row * p.d + e];
+  end = max(first, min(end, p.run_limit));
+  if (tid == 0) kept_s = 0, waiting_s = 0;
+  const int total = p.n_carried + (end - first), share = (total + splits - 1) / splits;
+  const int begin = min(total, split * share), stop = min(total, begin + share);
+
+  // The id of candidate c and the row of `vectors` it lies at (-1: neither).
+  auto candidate = [&](int c, int64_t &vec_row) -> int32_t {
+    vec_row = -1;
+    if (c >= stop) return -1;
+    int32_t id = c < p.n_carried ? p.carried[row * p.n_carried + c] : first + (c - p.n_carried);
+    if (id < 0) return -1;
+    vec_row = vector_base + id;
+    if (p.pages) {
+      // a request's logical bucket id sits at row id % page_rows of its page id / page_rows
+      const int page = id / p.page_rows < p.max_pages ? p.pages[row * p.max_pages + id / p.page_rows] : -1;
+      vec_row = page >= 0 ? (int64_t)page * p.page_rows + id % p.page_rows : -1;
+      if (page < 0) id = -1;
+    }
+    if (vec_row >= p.N) vec_row = -1, id = -1;
+    return id;
+  };
+  float4 v[kColumns];
+  auto ask = [&](const int64_t *rowof) {  // this thread's pieces of a tile's vectors, all in flight together
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int e = tid + i * kSelThreads;
+      const int64_t r = rowof[e / kColumns];
+      v[i] = r >= 0 ? __ldg(reinterpret_cast<const float4 *>(p.vectors + r * (NV * 4)) + e % kColumns)
+                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  };
+
+  int64_t vec_row, next_row = -1;
+  int32_t id = candidate(begin + tid, vec_row), next_id = -1;
+  rowof_s[0][tid] = vec_row;
+  if (tid < kRowKeep) held_s[0][tid] = kEmptyKey;
+  __syncthreads();
+  if constexpr (NV > 0) ask(rowof_s[0]);
+  int held = 0;  // which of held_s is the list so far
+  // A key of every thread into the list, or the list made of them.
+  auto fold = [&](int64_t key, bool merge) {
+    // a warp's 32 keys, best first (a bitonic network over the lanes)
+#pragma unroll
+    for (int span = 2; span <= 32; span <<= 1)
+#pragma unroll
+      for (int stride = span >> 1; stride > 0; stride >>= 1) {
+        const int64_t other = __shfl_xor_sync(0xffffffffu, key, stride);
+        const bool greater = ((lane & stride) == 0) == ((lane & span) == 0);
+        key = (key < other) == greater ? other : key;
+      }
+    runs_s[tid] = key;
+    __syncthreads();
+    int rank = lane;  // (its own run is searched as well: without a branch the searches wait side by side)
+#pragma unroll
+    for (int w = 0; w < kSelWarps; ++w) {
+      const int before = keys_before(runs_s + w * 32, 32, key, w < warp);
+      rank += w == warp ? 0 : before;
+    }
+    if (!merge) {
+      if (rank < kRowKeep) held_s[0][rank] = key;
+      return;
+    }
+    if (rank < kRowKeep) top_s[rank] = key;
+    __syncthreads();
+    const int64_t *old = held_s[held];
+    const int i = tid & (kRowKeep - 1);
+    key = tid < kRowKeep ? old[i] : top_s[i];
+    rank = i + keys_before(tid < kRowKeep ? top_s : old, kRowKeep, key, tid >= kRowKeep);
+    if (rank < kRowKeep) held_s[held ^ 1][rank] = key;
+    held ^= 1;
+  };
+  for (int t = begin; t < stop; t += kRowTile) {
+    const int parity = (t - begin) / kRowTile & 1;
+    const bool more = t + kRowTile < stop;
+    if (more) next_id = candidate(t + kRowTile + tid, next_row);
+    float acc = 0.0f;
+    if constexpr (NV > 0) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int e = tid + i * kSelThreads, cand = e / kColumns, c4 = e % kColumns;
+        tile_s[cand * NV + (c4 ^ (cand & (NV - 1)))] = v[i];
+      }
+      if (more) rowof_s[parity ^ 1][tid] = next_row;
+      __syncthreads();
+      if (more) ask(rowof_s[parity ^ 1]);
+#pragma unroll
+      for (int k4 = 0; k4 < NV; ++k4) {
+        const float4 w = tile_s[tid * NV + (k4 ^ (tid & (NV - 1)))];
+        const float4 q = *reinterpret_cast<const float4 *>(qs + k4 * 4);
+        acc = fmaf(q.x, w.x, acc), acc = fmaf(q.y, w.y, acc), acc = fmaf(q.z, w.z, acc), acc = fmaf(q.w, w.w, acc);
+      }
+    } else {
+      if (t > begin) __syncthreads();  // (the list and the runs of the tile before)
+      if (vec_row >= 0) {
+        const float4 *w4 = reinterpret_cast<const float4 *>(p.vectors + vec_row * p.d);
+#pragma unroll 4
+        for (int k4 = 0; k4 < p.d / 4; ++k4) {
+          const float4 w = __ldg(w4 + k4);
+          const float4 q = *reinterpret_cast<const float4 *>(qs + k4 * 4);
+          acc = fmaf(q.x, w.x, acc), acc = fmaf(q.y, w.y, acc), acc = fmaf(q.z, w.z, acc), acc = fmaf(q.w, w.w, acc);
+        }
+      }
+    }
+    if constexpr (SHAPED) {
+      if (vec_row >= 0) acc = shaped_score(acc, qs, p.d, p.shape, vec_row);
+    }
+    int64_t key = id >= 0 ? pack_key(acc, id + p.id_base) : kEmptyKey;
+    id = next_id, vec_row = next_row;
+    if (t == begin) {
+      fold(key, false);
+      continue;  // (the barrier before the list is read: the next tile's, or the one behind the loop)
+    }
+    // Later tiles hold few keys that beat the list: those wait side by side until there are enough of them for a round.
+    const bool beats = key > held_s[held][p.keep - 1];
+    const unsigned votes = __ballot_sync(0xffffffffu, beats);
+    int at = 0;
+    if (lane == 0 && votes) at = atomicAdd(&waiting_s, __popc(votes));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (beats) waits_s[at + __popc(votes & ((1u << lane) - 1))] = key;
+    __syncthreads();
+    const int n = waiting_s;  // (128 at most from before, and this tile's)
+    if (n <= kRowKeep && more) continue;
+    for (int w = 0; w < n; w += kRowTile) {
+      fold(w + tid < n ? waits_s[w + tid] : kEmptyKey, true);
+      __syncthreads();
+    }
+    if (tid == 0) waiting_s = 0;
+  }
+  __syncthreads();
+  const int64_t *list = held_s[held];
+
+  if (p.cluster == 1) {  // this CTA's list is a row's, or one that a merge takes
+    const int valid = __syncthreads_count(tid < my_keep && list[tid & (kRowKeep - 1)] != kEmptyKey);
+    const int64_t out_row = ((int64_t)split * p.R + row) * p.keep;
+    if (tid < p.keep) {
+      const int64_t key = tid < valid ? list[tid] : kEmptyKey;
+      if (p.keys_out) p.keys_out[out_row + tid] = key;
+      if (p.ids_out) p.ids_out[out_row + tid] = key == kEmptyKey ? LSA_PAD : key_id(key);
+    }
+    if (p.carried_out)
+      for (int e = tid; e < p.keep * p.fanout; e += kSelThreads) {
+        const int i = e / p.fanout, c = e - i * p.fanout;
+        p.carried_out[row * p.keep * p.fanout + e] =
+            i < valid ? (int32_t)p.children[(int64_t)(key_id(list[i]) - p.id_base) * p.fanout + c] : LSA_PAD;
+      }
+    return;
+  }
+
+  // ---- the cluster's lists become one: every CTA has them all, and places its own keys among them
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = p.cluster;
+  int size = 2;  // of the part of a list that can matter, as a power of two
+  while (size < p.keep) size <<= 1;
+  const int own = __syncthreads_count(tid < p.keep && list[tid & (kRowKeep - 1)] != kEmptyKey);
+  cluster_wait();  // (every CTA of the cluster is there)
+  {
+    const int i = tid & (kRowKeep - 1);
+    const int64_t key = i < p.keep ? list[i] : kEmptyKey;
+    if (i < size)
+      for (int peer = tid / kRowKeep; peer < C; peer += kSelThreads / kRowKeep)
+        cluster.map_shared_rank(&all_s[mine][0], peer)[i] = key;
+    if (tid < C) *cluster.map_shared_rank(&count_s[mine], tid) = own;
+  }
+  cluster_arrive();
+  cluster_wait();  // (nobody's shared memory is touched by another CTA from here on)
+  int found = 0;
+  for (int j = 0; j < C; ++j) found += count_s[j];
+  const int valid = min(found, my_keep);
+  const int64_t out_row = ((int64_t)(split / C) * p.R + row) * p.keep;
+  {
+    const int i = tid >> 1, half = tid & 1;  // two threads a key, every other list each
+    const int64_t key = i < p.keep ? list[i] : kEmptyKey;
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < kRowCluster; j += 2) {  // (lists past the cluster's hold whatever was there, and count for nothing)
+      const int before = keys_before(all_s[j + half], size, key, j + half < mine);
+      rank += j + half < C && j + half != mine ? before : 0;
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1) + i;
+    if (half == 0 && key != kEmptyKey && rank < valid) {
+      if (p.keys_out) p.keys_out[out_row + rank] = key;
+      if (p.ids_out) p.ids_out[out_row + rank] = key_id(key);
+      if (p.carried_out) {
+        const int slot = atomicAdd(&kept_s, 1);
+        kept_rank_s[slot] = rank, kept_id_s[slot] = key_id(key) - p.id_base;
+      }
+    }
+  }
+  if (mine == 0 && tid >= valid && tid < p.keep) {
+    if (p.keys_out) p.keys_out[out_row + tid] = kEmptyKey;
+    if (p.ids_out) p.ids_out[out_row + tid] = LSA_PAD;
+  }
+  if (p.carried_out) {  // (the cluster's list is the row's then)
+    int32_t *out = p.carried_out + row * p.keep * p.fanout;
+    if (mine == 0)
+      for (int e = valid * p.fanout + tid; e < p.keep * p.fanout; e += kSelThreads) out[e] = LSA_PAD;
+    __syncthreads();
+    for (int e = tid; e < kept_s * p.fanout; e += kSelThreads) {
+      const int slot = e / p.fanout, c = e - slot * p.fanout;
+      out[(int64_t)kept_rank_s[slot] * p.fanout + c] = (int32_t)p.children[(int64_t)kept_id_s[slot] * p.fanout + c];
+    }
+  }
+}
+
+// The best `keep` (128 at most) of up to 16 sorted lists a row, placed by counting. At least `keep` keys reach the least of the
+// lists' keys at place ceil(keep / parts), so only what reaches it is looked up in the other lists.
+constexpr int kMergeParts = 16;
+constexpr int kMergeThreads = 512;
+__global__ void __launch_bounds__(kMergeThreads)
+    merge_sorted_kernel(const int64_t *__restrict__ keys_in, int parts, int64_t R, int keep, int size,
+                        int64_t *__restrict__ keys_out, int32_t *__restrict__ ids_out, const int64_t *__restrict__ children,
+                        int fanout, int32_t *__restrict__ carried_out) {
+  __shared__ int64_t lists_s[kMergeParts * kRowKeep], out_s[kRowKeep];  // [parts][size]
+  const int tid = threadIdx.x;
+  const int64_t r = blockIdx.x;
+  dependents_may_launch();
+  wait_for_earlier_grids();
+  for (int e = tid; e < parts * size; e += kMergeThreads) {
+    const int part = e / size, i = e - part * size;
+    lists_s[e] = i < keep ? keys_in[((int64_t)part * R + r) * keep + i] : kEmptyKey;
+  }
+  if (tid < kRowKeep) out_s[tid] = kEmptyKey;
+  __syncthreads();
+  const int deep = (keep + parts - 1) / parts - 1;
+  int64_t least = INT64_MAX;
+  for (int j = 0; j < parts; ++j) least = min(least, lists_s[j * size + deep]);
+  for (int e = tid; e < parts * keep; e += kMergeThreads) {
+    const int i = e / parts, part = e - i * parts;  // (the lists' heads first: what is under the bar is whole warps)
+    const int64_t key = lists_s[part * size + i];
+    if (key < least || key == kEmptyKey) continue;
+    int rank = i;
+#pragma unroll 4
+    for (int j = 0; j < parts; ++j) {
+      const int before = keys_before(lists_s + j * size, size, key, j < part);
+      rank += j == part ? 0 : before;
+    }
+    if (rank < keep) out_s[rank] = key;
+  }
+  __syncthreads();
+  if (tid < keep) {
+    const int64_t key = out_s[tid];
+    if (keys_out) keys_out[r * keep + tid] = key;
+    if (ids_out) ids_out[r * keep + tid] = key == kEmptyKey ? LSA_PAD : key_id(key);
+  }
+  if (carried_out)
+    for (int e = tid; e < keep * fanout; e += kMergeThreads) {
+      const int i = e / fanout, c = e - i * fanout;
+      carried_out[r * keep * fanout + e] =
+          out_s[i] != kEmptyKey ? (int32_t)children[(int64_t)key_id(out_s[i]) * fanout + c] : LSA_PAD;
+    }
+}
+
+template <int NV>
+static int launch_row_select(const SelectParams &p, int splits, cudaStream_t s) {
+  const size_t smem = (size_t)kRowTile * NV * 16 + (size_t)p.d * 4;
+  const auto kernel = p.shape.floors ? row_select_kernel<NV, true> : row_select_kernel<NV, false>;
+  LSA_REQUIRE(smem <= kSelectShared, LSA_ERR_UNSUPPORTED);
+  if (!allow_shared(kernel, kSelectShared)) return LSA_ERR_LAUNCH;
+  launch_clusters(p.R <= kChainedRows, kernel, dim3((unsigned)p.R, (unsigned)splits), dim3(kSelThreads), smem, s, p, p.cluster);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
+// One row a CTA, or its candidates split over `splits` of them: the lists of p.cluster neighbouring CTAs leave as one.
+static int launch_one_row(SelectParams p, int splits, cudaStream_t s) {
+  if (p.cluster < 1) p.cluster = 1;
+  if (p.keep > kRowKeep) return launch_select<1>(p, splits, s);
+  return p.d == 64   ? launch_row_select<16>(p, splits, s)
+         : p.d == 32 ? launch_row_select<8>(p, splits, s)
+                     : launch_row_select<0>(p, splits, s);
 }
 
 // ---------------------------------------------------------------------------------------- flat prefill scan
@@ -964,12 +1189,6 @@ static int launch_flat(FlatParams p, cudaStream_t s) {
 }
 
 }  // namespace lsa
-
-#ifdef LSA_SELECT_TRACE
-extern "C" __attribute__((visibility("default"))) int lsa_select_trace_read(long long *host) {
-  return (int)cudaMemcpyFromSymbol(host, lsa::lsa_select_trace, sizeof(lsa::lsa_select_trace));
-}
-#endif
 
 // ================================================================================================ C ABI
 
@@ -1340,7 +1559,7 @@ LSA_API int lsa_scan_select(const float *queries, int64_t R, int d, const float 
     sel.keep = top_p;
     sel.id_base = bucket_id_base;
     sel.run_limit = INT32_MAX;
-    rc = lsa::launch_select<1>(sel, lsa::kScanRetrySplits, s);
+    rc = lsa::launch_one_row(sel, lsa::kScanRetrySplits, s);
     if (rc != LSA_OK) return rc;
     rc = lsa_merge_candidates(retry_parts, lsa::kScanRetrySplits, lsa::kScanRetry, top_p, retry_keys, nullptr, stream);
     if (rc != LSA_OK) return rc;
@@ -1540,6 +1759,12 @@ namespace lsa {
 // lists this file's own scans write).
 static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, int64_t *keys_out, int32_t *picked_out,
                        const int64_t *children, int fanout, int32_t *carried_out, bool sorted, cudaStream_t stream) {
+  if (sorted && parts <= kMergeParts && top_p <= kRowKeep) {
+    launch(R <= kChainedRows, merge_sorted_kernel, dim3((unsigned)R), dim3(kMergeThreads), 0, stream, keys_in, parts, R, top_p,
+           pow2_at_least(top_p), keys_out, picked_out, children, fanout, carried_out);
+    LSA_LAUNCH_CHECK();
+    return LSA_OK;
+  }
   // (the lists folded in registers pass through kSelWarps / 2 slots of 128 keys, whatever they hold themselves)
   const int room = max(pow2_at_least(parts * top_p), kSelWarps / 2 * kTopWarp);
   const size_t smem = (size_t)room * 8 + kHistBins * 4;
@@ -1551,29 +1776,33 @@ static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, 
   return LSA_OK;
 }
 
-// Splits of a row that are folded in a cluster, at most: a warp a list; and only for a few rows. (One row's 1,024 buckets over 8
-// CTAs, top 128: 13.3 us with the merge a launch of its own, 11.6 folded; a beam level of 1,024 nodes with 32 times 64 children
-// 18.2 and 13.3. The clusters of 64 rows wait for SMs that are free together: 4 CTAs a row took 22.5 and 26.7; and clusters of
-// 16, beyond the portable size, took a batch of 8 rows from 14.9 to 25.7.)
-constexpr int kFoldSplits = kSelWarps;
-
-// The best p.keep of each row's candidates, the row's split over `splits` CTAs: folded by a cluster where its registers take
-// the lists, else written to the workspace and merged by a launch of their own.
+// The best p.keep of each row's candidates, the row's split over `splits` CTAs. Up to kChainedRows rows are split over clusters: up
+// to eight CTAs are one and write the row, more are several whose lists a launch of its own merges. One B200, a graph of the call,
+// top 64, in us, the form with sorted lists folded pairwise first: 1,024 buckets over 8 CTAs 11.8 -> 6.5 (8 rows 11.9 -> 6.7),
+// 4,096 over 8 14.2 -> 10.1, 16,384 over 32 18.4 -> 13.2; a beam level of 1,024 nodes with 32 times 64 children 13.3 -> 7.1. Past
+// fifteen CTAs asked for, a row takes 32 (64 where it is alone and 32 are asked for): over 16,384 buckets one row takes 17.3 in 16,
+// 13.2 in 32 and 11.8 in 64, eight rows 24.8, 17.9 and 22.6 (the clusters of 512 CTAs wait for SMs that are free together; so would
+// those of more rows, whose CTAs are not clustered).
 static int select_split(SelectParams p, int splits, int64_t *keys_out, int32_t *ids_out, void *workspace, cudaStream_t s) {
-  size_t smem = 0;
-  p.fold = splits > 1 && splits <= kFoldSplits && p.R <= kChainedRows && p.keep <= kTopWarp &&
-           select_chunk(1, p.keep, p.d, &smem) >= (1 + kSelWarps / 2) * kTopWarp;
-  if (splits == 1 || p.fold) {
+  const bool clustered = splits > 1 && p.R <= kChainedRows && p.keep <= kRowKeep;
+  int lists = splits;
+  p.cluster = 1;
+  if (clustered) {
+    p.cluster = splits < kRowCluster ? splits : kRowCluster;
+    lists = splits < 2 * kRowCluster ? 1 : splits >= 32 && p.R == 1 ? 8 : 4;
+    splits = lists * p.cluster;
+  }
+  if (lists == 1) {
     p.keys_out = keys_out, p.ids_out = ids_out;
-    return launch_select<1>(p, splits, s);
+    return launch_one_row(p, splits, s);
   }
   const int64_t *children = p.children;
   int32_t *carried_out = p.carried_out;
   p.children = nullptr, p.carried_out = nullptr;
   p.keys_out = (int64_t *)workspace, p.ids_out = nullptr;
-  const int rc = launch_select<1>(p, splits, s);
+  const int rc = launch_one_row(p, splits, s);
   if (rc != LSA_OK) return rc;
-  return merge_lists((const int64_t *)workspace, splits, p.R, p.keep, keys_out, ids_out, children, p.fanout, carried_out, true, s);
+  return merge_lists((const int64_t *)workspace, lists, p.R, p.keep, keys_out, ids_out, children, p.fanout, carried_out, true, s);
 }
 }  // namespace lsa
 
@@ -1660,7 +1889,7 @@ LSA_API int lsa_beam_step(const float *queries, int64_t R, int d, const float *v
   p.keep = keep;
   p.fanout = fanout;
   p.run_limit = (int)N;
-  return lsa::launch_select<1>(p, 1, (cudaStream_t)stream);
+  return lsa::launch_one_row(p, 1, (cudaStream_t)stream);
 }
 
 LSA_API int lsa_flat_select_paged(const float *queries, int64_t R, int d, const float *centroids, int64_t rows,

@@ -653,11 +653,10 @@ class FlatLayer:
 
     @staticmethod
     def _decode_splits(rows: int, buckets: int) -> int:
-        """CTAs that a decode row's buckets are split over. A CTA sorts up to a thousand candidates of a row in registers; up to
-        4,096 go to the eight CTAs of a cluster, which fold their lists (one row over 1,024: 15.3 us in one CTA, 11.6 in eight;
-        over 4,096: 16.3 in 32 CTAs and a merge, 14.0 in eight), more to 32 CTAs and a merge, or 16 where there are several rows
-        (16,384 buckets: one row 18.8 us in 32; 8 rows 29.2 in 32, 20.5 in 16)."""
-        return 1 if buckets <= 512 else 8 if buckets <= 4096 else 32 if rows == 1 else 16
+        """CTAs that a decode row's buckets are split over: one ranks 256 at a time; up to 4,096 go to the eight CTAs of a cluster,
+        more to several clusters and a merge (one row over 512 buckets: 7.7 us in one CTA, 6.4 in eight; over 4,096: 10.1 in eight
+        and 9.6 in 32 with the merge; over 16,384: 21.8 and 11.8)."""
+        return 1 if buckets <= 256 else 8 if buckets <= 4096 else 32 if rows == 1 else 16
 
     def _decodes_in_one_call(self, q: torch.Tensor, positions: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                              index: FlatIndex) -> bool:

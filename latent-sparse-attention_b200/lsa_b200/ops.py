@@ -333,9 +333,9 @@ def _scan_samples(m: int, top_p: int, max_visible: int) -> bool:
 
 
 def _split_launches(rows: int, splits: int, keep: int) -> int:
-    """Launches of a scan whose rows are split: the lists of up to 8 CTAs of 128 keys of a few rows are folded by a cluster,
-    others merged by a launch of their own."""
-    return 1 if splits <= 1 or (rows <= 8 and splits <= 8 and keep <= 128) else 2
+    """Launches of a scan whose rows are split: the lists of the CTAs of a cluster become one in it (a few rows, 128 keys at
+    most, eight CTAs), others are merged by a launch of their own."""
+    return 1 if splits <= 1 or (rows <= 8 and splits < 16 and keep <= 128) else 2
 
 
 def flat_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, request_first: torch.Tensor | None,

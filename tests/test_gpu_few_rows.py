@@ -98,6 +98,38 @@ def test_lists_folded_in_a_cluster_are_the_scan_s(m, d, keep):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("keep", [1, 31, 64, 128])
+@pytest.mark.parametrize("m", [1, 255, 256, 257, 1025, 5000])
+@pytest.mark.parametrize("d", [32, 64, 20])
+def test_a_row_ranked_by_counting_is_the_row_scanned_whole(m, d, keep):
+    """Tiles of 256 candidates that are full, ragged and empty, in one CTA, in clusters of 2 to 8 and in several clusters that are
+    merged, against the scan that holds a row's best in one buffer: key for key, ties among them, rows that see few or no
+    buckets, budgets, candidates named twice or not at all."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m + d)
+    q = torch.randn(6, d, device="cuda", generator=gen)
+    c = torch.randn(m, d, device="cuda", generator=gen).mul(2).round().div(2)
+    c[m // 2:] = c[:m - m // 2].clone()  # (ties)
+    visible = torch.tensor([m, m // 2, 1, 0, max(0, m - 1), min(m, 300)], device="cuda", dtype=torch.int32)
+    want = ops.flat_select(q, c, visible, keep)
+    for splits in (1, 2, 5, 8, 11, 16, 32, 100):
+        got = ops.flat_select_decode(q, c, None, visible, keep, splits=splits)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        got = ops.flat_select_decode(q.repeat(3, 1), c, None, visible.repeat(3), keep, splits=splits)  # (too many for clusters)
+        assert torch.equal(got[0], want[0].repeat(3, 1)) and torch.equal(got[1], want[1].repeat(3, 1))
+    named = torch.randint(-1, m, (6, 300), device="cuda", generator=gen, dtype=torch.int32)
+    named[:, 150:] = named[:, :150].clone()
+    none = torch.zeros_like(visible)
+    scores = ops.flat_select(q, c, torch.full_like(visible, m), m)[0] if m <= 512 else None
+    for splits in (1, 8, 16):
+        kept, keys = ops.beam_step(q, c, named, none, none, keep, splits=splits)
+        for row in range(6 if scores is not None else 0):
+            by_id = {0x7FFFFFFF - (int(k) & 0xFFFFFFFF): int(k) for k in scores[row].tolist()}
+            best = sorted((by_id[i] for i in named[row].tolist() if i >= 0), reverse=True)[:keep]
+            assert keys[row].tolist()[:len(best)] == best and set(kept[row].tolist()[len(best):]) <= {-1}
+
+
 @pytest.mark.parametrize("T,R,splits,sizes", [
     (700, 1, 8, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200, sink_size=4, window_size=128)),
     (9000, 8, 1, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=700, sink_size=0, window_size=100))])
