@@ -225,8 +225,8 @@ int lsa_dense_scores(const float *queries, int64_t R, int d, const float *centro
                      float *scores_out, int64_t *keys_out, void *stream);
 
 /* Flat search, decode form: few rows, many buckets. The buckets of a row are split over `splits` CTAs whose
- * local top_p lists are merged: by the row's cluster of CTAs for up to 8 rows of up to 8 splits and 128 keys, else by a second
- * kernel. Reference: Selector.decode_flat
+ * local top_p lists are merged: for up to 8 rows and 128 keys by the row's cluster of up to 8 CTAs (and, from 16 splits on, by a
+ * second kernel over 4 or 8 such clusters), else by a second kernel. Reference: Selector.decode_flat
  * (src/lsa/sglang/index/selector.py:603-660), scan_paged (src/lsa/core/kernels/triton/paged.py:61-101),
  * DecodeSelect.listed (src/lsa/core/kernels/cutedsl/decode.py:1035-1068).
  *   request_first [R] int64 - first row of centroids of each request (requests hold their buckets contiguously)
@@ -403,7 +403,8 @@ int lsa_expand_batched(const int32_t *picked, int64_t R, int top_p, const int64_
  *          [first_slot, first_slot + slots) is skipped
  *   init_out / init_lse  [R, Hq, dh] / [R, Hq] fp32 or both NULL - a partial read over OTHER keys (the dense band
  *          of lsa_band_attend) the read starts from, as one more term of the online softmax
- *   splits CTAs-per-(row, KV head) the list is divided over; > 1 needs the workspace and runs the merge kernel
+ *   splits CTAs-per-(row, KV head) the list is divided over; > 1 needs the workspace and runs the merge kernel, except that up to
+ *          8 rows of up to 64 (row, KV head) pairs are divided over a cluster of as many CTAs as suits them, which merges on chip
  *   out    [R, Hq, dh] bf16 (out_bf16) and/or fp32 (out_f32); lse [R, Hq] fp32 or NULL
  * A row that reads nothing gives zeros and lse = -inf.
  * --------------------------------------------------------------------------------------------------------- */

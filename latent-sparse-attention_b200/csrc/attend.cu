@@ -6,10 +6,14 @@
 // mma.m16n8k16 instead of 5 of 16 M rows, which halves the instructions per key. Softmax is online in the log2
 // domain with fp32 statistics; the kernel emits the natural-log log-sum-exp so partial results over disjoint key
 // sets (splits of a list here, ranks of a sequence-sharded cache elsewhere) merge exactly.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "mma.cuh"
 
 namespace lsa {
+
+namespace cg = cooperative_groups;
 
 constexpr int kKeysPerStage = 32;  // two 16-key MMA tiles, interleaved for instruction-level parallelism
 
@@ -24,11 +28,36 @@ struct AttendParams {
   float scale_log2;
 };
 
+// A team: the warps of a CTA share one (row, KV head, split), a slice of its keys each. At most six, and eight CTAs a cluster.
+constexpr int kTeamWarps = 6;
+constexpr int kTeamCluster = 8;
+
+// What a team's warps and a cluster's CTAs hand one another: maxima (log2), sums and weights of a head, and the outputs.
+template <int DH, int NT>
+struct TeamShared {
+  float m[kTeamWarps][8 * NT], l[kTeamWarps][8 * NT], w[kTeamWarps][8 * NT];
+  float m_all[kTeamCluster][8 * NT], l_all[kTeamCluster][8 * NT], w_all[kTeamCluster][8 * NT];
+  float4 out_all[8 * NT * DH / 4 + kTeamCluster];  // [cluster][this CTA's share of the output]
+};
+template <bool TEAM, int DH, int NT>
+struct TeamSharedOf {
+  using type = TeamShared<DH, NT>;
+};
+template <int DH, int NT>
+struct TeamSharedOf<false, DH, NT> {
+  using type = int;
+};
+
 // DH: head dim (64 or 128). NT: 8-head tiles a group needs (1 or 2). W: warps a CTA, at most. STAGES: ring depth.
 // What bounds a chunk of prefill rows is the gather's bytes out of L2 (10 to 11 TB/s in the 256-byte rows of 1,024-byte
 // tokens): stages of 16 keys with 14 warps an SM, or three stages a warp, moved the same or less (1.70 ms became 1.73 to
 // 2.30 over 16,384 rows of 1,100 keys and 2 KV heads).
-template <int DH, int NT, int W, int STAGES>
+//
+// TEAM: a decode step's few items, a CTA each. What bounds those is latency - a warp has two stages in flight and waits for each of
+// them -, so an item's keys are dealt to up to six warps, whose results meet in shared memory, and the splits of a row are the CTAs
+// of a cluster, each of which adds up its share of the output out of its own shared memory: no partial output goes through memory
+// and no merge is launched.
+template <int DH, int NT, int W, int STAGES, bool TEAM = false>
 __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p) {
   constexpr int ROW_BYTES = DH * 2;
   constexpr int CHUNKS = ROW_BYTES / 16;                    // 16-byte chunks a row
@@ -43,14 +72,18 @@ __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+  // (a team's grid is (row x KV head, split), any other's the items of all splits, a warp each)
+  const int64_t item = TEAM ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+  if (TEAM && p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   dependents_may_launch();
   wait_for_earlier_grids();
-  if (item >= p.R * p.splits * p.Hkv) return;
+  if (!TEAM && item >= p.R * p.splits * p.Hkv) return;
   const int h = (int)(item % p.Hkv);
   const int64_t rs = item / p.Hkv;
-  const int split = (int)(rs % p.splits);
-  const int64_t r = rs / p.splits;
+  const int split = TEAM ? (int)blockIdx.y : (int)(rs % p.splits);
+  const int64_t r = TEAM ? rs : rs / p.splits;
+  const int slices = TEAM ? p.splits * (int)(blockDim.x >> 5) : p.splits;
+  const int slice = TEAM ? split * (int)(blockDim.x >> 5) + warp : split;
 
   unsigned char *mine = smem_raw + (size_t)warp * WARP_BYTES;
   const uint32_t smem_base = smem_u32(mine);
@@ -59,10 +92,10 @@ __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p
   int64_t n_total = p.lengths ? p.lengths[r] : p.list_stride;
   if (n_total > p.list_stride) n_total = p.list_stride;
   if (n_total < 0) n_total = 0;
-  int64_t per = (n_total + p.splits - 1) / p.splits;
-  per = (per + kKeysPerStage - 1) / kKeysPerStage * kKeysPerStage;
-  const int64_t begin = (int64_t)split * per;
-  const int64_t end = begin + per < n_total ? begin + per : n_total;
+  // (whole stages a slice, one more for the first ones)
+  const int64_t stages = (n_total + kKeysPerStage - 1) / kKeysPerStage, each = stages / slices, more = stages % slices;
+  const int64_t begin = min((each * slice + min((int64_t)slice, more)) * kKeysPerStage, n_total);
+  const int64_t end = min(begin + (each + (slice < more)) * kKeysPerStage, n_total);
   const int n = end > begin ? (int)(end - begin) : 0;
   const int iters = (n + kKeysPerStage - 1) / kKeysPerStage;
   const int32_t *list = p.ids + r * p.list_stride + begin;
@@ -98,8 +131,8 @@ __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p
   }
 
   // Start from a partial read over other keys (the dense band of the window): it enters as one more term of the
-  // online softmax, weight exp(lse) and value its normalised output. Only the first split carries it.
-  if (p.init_out && split == 0) {
+  // online softmax, weight exp(lse) and value its normalised output. Only the first slice carries it.
+  if (p.init_out && slice == 0) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -258,41 +291,129 @@ __global__ void __launch_bounds__(W * 32, 1) sparse_attend_kernel(AttendParams p
 
   // Finish: the row sums live per thread; add them over the eight key lanes of each head.
   constexpr float kLn2 = 0.6931471805599453f;
+  if constexpr (TEAM) {
+    __shared__ typename TeamSharedOf<TEAM, DH, NT>::type team;
+    float *outs = reinterpret_cast<float *>(smem_raw);  // [warps][8 * NT][DH], over the rings
+    const int tid = threadIdx.x, warps = blockDim.x >> 5;
+    __syncthreads();  // (every warp's ring is spent)
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      float l = l_run[nt][j];
-      l += __shfl_xor_sync(0xffffffffu, l, 4);
-      l += __shfl_xor_sync(0xffffffffu, l, 8);
-      l += __shfl_xor_sync(0xffffffffu, l, 16);
-      const int head = nt * 8 + t * 2 + j;
-      if (head >= p.group) continue;
-      const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-      const float lse = l > 0.0f ? (m_run[nt][j] + log2f(l)) * kLn2 : -INFINITY;
-      const int64_t out_row = r * p.Hq + h * p.group + head;
-      if (p.splits > 1) {
-        float *dst = p.part_out + ((int64_t)split * p.R * p.Hq + out_row) * DH;
-#pragma unroll
-        for (int mt = 0; mt < DH / 16; ++mt) {
-          dst[mt * 16 + g] = o[nt][mt][j] * inv;
-          dst[mt * 16 + g + 8] = o[nt][mt][2 + j] * inv;
-        }
-        if (g == 0) p.part_lse[(int64_t)split * p.R * p.Hq + out_row] = lse;
-      } else {
+      for (int j = 0; j < 2; ++j) {
+        float l = l_run[nt][j];
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        const int head = nt * 8 + t * 2 + j;
+        float *dst = outs + (warp * 8 * NT + head) * DH;
 #pragma unroll
         for (int mt = 0; mt < DH / 16; ++mt) {
-          const float lo = o[nt][mt][j] * inv, hi = o[nt][mt][2 + j] * inv;
-          if (p.out_bf16) {
-            p.out_bf16[out_row * DH + mt * 16 + g] = float_to_bf16_bits(lo);
-            p.out_bf16[out_row * DH + mt * 16 + g + 8] = float_to_bf16_bits(hi);
-          }
-          if (p.out_f32) {
-            p.out_f32[out_row * DH + mt * 16 + g] = lo;
-            p.out_f32[out_row * DH + mt * 16 + g + 8] = hi;
-          }
+          dst[mt * 16 + g] = o[nt][mt][j];
+          dst[mt * 16 + g + 8] = o[nt][mt][2 + j];
         }
-        if (g == 0 && p.lse) p.lse[out_row] = lse;
+        if (g == 0) team.m[warp][head] = m_run[nt][j], team.l[warp][head] = l;
+      }
+    __syncthreads();
+    // Weights of one head's parts: a thread a (part, head). (A head that saw no key has a maximum of -inf and weights of zero.)
+    auto weigh = [&](const float (*m)[8 * NT], float (*w)[8 * NT], int parts) {
+      for (int e = tid; e < parts * 8 * NT; e += blockDim.x) {
+        const int part = e / (8 * NT), head = e % (8 * NT);
+        float mx = -INFINITY;
+        for (int i = 0; i < parts; ++i) mx = fmaxf(mx, m[i][head]);
+        w[part][head] = mx > -INFINITY ? exp2f(m[part][head] - mx) : 0.0f;
+      }
+    };
+    weigh(team.m, team.w, warps);
+    const int own = split, C = p.splits, pieces = p.group * DH / 4, share = (pieces + C - 1) / C;  // (in pieces of four dims)
+    cg::cluster_group cluster = cg::this_cluster();
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // (every CTA of the cluster is there)
+    __syncthreads();
+    if (tid < p.group) {
+      float mx = -INFINITY, sum = 0.0f;
+      for (int i = 0; i < warps; ++i) mx = fmaxf(mx, team.m[i][tid]), sum = fmaf(team.w[i][tid], team.l[i][tid], sum);
+      for (int peer = 0; peer < C; ++peer) {
+        *cluster.map_shared_rank(&team.m_all[own][tid], peer) = mx;
+        *cluster.map_shared_rank(&team.l_all[own][tid], peer) = sum;
+      }
+    }
+    for (int e = tid; e < pieces; e += blockDim.x) {
+      const int head = e / (DH / 4), owner = e / share;
+      float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      for (int i = 0; i < warps; ++i) {
+        const float w = team.w[i][head];
+        const float4 x = reinterpret_cast<const float4 *>(outs)[i * (8 * NT * DH / 4) + e];
+        acc.x = fmaf(w, x.x, acc.x), acc.y = fmaf(w, x.y, acc.y), acc.z = fmaf(w, x.z, acc.z), acc.w = fmaf(w, x.w, acc.w);
+      }
+      *cluster.map_shared_rank(&team.out_all[own * share + (e - owner * share)], owner) = acc;
+    }
+    if (C > 1) {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // (no CTA reaches into another's from here on)
+    } else {
+      __syncthreads();
+    }
+    weigh(team.m_all, team.w_all, C);
+    __syncthreads();
+    const int64_t first_row = r * p.Hq + h * p.group;  // of the item's heads
+    for (int i = tid; i < share && own * share + i < pieces; i += blockDim.x) {
+      const int e = own * share + i, head = e / (DH / 4);
+      float mx = -INFINITY, sum = 0.0f;
+      float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int j = 0; j < kTeamCluster; ++j) {
+        if (j >= C) break;
+        const float w = team.w_all[j][head];
+        const float4 x = team.out_all[j * share + i];
+        mx = fmaxf(mx, team.m_all[j][head]), sum = fmaf(w, team.l_all[j][head], sum);
+        acc.x = fmaf(w, x.x, acc.x), acc.y = fmaf(w, x.y, acc.y), acc.z = fmaf(w, x.z, acc.z), acc.w = fmaf(w, x.w, acc.w);
+      }
+      const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+      const float out4[4] = {acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv};
+      const int64_t at = first_row * DH + 4 * e;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (p.out_bf16) p.out_bf16[at + c] = float_to_bf16_bits(out4[c]);
+        if (p.out_f32) p.out_f32[at + c] = out4[c];
+      }
+      if (p.lse && e % (DH / 4) == 0) p.lse[first_row + head] = sum > 0.0f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
+    }
+  } else {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float l = l_run[nt][j];
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        const int head = nt * 8 + t * 2 + j;
+        if (head >= p.group) continue;
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        const float lse = l > 0.0f ? (m_run[nt][j] + log2f(l)) * kLn2 : -INFINITY;
+        const int64_t out_row = r * p.Hq + h * p.group + head;
+        if (p.splits > 1) {
+          float *dst = p.part_out + ((int64_t)split * p.R * p.Hq + out_row) * DH;
+#pragma unroll
+          for (int mt = 0; mt < DH / 16; ++mt) {
+            dst[mt * 16 + g] = o[nt][mt][j] * inv;
+            dst[mt * 16 + g + 8] = o[nt][mt][2 + j] * inv;
+          }
+          if (g == 0) p.part_lse[(int64_t)split * p.R * p.Hq + out_row] = lse;
+        } else {
+#pragma unroll
+          for (int mt = 0; mt < DH / 16; ++mt) {
+            const float lo = o[nt][mt][j] * inv, hi = o[nt][mt][2 + j] * inv;
+            if (p.out_bf16) {
+              p.out_bf16[out_row * DH + mt * 16 + g] = float_to_bf16_bits(lo);
+              p.out_bf16[out_row * DH + mt * 16 + g + 8] = float_to_bf16_bits(hi);
+            }
+            if (p.out_f32) {
+              p.out_f32[out_row * DH + mt * 16 + g] = lo;
+              p.out_f32[out_row * DH + mt * 16 + g + 8] = hi;
+            }
+          }
+          if (g == 0 && p.lse) p.lse[out_row] = lse;
+        }
       }
     }
   }
@@ -402,6 +523,31 @@ static int launch_attend(const AttendParams &p, cudaStream_t s) {
   const int64_t grid = (items + warps - 1) / warps;
   if (grid > INT32_MAX) return LSA_ERR_ARGUMENT;
   launch(p.R <= kChainedRows, sparse_attend_kernel<DH, NT, W, STAGES>, dim3((unsigned)grid), dim3(warps * 32), smem, s, p);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
+// A few rows' items: a cluster each, of eight CTAs, or of four where eight would be more than the SMs hold side by side (clusters
+// of eight fill 112 SMs with one CTA of six warps each; two of three warps fit where one of six does not), and a team a CTA. 40 / 8
+// heads, lists out of HBM, one B200, a graph of the call, in us, a warp an item with 8 splits / 16 splits and a merge -> this: one
+// row of 600 keys 12.1 / 8.4 -> 6.5, of 3,076 24.4 / 15.1 -> 10.2, of 17,412 84.9 / 46.1 -> 24.8; four rows of 3,076 25.9 / 19.0 ->
+// 15.0; eight 31.3 / 26.0 -> 22.5, of 17,412 112 / 96 -> 89 (clusters of eight took 31 and 106). More than 64 items are work
+// enough for a warp an item.
+constexpr int64_t kTeamItems = 64;  // (row, KV head) pairs, at most
+template <int DH, int NT, int STAGES>
+static int launch_attend_team(AttendParams p, cudaStream_t s) {
+  constexpr int WARP_BYTES = STAGES * 2 * kKeysPerStage * DH * 2 + 16;
+  const auto kernel = sparse_attend_kernel<DH, NT, kTeamWarps, STAGES, true>;
+  const int64_t items = p.R * p.Hkv, stages = (p.list_stride + kKeysPerStage - 1) / kKeysPerStage;
+  p.splits = items <= 16 ? 8 : 4;
+  while (p.splits > 1 && p.splits > stages) p.splits >>= 1;
+  const int64_t ctas = items * p.splits;
+  int64_t warps = p.splits == 8 ? (ctas <= 112 ? kTeamWarps : kTeamWarps / 2) : kTeamWarps * sm_count() / ctas;
+  if (warps > (stages + p.splits - 1) / p.splits) warps = (stages + p.splits - 1) / p.splits;
+  warps = warps < 1 ? 1 : warps > kTeamWarps ? kTeamWarps : warps;
+  if (!allow_shared(kernel, (size_t)kTeamWarps * WARP_BYTES)) return LSA_ERR_LAUNCH;
+  launch_clusters(p.R <= kChainedRows, kernel, dim3((unsigned)items, (unsigned)p.splits), dim3((unsigned)warps * 32),
+                  (size_t)warps * WARP_BYTES, s, p, p.splits);
   LSA_LAUNCH_CHECK();
   return LSA_OK;
 }
@@ -673,6 +819,11 @@ LSA_API int lsa_sparse_attend(const uint16_t *q, int64_t R, int Hq, int dh, int6
   }
   cudaStream_t s = (cudaStream_t)stream;
   int rc;
+  // (a list read in one piece keeps its order of sums, whatever rows are beside it)
+  if (splits > 1 && R <= lsa::kChainedRows && R * Hkv <= lsa::kTeamItems) {
+    if (dh == 128) return group <= 8 ? lsa::launch_attend_team<128, 1, 2>(p, s) : lsa::launch_attend_team<128, 2, 2>(p, s);
+    return group <= 8 ? lsa::launch_attend_team<64, 1, 3>(p, s) : lsa::launch_attend_team<64, 2, 3>(p, s);
+  }
   // Shared memory a warp: dh 128 -> 2 stages of 16 KB (7 warps fill an SM), dh 64 -> 3 stages of 8 KB (9 warps).
   if (dh == 128)
     rc = group <= 8 ? lsa::launch_attend<128, 1, 7, 2>(p, s) : lsa::launch_attend<128, 2, 7, 2>(p, s);

@@ -637,8 +637,13 @@ def sparse_attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ids: torch.
          k.stride(1), ptr(ids), ids.shape[1], ptr(lengths), ptr(init[0]) if init else None,
          ptr(init[1]) if init else None, float(scale), splits, ptr(out_bf16), ptr(out_f32),
          ptr(lse), ptr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0,
-         stream(), launches=1 if splits == 1 else 2)
+         stream(), launches=_attend_launches(R, Hkv, splits))
     return (out_bf16 if out_bf16 is not None else out_f32), lse
+
+
+def _attend_launches(rows: int, kv_heads: int, splits: int) -> int:
+    """Launches of a gather: a few rows' splits (as many as suit them) meet in a cluster, others are merged by a launch."""
+    return 1 if splits == 1 or (rows <= 8 and rows * kv_heads <= 64) else 2
 
 
 def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh_used: int, positions: torch.Tensor,
@@ -656,7 +661,7 @@ def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh
          dh_off, dh_used, d_idx, ptr(positions), ptr(centroids), centroids.shape[0], ptr(members), members.shape[1], block_size,
          block_buckets, top_p, top_k, sink, window, select_splits, ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0), k.stride(1),
          float(scale), splits, ptr(out), ptr(expand_status), ptr(workspace), need, stream(),
-         launches=3 + _split_launches(R, select_splits, top_p) + (1 if splits == 1 else 2))
+         launches=3 + _split_launches(R, select_splits, top_p) + _attend_launches(R, k.shape[1], splits))
     return out
 
 

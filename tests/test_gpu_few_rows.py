@@ -130,6 +130,37 @@ def test_a_row_ranked_by_counting_is_the_row_scanned_whole(m, d, keep):
             assert keys[row].tolist()[:len(best)] == best and set(kept[row].tolist()[len(best):]) <= {-1}
 
 
+@pytest.mark.parametrize("heads,kv_heads,dh", [(40, 8, 128), (9, 1, 128), (8, 8, 64), (32, 2, 64)])
+def test_a_few_rows_attend_as_many_rows_do(heads, kv_heads, dh):
+    """A CTA of warps an item and its splits in a cluster, against the same rows among many (a warp an item): lists that are empty,
+    shorter than a warp's stage, ragged and longer than one cluster is given, slots outside the cache, a partial read to start from.
+    The probabilities are rounded to bf16 against other maxima: 2^-9 of an output's terms, which average out to a tenth of it."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    slots, R = 9000, 7
+    q = torch.randn(R, heads, dh, device="cuda", generator=gen).bfloat16()
+    k, v = (torch.randn(slots, kv_heads, dh, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    for width in (40, 3001, 8500):
+        ids = torch.stack([torch.randperm(slots + 50, device="cuda", generator=gen)[:width] for _ in range(R)]).to(torch.int32)
+        lengths = torch.tensor([width, 0, 1, 31, 33, width - 1, width // 2], device="cuda", dtype=torch.int32)
+        init = (torch.randn(R, heads, dh, device="cuda", generator=gen), torch.randn(R, heads, device="cuda", generator=gen))
+        init[1][0, 0] = -float("inf")
+        many = lambda x: torch.cat([x] * 2)
+        for start in (None, init):
+            want, want_lse = ops.sparse_attend(many(q), k, v, many(ids), many(lengths), dh ** -0.5, out_dtype=torch.float32,
+                                               init=None if start is None else tuple(many(x) for x in start))
+            for splits in (1, 2, 3, 8, 9, 16):
+                got, lse = ops.sparse_attend(q, k, v, ids, lengths, dh ** -0.5, splits=splits, out_dtype=torch.float32, init=start)
+                assert (got - want[:R]).abs().max() <= 2 ** -9 and (got - want[:R]).norm() <= 1e-3 * want[:R].norm()
+                seen = torch.isfinite(want_lse[:R])
+                assert torch.equal(torch.isfinite(lse), seen) and (lse - want_lse[:R])[seen].abs().max() <= 2e-5
+                if start is None:
+                    assert not got[1].any() and not seen[1].any()
+            half, _ = ops.sparse_attend(q, k, v, ids, lengths, dh ** -0.5, splits=8, init=start)
+            assert (half.float() - want[:R]).norm() <= 4e-3 * want[:R].norm()
+
+
 @pytest.mark.parametrize("T,R,splits,sizes", [
     (700, 1, 8, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200, sink_size=4, window_size=128)),
     (9000, 8, 1, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=700, sink_size=0, window_size=100))])
