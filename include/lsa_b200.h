@@ -181,6 +181,14 @@ int lsa_flat_select(const float *queries, int64_t R, int d, const float *centroi
                     const int32_t *visible, const int32_t *row_top_p, int top_p, int32_t bucket_id_base,
                     int64_t *keys_out, int32_t *picked_out, void *stream);
 
+/* The same search of many rows over few buckets (d 32 or 64, m up to 4,096, queries and centroids 16-byte aligned) through a
+ * scratch matrix of scores: the result is lsa_flat_select's, key for key. Other sizes and alignments: LSA_ERR_UNSUPPORTED.
+ *   workspace  lsa_flat_select_binned_workspace_bytes(R, d, m) bytes (at most 48 MiB; 0: not a size it takes), 16-byte aligned */
+size_t lsa_flat_select_binned_workspace_bytes(int64_t R, int d, int64_t m);
+int lsa_flat_select_binned(const float *queries, int64_t R, int d, const float *centroids, int64_t m, const int32_t *visible,
+                           const int32_t *row_top_p, int top_p, int32_t bucket_id_base, int64_t *keys_out, int32_t *picked_out,
+                           void *workspace, size_t workspace_bytes, void *stream);
+
 /* The same search with the scan on the tensor cores: the result is lsa_flat_select's, key for key. The bf16
  * scores of every (row, bucket) pair are made in tensor memory by tcgen05 products and never written; a row keeps
  * the buckets whose score, plus the bucket's own bf16 error bound, reaches a threshold bisected from 512 strided

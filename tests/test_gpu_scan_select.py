@@ -144,3 +144,78 @@ def test_index_vectors_in_a_narrow_cone_are_told_apart_about_their_centre(ops):
     assert 0.99 < float(unit) < 1.01 and torch.equal(plain, c.bfloat16())
     got, _ = ops.scan_select(q, c, plain, v, 64, lengths=ones, radius=unit)  # (the rows are crowded: scanned exactly)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("m,keep", [(1, 4), (2, 1), (127, 64), (129, 128), (1025, 700), (3072, 1024), (4095, 2048), (4096, 16)])
+def test_rows_placed_by_bins_are_the_rows_scanned(d, m, keep, monkeypatch):
+    """Scores in a scratch matrix and places counted bin by bin, against the scan that keeps a row's best in a buffer, key for key:
+    rows that see few or no buckets, budgets, ids that do not start at zero, and rows whose scores are all one number, two numbers,
+    one far from the rest or none at all; rows in several pieces; replayed from a graph."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m + d)
+    R = 300
+    q = torch.randn(R, d, device="cuda", generator=gen)
+    c = torch.randn(m, d, device="cuda", generator=gen)
+    c[::3] = c[::3].mul(2).round().div(2)
+    q[0], q[1, 1:], q[2], q[3, 0], q[4] = 0.0, 0.0, 1e30, float("inf"), float("nan")
+    q[5:40] = q[5:40].round()
+    c[m // 2] *= 1e5
+    visible = torch.randint(0, m + 3, (R,), device="cuda", generator=gen, dtype=torch.int32)
+    visible[:20], visible[20] = m, 0
+    row_p = torch.randint(0, keep + 1, (R,), device="cuda", generator=gen, dtype=torch.int32)
+    scratch = torch.empty(ops.query("lsa_flat_select_binned_workspace_bytes", R, d, m), device="cuda", dtype=torch.uint8)
+    taken = []
+
+    def both(*args):
+        monkeypatch.setattr(ops, "_binned_scratch", lambda *_: (taken.append(1), scratch)[1])
+        got = ops.flat_select(*args)
+        monkeypatch.setattr(ops, "_binned_scratch", lambda *_: None)
+        return got, ops.flat_select(*args)
+
+    for budget in (None, row_p):
+        got, want = both(q, c, visible, keep, budget, 1000)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert len(taken) == 2
+    if m == 4096:  # (pieces of 3,072 rows)
+        many, seen = q.repeat(25, 1), visible.repeat(25)
+        scratch = torch.empty(ops.query("lsa_flat_select_binned_workspace_bytes", 7500, d, m), device="cuda", dtype=torch.uint8)
+        got, want = both(many, c, seen, keep)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        keys, picked = torch.empty_like(got[0]), torch.empty_like(got[1])
+        monkeypatch.undo()
+        assert ops._binned_scratch(many, c, keep) is not None
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.flat_select(many, c, seen, keep, keys=keys, picked=picked)
+        keys.zero_()
+        graph.replay()
+        assert torch.equal(keys, want[0]) and torch.equal(picked, want[1])
+
+
+def test_a_search_without_memory_for_its_scores_goes_without(monkeypatch):
+    """No scratch, an unaligned query or a size the scores' form does not take: the other forms serve the call."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    q, c = torch.randn(256, 64, device="cuda", generator=gen), torch.randn(1500, 64, device="cuda", generator=gen)
+    visible = torch.full((256,), 1500, device="cuda", dtype=torch.int32)
+    want = ops.flat_select(q, c, visible, 600)
+    real = torch.empty
+
+    def none(*size, **kind):
+        if kind.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("no memory")
+        return real(*size, **kind)
+
+    with monkeypatch.context() as patch:
+        patch.setattr(ops.torch, "empty", none)
+        got = ops.flat_select(q, c, visible, 600)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    with pytest.raises(ValueError, match="shape"):
+        ops.flat_select(q, c.repeat(2, 1), visible, 2100)
+    apart = torch.empty(256 * 64 + 1, device="cuda")[1:].view(256, 64).copy_(q)
+    assert ops._binned_scratch(apart, c, 600) is None and ops._binned_scratch(q, c.repeat(3, 1), 600) is None
+    got = ops.flat_select(apart, c, visible, 600)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
