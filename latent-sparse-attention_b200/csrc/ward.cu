@@ -12,14 +12,18 @@
 // A round looks only at what the round before changed. A pair's cost depends on nothing but its two rows, so a row whose
 // cheapest partner neither merged nor went keeps it, unless a row that just merged is cheaper:
 //   dirty rows (merged, or their partner merged or went)  x  all open rows
-//   the other open rows                                   x  the rows that merged
-// and a row too large for the smallest row left is closed: it can never merge again (in a pairing, every pair). What
-// bounds it is fp32 multiply-adds in the first round and barriers in the last ones, where a handful of rows is dirty (a
-// round of a block of 80 pools takes 7 us, of which the tiles are 2).
+// and a row too large for the smallest row left is closed: it can never merge again (in a pairing, every pair). A pair's
+// cost has the same bits from either side, so two dirty rows meet once and a tile of theirs serves both, and the other open
+// rows learn of what merged from the same tiles. What bounds the first rounds is a tile's operands out of shared memory (of a
+// larger block's tile of 128 x 128 pairs, 25 k cycles, the products are 15 k, where their multiply-adds alone would be 8 k;
+// two sums a multiply-add with fma.rn.f32x2, whose operands are twice the bytes, came out alike), the last ones barriers,
+// where a handful of rows is dirty (a round of a block of 80 pools takes 7 us, of which the tiles are 2).
 // Measured on a B200, against every row searching all of its partners every round (one CTA a block up to 512 pools, two
 // launches a round, 256 rounds, above): the pairings of 16 blocks of 4,096, 2,048 and 1,024 buckets 26.0 -> 4.4 ms; 1,024
 // blocks of 256 pools with the pairings of 512, 256 and 128 buckets 7.2 -> 2.4 ms; 9 blocks of 128 pools 165 -> 57 us; one
-// block of 80 pools, sixteen rounds, 190 -> 119 us.
+// block of 80 pools, sixteen rounds, 190 -> 119 us. With every pair once, on the index of 1M clustered tokens: 1,024 blocks of 256
+// pools 2.10 -> 1.65 ms, the pairings of 16 blocks of 4,096 buckets 3.07 -> 2.28 (the first round 1.30 -> 0.76), of 2,048 0.92 ->
+// 0.77, of 1,024 384 -> 353 us, of 512 176 -> 158.
 //
 // Arithmetic order is the CPU specification's: a dot is an fma chain in ascending dim order, costs are evaluated as
 // written, so labels are bit-equal to a replay in that order.
@@ -134,6 +138,7 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   const int64_t apart = LOCAL ? (ctas > 1 ? P : 0) : (int64_t)(gridDim.x / ctas) * P;
   unsigned long long *mine = LOCAL ? s.cheapest : p.cheapest + g * P;
   __shared__ int warp_count[kThreads / 32], n_merge_s, smallest_s;
+  __shared__ float bound_s[TILE], known_s[TILE];  // costs that the cheapest of a tile's rows and of its partners are not above
   // What a CTA wrote before is seen by all of the block's after. (CTAs that are no cluster are launched as a cooperative grid,
   // so that all of them run: a wait that gives up all the same ends the block as one that did not reach its count.)
   bool gave_up = false;
@@ -272,9 +277,10 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   const float slack = __syncthreads_or(great) ? INFINITY : 9.5367431640625e-7f;
 
   for (; rounds < p.max_rounds && n_alive > p.bucket_count && !gave_up; ++rounds) {
-    // ---- the cheapest partners: tiles of (dirty x open) and (steady x merged), dealt to the CTAs in runs
-    auto stage = [&](float *tile, const uint16_t *list, int from, int n) {
-      for (int e = tid; e < TILE * (D / 4); e += kThreads) {
+    // ---- the cheapest partners: tiles of (dirty x open), dealt to the CTAs in runs. A pair's cost is the same from either side,
+    // bit for bit, so a tile serves its rows and its partners: two dirty rows meet once, and a steady row meets what merged.
+    auto stage = [&](float *tile, const uint16_t *list, int from, int n, int most) {
+      for (int e = tid; e < most * (D / 4); e += kThreads) {
         const int r = e / (D / 4), k = e - r * (D / 4);
         if (from + r < n) {
           const int id = list[from + r];
@@ -284,27 +290,31 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
         }
       }
     };
-    // One row tile against partner tiles first_tile .. end_tile - 1 of `lists` (two lists side by side, or one).
-    auto search = [&](auto rows_a_warp, const uint16_t *rows, int first_row, int n_rows, bool known,
-                      const uint16_t *list0, int n0, const uint16_t *list1, int n1, int first_tile, int end_tile) {
+    // A cost that a row's cheapest is not above: what it has so far.
+    auto known = [&](int id) {
+      const unsigned long long *at = mine + side * apart + id, v = LOCAL ? *(const volatile unsigned long long *)at : __ldcg(at);
+      return v == ~0ull ? INFINITY : cheapest_cost(v);
+    };
+    const int tiles0 = (n_dirty + TILE - 1) / TILE, tiles1 = (n_steady + TILE - 1) / TILE;
+    // One row tile of the dirty rows against partner tiles first_tile .. end_tile - 1 of the dirty and then the steady rows.
+    auto search = [&](auto rows_a_warp, int first_row, int first_tile, int end_tile) {
       constexpr int ROWS = decltype(rows_a_warp)::value;
-      const int tiles0 = (n0 + TILE - 1) / TILE;
-      const uint16_t *my_list = rows + first_row + warp * ROWS;
-      const int my_rows = min(ROWS, n_rows - first_row - warp * ROWS);  // (0 or less: this warp has none)
+      const uint16_t *my_list = s.dirty + first_row + warp * ROWS;
+      const int my_rows = min(ROWS, n_dirty - first_row - warp * ROWS);  // (0 or less: this warp has none)
       float best_c[ROWS];
       int best_j[ROWS];
 #pragma unroll
-      for (int i = 0; i < ROWS; ++i) {  // (a steady row keeps its partner unless a merged row is cheaper)
-        best_c[i] = known && i < my_rows ? s.cost[my_list[i]] : INFINITY;
-        best_j[i] = best_c[i] < INFINITY ? s.best[my_list[i]] : 0x7FFFFFFF;
-      }
+      for (int i = 0; i < ROWS; ++i) best_c[i] = INFINITY, best_j[i] = 0x7FFFFFFF;
       __syncthreads();  // (the tiles are free)
-      stage(s.a, rows + first_row, 0, min(ROWS * kThreads / 32, n_rows - first_row));
+      stage(s.a, s.dirty, first_row, n_dirty, ROWS * kThreads / 32);
+      if (!LOCAL && lane < my_rows) bound_s[warp * ROWS + lane] = known(my_list[lane]);
       for (int t = first_tile; t < end_tile; ++t) {
-        const uint16_t *others = t < tiles0 ? list0 : list1;
-        const int n_others = t < tiles0 ? n0 : n1, from = (t < tiles0 ? t : t - tiles0) * TILE;
+        const uint16_t *others = t < tiles0 ? s.dirty : s.steady;
+        const int n_others = t < tiles0 ? n_dirty : n_steady, from = (t < tiles0 ? t : t - tiles0) * TILE;
+        const bool both_ways = t != first_row / TILE;  // (the tile that the rows are of meets itself: every pair is there twice)
         if (t > first_tile) __syncthreads();
-        stage(s.b, others, from, n_others);
+        stage(s.b, others, from, n_others, TILE);
+        if (tid < TILE) known_s[tid] = both_ways && from + tid < n_others ? known(others[from + tid]) : -INFINITY;
         __syncthreads();
         if (my_rows <= 0) continue;
         float acc[ROWS][COLS];
@@ -330,8 +340,8 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
           }
         }
         // (rows and partners past the lists hold whatever the tiles held: they are not looked at)
-        int id_j[COLS];
-        float sq_j[COLS], al_j[COLS], sz_j[COLS];
+        int id_j[COLS], theirs_i[COLS];
+        float sq_j[COLS], al_j[COLS], sz_j[COLS], theirs_c[COLS];
 #pragma unroll
         for (int j = 0; j < COLS; ++j) {
           const int c = from + lane + 32 * j;
@@ -339,29 +349,47 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
           sq_j[j] = c < n_others ? s.sq[id_j[j]] : 0.0f;
           al_j[j] = c < n_others ? s.al[id_j[j]] : 0.0f;
           sz_j[j] = c < n_others ? s.sz[id_j[j]] : 0.0f;
+          theirs_c[j] = known_s[lane + 32 * j], theirs_i[j] = -1;
         }
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) {
           if (i >= my_rows) break;
           const int id_i = my_list[i];
           const float sq_i = s.sq[id_i], al_i = s.al[id_i], sz_i = s.sz[id_i];
+          const float bound_i = LOCAL ? INFINITY : bound_s[warp * ROWS + i], best_before = best_c[i];
 #pragma unroll
           for (int j = 0; j < COLS; ++j) {
             const float m2 = __fadd_rn(__fadd_rn(sq_i, sq_j[j]), __fmul_rn(2.0f, acc[i][j]));
             const float both = __fadd_rn(al_i, al_j[j]);
-            // Most pairs are far from the cheapest so far, and a product says so without the root: with
+            // Most pairs are far from the cheapest so far of either, and a product says so without the root: with
             // most = both - best - both / 2^20 positive and m2 <= most^2 (1 - 2^-20), the root is under `most` by more
             // than the roundings of all of these (a few 2^-24 of `both`), so the cost is above the best, and not a tie.
             // (That takes squares that are normal numbers: `most` is above 1e-15, and `slack` lets no pair through here in a
             // block whose norms may leave their range.)
-            const float most = (both - best_c[i]) - both * slack;
+            const float most = (both - fmaxf(fminf(bound_i, best_c[i]), theirs_c[j])) - both * slack;
             if (most > 1e-15f && m2 <= most * most * 0.99999904632568359375f) continue;
             if (id_j[j] < 0 || id_i == id_j[j] || __fadd_rn(sz_i, sz_j[j]) > p.bucket_cap) continue;
             const float whole = sqrtf(m2 > 0.0f ? m2 : 0.0f);
             const float cost = __fsub_rn(both, whole);
             if (cost < best_c[i] || (cost == best_c[i] && id_j[j] < best_j[i])) best_c[i] = cost, best_j[i] = id_j[j];
+            // (the lists ascend, so a tie of two of this thread's rows stays with the first; one with what the partner knows
+            // is settled where the minima are kept)
+            if (cost < theirs_c[j] || (cost == theirs_c[j] && theirs_i[j] < 0)) theirs_c[j] = cost, theirs_i[j] = id_i;
+          }
+          // (the lanes share what they found, so that in the next tile a pair is far from the cheapest of all of them; a local
+          // block has few tiles a row)
+          if (!LOCAL && __any_sync(0xffffffffu, best_c[i] < best_before && best_c[i] < bound_i)) {
+            float least = best_c[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+            if (lane == 0) bound_s[warp * ROWS + i] = fminf(bound_i, least);
           }
         }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+          if (both_ways && theirs_i[j] >= 0 && theirs_c[j] < INFINITY)
+            atomicMin(mine + side * apart + id_j[j], pack_cheapest(theirs_c[j], theirs_i[j]));
       }
       if (my_rows <= 0) return;
       // The lanes fold a row's minima, halving the rows a lane holds while there is more than one: a lane ends up with
@@ -391,28 +419,29 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
       if ((lane & (2 * left - 1)) == 0 && my_row < my_rows && best_c[0] < INFINITY)
         atomicMin(mine + side * apart + my_list[my_row], pack_cheapest(best_c[0], best_j[0]));
     };
-    // The tiles of a list of rows against its partners, this CTA's run of them, a row tile at a time.
-    auto search_all = [&](const uint16_t *rows, int n_rows, bool known, const uint16_t *list0, int n0,
-                          const uint16_t *list1, int n1) {
-      const int across = (n0 + TILE - 1) / TILE + (n1 + TILE - 1) / TILE;
+    // This CTA's run of the tiles, a row tile at a time. A row tile meets the dirty partners from its own tile on.
+    {
+      const int all = tiles0 + tiles1;
       // Eight rows a warp where that leaves every CTA a tile; else (a small block, a late round) two, for four times
       // the tiles.
       constexpr int SMALL = kWardFewRows * kThreads / 32;
-      int high = (n_rows + TILE - 1) / TILE;
-      const bool few = n_rows <= SMALL || high * across < ctas;
-      if (few) high = (n_rows + SMALL - 1) / SMALL;
-      const int lo = (int)((int64_t)high * across * rank / ctas), hi = (int)((int64_t)high * across * (rank + 1) / ctas);
-      for (int at = lo; at < hi;) {
-        const int rt = at / across, first = at - rt * across, end = min(across, first + hi - at);
+      const bool few = n_dirty <= SMALL || tiles0 * (tiles0 + 1) / 2 + tiles0 * tiles1 < ctas;
+      const int height = few ? SMALL : TILE, high = (n_dirty + height - 1) / height;
+      int64_t count = 0;
+      for (int rt = 0; rt < high; ++rt) count += all - rt * height / TILE;
+      const int64_t lo = count * rank / ctas, hi = count * (rank + 1) / ctas;
+      int64_t before = 0;
+      for (int rt = 0; rt < high && before < hi; ++rt) {
+        const int own = rt * height / TILE, across = all - own;
+        const int first = (int)max((int64_t)0, lo - before), end = (int)min((int64_t)across, hi - before);
+        before += across;
+        if (first >= end) continue;
         if (few)
-          search(std::integral_constant<int, kWardFewRows>(), rows, rt * SMALL, n_rows, known, list0, n0, list1, n1, first, end);
+          search(std::integral_constant<int, kWardFewRows>(), rt * height, own + first, own + end);
         else
-          search(std::integral_constant<int, kWardRows>(), rows, rt * TILE, n_rows, known, list0, n0, list1, n1, first, end);
-        at += end - first;
+          search(std::integral_constant<int, kWardRows>(), rt * height, own + first, own + end);
       }
-    };
-    search_all(s.dirty, n_dirty, false, s.dirty, n_dirty, s.steady, n_steady);
-    search_all(s.steady, n_steady, true, s.merged, n_merged, nullptr, 0);
+    }
     everyone();
     if (gave_up) break;
 
