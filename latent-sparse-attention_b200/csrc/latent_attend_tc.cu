@@ -20,7 +20,7 @@
 //   warp 4      tensor-memory allocation; issues S = Q K^T of every tile
 //   warp 9      issues O += P V of every tile (a warp of its own: the two products belong to tiles in
 //               different stages, and one warp for both makes each wait for the other's loads)
-//   warps 5-8   staging: a tile is up to 64 listed rows. 64 consecutive rows of the cache - what a bucket's pools
+//   warps 5-8   staging: the queries (warps 6-8, beside the first tiles), then tiles of up to 64 listed rows. 64 consecutive rows of the cache - what a bucket's pools
 //               and a window are made of - are ONE box of a tensor-map copy per plane, wherever they start;
 //               anything else is gathered with 16-byte asynchronous copies into the same swizzled planes
 //
@@ -35,6 +35,7 @@
 namespace lsa {
 
 constexpr int kLtThreads = 320;
+constexpr int kLtQueryThreads = 96;                 // the staging warps but the first bring the queries in
 constexpr int kLtKeys = 64;                         // gathered rows a tile
 constexpr int kLtPlanes = 9;                        // 576 dims = 9 planes of 64
 constexpr int kLtPlane = 64 * 128;                  // 64 rows x 64 dims of bf16
@@ -92,8 +93,8 @@ __global__ void __launch_bounds__(kLtThreads, 1)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // k_full / k_empty: a ring stage's rows have landed / may be overwritten; s_full / s_empty: an S buffer holds a
   // product / has been read; p_full: P is in place (and O rescaled); pv_done: the second product of a tile is over;
-  // drained: every product an issuing lane has issued is complete.
-  __shared__ __align__(8) uint64_t bars[3 * kLtStages + 2 * 2 + 4];
+  // drained: every product an issuing lane has issued is complete; q_full: the row's queries are in place.
+  __shared__ __align__(8) uint64_t bars[3 * kLtStages + 2 * 2 + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_s;
   __shared__ int32_t ids_s[kLtStages][kLtKeys];
@@ -106,7 +107,8 @@ __global__ void __launch_bounds__(kLtThreads, 1)
   enum { kFull = 0, kEmpty = kLtStages, kEmptyB = 2 * kLtStages, kSFull = 3 * kLtStages, kSEmpty = 3 * kLtStages + 2 };
   auto bar = [&](int kind, int i) { return smem_u32(&bars[kind + i]); };
   const uint32_t p_full = smem_u32(&bars[3 * kLtStages + 4]), pv_done = smem_u32(&bars[3 * kLtStages + 5]),
-                 drained_s = smem_u32(&bars[3 * kLtStages + 6]), drained_o = smem_u32(&bars[3 * kLtStages + 7]);
+                 drained_s = smem_u32(&bars[3 * kLtStages + 6]), drained_o = smem_u32(&bars[3 * kLtStages + 7]),
+                 q_full = smem_u32(&bars[3 * kLtStages + 8]);
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kLtThreads, 1)
     mbar_init(pv_done, 1);
     mbar_init(drained_s, 1);
     mbar_init(drained_o, 1);
+    mbar_init(q_full, kLtQueryThreads);
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -200,24 +203,20 @@ __global__ void __launch_bounds__(kLtThreads, 1)
     // ------------------------------------------------------------------------------------------ staging the rows
     const int ptid = tid - 5 * 32;
     auto gather_sync = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    // (the first entries of the list are asked for before the queries, which they do not depend on: a decode step's
-    // CTA lives for a few tiles and cannot afford one wait on memory after another)
-    int32_t head_a = -1, head_b = -1;
-    if (warp == 5) {
-      head_a = lane < n ? list[lane] : -1;
-      head_b = 32 + lane < n ? list[32 + lane] : -1;
+    // The row's query heads, by the last three warps: the first one starts on the list, and its first boxes are on their way
+    // beside them (a decode step's CTA lives for a few tiles and cannot afford one wait on memory after another).
+    if (warp > 5) {
+      for (int e = ptid - 32; e < kLatHeads * kLtChunks; e += kLtQueryThreads) {
+        const int qr = e / kLtChunks, c = e - qr * kLtChunks;
+        const bool ok = head0 + qr < p.Hq;
+        const uint16_t *src = ok ? p.q + r * p.q_row_stride + (int64_t)(head0 + qr) * p.q_head_stride + c * 8 : p.q;
+        cp_async_16(base + (c >> 3) * kLtPlane + qr * 128 + (((c & 7) ^ (qr & 7)) << 4), src, ok ? 16 : 0);
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      lt_proxy_fence();
+      lt_arrive(q_full);
     }
-    // the row's query heads
-    for (int e = ptid; e < kLatHeads * kLtChunks; e += 128) {
-      const int qr = e / kLtChunks, c = e - qr * kLtChunks;
-      const bool ok = head0 + qr < p.Hq;
-      const uint16_t *src = ok ? p.q + r * p.q_row_stride + (int64_t)(head0 + qr) * p.q_head_stride + c * 8 : p.q;
-      cp_async_16(base + (c >> 3) * kLtPlane + qr * 128 + (((c & 7) ^ (qr & 7)) << 4), src, ok ? 16 : 0);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    lt_proxy_fence();
-    gather_sync();  // the queries are in place before any tile is announced
     // The rows of a tile that is not one box, a quarter of the copies a warp.
     auto gather_rows = [&](int stage) {
       const uint32_t dst0 = base + kLtKOff + stage * kLtStage;
@@ -243,7 +242,7 @@ __global__ void __launch_bounds__(kLtThreads, 1)
         return dealt ? (int32_t)(id / deal_span * p.deal_granule + id % p.deal_granule) : id;
       };
       int x = 0, j = 0;
-      int32_t id_a = head_a, id_b = head_b;
+      int32_t id_a = lane < n ? list[lane] : -1, id_b = 32 + lane < n ? list[32 + lane] : -1;
       bool alive = true;
       while ((x < n || dealt) && alive) {
         const int stage = j & 1;
@@ -333,7 +332,7 @@ __global__ void __launch_bounds__(kLtThreads, 1)
     // (the whole warp walks the tiles and one lane of it issues: descriptors stay in uniform registers)
     const uint32_t s_col = __shfl_sync(0xffffffffu, tmem_base, 0) + kLtSCol;
     const uint64_t q_desc = smem_desc_sw128(base), k_desc = smem_desc_sw128(base + kLtKOff);
-    bool alive = true;
+    bool alive = wait(q_full, 0);
     for (int i = 0; alive; ++i) {
       const int sb = i & 1;
       alive = wait(bar(kFull, sb), (i >> 1) & 1);

@@ -19,6 +19,16 @@ from lsa_b200 import ops, probe
 from lsa_b200.layer import FlatDesign, FlatIndex, FlatLayer
 
 
+def wave_splits(items: int, keys: int, sms: int) -> int:
+    """CTAs that each of `items` alike lists of some `keys` keys is split over. A CTA takes an SM, so they run in waves; where the
+    last wave leaves SMs idle, pieces of a list fill it: as few as come within three hundredths of the least time for up to eight,
+    a piece costing what its partial output's trip does (a two-hundredth of a list; none is cut shorter than 1,024 keys, whose CTA
+    lasts four times as long as it takes to start and end)."""
+    most = max(1, min(8, keys // 1024))
+    times = [-(-items * s // sms) / s * (1.0 + 0.005 * (s - 1)) for s in range(1, most + 1)]
+    return next(s for s, time in enumerate(times, 1) if time <= 1.03 * min(times))
+
+
 class LatentLayer(FlatLayer):
     """Index build, prefill rows and decode steps over a latent cache [T, latent_dim] bf16; absorbed queries are
     [rows, heads, latent_dim] bf16 and outputs [rows, heads, value_dim]."""
@@ -119,6 +129,10 @@ class LatentLayer(FlatLayer):
                      out: torch.Tensor, warp_mma: bool = False) -> torch.Tensor:
         """The read of consecutive query rows [n, heads, latent_dim] at positions start.. over a cache whose index
         is built, into `out` [n, heads, value_dim] bf16."""
+        return self._read_rows(rows, start, latent, index, out, 1 if warp_mma else self._prefill_splits(rows, start), warp_mma)
+
+    def _read_rows(self, rows: torch.Tensor, start: int, latent: torch.Tensor, index: FlatIndex, out: torch.Tensor, splits: int,
+                   warp_mma: bool = False) -> torch.Tensor:
         n, dev = rows.shape[0], rows.device
         positions = torch.arange(start, start + n, device=dev)
         with probe.region("index map"):
@@ -126,9 +140,22 @@ class LatentLayer(FlatLayer):
                                                                     torch.float32, dev))
         lists, lengths = self._select(index_queries, positions, index, self._room, True, start + n - 1)
         with probe.region("attend"):
-            ops.latent_attend(rows, latent, lists, lengths, self.scale, value_dim=self.value_dim, out=out,
-                              warp_mma=warp_mma, status=self._attend_status)
+            workspace = None
+            if splits > 1:
+                try:  # (the allocator's again after the call: 131 KB a row of 64 heads and split)
+                    workspace = torch.empty(ops.query("lsa_latent_attend_workspace_bytes", n, self.heads, self.value_dim, splits),
+                                            device=dev, dtype=torch.uint8)
+                except torch.OutOfMemoryError:
+                    splits = 1
+            ops.latent_attend(rows, latent, lists, lengths, self.scale, value_dim=self.value_dim, splits=splits, out=out,
+                              workspace=workspace, warp_mma=warp_mma, status=self._attend_status)
         return out
+
+    def _prefill_splits(self, rows: torch.Tensor, start: int) -> int:
+        """CTAs that the list of a row of a chunk [n, heads, latent_dim] from position `start` on is split over."""
+        d, n = self.design, rows.shape[0]
+        keys = min(start + n, d.top_p * d.bucket_size + d.window_size + d.sink_size, d.list_width)
+        return wave_splits(n * -(-self.heads // 64), keys, torch.cuda.get_device_properties(rows.device).multi_processor_count)
 
     def prefill_from_host(self, q_host: torch.Tensor, rows_host: torch.Tensor, start: int, latent: torch.Tensor,
                           index: FlatIndex, out_host: torch.Tensor, pieces: int = 4) -> torch.Tensor:
@@ -159,9 +186,10 @@ class LatentLayer(FlatLayer):
                 arrived[i].record(self._copy_in)
         main.wait_event(rows_in)
         self.extend_index(latent, start, n)
+        splits = self._prefill_splits(q, start)  # (the chunk's, whatever it is cut into: a row's bits do not depend on that)
         for i, (first, stop) in enumerate(spans):
             main.wait_event(arrived[i])
-            self.prefill_rows(q[first:stop], start + first, latent, index, out[first:stop])
+            self._read_rows(q[first:stop], start + first, latent, index, out[first:stop], splits)
             done[i].record(main)
             with torch.cuda.stream(self._copy_out):
                 self._copy_out.wait_event(done[i])

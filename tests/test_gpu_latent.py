@@ -366,3 +366,48 @@ def test_latent_layer_end_to_end(oracle):
                                    lengths=want_lens)
     gap = np.abs(out.cpu().numpy() - want[:, :, :512])
     assert gap.max() <= 2e-2 and gap.mean() <= 2e-3, (gap.max(), gap.mean())
+
+
+@pytest.mark.parametrize("items,keys,sms,splits", [(148, 40000, 148, 1), (149, 40000, 148, 6), (48, 40000, 148, 3), (777, 40000, 148, 3),
+                                                   (8192, 40000, 148, 1), (48, 1500, 148, 1), (1, 40000, 148, 8), (200, 3000, 148, 2)])
+def test_pieces_of_a_chunk_s_lists_fill_its_last_wave(items, keys, sms, splits):
+    from lsa_b200.latent import wave_splits
+
+    assert wave_splits(items, keys, sms) == splits
+
+
+def test_a_chunk_read_in_pieces_of_its_lists_is_the_chunk(monkeypatch):
+    """Rows split where the last wave leaves SMs idle, against the same rows whole: the sums of up to eight pieces in fp32, rounded to
+    bf16 once (2^-9 of a value); and without the memory for the pieces."""
+    from lsa_b200 import latent as module
+    from lsa_b200 import workloads as W
+
+    cfg = W.cut(W.C4, 1 << 16)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    layer = module.LatentLayer(W.design_of(cfg), *W.latent_maps(cfg, gen), cfg["heads"], cfg["latent_dim"], cfg["value_dim"],
+                               W.latent_scale(cfg))
+    cache, _ = W.latent_cache(cfg, gen)
+    index = layer.build_index(cache)
+    n, first = 60, (1 << 16) - 60
+    q = W.latent_queries(cfg, cache[first:], gen)
+    out = [torch.empty(n, cfg["heads"], cfg["value_dim"], device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    layer.prefill_rows(q, first, cache, index, out[0])
+    real, taken = torch.empty, []
+
+    def none(*size, **kind):
+        if kind.get("dtype") == torch.uint8 and size[0] > 1 << 20:
+            taken.append(size[0])
+            raise torch.OutOfMemoryError("no memory")
+        return real(*size, **kind)
+
+    with monkeypatch.context() as patch:
+        patch.setattr(module.torch, "empty", none)
+        layer.prefill_rows(q, first, cache, index, out[1])
+    assert taken
+    monkeypatch.setattr(module, "wave_splits", lambda *_: 1)
+    layer.prefill_rows(q, first, cache, index, out[2])
+    layer.check()
+    assert torch.equal(out[1], out[2]) and not torch.equal(out[0], out[2])
+    scale = out[2].float().abs().max()
+    assert (out[0].float() - out[2].float()).abs().max() <= 2 ** -8 * scale
+    assert (out[0].float() - out[2].float()).norm() <= 4e-3 * out[2].float().norm()
