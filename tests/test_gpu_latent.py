@@ -378,7 +378,7 @@ def test_pieces_of_a_chunk_s_lists_fill_its_last_wave(items, keys, sms, splits):
 
 def test_a_chunk_read_in_pieces_of_its_lists_is_the_chunk(monkeypatch):
     """Rows split where the last wave leaves SMs idle, against the same rows whole: the sums of up to eight pieces in fp32, rounded to
-    bf16 once (2^-9 of a value); and without the memory for the pieces."""
+    bf16 once, so that the two lie a bf16 step apart at most, 2^-7 of a value; and without the memory for the pieces."""
     from lsa_b200 import latent as module
     from lsa_b200 import workloads as W
 
@@ -409,5 +409,5 @@ def test_a_chunk_read_in_pieces_of_its_lists_is_the_chunk(monkeypatch):
     layer.check()
     assert torch.equal(out[1], out[2]) and not torch.equal(out[0], out[2])
     scale = out[2].float().abs().max()
-    assert (out[0].float() - out[2].float()).abs().max() <= 2 ** -8 * scale
+    assert (out[0].float() - out[2].float()).abs().max() <= 2 ** -7 * scale
     assert (out[0].float() - out[2].float()).norm() <= 4e-3 * out[2].float().norm()
