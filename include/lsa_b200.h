@@ -158,6 +158,12 @@ int lsa_gather_sum(const void *src, int src_dtype, const void *index, int index_
                    int d, int64_t index_base, float *out, void *stream);
 
 /* ---------------------------------------------------------------------------------------------------------
+ * Whether rows [n, d] (f32 or bf16, side by side) are unit vectors (src/lsa/core/reference.py:42-60): out[0] = 1 where every
+ * element is finite, else 0; out[1] the greatest | |row| - 1 |.
+ * --------------------------------------------------------------------------------------------------------- */
+int lsa_unit_rows(const void *rows, int dtype, int64_t n, int d, float *out, void *stream);
+
+/* ---------------------------------------------------------------------------------------------------------
  * The buckets every row sees: visible[r] = min(positions[r] / block * per_block, limit), those of the cluster blocks
  * closed before its own (src/lsa/core/reference.py:228-232). positions [R] int64, visible [R] int32 out.
  * --------------------------------------------------------------------------------------------------------- */

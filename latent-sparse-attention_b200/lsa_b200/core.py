@@ -254,12 +254,15 @@ def check_unit_rows(name: str, vectors: torch.Tensor) -> None:
         raise ValueError(f"{name} must be float32 or bfloat16 - got {vectors.dtype}")
     if not vectors.numel():
         return
-    norms = vectors.float().norm(dim=1)
-    finite, off = torch.stack([vectors.isfinite().all().float(), (norms - 1).abs().max().nan_to_num(0.0)]).tolist()
+    if vectors.is_cuda and vectors.is_contiguous():
+        finite, off = ops.unit_rows(vectors).tolist()
+    else:
+        norms = vectors.float().norm(dim=1)
+        finite, off = torch.stack([vectors.isfinite().all().float(), (norms - 1).abs().max().nan_to_num(0.0)]).tolist()
     if not finite:
         raise ValueError(f"{name} holds a non-finite value")
     if off > NORM_TOLERANCE[vectors.dtype]:
-        raise ValueError(f"{name} must be unit rows - a row is {off:.3g} off unit length")
+        raise ValueError(f"{name} must be unit rows - a row is {min(off, torch.finfo(torch.float32).max):.3g} off unit length")
 
 
 def check_sizes(pool_size: int, bucket_size: int, bucket_cap: int, cluster_block_size: int) -> None:

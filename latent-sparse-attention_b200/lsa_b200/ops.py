@@ -241,6 +241,14 @@ def kmeans(pools: torch.Tensor, init_centroids: torch.Tensor, iters: int):
     return centroids, assign
 
 
+def unit_rows(vectors: torch.Tensor) -> torch.Tensor:
+    """[2] fp32: 1 where every element of `vectors` [n, d] (fp32 or bf16, contiguous) is finite, else 0; and the greatest distance of
+    a row's length from one (src/lsa/core/reference.py:42-60)."""
+    out = torch.empty(2, device=vectors.device, dtype=torch.float32)
+    call("lsa_unit_rows", ptr(vectors), _lib.dtype_code(vectors), vectors.shape[0], vectors.shape[1], ptr(out), stream(), launches=2)
+    return out
+
+
 def visible_buckets(positions: torch.Tensor, block_size: int, block_buckets: int, limit: int) -> torch.Tensor:
     """The buckets each of `positions` [R] sees [R] int32: those of the cluster blocks closed before its own, `limit` at
     most (src/lsa/core/reference.py:228-232)."""

@@ -862,3 +862,31 @@ def test_host_threads_that_launch_a_kernel_with_different_sizes(ops, kernel, mon
         thread.join()
     assert len(entries) == 2 and not wrong, (len(entries), wrong[:3])
     assert all(torch.equal(out, same) for out, same in zip(outs, want))
+
+
+@pytest.mark.parametrize("n,d", [(1, 1), (5, 64), (70001, 64), (3000, 20), (17, 200), (4, 30)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_unit_rows_in_one_pass_are_the_check_s(ops, n, d, dtype):
+    """The greatest distance from unit length against 64 bits (fp32 sums of up to 200 squares: 2e-6), what is not finite, and the
+    check's errors from either form."""
+    from lsa_b200 import core
+
+    gen = torch.Generator(device="cuda").manual_seed(n + d)
+    rows = torch.nn.functional.normalize(torch.randn(n, d, device="cuda", generator=gen), dim=-1).to(dtype)
+    rows[n // 2] *= 0.75
+    finite, off = ops.unit_rows(rows).tolist()
+    assert finite == 1.0 and abs(off - float((rows.double().norm(dim=1) - 1).abs().max())) <= 2e-6
+    apart = torch.empty(n, d + 1, device="cuda", dtype=dtype)[:, 1:].copy_(rows)
+    for x in (rows, apart):
+        with pytest.raises(ValueError, match="unit rows - a row is 0.2"):
+            core.check_unit_rows("rows", x)
+        for bad in (float("nan"), float("inf"), -float("inf")):
+            worse = x.clone()
+            worse[n - 1, d - 1] = bad
+            with pytest.raises(ValueError, match="non-finite"):
+                core.check_unit_rows("rows", worse)
+    core.check_unit_rows("rows", torch.nn.functional.normalize(rows.float(), dim=-1))
+    with pytest.raises(ValueError, match="unit rows"):
+        core.check_unit_rows("rows", torch.full((2, 8), 1e30, device="cuda"))
+    unaligned = torch.empty(n * d + 1, device="cuda", dtype=dtype)[1:].view(n, d).copy_(rows)
+    assert torch.equal(ops.unit_rows(unaligned)[0], torch.ones((), device="cuda")) and abs(float(ops.unit_rows(unaligned)[1]) - off) <= 2e-6
