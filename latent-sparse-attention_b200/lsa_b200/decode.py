@@ -61,8 +61,10 @@ class TreeDecoder:
             picked, _ = ops.beam_step(index_query, self.buckets.bucket_centroids, carried, first, end, d.top_p,
                                       splits=self.select_splits)
         with probe.region("expand"):
+            outs = (torch.empty(1, d.list_width, device=q.device, dtype=torch.int32),
+                    torch.empty(1, device=q.device, dtype=torch.int32), self.layer._expand_status)
             lists, lengths, _ = ops.expand(picked, plan["positions"], self.buckets.bucket_members, d.top_k, d.sink_size,
-                                           d.window_size)
+                                           d.window_size, outs=outs)
         return lists, lengths
 
     def step(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:

@@ -190,11 +190,9 @@ class FlatLayer:
                              dh_used=self.dh_used, out=out)
 
     def index_queries_rows(self, q: torch.Tensor) -> torch.Tensor:
-        """The same map for the few rows of a decode step, q [R <= 8, Hq, dh] bf16: a kernel that spreads one row's
-        contraction over many CTAs (with bf16 maps; other maps take `index_queries`)."""
-        if self.tensor_cores and q.shape[0] <= 8 and q.dtype == torch.bfloat16 and q.stride(2) == 1 \
-                and q.stride(1) == q.shape[2]:
-            return ops.rows_linear(q, self.query_map_t, normalize=True)
+        """The same map for the few rows of a decode step, q [R <= 8, Hq, dh] bf16: `index_queries`, whose kernel for few rows sums a
+        KV head's group before it multiplies (one row of 40 heads over 8: 5.0 us and one launch, where a map of all 40 heads'
+        dims, a fifth of them read as often, took 5.7 and 1.9 for the unit length)."""
         return self.index_queries(q)
 
     def index_keys(self, k: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
