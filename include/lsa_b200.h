@@ -164,6 +164,17 @@ int lsa_gather_sum(const void *src, int src_dtype, const void *index, int index_
 int lsa_unit_rows(const void *rows, int dtype, int64_t n, int d, float *out, void *stream);
 
 /* ---------------------------------------------------------------------------------------------------------
+ * Rows first .. first + n - 1 of a paged table (logical row i lies at row i % page_rows of page pages[i / page_rows]), up to three
+ * tables of 32-bit words beside one another: into the pages from dense [n, words], or out of them (into_pages 0; a row of a page
+ * that is not held, -1, reads as zeros and is not written). The bucket cache's tables
+ * (src/lsa/sglang/index/bucket_cache.py:484-601).
+ *   pages [max_pages] int32; table [rows, words], dense [n, words]; words 0: no such table
+ * --------------------------------------------------------------------------------------------------------- */
+int lsa_paged_rows(const int32_t *pages, int max_pages, int page_rows, int64_t first, int64_t n, int64_t rows, void *table0,
+                   void *dense0, int words0, void *table1, void *dense1, int words1, void *table2, void *dense2, int words2,
+                   int into_pages, void *stream);
+
+/* ---------------------------------------------------------------------------------------------------------
  * The buckets every row sees: visible[r] = min(positions[r] / block * per_block, limit), those of the cluster blocks
  * closed before its own (src/lsa/core/reference.py:228-232). positions [R] int64, visible [R] int32 out.
  * --------------------------------------------------------------------------------------------------------- */

@@ -13,7 +13,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblsa_b200.so")
-ABI_VERSION = 25
+ABI_VERSION = 26
 
 DTYPE_F32, DTYPE_BF16 = 0, 1
 PAD = -1
@@ -36,6 +36,7 @@ SIGNATURES = {
     "lsa_bucket_table": (_I, [_P, _I, _P, _L, _I, _I, _I, _I, _I, _L, _P, _P, _P, _P, _P, _P, _P]),
     "lsa_kmeans_update": (_I, [_P, _P, _P, _I, _I, _P, _P]),
     "lsa_gather_sum": (_I, [_P, _I, _P, _I, _L, _I, _I, _L, _P, _P]),
+    "lsa_paged_rows": (_I, [_P, _I, _I, _L, _L, _L, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _P]),
     "lsa_unit_rows": (_I, [_P, _I, _L, _I, _P, _P]),
     "lsa_visible_buckets": (_I, [_P, _L, _L, _L, _L, _P, _P]),
     "lsa_flat_select": (_I, [_P, _L, _I, _P, _L, _P, _P, _I, c_int32, _P, _P, _P]),

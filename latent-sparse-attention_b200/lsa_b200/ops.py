@@ -249,6 +249,21 @@ def unit_rows(vectors: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def paged_rows(pages: torch.Tensor, page_rows: int, first: int, tables: list, into_pages: bool) -> None:
+    """Rows first.. of up to three paged tables, [(table [rows, ...], dense [n, ...]), ...] of 32-bit elements, through a request's
+    `pages` [P] int32: dense into the pages, or out of them (src/lsa/sglang/index/bucket_cache.py:484-601)."""
+    (table, dense), n = tables[0], tables[0][1].shape[0]
+    flat = []
+    for held, side in tables:
+        if held.element_size() != 4 or side.dtype != held.dtype or held.shape[0] != table.shape[0] or side.shape != (n, *held.shape[1:]) \
+                or not held.is_contiguous() or not side.is_contiguous():
+            raise ValueError("paged tables and their dense sides hold 32-bit elements, contiguous, with rows alike")
+        flat += [ptr(held), ptr(side), held[0].numel() if held.shape[0] else 1]
+    flat += [None, None, 0] * (3 - len(tables))
+    call("lsa_paged_rows", ptr(_as(pages, torch.int32)), pages.shape[0], page_rows, first, n, table.shape[0], *flat, int(into_pages),
+         stream())
+
+
 def visible_buckets(positions: torch.Tensor, block_size: int, block_buckets: int, limit: int) -> torch.Tensor:
     """The buckets each of `positions` [R] sees [R] int32: those of the cluster blocks closed before its own, `limit` at
     most (src/lsa/core/reference.py:228-232)."""

@@ -127,7 +127,7 @@ class BucketCache:
         self.pending.pop(request, None)
         self.owner.pop(request, None)
         self.request_pages[request].fill_(-1)
-        self.bucket_counts[request] = 0
+        self.bucket_counts[request].fill_(0)
 
     def ensure(self, request: int, rid: object) -> None:
         """Start a row of the request table afresh when another request has taken it (bucket_cache.py:228-262)."""
@@ -197,7 +197,7 @@ class BucketCache:
         self.prints[request] = prints[:count]
         self.request_pages[request, :count] = torch.tensor(pages, dtype=torch.int32, device=self.request_pages.device)
         self.closed_keys[request] = count * page_keys
-        self.bucket_counts[request] = count * self.page_buckets
+        self.bucket_counts[request].fill_(count * self.page_buckets)
         return count
 
     def fingerprint(self, request: int, end: int, lookup) -> None:
@@ -237,8 +237,14 @@ class BucketCache:
     def gather(self, request: int, buckets: int) -> torch.Tensor:
         """The centroids of a request's first `buckets` buckets, side by side [buckets, index_dim] fp32
         (bucket_cache.py:560-601)."""
-        logical = torch.arange(buckets, device=self.centroids.device)
-        return self.centroids[self.rows_of(request, logical)]
+        return self._gathered(self.centroids, request, buckets)
+
+    def _gathered(self, table: torch.Tensor, request: int, buckets: int) -> torch.Tensor:
+        if not table.is_cuda:
+            return table[self.rows_of(request, torch.arange(buckets, device=table.device))]
+        out = torch.empty(buckets, table.shape[1], device=table.device, dtype=table.dtype)
+        ops.paged_rows(self.request_pages[request], self.page_buckets, 0, [(table, out)], into_pages=False)
+        return out
 
     def gather_shapes(self, request: int, buckets: int) -> ops.ShapeTable | None:
         """The shapes of the buckets `gather` returns, row for row, or None when buckets are not shaped
@@ -262,9 +268,16 @@ class BucketCache:
             self.holders[fresh[-1]] = 1
             pages.append(fresh[-1])
         if fresh:
-            first = len(pages) - len(fresh)
-            self.request_pages[request, first:len(pages)] = torch.tensor(fresh, dtype=torch.int32,
-                                                                         device=self.request_pages.device)
+            # (by runs of a kernel's own making: a copy from the host's list would wait for the GPU to come this far. Free pages
+            # are handed out in order as a rule, which is one run)
+            at, row = len(pages) - len(fresh), self.request_pages[request]
+            while fresh:
+                step = fresh[1] - fresh[0] if len(fresh) > 1 else 1
+                run = 1
+                while run < len(fresh) and fresh[run] == fresh[0] + run * step:
+                    run += 1
+                torch.arange(fresh[0], fresh[0] + run * step, step, dtype=row.dtype, device=row.device, out=row[at:at + run])
+                at, fresh = at + run, fresh[run:]
 
     def append(self, request: int, index_keys: torch.Tensor) -> int:
         """Take a request's next index keys [n, index_dim] (fp32 unit rows, in position order); cluster every
@@ -287,18 +300,17 @@ class BucketCache:
             labels, _ = ops.ward_rounds(pools, float(d.pool_size), per_block, d.bucket_cap)
             members, sizes, _, centroids, _, _ = ops.bucket_table(block_keys, labels, d.pool_size, per_block,
                                                                   d.bucket_cap, first_position=first_position)
-        rows = self.rows_of(request, first_bucket + torch.arange(blocks * per_block, device=members.device))
-        self.centroids[rows] = centroids
-        self.members[rows] = members
-        self.sizes[rows] = sizes
+        ops.paged_rows(self.request_pages[request], self.page_buckets, first_bucket,
+                       [(self.centroids, centroids), (self.members, members), (self.sizes, sizes)], into_pages=True)
         if self.bucket_shapes is not None:  # (bucket_cache.py:603-627; members are positions from `first_position`)
+            rows = self.rows_of(request, first_bucket + torch.arange(blocks * per_block, device=members.device))
             with probe.region("bucket shapes"):
                 built = ops.shape_build(block_keys, centroids, members, d.bucket_shape.rank, key_base=first_position)
             self.bucket_shapes.basis[rows] = built.basis
             self.bucket_shapes.variances[rows] = built.variances
             self.bucket_shapes.floor[rows] = built.floor
         self.closed_keys[request] = first_position + closed
-        self.bucket_counts[request] = first_bucket + blocks * per_block
+        self.bucket_counts[request].fill_(first_bucket + blocks * per_block)  # (an assignment would copy from the host, and wait)
         return blocks
 
 
@@ -359,7 +371,7 @@ class Selector:
         last = query_start + S - 1
         seen = min(last // d.cluster_block_size * d.block_bucket_count, cache.buckets_of(row))
         positions = positions.to(torch.int64)
-        visible = (positions // d.cluster_block_size * d.block_bucket_count).clamp_max(seen).to(torch.int32)
+        visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, seen)
         with probe.region("index q scan"):
             centroids = cache.gather(row, seen)
             if cache.bucket_shapes is not None:

@@ -133,3 +133,48 @@ def test_a_decode_graph_captured_for_a_context_range_reads_the_same_lists(oracle
     label["now"] = f"context_{4 * page_keys}"
     cut = selector.decode(cuda(queries), cuda(positions), rows)
     assert torch.equal(cut[:2], want[:2]) and not torch.equal(cut[2], want[2])
+
+
+def test_rows_of_a_paged_table_go_in_and_out_as_index_arithmetic_has_them():
+    """One to three tables of 32-bit words, runs that start and end inside a page, pages that are not held, pages handed out in and out
+    of order; and sides that do not fit."""
+    from lsa_b200 import ops
+    from lsa_b200.layer import FlatDesign
+    from lsa_b200.serving import BucketCache
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *shape: torch.randint(-9, 9, shape, device="cuda", generator=gen, dtype=torch.int32)
+    page_rows, pages = 6, torch.tensor([4, 0, -1, 7, 2], device="cuda", dtype=torch.int32)
+    tables = [rnd(48, 5), rnd(48), rnd(48, 3).float()]
+    for first, n in ((0, 1), (3, 7), (5, 25), (0, 30), (29, 1), (7, 0)):
+        logical = torch.arange(first, first + n, device="cuda")
+        rows = pages[logical // page_rows].long() * page_rows + logical % page_rows
+        held = pages[logical // page_rows] >= 0
+        for some in (tables[:1], tables[:2], tables):
+            outs = [torch.full((n, *t.shape[1:]), 77, device="cuda", dtype=t.dtype) for t in some]
+            ops.paged_rows(pages, page_rows, first, list(zip(some, outs)), into_pages=False)
+            for table, out in zip(some, outs):
+                want = table[rows.clamp_min(0)]
+                want[~held] = 0
+                assert torch.equal(out, want)
+            into, fresh = [t.clone() for t in some], [rnd(n, *t.shape[1:]).to(t.dtype) for t in some]
+            ops.paged_rows(pages, page_rows, first, list(zip(into, fresh)), into_pages=True)
+            for table, new, before in zip(into, fresh, some):
+                want = before.clone()
+                want[rows[held]] = new[held]
+                assert torch.equal(table, want)
+    with pytest.raises(ValueError, match="32-bit"):
+        ops.paged_rows(pages, page_rows, 0, [(tables[0], rnd(4, 6))], into_pages=True)
+    with pytest.raises(ValueError, match="32-bit"):
+        ops.paged_rows(pages, page_rows, 0, [(tables[0].long(), rnd(4, 5).long())], into_pages=False)
+    design = FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, top_p=4, top_k=32, sink_size=1, window_size=32, cluster_block_size=64)
+    cache = BucketCache(design, 32, pages=12, page_buckets=8, max_requests=3, max_request_pages=9)
+    cache.free_pages = [3, 11, 10, 9, 1, 4, 6, 8, 0]  # (handed out from the end: 0, a run of twos down, 1, runs up)
+    cache._grow(1, 8 * 8)
+    assert cache.request_pages[1].tolist() == cache.held[1] + [-1] and cache.held[1] == [0, 8, 6, 4, 1, 9, 10, 11]
+    cache._grow(1, 8 * 9)
+    assert cache.request_pages[1].tolist() == cache.held[1] and (cache.request_pages[[0, 2]] == -1).all()
+    cache.members.copy_(torch.randint(0, 99, cache.members.shape, device="cuda", generator=gen))
+    cache.centroids.normal_(generator=gen)
+    rows = cache.rows_of(1, torch.arange(50, device="cuda"))
+    assert torch.equal(cache.gather(1, 50), cache.centroids[rows])
