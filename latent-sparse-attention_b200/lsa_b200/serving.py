@@ -239,6 +239,10 @@ class BucketCache:
         (bucket_cache.py:560-601)."""
         return self._gathered(self.centroids, request, buckets)
 
+    def gather_members(self, request: int, buckets: int) -> torch.Tensor:
+        """Their members, side by side [buckets, bucket_cap] int32, -1 padded."""
+        return self._gathered(self.members, request, buckets)
+
     def _gathered(self, table: torch.Tensor, request: int, buckets: int) -> torch.Tensor:
         if not table.is_cuda:
             return table[self.rows_of(request, torch.arange(buckets, device=table.device))]
@@ -340,7 +344,7 @@ class Selector:
         return closed
 
     def prefill(self, row: int, index_queries: torch.Tensor, positions: torch.Tensor, index_keys: torch.Tensor,
-                query_start: int, local: bool = True) -> torch.Tensor:
+                query_start: int, local: bool = True, mask: torch.Tensor | None = None) -> torch.Tensor:
         """Read a prefill segment of one request: append its keys, select for its queries (selector.py:199-287).
 
         The keys go into the cache in one call and every query reads the buckets its own position sees - those of
@@ -354,6 +358,8 @@ class Selector:
             index_keys: The index keys the cache appends [S', index_dim] fp32, from the cache's end (S' >= S where
                 the segment's keys reach back before its first query).
             query_start: Position of the first query, from the scheduler: no device read.
+            mask: [key tiles, n, 4] int32 - the lists of the first n queries are written there as one bit a key
+                (`ops.list_bits`), and the others' returned.
 
         Returns:
             KV slots [S, width] int32, -1 padded, valid entries first.
@@ -384,6 +390,13 @@ class Selector:
             else:
                 _, picked = ops.flat_select(index_queries, centroids, visible, d.top_p)
         with probe.region("expand"):
+            if mask is not None:
+                n = mask.shape[1]
+                ops.list_bits(picked[:n], positions[:n], cache.gather_members(row, seen), d.top_k, d.sink_size, d.window_size,
+                              cache.end(row), mask.shape[0], out=mask)
+                picked, positions = picked[n:], positions[n:]
+                if n == S:
+                    return torch.empty(0, d.list_width, device=dev, dtype=torch.int32)
             table = self.slot_table()
             lists, _, _ = ops.expand_batched(picked, positions, None, cache.members, cache.request_pages[row:row + 1],
                                              cache.page_buckets, table[row:row + 1], self.kv_page_size, d.top_k,

@@ -208,17 +208,18 @@ class GroupedQueryIndexer:
         """Of each request of a prefill batch, the leading rows that read every key whatever is selected."""
         return self.ready().whole_rows(forward_batch.extend_seq_lens_cpu, forward_batch.extend_prefix_lens_cpu)
 
-    def select(self, q: torch.Tensor, k: torch.Tensor, forward_batch: Any, skip: list | None = None) -> torch.Tensor:
+    def select(self, q: torch.Tensor, k: torch.Tensor, forward_batch: Any, skip: list | None = None,
+               masks: list | None = None) -> torch.Tensor:
         """Select for every query of a forward, from the heads attention was handed: q [T, Hq * dh] or [T, Hq, dh]
         rotated on the prefix alone, k [T, Hkv, dh] the same, already in the pool at `out_cache_loc`. Returns KV
         slots [T, width] int32, -1 padded, valid entries first; with `skip` of the rows past each request's leading
-        ones alone."""
+        ones alone, and with `masks` of the rows past those whose lists a request's mask takes."""
         index = self.ready()
         inputs = index_space.key_and_query(q, k, self.geometry, self.heads)
         positions, slots = forward_batch.positions, forward_batch.out_cache_loc.long()
         if forward_batch.forward_mode.is_extend():
             return index.extend(inputs, positions, slots, forward_batch.lsa_rows, forward_batch.extend_seq_lens_cpu,
-                                forward_batch.extend_prefix_lens_cpu, skip)
+                                forward_batch.extend_prefix_lens_cpu, skip, masks)
         return index.decode(inputs, positions, slots, forward_batch.req_pool_indices.long())
 
 
@@ -321,19 +322,28 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
             or heads // kv_heads > 16 or not layer.scaling > 0 or keys.shape[2] != head_dim or values.shape[1:] != keys.shape[1:] \
             or k[0].numel() != v[0].numel() or k[0].numel() != kv_heads * head_dim or sum(lengths) != q.shape[0]:
         return None
-    tokens = q.shape[0]
-    lists = indexer.select(q, k, forward_batch, whole)
+    tokens, heads_of = q.shape[0], q
+    keys_of = k
     # (the dense read copies rows 16 bytes at a time out of the batch's own tensors, which may start anywhere in a larger one;
     # the lists' read takes keys and values from the pool)
     q, k, v = (x.contiguous() if x.data_ptr() % 16 == 0 or not x.is_contiguous() else x.clone() for x in (q, k, v))
     q, k, v = q.view(tokens, heads, head_dim), k.view(tokens, kv_heads, head_dim), v.view(tokens, kv_heads, head_dim)
     out = torch.empty(tokens, heads, head_dim, device=q.device, dtype=q.dtype)
-    rest, first, status = [], 0, indexer.read_status(q.device)
+    design = indexer.ready().selector.cache.design
+    masks, first = [], 0
     for count, dense in zip(lengths, whole, strict=True):
+        masks.append(_mask_of(q, k, v, out, first, count, dense, design))
+        first += count
+    lists = indexer.select(heads_of, keys_of, forward_batch, whole, masks)
+    rest, first, status = [], 0, indexer.read_status(q.device)
+    for count, dense, mask in zip(lengths, whole, masks, strict=True):
         if dense:
             piece = slice(first, first + dense)
             ops.causal_attend(q[piece], k[piece], v[piece], 0, layer.scaling, out=out[piece], status=status)
-        if dense < count:
+        if mask is not None:
+            piece, own = slice(first + dense, first + count), slice(first, first + count)
+            ops.listed_attend(q[piece], k[own], v[own], dense, mask, layer.scaling, out[piece], status)
+        elif dense < count:
             rest.append(slice(first + dense, first + count))
         first += count
     indexer.reads_done()
@@ -345,6 +355,27 @@ def whole_read(backend: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
             out[piece] = read[at:at + n]
             at += n
     return out.view(tokens, heads * head_dim)
+
+
+def _mask_of(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, first: int, count: int, dense: int,
+             design: Any) -> torch.Tensor | None:
+    """Memory for the lists of a prompt's rows past the `dense` ones as one bit a key, where those rows are read through them: a
+    prompt that starts in this batch, as long as the masked read takes it and is the faster. A CTA of it takes 256 rows of a head
+    through every key, 0.0216 us each; rows gathered one by one cost 58 ps a listed key and KV head, and 83 ps a key to list (400
+    rows at the end of 5,000 keys of 16 heads over 2: 109 us against 364)."""
+    n, heads, kv_heads = count - dense, q.shape[1], k.shape[1]
+    if not dense or n < 128 or count > 1600 * 128:
+        return None
+    rows, own = slice(first + dense, first + count), slice(first, first + count)
+    if not ops.dense_attend_supported(q[rows], k[own], v[own], out[rows]):
+        return None
+    waves = -(-(-(-n // 256) * heads) // 148)
+    if waves * count * 0.0216 >= n * design.list_width * (58e-6 * kv_heads + 83e-6):
+        return None
+    try:
+        return torch.empty(-(-count // 128), n, 4, device=q.device, dtype=torch.int32)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def select_and_read(original: Any, self: Any, *args: Any, **kwargs: Any) -> Any:

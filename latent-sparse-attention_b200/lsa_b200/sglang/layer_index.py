@@ -403,7 +403,7 @@ class LayerIndex:
                 for count, start, held in zip(lengths, starts, blocks, strict=True)]
 
     def extend(self, inputs: KeyAndQuery, positions: torch.Tensor, slots: torch.Tensor, rows: Sequence,
-               lengths: Sequence, starts: Sequence, skip: Sequence | None = None) -> torch.Tensor:
+               lengths: Sequence, starts: Sequence, skip: Sequence | None = None, masks: Sequence | None = None) -> torch.Tensor:
         """Write the keys of a prefill batch and select for its queries, request by request.
 
         Args:
@@ -413,22 +413,24 @@ class LayerIndex:
             rows: The requests' table rows; lengths: new tokens of each; starts: position of each request's first
                 new token, from the scheduler - no device read.
             skip: Leading rows of each request that need no list (`whole_rows`); their keys are indexed all the same.
+            masks: Of each request None, or [key tiles, n, 4] int32 that takes the lists of its next n rows as one bit a key.
 
         Returns:
-            KV slots [S, width] int32, -1 padded, valid entries first, of the rows not skipped.
+            KV slots [S, width] int32, -1 padded, valid entries first, of the rows neither skipped nor masked.
         """
         skip = [0] * len(lengths) if skip is None else skip
+        masks = [None] * len(lengths) if masks is None else masks
         index_queries, index_keys = self.project(inputs, slots)
         starts = [int(start) for start in starts]
         self.check_starts(positions, lengths, starts)
         lists, first = [], 0
-        for row, count, start, past in zip(rows, lengths, starts, skip, strict=True):
+        for row, count, start, past, mask in zip(rows, lengths, starts, skip, masks, strict=True):
             stop = first + count
             held = self.selector.cache.end(row)
             if held != start:  # (`maintain` brings a cached prefix's keys in before the forward)
                 raise ValueError(f"request {row}'s index holds {held} keys and its chunk starts at {start}")
             lists.append(self.selector.prefill(row, index_queries[first + past:stop], positions[first + past:stop],
-                                               index_keys[first:stop], start + past))
+                                               index_keys[first:stop], start + past, mask=mask))
             first = stop
         self.check(rows)
         return torch.cat(lists) if lists else torch.empty(0, self.settings.width, device=slots.device,

@@ -177,4 +177,4 @@ def test_rows_of_a_paged_table_go_in_and_out_as_index_arithmetic_has_them():
     cache.members.copy_(torch.randint(0, 99, cache.members.shape, device="cuda", generator=gen))
     cache.centroids.normal_(generator=gen)
     rows = cache.rows_of(1, torch.arange(50, device="cuda"))
-    assert torch.equal(cache.gather(1, 50), cache.centroids[rows])
+    assert torch.equal(cache.gather(1, 50), cache.centroids[rows]) and torch.equal(cache.gather_members(1, 50), cache.members[rows])

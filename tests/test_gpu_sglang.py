@@ -357,6 +357,9 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
                                                                  dtype=np.float32) / 14)).cuda().bfloat16() for _ in range(2))
     layer = types.SimpleNamespace(layer_id=0, tp_q_head_num=HQ, tp_k_head_num=HKV, head_dim=DH, scaling=DH ** -0.5)
 
+    masked, listed_attend = [], backend.ops.listed_attend  # rows read through masks
+    monkeypatch.setattr(backend.ops, "listed_attend", lambda q, *a: (masked.append(q.shape[0]), listed_attend(q, *a))[1])
+
     def served(dense: bool, save: bool = True):
         monkeypatch.setattr(backend, "ROWS", {})
         runner = types.SimpleNamespace(pool=Pool(slots_total), req_to_token=cuda(table))
@@ -366,6 +369,7 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
         if not dense:
             monkeypatch.setattr(indexer, "whole_rows", lambda batch: [0] * len(batch.rids))
         outs, taken = [], []
+        masked.clear()
         for first, stops in (([0, 0], [1200, 700]), ([1200], [1500])):  # a batch of prompts, then the first goes on
             some = range(len(stops))
             parts = [np.concatenate([data[i][x][a:b] for i, a, b in zip(some, first, stops)]) for x in range(3)]
@@ -383,8 +387,14 @@ def test_rows_that_read_everything_through_the_hooks_equal_their_lists(monkeypat
         return outs, taken
 
     dense, taken = served(True)
+    assert taken == [[512, 512], [0]] and masked == [688, 188], (taken, masked)
+    with monkeypatch.context() as patch:  # (and no memory for masks: the lists' read)
+        patch.setattr(backend, "_mask_of", lambda *a: None)
+        gathered, _ = served(True)
+        assert not masked
+    for one, other in zip(dense, gathered):
+        assert (one.float() - other.float()).abs().max() <= 2e-2 and (one.float() - other.float()).abs().mean() <= 1e-3
     lists, _ = served(False)
-    assert taken == [[512, 512], [0]], taken
     unsaved, _ = served(True, save=False)
     for got, want, plain in zip(dense, lists, unsaved):
         assert torch.equal(plain, want)
