@@ -11,7 +11,7 @@
 
 namespace lsa {
 
-constexpr int kBitsRows = 8;
+constexpr int kBitsRows = 8, kBitsQuads = 4;
 constexpr size_t kBitsShared = 200 * 1024;
 
 struct ListBitsParams {
@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
     const int64_t key_end = min(p.n_keys, (int64_t)p.tiles * 128);
     int counted = 0, bad = 0;
     const int in_step = 32 / p.lanes, first = lane % p.lanes * p.places, places = min(p.places, p.cap - first);
+    const bool sixteen = p.quads && p.places == 4 * kBitsQuads && p.cap % p.places == 0;  // (the same in every lane)
     int i0 = 0;
     for (; i0 < row_p && counted < row_k; i0 += in_step) {
       const int i = i0 + lane / p.lanes;
@@ -64,11 +65,24 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
             if (!see(row[j])) return;
         }
       };
+      // (a row of members ends in padding, whose ids are under every sink)
+      const uint32_t span = window_start > p.sink ? (uint32_t)(window_start - p.sink) : 0u;
+      auto counts = [&](int32_t id) { return (uint32_t)id - (uint32_t)p.sink < span && id >= 0; };
+      int4 held[kBitsQuads];  // sixteen places a lane, read once where they lie 16 bytes at a time
       int n = 0;
-      walk([&](int32_t id) {
-        n += id >= p.sink && id < window_start;
-        return id >= 0;  // (a row of members ends in padding)
-      });
+      if (sixteen) {
+        const int4 *row4 = reinterpret_cast<const int4 *>(row);
+#pragma unroll
+        for (int j = 0; j < kBitsQuads; ++j) held[j] = bucket >= 0 ? row4[j] : make_int4(-1, -1, -1, -1);
+#pragma unroll
+        for (int j = 0; j < kBitsQuads; ++j)
+          n += (counts(held[j].x) ? 1 : 0) + (counts(held[j].y) ? 1 : 0) + (counts(held[j].z) ? 1 : 0) + (counts(held[j].w) ? 1 : 0);
+      } else {
+        walk([&](int32_t id) {
+          n += counts(id);
+          return id >= 0;
+        });
+      }
       int incl = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -79,8 +93,8 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
       if (left > 0) {
         int at = 0;
         uint32_t bits = 0u;
-        walk([&](int32_t id) {
-          if (!(id >= p.sink && id < window_start)) return true;
+        auto add = [&](int32_t id) {
+          if (!counts(id)) return true;
           if (id < key_end) {
             if (id >> 5 != at) {
               if (bits) atomicOr(&words[at], bits);
@@ -89,7 +103,28 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
             bits |= 1u << (id & 31);
           }
           return --left > 0;
-        });
+        };
+        if (sixteen) {
+#pragma unroll
+          for (int j = 0; j < kBitsQuads; ++j) {
+            // (four keys that all count and are neighbours in a word, as a pool's are: one step)
+            const int4 v = held[j];
+            const bool run = left >= 4 && v.w == v.x + 3 && v.y == v.x + 1 && v.z == v.x + 2 && (v.x & 31) <= 28 && counts(v.x) &&
+                             counts(v.w) && v.w < key_end;
+            if (run) {
+              if (v.x >> 5 != at) {
+                if (bits) atomicOr(&words[at], bits);
+                at = v.x >> 5, bits = 0u;
+              }
+              bits |= 0xFu << (v.x & 31);
+              left -= 4;
+            } else if (left > 0) {
+              if (add(v.x) && add(v.y) && add(v.z)) add(v.w);
+            }
+          }
+        } else {
+          walk(add);
+        }
         if (bits) atomicOr(&words[at], bits);
       }
       counted += __shfl_sync(0xffffffffu, incl, 31);
