@@ -292,12 +292,15 @@ def flat_select(index_queries: torch.Tensor, centroids: torch.Tensor, visible: t
     return keys, picked
 
 
+BINNED_BUCKETS = 4096  # buckets that the search through a scratch matrix of scores takes, at most
+
+
 def _binned_scratch(q: torch.Tensor, c: torch.Tensor, top_p: int) -> torch.Tensor | None:
     """The scores' scratch of a search of many rows over few buckets, where that form takes the call, is the faster one and finds
     the memory. It is two launches a piece: 256 rows over 512 buckets, top 64, 26 us in one launch and 30 in two (a host's time),
     top 256 38 and 28; over 1,024 40 and 28; 8,192 rows over 256 buckets 57 and 45."""
     R, m = q.shape[0], c.shape[0]
-    if R < 128 or m > 4096 or top_p > 2048 or not (m >= 1024 or m * R >= 1 << 21 or m >= 512 and top_p > 128):
+    if R < 128 or m > BINNED_BUCKETS or top_p > 2048 or not (m >= 1024 or m * R >= 1 << 21 or m >= 512 and top_p > 128):
         return None  # (over 2,048 kept is refused in every form)
     if q.data_ptr() % 16 or c.data_ptr() % 16:
         return None

@@ -383,7 +383,7 @@ class Selector:
             if cache.bucket_shapes is not None:
                 _, picked = ops.shaped_select(index_queries, centroids, cache.gather_shapes(row, seen), visible,
                                               d.top_p)
-            elif S >= self.scan_rows and centroids.shape[1] == 64 and d.top_p <= 512:
+            elif S >= self.scan_rows and seen > ops.BINNED_BUCKETS and centroids.shape[1] == 64 and d.top_p <= 512:
                 operand, lengths, radius = ops.scan_centre(centroids, centroids.mean(0))
                 _, picked = ops.scan_select(index_queries, centroids, operand, visible, d.top_p, max_visible=seen,
                                             lengths=lengths, radius=radius)
