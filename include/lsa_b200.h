@@ -263,6 +263,12 @@ int lsa_flat_select_decode(const float *queries, int64_t R, int d, const float *
                            int64_t *keys_out, int32_t *picked_out, void *workspace, size_t workspace_bytes,
                            void *stream);
 
+/* lsa_visible_buckets and lsa_flat_select_decode in one (top_p up to 128, else LSA_ERR_UNSUPPORTED): row r sees the buckets of the
+ * cluster blocks closed before positions[r], m at most. */
+int lsa_flat_select_at(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
+                       int64_t block_buckets, int64_t m, int top_p, int splits, int64_t *keys_out, int32_t *picked_out,
+                       void *workspace, size_t workspace_bytes, void *stream);
+
 /* The same scan through page tables, as a serving cache holds its buckets: request r's logical bucket i is row
  * i % page_rows of page pages[r, i / page_rows] of `centroids` (-1 = no page: skipped); ids in the keys are the
  * LOGICAL bucket ids. Reference: scan_paged (src/lsa/core/kernels/triton/paged.py:61-101), DecodeSelect.listed

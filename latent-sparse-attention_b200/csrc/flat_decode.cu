@@ -1,4 +1,5 @@
-// A decode step over a flat index in one call: the launches of lsa_index_map, lsa_visible_buckets, lsa_flat_select_decode,
+// A decode step over a flat index in one call: the launches of lsa_index_map, lsa_flat_select_at (past a top_p of 128
+// lsa_visible_buckets and lsa_flat_select_decode),
 // lsa_expand and lsa_sparse_attend one after another, their intermediates in one workspace. On the GPU it is those calls; a host
 // that makes them from an interpreter, with a dozen allocations between, takes longer over them than the GPU does.
 #include "common.cuh"
@@ -55,8 +56,12 @@ LSA_API int lsa_flat_decode(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   LSA_REQUIRE(workspace_bytes >= room.total, LSA_ERR_WORKSPACE);
   int rc = lsa_index_map(q, LSA_DTYPE_BF16, R, Hq, Hq / Hkv, dh_off, dh_used, q_row_stride, q_head_stride, map, map_dtype, d_idx, 1,
                          room.index_queries, nullptr, stream);
-  if (rc == LSA_OK) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
-  if (rc == LSA_OK)
+  const bool at = top_p <= 128;  // (the scan finds what its rows see by itself)
+  if (rc == LSA_OK && at)
+    rc = lsa_flat_select_at(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, top_p, select_splits, room.keys,
+                            room.picked, room.select, room.select_bytes, stream);
+  if (rc == LSA_OK && !at) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
+  if (rc == LSA_OK && !at)
     rc = lsa_flat_select_decode(room.index_queries, R, d_idx, centroids, nullptr, room.visible, top_p, select_splits, room.keys,
                                 room.picked, room.select, room.select_bytes, stream);
   if (rc == LSA_OK)

@@ -3,10 +3,14 @@
 // out[s] = normalize( sum_kv (sum_{g < group} x[s, kv*group + g, off : off + dh_used]) @ W[kv*dh_used : (kv+1)*dh_used] )
 // with fp32 accumulation, in ascending input-dim order except for a few rows (up to 32, or 128 under a bf16 map), whose threads
 // share a row's dims. This is the exact-arithmetic form; rows are read once and the head sum never reaches memory.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "mma.cuh"
 
 namespace lsa {
+
+namespace cg = cooperative_groups;
 
 constexpr int kMapThreads = 256;
 constexpr int kMapRows = 64;    // rows a CTA maps, two a thread (half of them, one a thread, where 64 leave SMs without a second CTA)
@@ -369,7 +373,7 @@ static int launch_index_map(const void *x, int64_t rows, int heads, int group, i
 // A linear layer over a FEW rows (a decode step's queries): out[r, n] = act(sum_k xs[r, k] Wt[n, k]), xs = the row's
 // heads summed (fp32, rounded once to bf16) or the row itself. A warp owns an output column and walks its weights once
 // for all rows; eight columns a CTA, so even a single row's map spreads over N / 8 CTAs instead of one.
-constexpr int kLinMaxRows = 8;
+constexpr int kLinMaxRows = 8, kLinUnitCols = 64;  // (columns of a map whose grid is one cluster)
 constexpr size_t kLinStaged = 96 * 1024;  // a row's heads are staged whole where they take no more than this
 // 16-byte runs of a column's weights a lane takes before anything else: 8 (2,048 weights a column), or 20 (5,120) for
 // the widest maps - the kernel is built for both, so that a narrow map does not carry the registers of a wide one.
@@ -380,12 +384,14 @@ constexpr size_t kLinStaged = 96 * 1024;  // a row's heads are staged whole wher
 template <int kLinHeld, bool STAGED>
 __global__ void __launch_bounds__(STAGED ? 512 : 256)
     rows_linear_kernel(const uint16_t *__restrict__ x, int rows, int heads, int64_t x_row_stride, int64_t x_head_stride,
-                       int K, const uint16_t *__restrict__ Wt, int N, int gelu, float *__restrict__ out_f32,
+                       int K, const uint16_t *__restrict__ Wt, int N, int gelu, int unit, float *__restrict__ out_f32,
                        uint16_t *__restrict__ out_bf16) {
   constexpr int kLinThreads = STAGED ? 512 : 256;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float whole_s[kLinMaxRows][kLinUnitCols];  // the whole rows, where the grid is a cluster that makes them unit rows
   uint16_t *xs = reinterpret_cast<uint16_t *>(smem_raw);  // [rows][K] bf16
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (unit) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (waited for before the first write there)
   dependents_may_launch();
   // The weights of this warp's column do not depend on the kernel before: up to 5,120 of them are taken first, while
   // that kernel may still be running.
@@ -472,7 +478,7 @@ __global__ void __launch_bounds__(STAGED ? 512 : 256)
     }
   }
   __syncthreads();
-  if (n >= N) return;
+  if (n >= N && !unit) return;
   float acc[kLinMaxRows];
 #pragma unroll
   for (int r = 0; r < kLinMaxRows; ++r) acc[r] = 0.0f;
@@ -498,15 +504,43 @@ __global__ void __launch_bounds__(STAGED ? 512 : 256)
     if (k < K) fold(held[i], k);
   }
 #pragma unroll 4
-  for (int k = lane * 8 + kLinHeld * 256; k < K; k += 32 * 8) fold(*reinterpret_cast<const uint4 *>(w + k), k);
+  for (int k = lane * 8 + kLinHeld * 256; n < N && k < K; k += 32 * 8) fold(*reinterpret_cast<const uint4 *>(w + k), k);
 #pragma unroll
   for (int r = 0; r < kLinMaxRows; ++r) {
     if (r >= rows) break;
     float v = warp_sum(acc[r]);
     if (gelu) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
-    if (lane == 0) {
+    if (unit) {
+      acc[r] = v;
+    } else if (lane == 0) {
       if (out_f32) out_f32[(int64_t)r * N + n] = v;
       if (out_bf16) out_bf16[(int64_t)r * N + n] = float_to_bf16_bits(v);
+    }
+  }
+  if (unit) {
+    // A map of few columns is one cluster: every CTA gets the whole rows and divides its own columns by their length, the sums
+    // in rows_unit_kernel's order (a launch of its own was 1.9 us and the gap before it).
+    cg::cluster_group cluster = cg::this_cluster();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (n < N && lane < (int)gridDim.x) {
+#pragma unroll
+      for (int r = 0; r < kLinMaxRows; ++r)
+        if (r < rows) *cluster.map_shared_rank(&whole_s[r][n], lane) = acc[r];
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int first = blockIdx.x * (kLinThreads / 32);
+    for (int r = warp; r < rows; r += kLinThreads / 32) {
+      float ss = 0.0f;
+      for (int j = lane; j < N; j += 32) ss = fmaf(whole_s[r][j], whole_s[r][j], ss);
+      ss = warp_sum(ss);
+      const float den = fmaxf(sqrtf(ss), 1e-12f);
+      const int j = first + lane;
+      if (lane < kLinThreads / 32 && j < N) {
+        const float v = whole_s[r][j] / den;
+        if (out_f32) out_f32[(int64_t)r * N + j] = v;
+        if (out_bf16) out_bf16[(int64_t)r * N + j] = float_to_bf16_bits(v);
+      }
     }
   }
 }
@@ -551,9 +585,23 @@ LSA_API int lsa_rows_linear(const uint16_t *x, int rows, int heads, int64_t x_ro
   if (!lsa::allow_shared(kernel, most)) return LSA_ERR_LAUNCH;
   const unsigned threads = staged ? 512 : 256, grid = (unsigned)((d_out + threads / 32 - 1) / (threads / 32));
   const bool unit = flags & LSA_ROWS_NORMALIZE;
+  // (a grid of up to eight CTAs is a cluster that makes its rows unit rows itself)
+  const bool clustered = unit && !staged && d_out <= lsa::kLinUnitCols;
+  const int gelu = flags & LSA_ROWS_GELU ? 1 : 0;
+  uint16_t *const half = unit && !clustered ? nullptr : out_bf16;
+  if (clustered) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid), config.blockDim = dim3(threads), config.dynamicSmemBytes = smem, config.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = grid, attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute, config.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&config, kernel, x, rows, heads, x_row_stride, x_head_stride, d_in, Wt, d_out, gelu, 1, out_f32, half);
+    LSA_LAUNCH_CHECK();
+    return LSA_OK;
+  }
   lsa::launch(true, kernel, dim3(grid), dim3(threads), smem, (cudaStream_t)stream, x, rows,
-              heads, x_row_stride, x_head_stride, d_in, Wt, d_out, flags & LSA_ROWS_GELU ? 1 : 0, out_f32,
-              unit ? nullptr : out_bf16);
+              heads, x_row_stride, x_head_stride, d_in, Wt, d_out, gelu, 0, out_f32, half);
   LSA_LAUNCH_CHECK();
   if (unit) {
     lsa::launch(true, lsa::rows_unit_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, (cudaStream_t)stream,

@@ -349,6 +349,8 @@ struct SelectParams {
   int32_t *ids_out;             // [splits, R, keep] or NULL
   int32_t *carried_out;         // [R, keep * fanout] or NULL
   int64_t R, N;
+  const int64_t *positions;     // [R] in place of run_end: the run ends with the buckets of the blocks closed before it, or NULL
+  int64_t block, block_buckets; // (keys a block holds, and buckets)
   const int32_t *pages;         // [R, max_pages] page of every page_rows ids of a row (-1 = none), or NULL
   int d, n_carried, keep, fanout, id_base, chunk, run_limit, max_pages, page_rows;
   ShapeTable shape;             // the vectors' shapes, row for row (floors NULL: none)
@@ -731,6 +733,12 @@ __device__ __forceinline__ int keys_before(const int64_t *list, int size, int64_
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+// The buckets of the cluster blocks closed before a position's own, `limit` at most.
+__device__ __forceinline__ int32_t seen_buckets(int64_t pos, int64_t block, int64_t per_block, int64_t limit) {
+  const int64_t seen = (pos >= 0 ? pos / block : -((block - 1 - pos) / block)) * per_block;
+  return (int32_t)(seen < limit ? seen : limit);
+}
+
 // NV: 16-byte columns of a vector (8 or 16: tiles of vectors staged through shared memory, a half warp on a vector's bytes), or
 // 0: any width, every thread reading its own candidate's vector.
 template <int NV, bool SHAPED>
@@ -752,6 +760,7 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
 
   const int first = p.run_first ? p.run_first[row] : 0;
   int end = p.run_end ? p.run_end[row] : 0;
+  if (p.positions) end = seen_buckets(p.positions[row], p.block, p.block_buckets, p.run_limit);
   const int my_keep = p.row_keep ? max(0, min(p.row_keep[row], p.keep)) : p.keep;
   const int64_t vector_base = p.vector_base ? p.vector_base[row] : 0;
   for (int e = tid; e < p.d; e += kSelThreads) qs[e] = p.queries[row * p.d + e];
@@ -1654,8 +1663,7 @@ __global__ void __launch_bounds__(256)
                            int64_t limit, int32_t *__restrict__ visible) {
   const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (r >= R) return;
-  const int64_t pos = positions[r], seen = (pos >= 0 ? pos / block : -((block - 1 - pos) / block)) * per_block;
-  visible[r] = (int32_t)(seen < limit ? seen : limit);
+  visible[r] = seen_buckets(positions[r], block, per_block, limit);
 }
 }  // namespace lsa
 
@@ -1836,6 +1844,25 @@ LSA_API int lsa_flat_select_decode(const float *queries, int64_t R, int d, const
   p.d = d;
   p.keep = top_p;
   p.run_limit = INT32_MAX;
+  return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
+}
+
+LSA_API int lsa_flat_select_at(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
+                               int64_t block_buckets, int64_t m, int top_p, int splits, int64_t *keys_out, int32_t *picked_out,
+                               void *workspace, size_t workspace_bytes, void *stream) {
+  LSA_REQUIRE(queries && centroids && positions && keys_out, LSA_ERR_NULL);
+  LSA_REQUIRE(R >= 0 && d >= 4 && d % 4 == 0 && block >= 1 && block_buckets >= 1 && m >= 0 && m <= INT32_MAX && top_p >= 1 &&
+                  splits >= 1 && splits <= 1024,
+              LSA_ERR_ARGUMENT);
+  LSA_REQUIRE(top_p <= lsa::kRowKeep, LSA_ERR_UNSUPPORTED);
+  if (R == 0) return LSA_OK;
+  if (splits > 1) {
+    LSA_REQUIRE(workspace, LSA_ERR_NULL);
+    LSA_REQUIRE(workspace_bytes >= lsa_flat_select_decode_workspace_bytes(R, top_p, splits), LSA_ERR_WORKSPACE);
+  }
+  lsa::SelectParams p = {};
+  p.queries = queries, p.vectors = centroids, p.positions = positions, p.block = block, p.block_buckets = block_buckets;
+  p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = (int)m;
   return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 

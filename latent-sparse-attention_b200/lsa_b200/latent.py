@@ -204,10 +204,13 @@ class LatentLayer(FlatLayer):
         d, b = self.design, index.buckets
         with probe.region("index map"):
             index_queries = self.index_queries(q)
-        visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
         with probe.region("select"):
-            _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p,
-                                               splits=select_splits)
+            if d.top_p <= 128:
+                _, picked = ops.flat_select_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size, d.block_bucket_count,
+                                               d.top_p, splits=select_splits)
+            else:
+                visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
+                _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p, splits=select_splits)
         with probe.region("expand"):
             outs = (torch.empty(q.shape[0], d.list_width, device=q.device, dtype=torch.int32),
                     torch.empty(q.shape[0], device=q.device, dtype=torch.int32), self._expand_status)

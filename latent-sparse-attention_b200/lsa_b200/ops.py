@@ -127,7 +127,7 @@ def rows_linear(x: torch.Tensor, weight_t: torch.Tensor, sum_heads: bool = False
     out_bf16 = torch.empty(rows, d_out, device=x.device, dtype=torch.bfloat16) if out_dtype == torch.bfloat16 else None
     call("lsa_rows_linear", ptr(x), rows, heads, x.stride(0), x.stride(1) if heads > 1 else 0, d_in, ptr(w), d_out,
          (1 if gelu else 0) | (2 if normalize else 0), ptr(out_f32), ptr(out_bf16), stream(),
-         launches=2 if normalize else 1)
+         launches=2 if normalize and (sum_heads or d_out > 64) else 1)
     return out_f32 if out_dtype == torch.float32 else out_bf16
 
 
@@ -402,6 +402,20 @@ def flat_select_decode(index_queries: torch.Tensor, centroids: torch.Tensor, req
          top_p, splits, ptr(keys), ptr(picked), ptr(workspace),
          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream(),
          launches=_split_launches(R, splits, top_p))
+    return keys, picked
+
+
+def flat_select_at(index_queries: torch.Tensor, centroids: torch.Tensor, positions: torch.Tensor, block_size: int, block_buckets: int,
+                   top_p: int, splits: int = 1):
+    """`visible_buckets` and `flat_select_decode` of a few rows in one launch fewer (top_p up to 128)."""
+    q, c, positions = _as(index_queries, torch.float32), _as(centroids, torch.float32), _as(positions, torch.int64)
+    R, d = q.shape
+    keys = torch.empty(R, top_p, device=q.device, dtype=torch.int64)
+    picked = torch.empty(R, top_p, device=q.device, dtype=torch.int32)
+    need = query("lsa_flat_select_decode_workspace_bytes", R, top_p, splits)
+    workspace = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
+    call("lsa_flat_select_at", ptr(q), R, d, ptr(c), ptr(positions), block_size, block_buckets, c.shape[0], top_p, splits, ptr(keys),
+         ptr(picked), ptr(workspace), need, stream(), launches=_split_launches(R, splits, top_p))
     return keys, picked
 
 
@@ -711,7 +725,7 @@ def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh
          dh_off, dh_used, d_idx, ptr(positions), ptr(centroids), centroids.shape[0], ptr(members), members.shape[1], block_size,
          block_buckets, top_p, top_k, sink, window, select_splits, ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0), k.stride(1),
          float(scale), splits, ptr(out), ptr(expand_status), ptr(workspace), need, stream(),
-         launches=3 + _split_launches(R, select_splits, top_p) + _attend_launches(R, k.shape[1], splits))
+         launches=(2 if top_p <= 128 else 3) + _split_launches(R, select_splits, top_p) + _attend_launches(R, k.shape[1], splits))
     return out
 
 

@@ -130,6 +130,40 @@ def test_a_row_ranked_by_counting_is_the_row_scanned_whole(m, d, keep):
             assert keys[row].tolist()[:len(best)] == best and set(kept[row].tolist()[len(best):]) <= {-1}
 
 
+@pytest.mark.parametrize("m,d,keep,splits", [(0, 64, 3, 1), (5, 64, 128, 8), (300, 32, 64, 1), (5000, 64, 100, 32), (700, 20, 7, 8)])
+def test_rows_at_their_positions_see_what_the_visible_counts_say(m, d, keep, splits):
+    """The scan that counts a row's closed blocks itself, against the counts written first: positions before the first block closes,
+    at a block's ends, past the table and negative."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    q, c = torch.randn(7, d, device="cuda", generator=gen), torch.randn(max(m, 1), d, device="cuda", generator=gen)[:max(m, 1)]
+    positions = torch.tensor([0, 63, 64, 127, 1 << 40, -1, -70], device="cuda")
+    for block, per in ((64, 4), (64, 1), (7, 40)):
+        visible = ops.visible_buckets(positions, block, per, c.shape[0])
+        want = ops.flat_select_decode(q, c, None, visible, keep, splits=splits)
+        got = ops.flat_select_at(q, c, positions, block, per, keep, splits=splits)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    with pytest.raises(ValueError, match="shape"):
+        ops.flat_select_at(q, c, positions, 64, 4, 129)
+
+
+@pytest.mark.parametrize("rows,d_in,d_out", [(1, 2048, 64), (8, 264, 33), (3, 5120, 8), (8, 8, 1), (5, 2048, 65)])
+def test_unit_rows_in_the_map_s_own_cluster(rows, d_in, d_out):
+    """Maps of up to 64 columns, whose CTAs swap their columns and divide them, and a wider one in two launches: unit rows of the same
+    map's plain output, in the same order of sums."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(d_in)
+    x = torch.randn(rows, d_in, device="cuda", generator=gen).bfloat16()
+    w = torch.randn(d_out, d_in, device="cuda", generator=gen).bfloat16()
+    plain, got = ops.rows_linear(x, w), ops.rows_linear(x, w, normalize=True)
+    want = plain.double() / plain.double().norm(dim=1, keepdim=True)
+    assert (got.double() - want).abs().max() <= 2e-7  # (an fp32 sum of 64 squares, a root and a division)
+    zero = ops.rows_linear(torch.zeros_like(x), w, normalize=True)
+    assert not zero.any()
+
+
 @pytest.mark.parametrize("heads,kv_heads,dh", [(40, 8, 128), (9, 1, 128), (8, 8, 64), (32, 2, 64)])
 def test_a_few_rows_attend_as_many_rows_do(heads, kv_heads, dh):
     """A CTA of warps an item and its splits in a cluster, against the same rows among many (a warp an item): lists that are empty,
