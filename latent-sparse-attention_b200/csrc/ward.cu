@@ -23,7 +23,9 @@
 // blocks of 256 pools with the pairings of 512, 256 and 128 buckets 7.2 -> 2.4 ms; 9 blocks of 128 pools 165 -> 57 us; one
 // block of 80 pools, sixteen rounds, 190 -> 119 us. With every pair once, on the index of 1M clustered tokens: 1,024 blocks of 256
 // pools 2.10 -> 1.65 ms, the pairings of 16 blocks of 4,096 buckets 3.07 -> 2.28 (the first round 1.30 -> 0.76), of 2,048 0.92 ->
-// 0.77, of 1,024 384 -> 353 us, of 512 176 -> 158.
+// 0.77, of 1,024 384 -> 353 us, of 512 176 -> 158. With the dirty and the steady partners as one run of tiles, a last row tile's few
+// rows over all warps, and one branch for a lane's pairs of a row, 1,024 blocks of 256 pools 1.66 -> 1.47 ms, the pairings of 4,096
+// buckets 2.28 -> 2.21, of 1,024 352 -> 335 us.
 //
 // Arithmetic order is the CPU specification's: a dot is an fma chain in ascending dim order, costs are evaluated as
 // written, so labels are bit-equal to a replay in that order.
@@ -274,16 +276,18 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
   // range. (Norms that are not numbers count as greater; an infinite slack leaves `most` infinitely below zero, or no number.)
   bool great = false;
   for (int i = tid; i < P; i += kThreads) great = great || !(s.al[i] <= 1e15f);
-  const float slack = __syncthreads_or(great) ? INFINITY : 9.5367431640625e-7f;
+  const float keep = __syncthreads_or(great) ? -INFINITY : 1.0f - 9.5367431640625e-7f;
 
   for (; rounds < p.max_rounds && n_alive > p.bucket_count && !gave_up; ++rounds) {
     // ---- the cheapest partners: tiles of (dirty x open), dealt to the CTAs in runs. A pair's cost is the same from either side,
     // bit for bit, so a tile serves its rows and its partners: two dirty rows meet once, and a steady row meets what merged.
-    auto stage = [&](float *tile, const uint16_t *list, int from, int n, int most) {
+    const int n_open = n_dirty + n_steady;
+    auto open_row = [&](int at) { return at < n_dirty ? s.dirty[at] : s.steady[at - n_dirty]; };  // (no tile ends with the dirty ones)
+    auto stage = [&](float *tile, int from, int n, int most) {
       for (int e = tid; e < most * (D / 4); e += kThreads) {
         const int r = e / (D / 4), k = e - r * (D / 4);
         if (from + r < n) {
-          const int id = list[from + r];
+          const int id = open_row(from + r);
           *reinterpret_cast<float4 *>(tile + r * LD + 4 * k) =
               LOCAL ? *reinterpret_cast<const float4 *>(s.sums + (size_t)id * LD + 4 * k)
                     : __ldcg(reinterpret_cast<const float4 *>(sums_g + (size_t)id * D + 4 * k));
@@ -295,7 +299,6 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
       const unsigned long long *at = mine + side * apart + id, v = LOCAL ? *(const volatile unsigned long long *)at : __ldcg(at);
       return v == ~0ull ? INFINITY : cheapest_cost(v);
     };
-    const int tiles0 = (n_dirty + TILE - 1) / TILE, tiles1 = (n_steady + TILE - 1) / TILE;
     // One row tile of the dirty rows against partner tiles first_tile .. end_tile - 1 of the dirty and then the steady rows.
     auto search = [&](auto rows_a_warp, int first_row, int first_tile, int end_tile) {
       constexpr int ROWS = decltype(rows_a_warp)::value;
@@ -306,15 +309,15 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) best_c[i] = INFINITY, best_j[i] = 0x7FFFFFFF;
       __syncthreads();  // (the tiles are free)
-      stage(s.a, s.dirty, first_row, n_dirty, ROWS * kThreads / 32);
-      if (!LOCAL && lane < my_rows) bound_s[warp * ROWS + lane] = known(my_list[lane]);
+      stage(s.a, first_row, n_dirty, ROWS * kThreads / 32);
+      if (lane < my_rows) bound_s[warp * ROWS + lane] = known(my_list[lane]);
       for (int t = first_tile; t < end_tile; ++t) {
-        const uint16_t *others = t < tiles0 ? s.dirty : s.steady;
-        const int n_others = t < tiles0 ? n_dirty : n_steady, from = (t < tiles0 ? t : t - tiles0) * TILE;
-        const bool both_ways = t != first_row / TILE;  // (the tile that the rows are of meets itself: every pair is there twice)
+        const int from = t * TILE;
+        // (the dirty rows of the tile that the rows are of meet themselves: every pair is there twice)
+        const int one_way = t == first_row / TILE ? n_dirty : 0;
         if (t > first_tile) __syncthreads();
-        stage(s.b, others, from, n_others, TILE);
-        if (tid < TILE) known_s[tid] = both_ways && from + tid < n_others ? known(others[from + tid]) : -INFINITY;
+        stage(s.b, from, n_open, TILE);
+        if (tid < TILE) known_s[tid] = from + tid >= one_way && from + tid < n_open ? known(open_row(from + tid)) : -INFINITY;
         __syncthreads();
         if (my_rows <= 0) continue;
         float acc[ROWS][COLS];
@@ -345,10 +348,10 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
 #pragma unroll
         for (int j = 0; j < COLS; ++j) {
           const int c = from + lane + 32 * j;
-          id_j[j] = c < n_others ? others[c] : -1;
-          sq_j[j] = c < n_others ? s.sq[id_j[j]] : 0.0f;
-          al_j[j] = c < n_others ? s.al[id_j[j]] : 0.0f;
-          sz_j[j] = c < n_others ? s.sz[id_j[j]] : 0.0f;
+          id_j[j] = c < n_open ? open_row(c) : -1;
+          sq_j[j] = c < n_open ? s.sq[id_j[j]] : 0.0f;
+          al_j[j] = c < n_open ? s.al[id_j[j]] : 0.0f;
+          sz_j[j] = c < n_open ? s.sz[id_j[j]] : 0.0f;
           theirs_c[j] = known_s[lane + 32 * j], theirs_i[j] = -1;
         }
 #pragma unroll
@@ -356,25 +359,34 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
           if (i >= my_rows) break;
           const int id_i = my_list[i];
           const float sq_i = s.sq[id_i], al_i = s.al[id_i], sz_i = s.sz[id_i];
-          const float bound_i = LOCAL ? INFINITY : bound_s[warp * ROWS + i], best_before = best_c[i];
+          const float bound_i = bound_s[warp * ROWS + i], best_before = best_c[i];
+          const float row_least = fminf(bound_i, best_before);
+          // Most pairs are far from the cheapest so far of either, and a product says so without the root: with
+          // most = both - best - both / 2^20 positive and m2 <= most^2 (1 - 2^-20), the root is under `most` by more
+          // than the roundings of all of these (a few 2^-24 of `both`), so the cost is above the best, and not a tie.
+          // (That takes squares that are normal numbers: `most` is above 1e-15, and `slack` lets no pair through here in a
+          // block whose norms may leave their range.) The lane's pairs of a row are looked at together: one branch for all.
+          float m2[COLS], both[COLS];
+          bool close[COLS], any = false;
 #pragma unroll
           for (int j = 0; j < COLS; ++j) {
-            const float m2 = __fadd_rn(__fadd_rn(sq_i, sq_j[j]), __fmul_rn(2.0f, acc[i][j]));
-            const float both = __fadd_rn(al_i, al_j[j]);
-            // Most pairs are far from the cheapest so far of either, and a product says so without the root: with
-            // most = both - best - both / 2^20 positive and m2 <= most^2 (1 - 2^-20), the root is under `most` by more
-            // than the roundings of all of these (a few 2^-24 of `both`), so the cost is above the best, and not a tie.
-            // (That takes squares that are normal numbers: `most` is above 1e-15, and `slack` lets no pair through here in a
-            // block whose norms may leave their range.)
-            const float most = (both - fmaxf(fminf(bound_i, best_c[i]), theirs_c[j])) - both * slack;
-            if (most > 1e-15f && m2 <= most * most * 0.99999904632568359375f) continue;
-            if (id_j[j] < 0 || id_i == id_j[j] || __fadd_rn(sz_i, sz_j[j]) > p.bucket_cap) continue;
-            const float whole = sqrtf(m2 > 0.0f ? m2 : 0.0f);
-            const float cost = __fsub_rn(both, whole);
-            if (cost < best_c[i] || (cost == best_c[i] && id_j[j] < best_j[i])) best_c[i] = cost, best_j[i] = id_j[j];
-            // (the lists ascend, so a tie of two of this thread's rows stays with the first; one with what the partner knows
-            // is settled where the minima are kept)
-            if (cost < theirs_c[j] || (cost == theirs_c[j] && theirs_i[j] < 0)) theirs_c[j] = cost, theirs_i[j] = id_i;
+            m2[j] = __fadd_rn(__fadd_rn(sq_i, sq_j[j]), __fmul_rn(2.0f, acc[i][j]));
+            both[j] = __fadd_rn(al_i, al_j[j]);
+            const float most = fmaf(both[j], keep, -fmaxf(row_least, theirs_c[j]));
+            close[j] = !(most > 1e-15f && m2[j] <= most * most * 0.99999904632568359375f);
+            any = any || close[j];
+          }
+          if (any) {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) {
+              if (!close[j] || id_j[j] < 0 || id_i == id_j[j] || __fadd_rn(sz_i, sz_j[j]) > p.bucket_cap) continue;
+              const float whole = sqrtf(m2[j] > 0.0f ? m2[j] : 0.0f);
+              const float cost = __fsub_rn(both[j], whole);
+              if (cost < best_c[i] || (cost == best_c[i] && id_j[j] < best_j[i])) best_c[i] = cost, best_j[i] = id_j[j];
+              // (the lists ascend, so a tie of two of this thread's rows stays with the first; one with what the partner knows
+              // is settled where the minima are kept)
+              if (cost < theirs_c[j] || (cost == theirs_c[j] && theirs_i[j] < 0)) theirs_c[j] = cost, theirs_i[j] = id_i;
+            }
           }
           // (the lanes share what they found, so that in the next tile a pair is far from the cheapest of all of them; a local
           // block has few tiles a row)
@@ -388,7 +400,7 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < COLS; ++j)
-          if (both_ways && theirs_i[j] >= 0 && theirs_c[j] < INFINITY)
+          if (theirs_i[j] >= 0 && theirs_c[j] < INFINITY)
             atomicMin(mine + side * apart + id_j[j], pack_cheapest(theirs_c[j], theirs_i[j]));
       }
       if (my_rows <= 0) return;
@@ -421,23 +433,26 @@ __global__ void __launch_bounds__(ward_threads(LOCAL), LOCAL ? 2 : 1) ward_kerne
     };
     // This CTA's run of the tiles, a row tile at a time. A row tile meets the dirty partners from its own tile on.
     {
-      const int all = tiles0 + tiles1;
+      const int all = (n_open + TILE - 1) / TILE, high = (n_dirty + TILE - 1) / TILE;
       // Eight rows a warp where that leaves every CTA a tile; else (a small block, a late round) two, for four times
-      // the tiles.
+      // the tiles. A last row tile of few rows gives every warp two or four of them. The last row tiles come first: where a CTA has
+      // a block to itself, the rows that a later row tile meets have met their own by then, and know how cheap they are.
       constexpr int SMALL = kWardFewRows * kThreads / 32;
-      const bool few = n_dirty <= SMALL || tiles0 * (tiles0 + 1) / 2 + tiles0 * tiles1 < ctas;
-      const int height = few ? SMALL : TILE, high = (n_dirty + height - 1) / height;
+      const bool few = n_dirty <= SMALL || high * all - high * (high - 1) / 2 < ctas;
+      const int height = few ? SMALL : TILE, row_tiles = (n_dirty + height - 1) / height;
       int64_t count = 0;
-      for (int rt = 0; rt < high; ++rt) count += all - rt * height / TILE;
+      for (int rt = 0; rt < row_tiles; ++rt) count += all - rt * height / TILE;
       const int64_t lo = count * rank / ctas, hi = count * (rank + 1) / ctas;
       int64_t before = 0;
-      for (int rt = 0; rt < high && before < hi; ++rt) {
-        const int own = rt * height / TILE, across = all - own;
+      for (int rt = row_tiles - 1; rt >= 0 && before < hi; --rt) {
+        const int own = rt * height / TILE, across = all - own, rows = n_dirty - rt * height;
         const int first = (int)max((int64_t)0, lo - before), end = (int)min((int64_t)across, hi - before);
         before += across;
         if (first >= end) continue;
-        if (few)
+        if (few || rows <= SMALL)
           search(std::integral_constant<int, kWardFewRows>(), rt * height, own + first, own + end);
+        else if (rows <= 2 * SMALL)
+          search(std::integral_constant<int, 2 * kWardFewRows>(), rt * height, own + first, own + end);
         else
           search(std::integral_constant<int, kWardRows>(), rt * height, own + first, own + end);
       }

@@ -159,6 +159,20 @@ def test_ward_blocks_over_one_to_eight_ctas_are_bit_exact(ops, oracle, G, P, d, 
         assert np.array_equal(rounds.cpu().numpy(), want_rounds)
 
 
+@pytest.mark.parametrize("G,whole,tile", [(150, 64, 64), (80, 512, 128)])
+@pytest.mark.parametrize("quarters", [(0, 1), (1, 0), (1, 1), (2, 0), (2, 1), (4, -1)])
+def test_ward_of_a_last_row_tile_with_few_rows_is_bit_exact(ops, oracle, G, whole, tile, quarters):
+    """A last row tile of one row, of up to two rows a warp, of up to four and of more, beside whole ones, the partners' tiles ragged
+    the same way; later rounds leave tiles that are part dirty and part steady."""
+    P = whole + quarters[0] * tile // 4 + quarters[1]
+    keys = unit_rows(mixture(G * P, 16, 24, 0.4, P)).reshape(G, P, 16) * np.float32(2.0)
+    size_rows = np.full((G, P), 4.0, dtype=np.float32)
+    want, want_reached, want_rounds = oracle.ward_rounds(keys, size_rows, P // 4, 32.0, return_rounds=True)
+    got, reached, rounds = ops.ward_rounds(cuda(keys), 4.0, P // 4, 32.0, return_rounds=True)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(reached.cpu().numpy(), want_reached) and np.array_equal(rounds.cpu().numpy(), want_rounds)
+
+
 @pytest.mark.parametrize("scale", [1e-30, 1e-22, 1e-19, 3e-17, 1e-10, 1e14, 1e15, 4e18, 1.2e19])
 @pytest.mark.parametrize("P", [96, 600])
 def test_ward_of_keys_whose_squares_leave_fp32s_range_is_bit_exact(ops, oracle, scale, P):
