@@ -1,6 +1,7 @@
 // Expansion: a row's picked buckets become its read list - members best bucket first, then the window, then
 // the sinks. Pure integer work, one warp a row, ballot-compacted so the order is the table's order.
 #include "common.cuh"
+#include "expand.cuh"
 
 namespace lsa {
 
@@ -321,89 +322,28 @@ __global__ void __launch_bounds__(kSpreadThreads) expand_spread_kernel(ExpandPar
     from_s[i] = bucket >= 0 ? bucket * p.cap : -1;
   }
   __syncthreads();
-  const int step = (p.cap + 31) / 32;
-  auto before_window = [&](int32_t id) { return id >= 0 && id < window_start; };
   for (int i0 = warp * kSpreadPicks; i0 < row_p; i0 += kWarps * kSpreadPicks) {
     int64_t at[kSpreadPicks];
-    int32_t sample[kSpreadPicks], head[kSpreadPicks];
+    int first[kSpreadPicks], count[kSpreadPicks];
 #pragma unroll
-    for (int j = 0; j < kSpreadPicks; ++j) {
-      at[j] = i0 + j < row_p ? from_s[i0 + j] : -1;
-      // the last place of each 32nd of the row, and the row's first 32 places
-      const int place = min(p.cap, (lane + 1) * step) - 1;
-      sample[j] = at[j] >= 0 && lane * step < p.cap ? p.members[at[j] + place] : LSA_PAD;
-      head[j] = at[j] >= 0 && lane < p.cap ? p.members[at[j] + lane] : LSA_PAD;
-    }
-    int whole[kSpreadPicks];  // 32nds that lie before the window
-    int32_t inner[kSpreadPicks];
+    for (int j = 0; j < kSpreadPicks; ++j) at[j] = i0 + j < row_p ? from_s[i0 + j] : -1;
+    member_runs(p.members, p.cap, at, window_start, p.sink, first, count);
 #pragma unroll
-    for (int j = 0; j < kSpreadPicks; ++j) {
-      whole[j] = __popc(__ballot_sync(0xffffffffu, before_window(sample[j])));
-      const int place = whole[j] * step + lane;
-      inner[j] = at[j] >= 0 && lane < step && place < p.cap ? p.members[at[j] + place] : LSA_PAD;
-    }
-#pragma unroll
-    for (int j = 0; j < kSpreadPicks; ++j) {
-      int end = min(p.cap, whole[j] * step) + __popc(__ballot_sync(0xffffffffu, before_window(inner[j])));
-      for (int l0 = 32; l0 < step; l0 += 32) {  // (rows of more than 1,024 places)
-        const int place = whole[j] * step + l0 + lane;
-        const int32_t id = at[j] >= 0 && l0 + lane < step && place < p.cap ? p.members[at[j] + place] : LSA_PAD;
-        end += __popc(__ballot_sync(0xffffffffu, before_window(id)));
-      }
-      int first = __popc(__ballot_sync(0xffffffffu, head[j] >= 0 && head[j] < p.sink));
-      if (first == 32)  // (more sinks in the bucket than that: one after another)
-        while (first < end && p.members[at[j] + first] < p.sink) ++first;
-      first = min(first, end);
+    for (int j = 0; j < kSpreadPicks; ++j)
       if (lane == 0 && i0 + j < row_p) {
-        count_s[i0 + j] = end - first;
-        if (at[j] >= 0) from_s[i0 + j] = at[j] + first;
+        count_s[i0 + j] = count[j];
+        if (at[j] >= 0) from_s[i0 + j] = at[j] + first[j];
       }
-    }
   }
   __syncthreads();
-  if (warp == 0) {
-    int carry = 0;
-    for (int base = 0; base < row_p; base += 32) {
-      const int v = base + lane < row_p ? count_s[base + lane] : 0;
-      int incl = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      if (base + lane < row_p) start_s[base + lane] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) start_s[row_p] = carry;
-  }
+  if (warp == 0) run_starts(count_s, row_p, start_s);
   __syncthreads();
   const int listed = min(start_s[row_p], row_k);
   const int in_window = p.flags & LSA_EXPAND_NO_LOCAL ? 0 : (int)max((int64_t)0, pos + 1 - window_start);
   const int sinks = p.flags & LSA_EXPAND_NO_LOCAL ? 0 : (int)max((int64_t)0, min((int64_t)p.sink, min(window_start, pos + 1)));
   const int total = listed + in_window + sinks;
   const int gtid = blockIdx.x * kSpreadThreads + tid, gthreads = gridDim.x * kSpreadThreads;
-  constexpr int kAhead = 4;
-  for (int e0 = gtid; e0 < listed; e0 += kAhead * gthreads) {
-    int32_t ids[kAhead];
-#pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const int e = e0 + j * gthreads;
-      ids[j] = LSA_PAD;
-      if (e < listed) {
-        int lo = 0, hi = row_p;  // the last pick whose run starts at or before e
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (start_s[mid] <= e) lo = mid; else hi = mid;
-        }
-        ids[j] = p.members[from_s[lo] + (e - start_s[lo])];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const int e = e0 + j * gthreads;
-      if (e < listed) out[e] = stored_id(p, table, ids[j]);
-    }
-  }
+  list_members(p.members, from_s, start_s, row_p, listed, gtid, gthreads, [&](int e, int32_t id) { out[e] = stored_id(p, table, id); });
   for (int i = gtid; i < in_window; i += gthreads) out[listed + i] = stored_id(p, table, window_start + i);
   for (int i = gtid; i < sinks; i += gthreads) out[listed + in_window + i] = stored_id(p, table, i);
   if (!(p.flags & LSA_EXPAND_NO_PAD))

@@ -1,8 +1,9 @@
 // A decode step over a flat index in one call: the launches of lsa_index_map, lsa_flat_select_at (past a top_p of 128
-// lsa_visible_buckets and lsa_flat_select_decode),
-// lsa_expand and lsa_sparse_attend one after another, their intermediates in one workspace. On the GPU it is those calls; a host
+// lsa_visible_buckets and lsa_flat_select_decode), lsa_expand - short lists are the scan's own output, a launch fewer - and
+// lsa_sparse_attend one after another, their intermediates in one workspace. On the GPU it is those calls; a host
 // that makes them from an interpreter, with a dozen allocations between, takes longer over them than the GPU does.
 #include "common.cuh"
+#include "expand.cuh"
 
 namespace lsa {
 
@@ -56,15 +57,23 @@ LSA_API int lsa_flat_decode(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   LSA_REQUIRE(workspace_bytes >= room.total, LSA_ERR_WORKSPACE);
   int rc = lsa_index_map(q, LSA_DTYPE_BF16, R, Hq, Hq / Hkv, dh_off, dh_used, q_row_stride, q_head_stride, map, map_dtype, d_idx, 1,
                          room.index_queries, nullptr, stream);
-  const bool at = top_p <= 128;  // (the scan finds what its rows see by itself)
+  // Short lists are the scan's own output.
+  const bool listed = centroids && members && bucket_cap >= 1 && block >= 1 &&
+                      lsa::flat_lists_takes(R, m, top_p, select_splits, bucket_cap, top_k, sink, window);
+  if (rc == LSA_OK && listed) {
+    const lsa::RowLists lists = {members, room.lists, room.lengths, width, bucket_cap, top_k, sink, window};
+    rc = lsa::flat_lists(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, top_p, select_splits, lists,
+                         (cudaStream_t)stream);
+  }
+  const bool at = !listed && top_p <= 128;  // (the scan finds what its rows see by itself)
   if (rc == LSA_OK && at)
     rc = lsa_flat_select_at(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, top_p, select_splits, room.keys,
                             room.picked, room.select, room.select_bytes, stream);
-  if (rc == LSA_OK && !at) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
-  if (rc == LSA_OK && !at)
+  if (rc == LSA_OK && !listed && !at) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
+  if (rc == LSA_OK && !listed && !at)
     rc = lsa_flat_select_decode(room.index_queries, R, d_idx, centroids, nullptr, room.visible, top_p, select_splits, room.keys,
                                 room.picked, room.select, room.select_bytes, stream);
-  if (rc == LSA_OK)
+  if (rc == LSA_OK && !listed)
     rc = lsa_expand(room.picked, R, top_p, positions, members, m, bucket_cap, nullptr, nullptr, top_k, sink, window, nullptr, 0, 0,
                     INT64_MAX, 1, 1, 0, LSA_EXPAND_NO_PAD, room.lists, room.lengths, expand_status, stream);
   if (rc == LSA_OK)

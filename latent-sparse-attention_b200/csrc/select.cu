@@ -7,6 +7,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "expand.cuh"
 #include "scan_select.cuh"
 #include "shape.cuh"
 
@@ -355,6 +356,7 @@ struct SelectParams {
   int d, n_carried, keep, fanout, id_base, chunk, run_limit, max_pages, page_rows;
   ShapeTable shape;             // the vectors' shapes, row for row (floors NULL: none)
   int cluster;                  // CTAs a cluster, whose lists become one (row_select_kernel)
+  RowLists read;                // where the rows' read lists go (row_select_kernel's LISTED form)
 };
 
 // RB rows a CTA. Shared memory: queries [RB][d], per-row key buffers [RB][keep_pow2 + chunk], histograms.
@@ -741,7 +743,12 @@ __device__ __forceinline__ int32_t seen_buckets(int64_t pos, int64_t block, int6
 
 // NV: 16-byte columns of a vector (8 or 16: tiles of vectors staged through shared memory, a half warp on a vector's bytes), or
 // 0: any width, every thread reading its own candidate's vector.
-template <int NV, bool SHAPED>
+// LISTED: the row's read list leaves the kernel, not its picks: every CTA of the cluster has all picks written into its shared
+// memory, counts the members of its share of them, has the counts written into the others' and lists its share of the places. What
+// bounds the list is two rounds of loads for the counts and one for the ids, and two cluster barriers. (64 of 1,024 buckets, 3,100
+// ids, one B200: scan and expansion 7.2 + 5.6 us as two launches, 11.8 as one; the step, which its host bounds at 4.1 us a launch,
+// 35.1 -> 32.4.)
+template <int NV, bool SHAPED, bool LISTED>
 __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p) {
   constexpr int kColumns = NV > 0 ? NV : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -749,6 +756,8 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
   float *qs = reinterpret_cast<float *>(tile_s + (size_t)kRowTile * NV);  // [d]
   __shared__ int64_t rowof_s[2][kRowTile], runs_s[kRowTile], top_s[kRowKeep], held_s[2][kRowKeep], all_s[kRowCluster][kRowKeep];
   __shared__ int64_t waits_s[kRowKeep + kRowTile];
+  __shared__ int64_t from_s[LISTED ? kRowKeep : 1];  // of each pick: where its run starts in the member table,
+  __shared__ int pick_s[LISTED ? kRowKeep : 1], members_s[LISTED ? kRowKeep : 1], start_s[LISTED ? kRowKeep + 1 : 1];  // id, length, place
   __shared__ int count_s[kRowCluster], kept_rank_s[kRowKeep], kept_id_s[kRowKeep], kept_s, waiting_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -766,6 +775,7 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
   for (int e = tid; e < p.d; e += kSelThreads) qs[e] = p.queries[row * p.d + e];
   end = max(first, min(end, p.run_limit));
   if (tid == 0) kept_s = 0, waiting_s = 0;
+  if (LISTED && tid < kRowKeep) pick_s[tid] = LSA_PAD;
   const int total = p.n_carried + (end - first), share = (total + splits - 1) / splits;
   const int begin = min(total, split * share), stop = min(total, begin + share);
 
@@ -894,9 +904,55 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
   }
   __syncthreads();
   const int64_t *list = held_s[held];
+  // The row's read list, once every CTA has the picks.
+  auto write_list = [&] {
+    if constexpr (LISTED) {
+      constexpr int kPicks = 4;  // a warp looks at side by side
+      const RowLists &to = p.read;
+      const int64_t pos = p.positions[row], window_start = max((int64_t)0, pos + 1 - to.window);
+      for (int i0 = (mine * kSelWarps + warp) * kPicks; i0 < p.keep; i0 += p.cluster * kSelWarps * kPicks) {
+        int64_t at[kPicks];
+        int begin[kPicks], count[kPicks];
+#pragma unroll
+        for (int j = 0; j < kPicks; ++j) {
+          const int pick = i0 + j < p.keep ? pick_s[i0 + j] : LSA_PAD;
+          at[j] = pick >= 0 ? (int64_t)pick * to.cap : -1;
+        }
+        member_runs(to.members, to.cap, at, window_start, to.sink, begin, count);
+#pragma unroll
+        for (int j = 0; j < kPicks; ++j)
+          if (lane < p.cluster && i0 + j < p.keep) {
+            int64_t *from = &from_s[i0 + j];
+            int *n = &members_s[i0 + j];
+            if (p.cluster > 1) from = cg::this_cluster().map_shared_rank(from, lane), n = cg::this_cluster().map_shared_rank(n, lane);
+            *from = at[j] + begin[j], *n = count[j];  // (a pick of no bucket has no member)
+          }
+      }
+      if (p.cluster > 1)
+        cluster_arrive(), cluster_wait();  // (nobody's shared memory is touched by another CTA from here on)
+      else
+        __syncthreads();
+      if (warp == 0) run_starts(members_s, p.keep, start_s);
+      __syncthreads();
+      const int listed = min(start_s[p.keep], to.top_k), in_window = (int)max((int64_t)0, pos + 1 - window_start);
+      const int sinks = (int)max((int64_t)0, min((int64_t)to.sink, min(window_start, pos + 1)));
+      const int at = mine * kSelThreads + tid, step = p.cluster * kSelThreads;
+      int32_t *out = to.lists + row * to.width;
+      list_members(to.members, from_s, start_s, p.keep, listed, at, step, [&](int e, int32_t id) { out[e] = id; });
+      for (int i = at; i < in_window; i += step) out[listed + i] = (int32_t)(window_start + i);
+      for (int i = at; i < sinks; i += step) out[listed + in_window + i] = i;
+      if (at == 0) to.lengths[row] = listed + in_window + sinks;
+    }
+  };
 
   if (p.cluster == 1) {  // this CTA's list is a row's, or one that a merge takes
     const int valid = __syncthreads_count(tid < my_keep && list[tid & (kRowKeep - 1)] != kEmptyKey);
+    if constexpr (LISTED) {
+      if (tid < valid) pick_s[tid] = key_id(list[tid]);
+      __syncthreads();
+      write_list();
+      return;
+    }
     const int64_t out_row = ((int64_t)split * p.R + row) * p.keep;
     if (tid < p.keep) {
       const int64_t key = tid < valid ? list[tid] : kEmptyKey;
@@ -928,7 +984,7 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
     if (tid < C) *cluster.map_shared_rank(&count_s[mine], tid) = own;
   }
   cluster_arrive();
-  cluster_wait();  // (nobody's shared memory is touched by another CTA from here on)
+  cluster_wait();  // (but for the picks of a list, nobody's shared memory is touched by another CTA from here on)
   int found = 0;
   for (int j = 0; j < C; ++j) found += count_s[j];
   const int valid = min(found, my_keep);
@@ -943,7 +999,10 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
       rank += j + half < C && j + half != mine ? before : 0;
     }
     rank += __shfl_xor_sync(0xffffffffu, rank, 1) + i;
-    if (half == 0 && key != kEmptyKey && rank < valid) {
+    if (LISTED) {
+      if (key != kEmptyKey && rank < valid)
+        for (int peer = half; peer < C; peer += 2) *cluster.map_shared_rank(&pick_s[rank], peer) = key_id(key);
+    } else if (half == 0 && key != kEmptyKey && rank < valid) {
       if (p.keys_out) p.keys_out[out_row + rank] = key;
       if (p.ids_out) p.ids_out[out_row + rank] = key_id(key);
       if (p.carried_out) {
@@ -951,6 +1010,12 @@ __global__ void __launch_bounds__(kSelThreads) row_select_kernel(SelectParams p)
         kept_rank_s[slot] = rank, kept_id_s[slot] = key_id(key) - p.id_base;
       }
     }
+  }
+  if constexpr (LISTED) {
+    cluster_arrive();
+    cluster_wait();  // (the picks are everywhere)
+    write_list();
+    return;
   }
   if (mine == 0 && tid >= valid && tid < p.keep) {
     if (p.keys_out) p.keys_out[out_row + tid] = kEmptyKey;
@@ -1019,7 +1084,9 @@ __global__ void __launch_bounds__(kMergeThreads)
 template <int NV>
 static int launch_row_select(const SelectParams &p, int splits, cudaStream_t s) {
   const size_t smem = (size_t)kRowTile * NV * 16 + (size_t)p.d * 4;
-  const auto kernel = p.shape.floors ? row_select_kernel<NV, true> : row_select_kernel<NV, false>;
+  const auto kernel = p.read.members   ? row_select_kernel<NV, false, true>
+                      : p.shape.floors ? row_select_kernel<NV, true, false>
+                                       : row_select_kernel<NV, false, false>;
   LSA_REQUIRE(smem <= kSelectShared, LSA_ERR_UNSUPPORTED);
   if (!allow_shared(kernel, kSelectShared)) return LSA_ERR_LAUNCH;
   launch_clusters(p.R <= kChainedRows, kernel, dim3((unsigned)p.R, (unsigned)splits), dim3(kSelThreads), smem, s, p, p.cluster);
@@ -1865,6 +1932,25 @@ LSA_API int lsa_flat_select_at(const float *queries, int64_t R, int d, const flo
   p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = (int)m;
   return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
+
+namespace lsa {
+// (Eight ids a thread at most; a longer list is a launch's own, over up to 32 larger CTAs.)
+bool flat_lists_takes(int64_t R, int64_t m, int top_p, int splits, int cap, int top_k, int sink, int window) {
+  const int64_t ctas = splits < kRowCluster ? splits : kRowCluster;
+  return R >= 1 && R <= kChainedRows && m >= 1 && m <= INT32_MAX && top_p <= kRowKeep && splits >= 1 && splits < 2 * kRowCluster &&
+         (int64_t)top_k + window + sink < INT32_MAX && (int64_t)top_p * cap + window <= ctas * kSelThreads * 8;
+}
+
+int flat_lists(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
+               int64_t block_buckets, int64_t m, int top_p, int splits, const RowLists &lists, cudaStream_t stream) {
+  LSA_REQUIRE(queries && centroids && positions && lists.members, LSA_ERR_NULL);
+  LSA_REQUIRE(d >= 4 && d % 4 == 0 && block >= 1 && block_buckets >= 1 && top_p >= 1, LSA_ERR_ARGUMENT);
+  SelectParams p = {};
+  p.queries = queries, p.vectors = centroids, p.positions = positions, p.block = block, p.block_buckets = block_buckets;
+  p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = (int)m, p.read = lists;
+  return select_split(p, splits, nullptr, nullptr, nullptr, stream);
+}
+}  // namespace lsa
 
 LSA_API int lsa_shaped_select_decode(const float *queries, int64_t R, int d, const float *centroids,
                                      const uint8_t *basis, const float *variances, const float *floors, int rank,

@@ -725,8 +725,15 @@ def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh
          dh_off, dh_used, d_idx, ptr(positions), ptr(centroids), centroids.shape[0], ptr(members), members.shape[1], block_size,
          block_buckets, top_p, top_k, sink, window, select_splits, ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0), k.stride(1),
          float(scale), splits, ptr(out), ptr(expand_status), ptr(workspace), need, stream(),
-         launches=(2 if top_p <= 128 else 3) + _split_launches(R, select_splits, top_p) + _attend_launches(R, k.shape[1], splits))
+         launches=_flat_decode_launches(R, k.shape[1], top_p, top_p * members.shape[1] + window, select_splits, splits))
     return out
+
+
+def _flat_decode_launches(rows: int, kv_heads: int, top_p: int, ids: int, select_splits: int, splits: int) -> int:
+    """Launches of a decode step in one call: the scan of a few rows leaves their lists itself where eight ids a thread do."""
+    listed = rows <= 8 and top_p <= 128 and select_splits < 16 and ids <= min(select_splits, 8) * 256 * 8
+    select = 1 if listed else (1 if top_p <= 128 else 2) + _split_launches(rows, select_splits, top_p)
+    return 1 + select + _attend_launches(rows, kv_heads, splits)
 
 
 def latent_attend(q: torch.Tensor, latent: torch.Tensor, ids: torch.Tensor, lengths: torch.Tensor | None,

@@ -197,9 +197,15 @@ def test_a_few_rows_attend_as_many_rows_do(heads, kv_heads, dh):
 
 @pytest.mark.parametrize("T,R,splits,sizes", [
     (700, 1, 8, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=40, top_k=200, sink_size=4, window_size=128)),
-    (9000, 8, 1, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=700, sink_size=0, window_size=100))])
+    (9000, 8, 1, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=256, top_p=64, top_k=700, sink_size=0, window_size=100)),
+    # (lists out of the scan itself up to eight ids a thread, and one id past that: 127 picks of 128 and the window)
+    (20000, 3, 8, dict(pool_size=4, bucket_size=64, bucket_cap=128, cluster_block_size=512, top_p=127, top_k=3000, sink_size=40,
+                       window_size=128)),
+    (20000, 8, 8, dict(pool_size=4, bucket_size=64, bucket_cap=128, cluster_block_size=512, top_p=127, top_k=9000, sink_size=3,
+                       window_size=129))])
 def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monkeypatch):
-    """The same rows bit for bit, at the end, in the middle and before the first block; strided queries; a status that is raised."""
+    """The same rows bit for bit, at the end, in the middle and before the first block; strided queries; a status that is raised. Lists
+    that the scan writes itself are the expansion's."""
     from helpers import layer_inputs
     from lsa_b200 import ops
     from lsa_b200.layer import FlatDesign, FlatLayer
