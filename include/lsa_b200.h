@@ -269,6 +269,15 @@ int lsa_flat_select_at(const float *queries, int64_t R, int d, const float *cent
                        int64_t block_buckets, int64_t m, int top_p, int splits, int64_t *keys_out, int32_t *picked_out,
                        void *workspace, size_t workspace_bytes, void *stream);
 
+/* lsa_flat_select_at and lsa_expand of what it picks (no page table, no ranges, no padding), members [m, bucket_cap], as one call: a
+ * launch or two where the lists are a decode step's. selected [R, top_k + window + sink], lengths [R].
+ *   workspace  lsa_flat_lists_at_workspace_bytes(R, top_p, splits), 8-byte aligned */
+size_t lsa_flat_lists_at_workspace_bytes(int64_t R, int top_p, int splits);
+int lsa_flat_lists_at(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
+                      int64_t block_buckets, int64_t m, const int32_t *members, int bucket_cap, int top_p, int top_k, int sink,
+                      int window, int splits, int32_t *selected, int32_t *lengths, void *workspace, size_t workspace_bytes,
+                      void *stream);
+
 /* The same scan through page tables, as a serving cache holds its buckets: request r's logical bucket i is row
  * i % page_rows of page pages[r, i / page_rows] of `centroids` (-1 = no page: skipped); ids in the keys are the
  * LOGICAL bucket ids. Reference: scan_paged (src/lsa/core/kernels/triton/paged.py:61-101), DecodeSelect.listed

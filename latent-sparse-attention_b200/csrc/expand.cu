@@ -24,6 +24,8 @@ struct ExpandParams {
   int32_t *status;
   int64_t R, m, owner_first, owner_end;
   int top_p, cap, top_k, sink, window, page_size, width, granule, world, rank, flags;
+  const int64_t *keys;   // in place of the picks: `parts` lists a row of sorted keys [parts, R, top_p] (expand_spread_kernel's SORTED)
+  int parts, size;       // (size: top_p as the next power of two)
   uint32_t cap_inverse;  // ceil(2^21 / cap)
   bool keeps_all;        // no owner range and no dealt granules: every id is kept
 };
@@ -290,6 +292,12 @@ constexpr int kSpreadMaxPicks = 1024;
 constexpr int kSpreadMaxCtas = 32;
 constexpr int kSpreadPicks = 4;  // picks a warp looks at side by side
 
+// SORTED: the picks are the best of several lists, placed by counting as in a merge of its own - every CTA all of them, a thread a
+// key. (128 picks of 16,384 buckets out of the lists of eight clusters, a row of 83,000 ids: the merge 6.2 and the expansion 9.3 us as
+// two launches, 13.6 as one; the decode step over 10M positions 68.5 -> 66.3.)
+constexpr int kSortedParts = 8, kSortedPicks = 128;
+
+template <bool SORTED>
 __global__ void __launch_bounds__(kSpreadThreads) expand_spread_kernel(ExpandParams p) {
   __shared__ int64_t from_s[kSpreadMaxPicks];  // where the pick's run starts in the member table
   __shared__ int count_s[kSpreadMaxPicks];
@@ -307,9 +315,35 @@ __global__ void __launch_bounds__(kSpreadThreads) expand_spread_kernel(ExpandPar
   const int64_t window_start = max((int64_t)0, pos + 1 - p.window);
   int32_t *out = p.selected + r * p.width;
   if (tid == 0) bad_s = 0;
+  __shared__ int64_t keys_s[SORTED ? kSortedParts * kSortedPicks : 1];
+  __shared__ int32_t pick_s[SORTED ? kSortedPicks : 1];
+  if constexpr (SORTED) {
+    static_assert(kSortedParts * kSortedPicks <= kSpreadThreads, "a thread a key");
+    if (tid < p.parts * p.size) {
+      const int part = tid / p.size, i = tid - part * p.size;
+      keys_s[tid] = i < p.top_p ? p.keys[((int64_t)part * p.R + r) * p.top_p + i] : kEmptyKey;
+    }
+    if (tid < p.top_p) pick_s[tid] = LSA_PAD;
+    __syncthreads();
+    // (at least top_p keys reach the least of the lists' keys at place ceil(top_p / parts))
+    const int deep = (p.top_p + p.parts - 1) / p.parts - 1;
+    int64_t least = INT64_MAX;
+    for (int j = 0; j < p.parts; ++j) least = min(least, keys_s[j * p.size + deep]);
+    const int i = tid / p.parts, part = tid - i * p.parts;  // (the lists' heads first: what is under the bar is whole warps)
+    const int64_t key = i < p.top_p ? keys_s[part * p.size + i] : kEmptyKey;
+    if (key >= least && key != kEmptyKey) {
+      int rank = i;
+#pragma unroll 4
+      for (int j = 0; j < p.parts; ++j) {
+        const int before = keys_before(keys_s + j * p.size, p.size, key, j < part);
+        rank += j == part ? 0 : before;
+      }
+      if (rank < p.top_p) pick_s[rank] = key_id(key);
+    }
+  }
   __syncthreads();
   for (int i = tid; i < row_p; i += kSpreadThreads) {
-    int64_t bucket = p.picked[r * p.top_p + i];
+    int64_t bucket = SORTED ? pick_s[i] : p.picked[r * p.top_p + i];
     if (bucket >= 0 && p.bucket_pages) {
       const int64_t slot = bucket / p.bucket_page_rows;
       const int page = slot < p.bucket_max_pages ? p.bucket_pages[request * p.bucket_pages_stride + slot] : -1;
@@ -354,6 +388,35 @@ __global__ void __launch_bounds__(kSpreadThreads) expand_spread_kernel(ExpandPar
   }
 }
 
+bool expands_spread(int64_t R, int top_p, int cap, int window) {
+  return top_p <= kSpreadMaxPicks && (int64_t)top_p * cap + window >= (R <= 8 ? 1024 : (R <= 64 ? 4096 : INT64_MAX));
+}
+
+// As many CTAs a row as give a thread two ids of half-full buckets, a wave of them at most.
+static int launch_spread(const ExpandParams &p, cudaStream_t stream) {
+  const int64_t wanted = ((int64_t)p.top_p * p.cap / 2 + p.window) / (2 * kSpreadThreads);
+  const int64_t most = sm_count() / p.R < kSpreadMaxCtas ? sm_count() / p.R : kSpreadMaxCtas;
+  const int64_t ctas = wanted < most ? wanted : most;
+  const dim3 grid((unsigned)(ctas < 1 ? 1 : ctas), (unsigned)p.R);
+  launch(p.R <= kChainedRows, p.keys ? expand_spread_kernel<true> : expand_spread_kernel<false>, grid, dim3(kSpreadThreads), 0, stream,
+         p);
+  LSA_LAUNCH_CHECK();
+  return LSA_OK;
+}
+
+int expand_sorted(const int64_t *keys, int parts, int64_t R, int top_p, const int64_t *positions, int64_t m, const RowLists &to,
+                  cudaStream_t stream) {
+  LSA_REQUIRE(parts <= kSortedParts && top_p <= kSortedPicks, LSA_ERR_UNSUPPORTED);
+  ExpandParams p = {};
+  p.keys = keys, p.parts = parts, p.size = 2;
+  while (p.size < top_p) p.size <<= 1;
+  p.positions = positions, p.members = to.members, p.selected = to.lists, p.lengths = to.lengths;
+  p.R = R, p.m = m, p.owner_end = INT64_MAX, p.world = p.granule = 1, p.keeps_all = true;
+  p.top_p = top_p, p.cap = to.cap, p.top_k = to.top_k, p.sink = to.sink, p.window = to.window, p.width = (int)to.width;
+  p.flags = LSA_EXPAND_NO_PAD;
+  return launch_spread(p, stream);
+}
+
 }  // namespace lsa
 
 LSA_API int lsa_expand_batched(const int32_t *picked, int64_t R, int top_p, const int64_t *positions,
@@ -374,7 +437,7 @@ LSA_API int lsa_expand_batched(const int32_t *picked, int64_t R, int top_p, cons
               LSA_ERR_ARGUMENT);
   LSA_REQUIRE((int64_t)top_k + window + sink < INT32_MAX, LSA_ERR_ARGUMENT);
   if (R == 0) return LSA_OK;
-  lsa::ExpandParams p;
+  lsa::ExpandParams p = {};
   p.picked = picked;
   p.positions = positions;
   p.members = members;
@@ -408,17 +471,7 @@ LSA_API int lsa_expand_batched(const int32_t *picked, int64_t R, int top_p, cons
   const bool keeps_all = owner_world <= 1 && owner_first <= 0 && owner_end == INT64_MAX;
   p.keeps_all = keeps_all;
   p.cap_inverse = ((1u << 21) + (uint32_t)bucket_cap - 1) / (uint32_t)bucket_cap;
-  if (keeps_all && top_p <= lsa::kSpreadMaxPicks &&
-      (int64_t)top_p * bucket_cap + window >= (R <= 8 ? 1024 : (R <= 64 ? 4096 : INT64_MAX))) {
-    // a decode step's long lists: as many CTAs a row as give a thread two ids of half-full buckets, a wave of them at most
-    const int64_t wanted = ((int64_t)top_p * bucket_cap / 2 + window) / (2 * lsa::kSpreadThreads);
-    const int64_t most = lsa::sm_count() / R < lsa::kSpreadMaxCtas ? lsa::sm_count() / R : lsa::kSpreadMaxCtas;
-    const int64_t ctas = wanted < most ? wanted : most;
-    const dim3 grid((unsigned)(ctas < 1 ? 1 : ctas), (unsigned)R);
-    lsa::launch(R <= lsa::kChainedRows, lsa::expand_spread_kernel, grid, dim3(lsa::kSpreadThreads), 0, (cudaStream_t)stream, p);
-    LSA_LAUNCH_CHECK();
-    return LSA_OK;
-  }
+  if (keeps_all && lsa::expands_spread(R, top_p, bucket_cap, window)) return lsa::launch_spread(p, (cudaStream_t)stream);  // (a decode step's long lists)
   // Many rows of long runs: a CTA a row (8,192 rows of 128 picks of 640 ids: 1,391 -> 459 us against a warp a row; 777 rows:
   // 497 -> 70 us). Short rows do not pay for the CTA's scan.
   if (keeps_all && top_p <= lsa::kRunMaxPicks && bucket_cap > lsa::kFlatCap && (int64_t)top_p * bucket_cap >= 8192) {

@@ -1,9 +1,21 @@
-// What the expansion of a decode step's rows shares between a launch of its own and the tail of a scan.
+// What a decode step's scan and its expansion share: the expansion is a launch of its own or the tail of the scan, the last merge of
+// a scan's lists a launch of its own or the head of the expansion.
 #pragma once
 
 #include "common.cuh"
 
 namespace lsa {
+
+// How many of list[0..size) (descending, size a power of two) come before `key`: those greater, and equal ones too if `ties`.
+__device__ __forceinline__ int keys_before(const int64_t *list, int size, int64_t key, bool ties) {
+  int at = 0;
+  for (int step = size >> 1; step; step >>= 1) {
+    const int64_t other = list[at + step - 1];
+    at += other > key || (ties && other == key) ? step : 0;
+  }
+  const int64_t other = list[at];
+  return at + (other > key || (ties && other == key) ? 1 : 0);
+}
 
 // The run of N buckets' members that lie from the sinks on and before the window: where it starts in the bucket's row and how many
 // there are. Members ascend, so a warp looks at 32 places spread over a row and then at the places between two of them: two rounds
@@ -101,9 +113,10 @@ struct RowLists {
   int cap, top_k, sink, window;
 };
 
-// lsa_flat_select_at and the expansion of what it picks as one launch. `flat_lists_takes`: whether it has a form for the sizes.
-bool flat_lists_takes(int64_t R, int64_t m, int top_p, int splits, int cap, int top_k, int sink, int window);
-int flat_lists(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
-               int64_t block_buckets, int64_t m, int top_p, int splits, const RowLists &lists, cudaStream_t stream);
+// Whether rows of such picks are expanded by several CTAs each (expand_spread_kernel), and that expansion over the picks of `parts`
+// lists a row, sorted keys [parts][R][top_p]: the best top_p of them all.
+bool expands_spread(int64_t R, int top_p, int cap, int window);
+int expand_sorted(const int64_t *keys, int parts, int64_t R, int top_p, const int64_t *positions, int64_t m, const RowLists &to,
+                  cudaStream_t stream);
 
 }  // namespace lsa

@@ -1,9 +1,8 @@
-// A decode step over a flat index in one call: the launches of lsa_index_map, lsa_flat_select_at (past a top_p of 128
-// lsa_visible_buckets and lsa_flat_select_decode), lsa_expand - short lists are the scan's own output, a launch fewer - and
-// lsa_sparse_attend one after another, their intermediates in one workspace. On the GPU it is those calls; a host
+// A decode step over a flat index in one call: the launches of lsa_index_map, lsa_flat_lists_at (past a top_p of 128
+// lsa_visible_buckets, lsa_flat_select_decode and lsa_expand) and lsa_sparse_attend one after another, their intermediates in one
+// workspace. On the GPU it is those calls; a host
 // that makes them from an interpreter, with a dozen allocations between, takes longer over them than the GPU does.
 #include "common.cuh"
-#include "expand.cuh"
 
 namespace lsa {
 
@@ -22,7 +21,7 @@ struct FlatDecodeRoom {
       total += (bytes + 255) & ~(size_t)255;
       return (void *)p;
     };
-    select_bytes = lsa_flat_select_decode_workspace_bytes(R, top_p, select_splits);
+    select_bytes = lsa_flat_lists_at_workspace_bytes(R, top_p, select_splits);
     attend_bytes = lsa_sparse_attend_workspace_bytes(R, Hq, dh, splits);
     index_queries = (float *)take((size_t)R * d_idx * 4), lse = (float *)take((size_t)R * Hq * 4);
     visible = (int32_t *)take((size_t)R * 4), picked = (int32_t *)take((size_t)R * top_p * 4);
@@ -57,23 +56,15 @@ LSA_API int lsa_flat_decode(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   LSA_REQUIRE(workspace_bytes >= room.total, LSA_ERR_WORKSPACE);
   int rc = lsa_index_map(q, LSA_DTYPE_BF16, R, Hq, Hq / Hkv, dh_off, dh_used, q_row_stride, q_head_stride, map, map_dtype, d_idx, 1,
                          room.index_queries, nullptr, stream);
-  // Short lists are the scan's own output.
-  const bool listed = centroids && members && bucket_cap >= 1 && block >= 1 &&
-                      lsa::flat_lists_takes(R, m, top_p, select_splits, bucket_cap, top_k, sink, window);
-  if (rc == LSA_OK && listed) {
-    const lsa::RowLists lists = {members, room.lists, room.lengths, width, bucket_cap, top_k, sink, window};
-    rc = lsa::flat_lists(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, top_p, select_splits, lists,
-                         (cudaStream_t)stream);
-  }
-  const bool at = !listed && top_p <= 128;  // (the scan finds what its rows see by itself)
+  const bool at = top_p <= 128;  // (the scan finds what its rows see by itself, and leaves lists)
   if (rc == LSA_OK && at)
-    rc = lsa_flat_select_at(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, top_p, select_splits, room.keys,
-                            room.picked, room.select, room.select_bytes, stream);
-  if (rc == LSA_OK && !listed && !at) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
-  if (rc == LSA_OK && !listed && !at)
+    rc = lsa_flat_lists_at(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, members, bucket_cap, top_p,
+                           top_k, sink, window, select_splits, room.lists, room.lengths, room.select, room.select_bytes, stream);
+  if (rc == LSA_OK && !at) rc = lsa_visible_buckets(positions, R, block, block_buckets, m, room.visible, stream);
+  if (rc == LSA_OK && !at)
     rc = lsa_flat_select_decode(room.index_queries, R, d_idx, centroids, nullptr, room.visible, top_p, select_splits, room.keys,
                                 room.picked, room.select, room.select_bytes, stream);
-  if (rc == LSA_OK && !listed)
+  if (rc == LSA_OK && !at)
     rc = lsa_expand(room.picked, R, top_p, positions, members, m, bucket_cap, nullptr, nullptr, top_k, sink, window, nullptr, 0, 0,
                     INT64_MAX, 1, 1, 0, LSA_EXPAND_NO_PAD, room.lists, room.lengths, expand_status, stream);
   if (rc == LSA_OK)

@@ -721,17 +721,6 @@ constexpr int kRowTile = kSelThreads;
 constexpr int kRowKeep = 128;
 constexpr int kRowCluster = 8;
 
-// How many of list[0..size) (descending, size a power of two) come before `key`: those greater, and equal ones too if `ties`.
-__device__ __forceinline__ int keys_before(const int64_t *list, int size, int64_t key, bool ties) {
-  int at = 0;
-  for (int step = size >> 1; step; step >>= 1) {
-    const int64_t other = list[at + step - 1];
-    at += other > key || (ties && other == key) ? step : 0;
-  }
-  const int64_t other = list[at];
-  return at + (other > key || (ties && other == key) ? 1 : 0);
-}
-
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
@@ -1851,6 +1840,17 @@ static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, 
   return LSA_OK;
 }
 
+// The CTAs that a row's candidates are split over, of the `splits` asked for, and the clusters of p.cluster that they are; returns
+// the lists that they leave a row.
+static int split_over_clusters(SelectParams &p, int &splits) {
+  p.cluster = 1;
+  if (splits <= 1 || p.R > kChainedRows || p.keep > kRowKeep) return splits;
+  p.cluster = splits < kRowCluster ? splits : kRowCluster;
+  const int lists = splits < 2 * kRowCluster ? 1 : splits >= 32 && p.R == 1 ? 8 : 4;
+  splits = lists * p.cluster;
+  return lists;
+}
+
 // The best p.keep of each row's candidates, the row's split over `splits` CTAs. Up to kChainedRows rows are split over clusters: up
 // to eight CTAs are one and write the row, more are several whose lists a launch of its own merges. One B200, a graph of the call,
 // top 64, in us, the form with sorted lists folded pairwise first: 1,024 buckets over 8 CTAs 11.8 -> 6.5 (8 rows 11.9 -> 6.7),
@@ -1859,14 +1859,7 @@ static int merge_lists(const int64_t *keys_in, int parts, int64_t R, int top_p, 
 // 13.2 in 32 and 11.8 in 64, eight rows 24.8, 17.9 and 22.6 (the clusters of 512 CTAs wait for SMs that are free together; so would
 // those of more rows, whose CTAs are not clustered).
 static int select_split(SelectParams p, int splits, int64_t *keys_out, int32_t *ids_out, void *workspace, cudaStream_t s) {
-  const bool clustered = splits > 1 && p.R <= kChainedRows && p.keep <= kRowKeep;
-  int lists = splits;
-  p.cluster = 1;
-  if (clustered) {
-    p.cluster = splits < kRowCluster ? splits : kRowCluster;
-    lists = splits < 2 * kRowCluster ? 1 : splits >= 32 && p.R == 1 ? 8 : 4;
-    splits = lists * p.cluster;
-  }
+  const int lists = split_over_clusters(p, splits);
   if (lists == 1) {
     p.keys_out = keys_out, p.ids_out = ids_out;
     return launch_one_row(p, splits, s);
@@ -1933,24 +1926,51 @@ LSA_API int lsa_flat_select_at(const float *queries, int64_t R, int d, const flo
   return lsa::select_split(p, splits, keys_out, picked_out, workspace, (cudaStream_t)stream);
 }
 
-namespace lsa {
-// (Eight ids a thread at most; a longer list is a launch's own, over up to 32 larger CTAs.)
-bool flat_lists_takes(int64_t R, int64_t m, int top_p, int splits, int cap, int top_k, int sink, int window) {
-  const int64_t ctas = splits < kRowCluster ? splits : kRowCluster;
-  return R >= 1 && R <= kChainedRows && m >= 1 && m <= INT32_MAX && top_p <= kRowKeep && splits >= 1 && splits < 2 * kRowCluster &&
-         (int64_t)top_k + window + sink < INT32_MAX && (int64_t)top_p * cap + window <= ctas * kSelThreads * 8;
+LSA_API size_t lsa_flat_lists_at_workspace_bytes(int64_t R, int top_p, int splits) {
+  if (R <= 0 || top_p <= 0 || splits <= 0) return 0;  // (the scans' lists, and a row's keys and picks)
+  return lsa_flat_select_decode_workspace_bytes(R, top_p, splits) + (size_t)R * top_p * (sizeof(int64_t) + sizeof(int32_t));
 }
 
-int flat_lists(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
-               int64_t block_buckets, int64_t m, int top_p, int splits, const RowLists &lists, cudaStream_t stream) {
-  LSA_REQUIRE(queries && centroids && positions && lists.members, LSA_ERR_NULL);
-  LSA_REQUIRE(d >= 4 && d % 4 == 0 && block >= 1 && block_buckets >= 1 && top_p >= 1, LSA_ERR_ARGUMENT);
-  SelectParams p = {};
+LSA_API int lsa_flat_lists_at(const float *queries, int64_t R, int d, const float *centroids, const int64_t *positions, int64_t block,
+                              int64_t block_buckets, int64_t m, const int32_t *members, int bucket_cap, int top_p, int top_k, int sink,
+                              int window, int splits, int32_t *selected, int32_t *lengths, void *workspace, size_t workspace_bytes,
+                              void *stream) {
+  LSA_REQUIRE(queries && centroids && positions && selected && lengths && (m == 0 || members), LSA_ERR_NULL);
+  LSA_REQUIRE(R >= 0 && d >= 4 && d % 4 == 0 && block >= 1 && block_buckets >= 1 && m >= 0 && m <= INT32_MAX && bucket_cap >= 1 &&
+                  top_p >= 1 && top_k >= 1 && sink >= 0 && window >= 1 && splits >= 1 && splits <= 1024 &&
+                  (int64_t)top_k + window + sink < INT32_MAX,
+              LSA_ERR_ARGUMENT);
+  LSA_REQUIRE(top_p <= lsa::kRowKeep, LSA_ERR_UNSUPPORTED);
+  if (R == 0) return LSA_OK;
+  LSA_REQUIRE(workspace, LSA_ERR_NULL);
+  LSA_REQUIRE(workspace_bytes >= lsa_flat_lists_at_workspace_bytes(R, top_p, splits), LSA_ERR_WORKSPACE);
+  const cudaStream_t s = (cudaStream_t)stream;
+  const lsa::RowLists to = {members, selected, lengths, (int64_t)top_k + window + sink, bucket_cap, top_k, sink, window};
+  const int64_t ids = (int64_t)top_p * bucket_cap + window;
+  lsa::SelectParams p = {};
   p.queries = queries, p.vectors = centroids, p.positions = positions, p.block = block, p.block_buckets = block_buckets;
-  p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = (int)m, p.read = lists;
-  return select_split(p, splits, nullptr, nullptr, nullptr, stream);
+  p.R = R, p.N = INT64_MAX, p.d = d, p.keep = top_p, p.run_limit = (int)m;
+  int ctas = splits;
+  const int lists = lsa::split_over_clusters(p, ctas);
+  // Lists of up to eight ids a thread leave the scan itself; of longer ones the rows' expansion takes the lists of several clusters
+  // as they are, where it has the form of its own for such rows.
+  if (lists == 1 && R <= lsa::kChainedRows && m > 0 && ids <= (int64_t)p.cluster * lsa::kSelThreads * 8) {
+    p.read = to;
+    return lsa::launch_one_row(p, ctas, s);
+  }
+  if (lists > 1 && p.cluster > 1 && m > 0 && lsa::expands_spread(R, top_p, bucket_cap, window)) {
+    p.keys_out = (int64_t *)workspace;
+    const int rc = lsa::launch_one_row(p, ctas, s);
+    return rc != LSA_OK ? rc : lsa::expand_sorted(p.keys_out, lists, R, top_p, positions, m, to, s);
+  }
+  unsigned char *at = (unsigned char *)workspace + lsa_flat_select_decode_workspace_bytes(R, top_p, splits);
+  int64_t *keys = (int64_t *)at;
+  int32_t *picked = (int32_t *)(keys + R * top_p);
+  const int rc = lsa::select_split(p, splits, keys, picked, workspace, s);
+  if (rc != LSA_OK) return rc;
+  return lsa_expand(picked, R, top_p, positions, members, m, bucket_cap, nullptr, nullptr, top_k, sink, window, nullptr, 0, 0,
+                    INT64_MAX, 1, 1, 0, LSA_EXPAND_NO_PAD, selected, lengths, nullptr, stream);
 }
-}  // namespace lsa
 
 LSA_API int lsa_shaped_select_decode(const float *queries, int64_t R, int d, const float *centroids,
                                      const uint8_t *basis, const float *variances, const float *floors, int rank,

@@ -204,18 +204,22 @@ class LatentLayer(FlatLayer):
         d, b = self.design, index.buckets
         with probe.region("index map"):
             index_queries = self.index_queries(q)
-        with probe.region("select"):
-            if d.top_p <= 128:
-                _, picked = ops.flat_select_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size, d.block_bucket_count,
-                                               d.top_p, splits=select_splits)
-            else:
-                visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
-                _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p, splits=select_splits)
-        with probe.region("expand"):
-            outs = (torch.empty(q.shape[0], d.list_width, device=q.device, dtype=torch.int32),
-                    torch.empty(q.shape[0], device=q.device, dtype=torch.int32), self._expand_status)
-            lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
-                                           outs=outs, pad=False)  # (the read goes by the lengths)
+        if d.top_p <= 128 and b.bucket_members.shape[0] == b.bucket_centroids.shape[0] and not probe.listening():
+            lists, lengths = ops.flat_lists_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size, d.block_bucket_count,
+                                               b.bucket_members, d.top_p, d.top_k, d.sink_size, d.window_size, splits=select_splits)
+        else:  # (a stage at a time)
+            with probe.region("select"):
+                if d.top_p <= 128:
+                    _, picked = ops.flat_select_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size,
+                                                   d.block_bucket_count, d.top_p, splits=select_splits)
+                else:
+                    visible = ops.visible_buckets(positions, d.cluster_block_size, d.block_bucket_count, b.bucket_centroids.shape[0])
+                    _, picked = ops.flat_select_decode(index_queries, b.bucket_centroids, None, visible, d.top_p, splits=select_splits)
+            with probe.region("expand"):
+                outs = (torch.empty(q.shape[0], d.list_width, device=q.device, dtype=torch.int32),
+                        torch.empty(q.shape[0], device=q.device, dtype=torch.int32), self._expand_status)
+                lists, lengths, _ = ops.expand(picked, positions, b.bucket_members, d.top_k, d.sink_size, d.window_size,
+                                               outs=outs, pad=False)  # (the read goes by the lengths)
         with probe.region("attend"):
             out, _ = ops.latent_attend(q, latent, lists, lengths, self.scale, value_dim=self.value_dim, splits=splits,
                                        warp_mma=warp_mma, status=self._attend_status)

@@ -419,6 +419,32 @@ def flat_select_at(index_queries: torch.Tensor, centroids: torch.Tensor, positio
     return keys, picked
 
 
+def flat_lists_at(index_queries: torch.Tensor, centroids: torch.Tensor, positions: torch.Tensor, block_size: int, block_buckets: int,
+                  members: torch.Tensor, top_p: int, top_k: int, sink: int, window: int, splits: int = 1) -> tuple:
+    """`flat_select_at` and the `expand` of what it picks (no padding) in one call of a launch or two: lists [R, top_k + window + sink]
+    and their lengths. `members` has a row a centroid."""
+    q, c, positions = _as(index_queries, torch.float32), _as(centroids, torch.float32), _as(positions, torch.int64)
+    members, (R, d) = _as(members, torch.int32), q.shape
+    if members.shape[0] != c.shape[0]:
+        raise ValueError(f"{members.shape[0]} rows of members for {c.shape[0]} centroids")
+    lists = torch.empty(R, top_k + window + sink, device=q.device, dtype=torch.int32)
+    lengths = torch.empty(R, device=q.device, dtype=torch.int32)
+    need = query("lsa_flat_lists_at_workspace_bytes", R, top_p, splits)
+    workspace = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8)
+    call("lsa_flat_lists_at", ptr(q), R, d, ptr(c), ptr(positions), block_size, block_buckets, c.shape[0], ptr(members),
+         members.shape[1], top_p, top_k, sink, window, splits, ptr(lists), ptr(lengths), ptr(workspace), need, stream(),
+         launches=_list_launches(R, top_p, top_p * members.shape[1] + window, splits))
+    return lists, lengths
+
+
+def _list_launches(rows: int, top_p: int, ids: int, splits: int) -> int:
+    """Launches of `flat_lists_at`: the scan of a few rows leaves their lists itself where eight ids a thread do, and the expansion
+    of longer ones merges the lists of several clusters."""
+    if rows <= 8 and splits < 16:
+        return 1 if ids <= min(splits, 8) * 256 * 8 else 2
+    return 2 if rows <= 8 and ids >= 1024 else 1 + _split_launches(rows, splits, top_p)
+
+
 def flat_select_paged(index_queries: torch.Tensor, centroids: torch.Tensor, pages: torch.Tensor,
                       counts: torch.Tensor, page_rows: int, top_p: int, splits: int = 1,
                       workspace: torch.Tensor | None = None):
@@ -725,15 +751,11 @@ def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh
          dh_off, dh_used, d_idx, ptr(positions), ptr(centroids), centroids.shape[0], ptr(members), members.shape[1], block_size,
          block_buckets, top_p, top_k, sink, window, select_splits, ptr(k), ptr(v), k.shape[0], k.shape[1], k.stride(0), k.stride(1),
          float(scale), splits, ptr(out), ptr(expand_status), ptr(workspace), need, stream(),
-         launches=_flat_decode_launches(R, k.shape[1], top_p, top_p * members.shape[1] + window, select_splits, splits))
+         launches=1 + _attend_launches(R, k.shape[1], splits) +
+         (_list_launches(R, top_p, top_p * members.shape[1] + window, select_splits) if top_p <= 128 else
+          2 + _split_launches(R, select_splits, top_p)))
     return out
 
-
-def _flat_decode_launches(rows: int, kv_heads: int, top_p: int, ids: int, select_splits: int, splits: int) -> int:
-    """Launches of a decode step in one call: the scan of a few rows leaves their lists itself where eight ids a thread do."""
-    listed = rows <= 8 and top_p <= 128 and select_splits < 16 and ids <= min(select_splits, 8) * 256 * 8
-    select = 1 if listed else (1 if top_p <= 128 else 2) + _split_launches(rows, select_splits, top_p)
-    return 1 + select + _attend_launches(rows, kv_heads, splits)
 
 
 def latent_attend(q: torch.Tensor, latent: torch.Tensor, ids: torch.Tensor, lengths: torch.Tensor | None,

@@ -229,6 +229,36 @@ def test_a_step_in_one_call_is_the_calls_it_is_made_of(T, R, splits, sizes, monk
     layer.check()
 
 
+@pytest.mark.parametrize("m,cap,top_p,top_k,window,sink", [(1024, 64, 64, 3000, 128, 4), (1024, 1, 1, 1, 1, 0),
+                                                            (1000, 1280, 128, 163840, 5120, 4), (4100, 33, 127, 1000, 50, 40),
+                                                            (300, 128, 127, 9000, 128, 0), (300, 128, 127, 9000, 129, 0), (40, 7, 9, 60, 3, 2)])
+def test_lists_out_of_the_scan_are_the_expansion_s_of_its_picks(m, cap, top_p, top_k, window, sink):
+    """One to nine rows over one CTA, a cluster and several, before the first block, at its end and at the last; lists out of the scan
+    itself (2,048 ids a CTA at most), of an expansion that merges, and of the calls one after another: the same ids."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m + cap)
+    per, block = 10, 10 * cap
+    q, c = (torch.nn.functional.normalize(torch.randn(n, 64, device="cuda", generator=gen), dim=-1) for n in (9, m))
+    c[m // 2:m // 2 + 5] = c[:5]  # (ties)
+    bucket, place = torch.arange(m, device="cuda")[:, None], torch.arange(cap, device="cuda")
+    members = (bucket // per * block + bucket % per + place * per).to(torch.int32)
+    members[torch.rand(m, cap, device="cuda", generator=gen).sort(-1, descending=True).values < 0.2] = -1  # (ragged: pads at the end)
+    last = m * cap - 1
+    positions = torch.tensor([last, 0, block - 1, block, last // 2, last // 3, 3 * block + 5, last - 1, block * (m // per)], device="cuda")
+    for rows in (1, 3, 8, 9):
+        for splits in (1, 2, 8, 15, 16, 32):
+            _, picked = ops.flat_select_at(q[:rows], c, positions[:rows], block, per, top_p, splits=splits)
+            want, lengths, _ = ops.expand(picked, positions[:rows], members, top_k, sink, window)
+            got, got_lengths = ops.flat_lists_at(q[:rows], c, positions[:rows], block, per, members, top_p, top_k, sink, window,
+                                                 splits=splits)
+            assert torch.equal(got_lengths, lengths)
+            seen = torch.arange(want.shape[1], device="cuda") < lengths[:, None]
+            assert torch.equal(torch.where(seen, got, -1), torch.where(seen, want, -1))
+    with pytest.raises(ValueError):  # (128 picks at most)
+        ops.flat_lists_at(q, c, positions, block, per, members, 129, top_k, sink, window)
+
+
 def test_a_step_before_the_first_block_has_closed_is_refused_either_way(monkeypatch):
     """An index without a bucket (a cache shorter than a cluster block): the scan of a few rows takes no empty table, in one call
     or one by one."""
