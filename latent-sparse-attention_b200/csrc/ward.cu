@@ -14,10 +14,10 @@
 //   dirty rows (merged, or their partner merged or went)  x  all open rows
 // and a row too large for the smallest row left is closed: it can never merge again (in a pairing, every pair). A pair's
 // cost has the same bits from either side, so two dirty rows meet once and a tile of theirs serves both, and the other open
-// rows learn of what merged from the same tiles. What bounds the first rounds is a tile's operands out of shared memory (of a
-// larger block's tile of 128 x 128 pairs, 25 k cycles, the products are 15 k, where their multiply-adds alone would be 8 k;
-// two sums a multiply-add with fma.rn.f32x2, whose operands are twice the bytes, came out alike), the last ones barriers,
-// where a handful of rows is dirty (a round of a block of 80 pools takes 7 us, of which the tiles are 2).
+// rows learn of what merged from the same tiles. What bounds the first rounds is a warp's way through a tile (of a
+// larger block's tile of 128 x 128 pairs, 23 k cycles, the products are 13.5 k, where their multiply-adds alone would be 8 k,
+// and the costs 5 k; two sums a multiply-add with fma.rn.f32x2, lanes that share operands so that these leave shared memory in
+// three quarters of the time, and two teams of warps with a tile each came out alike or slower), the last ones barriers, where a handful of rows is dirty (a round of a block of 80 pools takes 7 us, of which the tiles are 2).
 // Measured on a B200, against every row searching all of its partners every round (one CTA a block up to 512 pools, two
 // launches a round, 256 rounds, above): the pairings of 16 blocks of 4,096, 2,048 and 1,024 buckets 26.0 -> 4.4 ms; 1,024
 // blocks of 256 pools with the pairings of 512, 256 and 128 buckets 7.2 -> 2.4 ms; 9 blocks of 128 pools 165 -> 57 us; one
