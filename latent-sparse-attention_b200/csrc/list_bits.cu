@@ -72,8 +72,9 @@ __global__ void __launch_bounds__(kBitsRows * 32) list_bits_kernel(ListBitsParam
       int n = 0;
       if (sixteen) {
         const int4 *row4 = reinterpret_cast<const int4 *>(row);
+        const bool any = bucket >= 0 && places > 0;  // (the lanes are a power of two: 112 places are seven lanes', and the eighth has none)
 #pragma unroll
-        for (int j = 0; j < kBitsQuads; ++j) held[j] = bucket >= 0 ? row4[j] : make_int4(-1, -1, -1, -1);
+        for (int j = 0; j < kBitsQuads; ++j) held[j] = any ? row4[j] : make_int4(-1, -1, -1, -1);
 #pragma unroll
         for (int j = 0; j < kBitsQuads; ++j)
           n += (counts(held[j].x) ? 1 : 0) + (counts(held[j].y) ? 1 : 0) + (counts(held[j].z) ? 1 : 0) + (counts(held[j].w) ? 1 : 0);

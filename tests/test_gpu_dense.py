@@ -196,7 +196,30 @@ def test_lists_as_bits_are_the_lists(cap, top_p, top_k, sink, window, sizes):
             assert int(status) == ((picked >= m) & within).sum()  # (every one, where `expand` may stop at the cut)
 
 
+@pytest.mark.parametrize("cap", [112, 208, 224, 240, 400, 464, 496])
+def test_a_bucket_that_ends_before_its_lanes_lends_no_key_of_the_next(cap):
+    """Caps whose sixteen-place lanes, a power of two of them, pass the bucket's end: the bits are `expand`'s lists where every
+    bucket of the table is full, its last one too, and no row picks two neighbours; with and without a cut at top-k."""
+    from lsa_b200 import ops
+
+    rng = np.random.default_rng(cap)
+    m, R, top_p, sink, window = 9, 40, 4, 4, 64
+    T = m * cap
+    members = np.sort(rng.permutation(T).astype(np.int32).reshape(m, cap), axis=1)
+    picked = np.stack([rng.permutation(np.arange(r % 2, m, 2))[:top_p] for r in range(R)]).astype(np.int32)
+    positions = np.concatenate([[T - 1, T // 2], rng.integers(0, T, R - 2)])
+    for top_k in (top_p * cap, cap + 37):
+        args = (cuda(picked), cuda(positions), cuda(members), top_k, sink, window)
+        lists, lengths, _ = ops.expand(*args)
+        words = ops.list_bits(*args, T, -(-T // 128)).cpu().numpy().view(np.uint32)
+        bits = np.unpackbits(words.transpose(1, 0, 2).copy().view(np.uint8), axis=-1, bitorder="little").reshape(R, -1)
+        for r in range(R):
+            assert np.array_equal(np.flatnonzero(bits[r]), np.sort(lists[r, :lengths[r]].cpu().numpy())), r
+
+
 @pytest.mark.parametrize("T,Hq,Hkv,chunk,sizes", [
+    (2500, 8, 2, 512, dict(pool_size=16, bucket_size=32, bucket_cap=112, cluster_block_size=512, top_p=8, top_k=300, sink_size=4,
+                           window_size=300)),   # (the lanes of a bucket's bits pass its end)
     (2500, 8, 2, 512, dict(pool_size=4, bucket_size=8, bucket_cap=16, cluster_block_size=128, top_p=64, top_k=300, sink_size=4,
                            window_size=128)),   # gathered else
     (3000, 5, 1, 1024, dict(pool_size=16, bucket_size=32, bucket_cap=64, cluster_block_size=512, top_p=16, top_k=300,
