@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kBinThreads) bin_select_kernel(BinParams p) {
     low = low_s, high = high_s;
     top = score_of(high);
     const float range = top - score_of(low);
-    by_id = !(range > 0.0f);
+    by_id = low >= high;  // (of the ordered integers, as the keys have them: -0 and +0 are two scores, in one bin)
     scale = (float)(kBins - 2) / (by_id ? (float)n : range);
     if (!isfinite(scale)) scale = 0.0f;
 #pragma unroll

@@ -194,6 +194,31 @@ def test_rows_placed_by_bins_are_the_rows_scanned(d, m, keep, monkeypatch):
         assert torch.equal(keys, want[0]) and torch.equal(picked, want[1])
 
 
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("m", [100, 150, 2048])
+def test_scores_of_zero_are_placed_by_their_signs(d, m, monkeypatch):
+    """Products that underflow leave -0 and +0, which a key tells apart: rows that score nothing else, among them few enough for a bin
+    and more, and rows of other scores, as the scan in a buffer places them."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(m + d)
+    R, keep = 40, 64
+    c = torch.randn(m, d, device="cuda", generator=gen)
+    c[:, -1] = torch.where(torch.rand(m, device="cuda", generator=gen) < 0.8, -1e-30, 1e-30)
+    q = torch.randn(R, d, device="cuda", generator=gen)
+    q[:30], q[:30, -1] = 0.0, 1e-30
+    q[10:20, 0] = c[5, 0] * 1e-38  # (and some score a few subnormal numbers)
+    visible = torch.randint(1, m + 1, (R,), device="cuda", generator=gen, dtype=torch.int32)
+    visible[0] = m
+    scratch = torch.empty(ops.query("lsa_flat_select_binned_workspace_bytes", R, d, m), device="cuda", dtype=torch.uint8)
+    monkeypatch.setattr(ops, "_binned_scratch", lambda *_: None)
+    want = ops.flat_select(q, c, visible, keep)
+    assert len(set(((want[0][0][:min(m, keep)] >> 32) & 0xFFFFFFFF).tolist())) <= 2
+    monkeypatch.setattr(ops, "_binned_scratch", lambda *_: scratch)
+    got = ops.flat_select(q, c, visible, keep)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 def test_a_search_without_memory_for_its_scores_goes_without(monkeypatch):
     """No scratch, an unaligned query or a size the scores' form does not take: the other forms serve the call."""
     from lsa_b200 import ops
