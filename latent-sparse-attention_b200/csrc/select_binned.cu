@@ -108,7 +108,7 @@ __device__ __forceinline__ float score_of(int32_t ordered) {
 
 __global__ void __launch_bounds__(kBinThreads) bin_select_kernel(BinParams p) {
   extern __shared__ __align__(16) int64_t area[];  // the keys of the bins that hold the best ones
-  __shared__ int bins_s[kBins];                    // counts, then where the next key of a bin goes
+  __shared__ __align__(16) int bins_s[kBins];      // counts (read four at a time), then where the next key of a bin goes
   __shared__ int low_s, high_s, most_s, last_s, count_s, sums_s[kBinThreads / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t row = blockIdx.x;
