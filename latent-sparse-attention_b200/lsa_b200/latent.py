@@ -128,34 +128,42 @@ class LatentLayer(FlatLayer):
     def prefill_rows(self, rows: torch.Tensor, start: int, latent: torch.Tensor, index: FlatIndex,
                      out: torch.Tensor, warp_mma: bool = False) -> torch.Tensor:
         """The read of consecutive query rows [n, heads, latent_dim] at positions start.. over a cache whose index
-        is built, into `out` [n, heads, value_dim] bf16."""
-        return self._read_rows(rows, start, latent, index, out, 1 if warp_mma else self._prefill_splits(rows, start), warp_mma)
+        is built, into `out` [n, heads, value_dim] bf16. Over how many CTAs a row's list is split goes by how many rows the call
+        has (`wave_splits`; and is one where there is no memory for the pieces' outputs), so a row read with others may differ
+        from the same row read alone: by the order of fp32 sums, a bf16 step at most."""
+        lists, lengths = self._row_lists(rows, start, index)
+        splits, workspace = (1, None) if warp_mma else self._list_pieces(rows, start, rows.shape[0])
+        return self._read_lists(rows, latent, lists, lengths, out, splits, workspace, warp_mma)
 
-    def _read_rows(self, rows: torch.Tensor, start: int, latent: torch.Tensor, index: FlatIndex, out: torch.Tensor, splits: int,
-                   warp_mma: bool = False) -> torch.Tensor:
+    def _row_lists(self, rows: torch.Tensor, start: int, index: FlatIndex) -> tuple:
+        """The lists of consecutive query rows from position `start` on, and their lengths."""
         n, dev = rows.shape[0], rows.device
         positions = torch.arange(start, start + n, device=dev)
         with probe.region("index map"):
             index_queries = self.index_queries(rows, out=self._room("index queries", (n, self.index_dim),
                                                                     torch.float32, dev))
-        lists, lengths = self._select(index_queries, positions, index, self._room, True, start + n - 1)
+        return self._select(index_queries, positions, index, self._room, True, start + n - 1)
+
+    def _list_pieces(self, rows: torch.Tensor, start: int, most: int) -> tuple:
+        """CTAs that the list of a row of a chunk [n, heads, latent_dim] from position `start` on is split over, and the memory for
+        the partial outputs of `most` of its rows (the allocator's again after the call: 131 KB a row of 64 heads and split)."""
+        d, n = self.design, rows.shape[0]
+        keys = min(start + n, d.top_p * d.bucket_size + d.window_size + d.sink_size, d.list_width)
+        splits = wave_splits(n * -(-self.heads // 64), keys, torch.cuda.get_device_properties(rows.device).multi_processor_count)
+        if splits == 1:
+            return 1, None
+        try:
+            return splits, torch.empty(ops.query("lsa_latent_attend_workspace_bytes", most, self.heads, self.value_dim, splits),
+                                       device=rows.device, dtype=torch.uint8)
+        except torch.OutOfMemoryError:
+            return 1, None
+
+    def _read_lists(self, rows: torch.Tensor, latent: torch.Tensor, lists: torch.Tensor, lengths: torch.Tensor, out: torch.Tensor,
+                    splits: int, workspace: torch.Tensor | None, warp_mma: bool = False) -> torch.Tensor:
         with probe.region("attend"):
-            workspace = None
-            if splits > 1:
-                try:  # (the allocator's again after the call: 131 KB a row of 64 heads and split)
-                    workspace = torch.empty(ops.query("lsa_latent_attend_workspace_bytes", n, self.heads, self.value_dim, splits),
-                                            device=dev, dtype=torch.uint8)
-                except torch.OutOfMemoryError:
-                    splits = 1
             ops.latent_attend(rows, latent, lists, lengths, self.scale, value_dim=self.value_dim, splits=splits, out=out,
                               workspace=workspace, warp_mma=warp_mma, status=self._attend_status)
         return out
-
-    def _prefill_splits(self, rows: torch.Tensor, start: int) -> int:
-        """CTAs that the list of a row of a chunk [n, heads, latent_dim] from position `start` on is split over."""
-        d, n = self.design, rows.shape[0]
-        keys = min(start + n, d.top_p * d.bucket_size + d.window_size + d.sink_size, d.list_width)
-        return wave_splits(n * -(-self.heads // 64), keys, torch.cuda.get_device_properties(rows.device).multi_processor_count)
 
     def prefill_from_host(self, q_host: torch.Tensor, rows_host: torch.Tensor, start: int, latent: torch.Tensor,
                           index: FlatIndex, out_host: torch.Tensor, pieces: int = 4) -> torch.Tensor:
@@ -186,10 +194,12 @@ class LatentLayer(FlatLayer):
                 arrived[i].record(self._copy_in)
         main.wait_event(rows_in)
         self.extend_index(latent, start, n)
-        splits = self._prefill_splits(q, start)  # (the chunk's, whatever it is cut into: a row's bits do not depend on that)
         for i, (first, stop) in enumerate(spans):
             main.wait_event(arrived[i])
-            self._read_rows(q[first:stop], start + first, latent, index, out[first:stop], splits)
+            lists, lengths = self._row_lists(q[first:stop], start + first, index)
+            if i == 0:  # (once for the chunk, with room for its largest piece: a row's bits do not depend on what it is cut into)
+                splits, workspace = self._list_pieces(q, start, stop - first)
+            self._read_lists(q[first:stop], latent, lists, lengths, out[first:stop], splits, workspace)
             done[i].record(main)
             with torch.cuda.stream(self._copy_out):
                 self._copy_out.wait_event(done[i])

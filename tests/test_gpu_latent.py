@@ -411,3 +411,54 @@ def test_a_chunk_read_in_pieces_of_its_lists_is_the_chunk(monkeypatch):
     scale = out[2].float().abs().max()
     assert (out[0].float() - out[2].float()).abs().max() <= 2 ** -7 * scale
     assert (out[0].float() - out[2].float()).norm() <= 4e-3 * out[2].float().norm()
+
+
+def _short_of(monkeypatch, module, which):
+    """The `which`-th allocation of partial outputs finds no memory; returns the list of those asked for."""
+    real, asked = torch.empty, []
+
+    def empty(*size, **kind):
+        if kind.get("dtype") == torch.uint8 and size[0] > 1 << 20:
+            asked.append(size[0])
+            if len(asked) == which:
+                raise torch.OutOfMemoryError("no memory")
+        return real(*size, **kind)
+
+    monkeypatch.setattr(module.torch, "empty", empty)
+    return asked
+
+
+@pytest.mark.parametrize("pieces", [1, 3, 4])
+def test_a_chunk_from_the_host_is_split_alike_in_all_of_its_pieces(pieces, monkeypatch):
+    """Whatever a chunk is cut into, and wherever memory for partial outputs runs out, its rows are the chunk's bits: all of them read
+    in pieces of their lists, or none."""
+    from lsa_b200 import latent as module
+    from lsa_b200 import workloads as W
+
+    cfg = W.cut(W.C4, 1 << 16)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    layer = module.LatentLayer(W.design_of(cfg), *W.latent_maps(cfg, gen), cfg["heads"], cfg["latent_dim"], cfg["value_dim"],
+                               W.latent_scale(cfg))
+    cache, _ = W.latent_cache(cfg, gen)
+    index = layer.build_index(cache)
+    n, first = 200, (1 << 16) - 200
+    q, rows = W.latent_queries(cfg, cache[first:], gen), cache[first:].cpu().pin_memory()
+    q_host = q.cpu().pin_memory()
+
+    def from_host():
+        out = torch.empty(n, cfg["heads"], cfg["value_dim"], dtype=torch.bfloat16, pin_memory=True)
+        layer.prefill_from_host(q_host, rows, first, cache, index, out, pieces=pieces)
+        torch.cuda.synchronize()
+        return out.cuda()
+
+    split, whole = (torch.empty(n, cfg["heads"], cfg["value_dim"], device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    layer.prefill_rows(q, first, cache, index, split)
+    with monkeypatch.context() as patch:
+        patch.setattr(module, "wave_splits", lambda *_: 1)
+        layer.prefill_rows(q, first, cache, index, whole)
+    assert not torch.equal(split, whole) and torch.equal(from_host(), split)
+    for short, want in ((1, whole), (2, split), (3, split)):
+        with monkeypatch.context() as patch:
+            asked = _short_of(patch, module, short)
+            assert torch.equal(from_host(), want) and len(asked) == 1, (short, asked)
+    layer.check()
