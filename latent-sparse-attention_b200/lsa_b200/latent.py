@@ -194,12 +194,16 @@ class LatentLayer(FlatLayer):
                 arrived[i].record(self._copy_in)
         main.wait_event(rows_in)
         self.extend_index(latent, start, n)
+        own = type(self).prefill_rows is LatentLayer.prefill_rows and "prefill_rows" not in self.__dict__
         for i, (first, stop) in enumerate(spans):
             main.wait_event(arrived[i])
-            lists, lengths = self._row_lists(q[first:stop], start + first, index)
-            if i == 0:  # (once for the chunk, with room for its largest piece: a row's bits do not depend on what it is cut into)
-                splits, workspace = self._list_pieces(q, start, stop - first)
-            self._read_lists(q[first:stop], latent, lists, lengths, out[first:stop], splits, workspace)
+            if not own:  # (a layer that reads rows its own way has that called)
+                self.prefill_rows(q[first:stop], start + first, latent, index, out[first:stop])
+            else:
+                lists, lengths = self._row_lists(q[first:stop], start + first, index)
+                if i == 0:  # (once for the chunk, with room for its largest piece: a row's bits do not depend on what it is cut into)
+                    splits, workspace = self._list_pieces(q, start, stop - first)
+                self._read_lists(q[first:stop], latent, lists, lengths, out[first:stop], splits, workspace)
             done[i].record(main)
             with torch.cuda.stream(self._copy_out):
                 self._copy_out.wait_event(done[i])

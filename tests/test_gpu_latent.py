@@ -462,3 +462,36 @@ def test_a_chunk_from_the_host_is_split_alike_in_all_of_its_pieces(pieces, monke
             asked = _short_of(patch, module, short)
             assert torch.equal(from_host(), want) and len(asked) == 1, (short, asked)
     layer.check()
+
+
+@pytest.mark.parametrize("on", ["class", "object"])
+def test_a_layer_that_reads_rows_its_own_way_reads_a_host_chunk_so(on):
+    """`prefill_rows` of a subclass, or set on one layer, is what `prefill_from_host` calls for every piece."""
+    from lsa_b200 import latent as module
+    from lsa_b200 import workloads as W
+
+    cfg = W.cut(W.C4, 1 << 14)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    seen = []
+
+    class Watched(module.LatentLayer):
+        def prefill_rows(self, rows, start, latent, index, out, warp_mma=False):
+            seen.append((start, rows.shape[0]))
+            return super().prefill_rows(rows, start, latent, index, out, warp_mma)
+
+    kind = Watched if on == "class" else module.LatentLayer
+    layer = kind(W.design_of(cfg), *W.latent_maps(cfg, gen), cfg["heads"], cfg["latent_dim"], cfg["value_dim"], W.latent_scale(cfg))
+    if on == "object":
+        given = layer.prefill_rows
+        layer.prefill_rows = lambda rows, start, *args: (seen.append((start, rows.shape[0])), given(rows, start, *args))[1]
+    cache, _ = W.latent_cache(cfg, gen)
+    index = layer.build_index(cache)
+    n, first = 40, (1 << 14) - 40
+    q = W.latent_queries(cfg, cache[first:], gen)
+    out = torch.empty(n, cfg["heads"], cfg["value_dim"], dtype=torch.bfloat16, pin_memory=True)
+    layer.prefill_from_host(q.cpu().pin_memory(), cache[first:].cpu().pin_memory(), first, cache, index, out, pieces=2)
+    torch.cuda.synchronize()
+    assert seen == [(first, 20), (first + 20, 20)]
+    want = torch.empty(20, cfg["heads"], cfg["value_dim"], device="cuda", dtype=torch.bfloat16)
+    module.LatentLayer.prefill_rows(layer, q[20:], first + 20, cache, index, want)
+    assert torch.equal(out[20:].cuda(), want)
