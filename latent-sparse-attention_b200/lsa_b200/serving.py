@@ -272,16 +272,14 @@ class BucketCache:
             self.holders[fresh[-1]] = 1
             pages.append(fresh[-1])
         if fresh:
-            # (by runs of a kernel's own making: a copy from the host's list would wait for the GPU to come this far. Free pages
-            # are handed out in order as a rule, which is one run)
-            at, row = len(pages) - len(fresh), self.request_pages[request]
-            while fresh:
-                step = fresh[1] - fresh[0] if len(fresh) > 1 else 1
-                run = 1
-                while run < len(fresh) and fresh[run] == fresh[0] + run * step:
-                    run += 1
-                torch.arange(fresh[0], fresh[0] + run * step, step, dtype=row.dtype, device=row.device, out=row[at:at + run])
-                at, fresh = at + run, fresh[run:]
+            # (neither way waits for the GPU to come this far, as a copy from pageable memory would. Free pages are handed out in
+            # order as a rule, which a kernel counts up or down; others cross from pinned memory, whose allocator holds it until then)
+            row = self.request_pages[request, len(pages) - len(fresh):len(pages)]
+            step = fresh[1] - fresh[0] if len(fresh) > 1 else 1
+            if all(b - a == step for a, b in zip(fresh, fresh[1:])):
+                torch.arange(fresh[0], fresh[0] + len(fresh) * step, step, dtype=row.dtype, device=row.device, out=row)
+            else:
+                row.copy_(torch.tensor(fresh, dtype=row.dtype, pin_memory=row.is_cuda), non_blocking=True)
 
     def append(self, request: int, index_keys: torch.Tensor) -> int:
         """Take a request's next index keys [n, index_dim] (fp32 unit rows, in position order); cluster every

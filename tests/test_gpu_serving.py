@@ -178,3 +178,36 @@ def test_rows_of_a_paged_table_go_in_and_out_as_index_arithmetic_has_them():
     cache.centroids.normal_(generator=gen)
     rows = cache.rows_of(1, torch.arange(50, device="cuda"))
     assert torch.equal(cache.gather(1, 50), cache.centroids[rows]) and torch.equal(cache.gather_members(1, 50), cache.members[rows])
+
+
+def test_pages_in_any_order_are_written_by_one_operation():
+    """A prompt over pages that came back in mixed order: its page numbers in one copy that does not wait for the GPU; in order, up or
+    down, by a kernel; later growth behind them."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from lsa_b200.layer import FlatDesign
+    from lsa_b200.serving import BucketCache
+
+    class Watched(TorchDispatchMode):
+        def __torch_dispatch__(self, op, types, args=(), kwargs=None):
+            done.append(op.overloadpacket.__name__)
+            return op(*args, **(kwargs or {}))
+
+    design = FlatDesign(pool_size=4, bucket_size=8, bucket_cap=16, top_p=4, top_k=32, sink_size=1, window_size=32, cluster_block_size=64)
+    mixed = np.random.default_rng(0).permutation(400).tolist()
+    for free in (mixed, list(range(400)), list(range(399, -1, -1)), list(range(0, 800, 2))[:400]):
+        cache = BucketCache(design, 32, pages=800, page_buckets=8, max_requests=3, max_request_pages=300)
+        cache.free_pages = list(free)
+        done = []
+        torch.cuda._sleep(10_000_000)
+        torch.cuda.set_sync_debug_mode("error")
+        try:
+            with Watched():
+                cache._grow(1, 8 * 290)
+                cache._grow(1, 8 * 291)
+                cache._grow(1, 8 * 300)
+        finally:
+            torch.cuda.set_sync_debug_mode("default")
+        assert sum(name in ("arange", "copy_", "_to_copy") for name in done) == 3, done
+        assert cache.held[1] == free[::-1][:300] and cache.request_pages[1].tolist() == cache.held[1]
+        assert (cache.request_pages[[0, 2]] == -1).all()
