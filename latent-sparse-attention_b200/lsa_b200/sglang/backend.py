@@ -19,6 +19,7 @@ import torch
 
 from lsa_b200 import ops
 from lsa_b200.constants import Sentinel
+from lsa_b200.layer import FlatLayer
 from lsa_b200.sglang import index_space, weights
 from lsa_b200.sglang.layer_index import KeySplit, LayerIndex, Shard
 from lsa_b200.sglang.settings import DesignSettings
@@ -362,14 +363,20 @@ def _mask_of(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tenso
     """Memory for the lists of a prompt's rows past the `dense` ones as one bit a key, where those rows are read through them: a
     prompt that starts in this batch, as long as the masked read takes it and is the faster. A CTA of it takes 256 rows of a head
     through every key, 0.0216 us each; rows gathered one by one cost 58 ps a listed key and KV head, and 83 ps a key to list (400
-    rows at the end of 5,000 keys of 16 heads over 2: 109 us against 364)."""
+    rows at the end of 5,000 keys of 16 heads over 2: 109 us against 364). These are not the rates of `FlatLayer._listed_until`:
+    that line is drawn for chunks of several waves, whose cost a row and head is an average (0.0216 us a key and CTA is 0.57 ps a
+    row and head where every SM has a CTA; 0.68 there), and against lists of positions, where a served list is padded and
+    translated to KV slots. (Whole batches of a prompt of 4,800 to 50,000 tokens beside one of 64, lists against masks: 0.92 / 0.78
+    to 29.9 / 19.6 ms under 16 heads over 2, 1.54 / 1.11 to 96 / 34 under 32 over 8; the rule takes the faster of them but at
+    50,000 under 32 over 2, 34.6 / 31.3.)"""
     n, heads, kv_heads = count - dense, q.shape[1], k.shape[1]
-    if not dense or n < 128 or count > 1600 * 128:
+    if not dense or n < 128 or count > FlatLayer.most_listed:
         return None
     rows, own = slice(first + dense, first + count), slice(first, first + count)
     if not ops.dense_attend_supported(q[rows], k[own], v[own], out[rows]):
         return None
-    waves = -(-(-(-n // 256) * heads) // 148)
+    sms = torch.cuda.get_device_properties(q.device).multi_processor_count
+    waves = -(-(-(-n // 256) * heads) // sms)
     if waves * count * 0.0216 >= n * design.list_width * (58e-6 * kv_heads + 83e-6):
         return None
     try:

@@ -403,3 +403,17 @@ def test_a_dense_read_that_gave_up_is_told_before_the_next_forward(monkeypatch):
         indexer.maintain(batch)
     indexer.maintain(batch)
     assert len(seen) == 3
+
+
+@pytest.mark.parametrize("sms,masked", [(148, True), (8, False), (4096, True)])
+def test_rows_are_read_through_masks_by_the_sms_there_are(sms, masked, monkeypatch):
+    """400 rows at the end of 5,000 keys of 16 heads over 2: four waves of CTAs on eight SMs cost more than their lists."""
+    from lsa_b200 import layer
+
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: types.SimpleNamespace(multi_processor_count=sms))
+    monkeypatch.setattr(backend.ops, "dense_attend_supported", lambda *tensors: True)
+    q, k = torch.empty(5000, 16, 128, dtype=torch.bfloat16), torch.empty(5000, 2, 128, dtype=torch.bfloat16)
+    mask = backend._mask_of(q, k, k, q, 0, 5000, 4600, layer.FlatDesign())
+    assert (mask is not None) == masked and (mask is None or mask.shape == (40, 400, 4))
+    assert backend._mask_of(q, k, k, q, 0, 5000, 0, layer.FlatDesign()) is None
+    assert backend._mask_of(q, k, k, q, 0, 5000, 4900, layer.FlatDesign()) is None
