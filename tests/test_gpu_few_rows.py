@@ -130,14 +130,14 @@ def test_a_row_ranked_by_counting_is_the_row_scanned_whole(m, d, keep):
             assert keys[row].tolist()[:len(best)] == best and set(kept[row].tolist()[len(best):]) <= {-1}
 
 
-@pytest.mark.parametrize("m,d,keep,splits", [(0, 64, 3, 1), (5, 64, 128, 8), (300, 32, 64, 1), (5000, 64, 100, 32), (700, 20, 7, 8)])
+@pytest.mark.parametrize("m,d,keep,splits", [(1, 64, 3, 1), (5, 64, 128, 8), (300, 32, 64, 1), (5000, 64, 100, 32), (700, 20, 7, 8)])
 def test_rows_at_their_positions_see_what_the_visible_counts_say(m, d, keep, splits):
     """The scan that counts a row's closed blocks itself, against the counts written first: positions before the first block closes,
     at a block's ends, past the table and negative."""
     from lsa_b200 import ops
 
     gen = torch.Generator(device="cuda").manual_seed(m)
-    q, c = torch.randn(7, d, device="cuda", generator=gen), torch.randn(max(m, 1), d, device="cuda", generator=gen)[:max(m, 1)]
+    q, c = torch.randn(7, d, device="cuda", generator=gen), torch.randn(m, d, device="cuda", generator=gen)
     positions = torch.tensor([0, 63, 64, 127, 1 << 40, -1, -70], device="cuda")
     for block, per in ((64, 4), (64, 1), (7, 40)):
         visible = ops.visible_buckets(positions, block, per, c.shape[0])
@@ -146,6 +146,8 @@ def test_rows_at_their_positions_see_what_the_visible_counts_say(m, d, keep, spl
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     with pytest.raises(ValueError, match="shape"):
         ops.flat_select_at(q, c, positions, 64, 4, 129)
+    with pytest.raises(ValueError, match="NULL"):  # (a table without a row)
+        ops.flat_select_at(q, c[:0], positions, 64, 4, keep, splits=splits)
 
 
 @pytest.mark.parametrize("rows,d_in,d_out", [(1, 2048, 64), (8, 264, 33), (3, 5120, 8), (8, 8, 1), (5, 2048, 65)])
@@ -193,6 +195,38 @@ def test_a_few_rows_attend_as_many_rows_do(heads, kv_heads, dh):
                     assert not got[1].any() and not seen[1].any()
             half, _ = ops.sparse_attend(q, k, v, ids, lengths, dh ** -0.5, splits=8, init=start)
             assert (half.float() - want[:R]).norm() <= 4e-3 * want[:R].norm()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dh", [(40, 8, 128), (9, 1, 128), (8, 8, 64), (32, 2, 64)])
+@pytest.mark.parametrize("where,what", [("k", float("nan")), ("k", float("inf")), ("k", -float("inf")), ("v", float("inf")),
+                                        ("v", float("nan"))])
+def test_what_is_not_finite_reaches_the_few_rows_it_reaches_among_many(heads, kv_heads, dh, where, what):
+    """One infinity or NaN in a listed key or value, at a list's start, in its second stage and at its end (another warp's and another
+    CTA's share): the weights of zero that meet in the cluster leave what a warp an item leaves, element by element. A key of
+    -inf scores -inf under half of the heads, which do not see it."""
+    from lsa_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    slots, R = 9000, 7
+    q = torch.randn(R, heads, dh, device="cuda", generator=gen).bfloat16()
+    k, v = (torch.randn(slots, kv_heads, dh, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    held = {"k": k, "v": v}[where]
+    for width in (40, 3001, 8500):
+        ids = torch.stack([torch.randperm(slots, device="cuda", generator=gen)[:width] for _ in range(R)]).to(torch.int32)
+        lengths = torch.tensor([width, 0, 1, 31, 33, width - 1, width // 2], device="cuda", dtype=torch.int32)
+        many = lambda x: torch.cat([x] * 2)
+        for at in (0, 32, width - 1):
+            kept = held.clone()
+            held[ids[:, at].long(), 0, 3] = what
+            want, want_lse = (x[:R] for x in ops.sparse_attend(many(q), k, v, many(ids), many(lengths), dh ** -0.5,
+                                                               out_dtype=torch.float32))
+            assert (where == "k" and abs(what) == float("inf")) or not want[0].isfinite().all()
+            for splits in (2, 8, 16):
+                got, lse = ops.sparse_attend(q, k, v, ids, lengths, dh ** -0.5, splits=splits, out_dtype=torch.float32)
+                assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()), (width, at, splits)
+                finite = want.isfinite()
+                assert (got - want)[finite].abs().max() <= 2 ** -9 and torch.equal(lse.isfinite(), want_lse.isfinite())
+            held.copy_(kept)
 
 
 @pytest.mark.parametrize("T,R,splits,sizes", [
