@@ -125,9 +125,12 @@ def rows_linear(x: torch.Tensor, weight_t: torch.Tensor, sum_heads: bool = False
     out_f32 = torch.empty(rows, d_out, device=x.device, dtype=torch.float32) \
         if (out_dtype == torch.float32 or normalize) else None
     out_bf16 = torch.empty(rows, d_out, device=x.device, dtype=torch.bfloat16) if out_dtype == torch.bfloat16 else None
+    # (unit rows are a launch of their own where the map is wide, or stages a row's heads)
+    staged = heads > 1 and d_in <= 2048 and heads * d_in * 2 <= 96 << 10 and (rows + heads) * d_in * 2 <= 160 << 10 \
+        and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
     call("lsa_rows_linear", ptr(x), rows, heads, x.stride(0), x.stride(1) if heads > 1 else 0, d_in, ptr(w), d_out,
          (1 if gelu else 0) | (2 if normalize else 0), ptr(out_f32), ptr(out_bf16), stream(),
-         launches=2 if normalize and (sum_heads or d_out > 64) else 1)
+         launches=2 if normalize and rows and (staged or d_out > 64) else 1)
     return out_f32 if out_dtype == torch.float32 else out_bf16
 
 
@@ -755,7 +758,6 @@ def flat_decode(q: torch.Tensor, index_map_weight: torch.Tensor, dh_off: int, dh
          (_list_launches(R, top_p, top_p * members.shape[1] + window, select_splits) if top_p <= 128 else
           2 + _split_launches(R, select_splits, top_p)))
     return out
-
 
 
 def latent_attend(q: torch.Tensor, latent: torch.Tensor, ids: torch.Tensor, lengths: torch.Tensor | None,
