@@ -56,7 +56,7 @@ LSA_API int lsa_flat_decode(const uint16_t *q, int64_t R, int Hq, int dh, int64_
   LSA_REQUIRE(workspace_bytes >= room.total, LSA_ERR_WORKSPACE);
   int rc = lsa_index_map(q, LSA_DTYPE_BF16, R, Hq, Hq / Hkv, dh_off, dh_used, q_row_stride, q_head_stride, map, map_dtype, d_idx, 1,
                          room.index_queries, nullptr, stream);
-  const bool at = top_p <= 128;  // (the scan finds what its rows see by itself, and leaves lists)
+  const bool at = top_p <= 128;  // (the scan finds what its rows see by itself, and leaves lists; a layer makes no other call)
   if (rc == LSA_OK && at)
     rc = lsa_flat_lists_at(room.index_queries, R, d_idx, centroids, positions, block, block_buckets, m, members, bucket_cap, top_p,
                            top_k, sink, window, select_splits, room.lists, room.lengths, room.select, room.select_bytes, stream);

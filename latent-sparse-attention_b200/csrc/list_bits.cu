@@ -1,12 +1,13 @@
 // Which keys a row's list names, as one bit a key: what the listed form of the dense read masks with. The list is that of
 // lsa_expand - members best bucket first up to the row's top-k, the window, the sinks - without its order.
 //
-// A warp a row, eight rows a CTA. Buckets of 16 places are a lane each, wider ones several; a lane walks its places twice - how
+// A warp a row, eight rows a CTA. Buckets of 16 places are a lane each, wider ones several. A lane takes its places twice - how
 // many count, then, once the counts before it are summed, its share of the top-k - and sets their bits in the row's words in
-// shared memory; a pool's keys are neighbours, so a lane gathers a word's bits before it adds them. The eight rows' words leave
-// together, 128 bytes a key tile. What bounds it is the warps' own instructions (20,096 rows of up to 4,096 keys out of 1,024 picks
-// of 16 places: 372 us, where expansion into lists took 866; a list and a walk of it would write and read four bytes a key in
-// place of a bit).
+// shared memory: sixteen places are held in registers from one read where they lie 16 bytes at a time, others are walked. A pool's
+// keys are neighbours, so four of them are one step and a lane gathers a word's bits before it adds them. The eight rows' words
+// leave together, 128 bytes a key tile. What bounds it is the warps' own instructions (20,096 rows of up to 4,096 keys out of 1,024
+// picks of 16 places, half full: 303 us, where expansion into lists takes 696; a list and a walk of it would write and read four
+// bytes a key in place of a bit).
 #include "common.cuh"
 
 namespace lsa {

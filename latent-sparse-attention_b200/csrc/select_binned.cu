@@ -12,7 +12,8 @@
 // below it in the first and the last, or where those are one score the range of their ids; what two such rounds do not spread is
 // sorted.
 //
-// What bounds it is a CTA's chain of passes and barriers a row, eight CTAs an SM side by side; the scores are a fifth of it. 8,192
+// What bounds it is a CTA's chain of passes and barriers a row, six CTAs an SM side by side (eight up to 2,048 buckets; a row's keys
+// have room for the last resort's sort, a power of two of them); the scores are a fifth of it. 8,192
 // rows of 64 dims over 3,072 buckets, one B200: top 1,024 990 us as a warp a row that cut and sorted its buffer in one CTA of eight
 // warps an SM, 222 so; top 64 291 and 172; equal scores 958 and 232.
 #include "common.cuh"

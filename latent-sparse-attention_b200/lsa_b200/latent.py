@@ -23,7 +23,8 @@ def wave_splits(items: int, keys: int, sms: int) -> int:
     """CTAs that each of `items` alike lists of some `keys` keys is split over. A CTA takes an SM, so they run in waves; where the
     last wave leaves SMs idle, pieces of a list fill it: as few as come within three hundredths of the least time for up to eight,
     a piece costing what its partial output's trip does (a two-hundredth of a list; none is cut shorter than 1,024 keys, whose CTA
-    lasts four times as long as it takes to start and end)."""
+    lasts four times as long as it takes to start and end). Whole against in pieces: 186 rows 6.26 / 4.21 ms, 777 13.4 to 15.3 /
+    12.7 to 13.7; 1,184, which stay whole, 15.7."""
     most = max(1, min(8, keys // 1024))
     times = [-(-items * s // sms) / s * (1.0 + 0.005 * (s - 1)) for s in range(1, most + 1)]
     return next(s for s, time in enumerate(times, 1) if time <= 1.03 * min(times))
@@ -221,7 +222,7 @@ class LatentLayer(FlatLayer):
         if d.top_p <= 128 and b.bucket_members.shape[0] == b.bucket_centroids.shape[0] and not probe.listening():
             lists, lengths = ops.flat_lists_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size, d.block_bucket_count,
                                                b.bucket_members, d.top_p, d.top_k, d.sink_size, d.window_size, splits=select_splits)
-        else:  # (a stage at a time)
+        else:  # (a stage at a time: somebody listens to their times, or the picks or the tables are not those of one call)
             with probe.region("select"):
                 if d.top_p <= 128:
                     _, picked = ops.flat_select_at(index_queries, b.bucket_centroids, positions, d.cluster_block_size,

