@@ -126,11 +126,11 @@ def rows_linear(x: torch.Tensor, weight_t: torch.Tensor, sum_heads: bool = False
         if (out_dtype == torch.float32 or normalize) else None
     out_bf16 = torch.empty(rows, d_out, device=x.device, dtype=torch.bfloat16) if out_dtype == torch.bfloat16 else None
     # (unit rows are a launch of their own where the map is wide, or stages a row's heads)
-    staged = heads > 1 and d_in <= 2048 and heads * d_in * 2 <= 96 << 10 and (rows + heads) * d_in * 2 <= 160 << 10 \
+    staged = normalize and heads > 1 and d_in <= 2048 and heads * d_in * 2 <= 96 << 10 and (rows + heads) * d_in * 2 <= 160 << 10 \
         and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
     call("lsa_rows_linear", ptr(x), rows, heads, x.stride(0), x.stride(1) if heads > 1 else 0, d_in, ptr(w), d_out,
          (1 if gelu else 0) | (2 if normalize else 0), ptr(out_f32), ptr(out_bf16), stream(),
-         launches=2 if normalize and rows and (staged or d_out > 64) else 1)
+         launches=2 if rows and (staged or normalize and d_out > 64) else 1)
     return out_f32 if out_dtype == torch.float32 else out_bf16
 
 
